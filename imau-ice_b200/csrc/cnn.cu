@@ -6,22 +6,23 @@
 //   forward  D[pixel][cout] = sum_(tap,cin)  X[pixel+tap][cin]     W[tap][cout][cin]
 //   dgrad    D[pixel][cin]  = sum_(tap,cout) dZ[pixel-tap][cout]   W[tap][cout][cin]
 //   wgrad    D[cout][cin]   = sum_pixel      dZ[pixel][cout]       X[pixel+tap][cin]
-// (dZ = dY masked by the ReLU of the layer's output).  A CTA of 128 threads owns one
-// 128-row tile of D in tensor memory (FP32 accumulators, tcgen05.alloc), its threads
-// gather the BF16 operand tiles for one tap (or one 64-pixel slice) from HBM into
-// shared memory in the no-swizzle K-major core-matrix layout -- 8 rows x 16 bytes
-// per core matrix, rows 16 bytes apart, K halves LBO apart, 8-row groups SBO apart --
-// while the tensor core works on the other of two stages; one elected thread issues
-// the tcgen05.mma instructions (M = 128, K = 16 each) and commits them to the stage's
-// mbarrier.  The epilogue reads the accumulators with tcgen05.ld (warp w owns lanes
-// 32w..32w+31 = rows), adds the bias and applies the ReLU, and stores BF16 (forward,
-// dgrad) or FP32 partial sums (wgrad, one slice of pixels per CTA, reduced in a fixed
-// order afterwards so that training is deterministic).
+// (dZ: the gradient of a layer's output masked by its ReLU; the kernel that writes a
+// gradient masks it, so every later reader takes it as it stands).  A persistent CTA
+// copies an image tile with its one-pixel halo into shared memory once (cp.async, zeros
+// outside the image), in the no-swizzle core-matrix layout -- 16-byte chunks of 8
+// channels, consecutive pixels 16 bytes apart, one plane per chunk -- so that a tap is a
+// shifted start address of the same tile: no operand is gathered twice.  One elected
+// thread issues the tcgen05.mma instructions (K = 16 each) with FP32 accumulators in
+// tensor memory and commits them to an mbarrier; the epilogue reads them back with
+// tcgen05.ld.  The weight gradient takes the same pixel-major tiles as MN-major operands
+// and keeps the sums of all its taps in tensor memory over every tile of the CTA; the
+// CTAs' sums are added in a fixed order afterwards, so training is deterministic.
 //
-// Pooling, upsampling + concatenation, the 1x1 head with the masked squared-error
-// loss, and Adam are elementwise or reduction kernels on CUDA cores.  Every mbarrier
-// wait is bounded; on time-out the kernel raises the network's error flag and frees
-// its tensor memory, and the host returns DIVA_TIMEOUT.
+// Pooling, the 1x1 head with the masked squared-error loss, and Adam are elementwise or
+// reduction kernels on CUDA cores; upsampling + concatenation happens in the loads of
+// the convolutions that read it.  Every mbarrier wait is bounded; on time-out the kernel
+// raises the network's error flag and frees its tensor memory, and the host returns
+// DIVA_TIMEOUT.
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cmath>
@@ -39,7 +40,6 @@ using bf16 = __nv_bfloat16;
 constexpr int kInC = 16;            // input channels (8 used)
 constexpr double kVelScale = 10.0;  // m/yr; outputs are asinh(u / kVelScale)
 constexpr long kSpin = 1L << 22;    // mbarrier polls before a wait gives up
-constexpr int kPixChunk = 64;       // wgrad K slice (pixels) per stage
 
 // ---------------------------------------------------------------------------
 // PTX wrappers (sm_100a)
@@ -113,6 +113,13 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t
   return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
+// A descriptor whose start address lies `off` 16-byte units further on (the addresses of a
+// CTA's shared memory stay below the 14-bit field's end).  One thread issues all MMAs, so
+// their rate is that of its instructions: forming each descriptor from scratch took longer
+// than the MMA itself at these tile sizes.
+__device__ __forceinline__ uint64_t sdesc_at(uint64_t d, uint32_t off) {
+  return (d & 0xFFFFFFFF00000000ull) | (uint64_t)((uint32_t)d + off);
+}
 // Instruction descriptor, kind::f16: D FP32 (bits 4-5 = 1), A and B BF16 (bits 7-9,
 // 10-12 = 1), both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
@@ -121,7 +128,7 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
 
 template <int N>
 __host__ __device__ constexpr int tmem_cols() {
-  return N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
+  return N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : N <= 256 ? 256 : 512;
 }
 
 // zero the lanes of v whose BF16 gate value is not > 0 (ReLU derivative)
@@ -138,134 +145,226 @@ __device__ __forceinline__ uint4 relu_gate(uint4 v, uint4 g) {
   return v;
 }
 
-__device__ __forceinline__ unsigned char* align1024(unsigned char* p) {
-  return reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
+__device__ __forceinline__ unsigned char* align128(unsigned char* p) {
+  return reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 127) & ~uintptr_t(127));
+}
+// 16 bytes global -> shared without registers; zeros when !in (src is then not read)
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The input of a 3x3 layer: one tensor [n][H][W][C], or the concatenation of a tensor at half
+// the resolution (lo, its first C1 channels, read at (y/2, x/2)) and one at the full (x).
+struct Input {
+  const bf16 *x, *lo;
+  int c1;   // channels from lo (0: none)
+};
+// Planes of 16-byte chunks are `px` pixels long; a warp stores chunks c8 = 0.. of one or more
+// consecutive pixels, so px is rounded up to the residue mod 8 that puts those 8 stores of a
+// phase into different banks (C = 16: 2 chunks x 4 pixels, 32: 4 x 2, 64 and more: 8 x 1).
+__host__ __device__ constexpr int plane_px(int px, int C) {
+  const int r = C == 16 ? 4 : C == 32 ? 2 : 1;
+  return px + ((r - px % 8) + 8) % 8;
 }
 
-// Occupancy guard: dynamic shared memory large enough that the CTAs resident on one
-// SM never ask for more than its 512 tensor-memory columns together.
-__host__ constexpr int smem_floor(int ncols) { return ncols >= 128 ? 47 * 1024 : ncols >= 64 ? 27 * 1024 : 0; }
+constexpr int kConvThreads = 256;
+
+// Stage `rows` image rows from y0 (possibly -1) and `cols` pixels from x0 (possibly -1) of the
+// C-channel input of image b: pixel (r, xx), chunk c8 at dst + r rpitch + c8 cpitch + 16 xx
+// bytes, zeros outside the image.  A thread keeps its (pixel, chunk) positions of a row and
+// walks down the rows with two additions per copy; recomputing every chunk's address from
+// scratch made the copies' instructions the bound of the tiles.
+template <int C>
+__device__ __forceinline__ void stage_rows(uint32_t dst, int rpitch, int cpitch, const Input& in, int H, int W, int b,
+                                           int y0, int rows, int x0, int cols) {
+  constexpr int C8 = C / 8;
+  for (int e = threadIdx.x; e < cols * C8; e += kConvThreads) {
+    const int c8 = e % C8, xx = e / C8, x = x0 + xx;
+    const bool xin = x >= 0 && x < W, low = c8 * 8 < in.c1;
+    const int xc = xin ? x : 0;
+    const char* src;   // row 0 of the image
+    int stride;        // bytes per row
+    if (low) {
+      src = reinterpret_cast<const char*>(in.lo + ((long)b * (H / 2) * (W / 2) + xc / 2) * in.c1 + c8 * 8);
+      stride = (W / 2) * in.c1 * 2;
+    } else {
+      src = reinterpret_cast<const char*>(in.x + ((long)b * H * W + xc) * (C - in.c1) + c8 * 8 - in.c1);
+      stride = W * (C - in.c1) * 2;
+    }
+    uint32_t d = dst + c8 * cpitch + xx * 16;
+    const int sh = low ? 1 : 0;
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r, d += rpitch) {
+      const int y = y0 + r;
+      const bool ok = xin && y >= 0 && y < H;
+      cp16(d, src + (ok ? (long)(y >> sh) * stride : 0), ok);
+    }
+  }
+}
 
 // ---------------------------------------------------------------------------
 // forward / dgrad 3x3 convolution
 // ---------------------------------------------------------------------------
+// A tile is TH x TW output pixels; its input, with the halo, is staged as (TH+2) rows of
+// P = TW + 2 pixels, row after row.  An accumulator block is 128 consecutive positions of
+// that pitch-P order (row m of D = position 128 blk + m), so that tap (ty, tx) of every
+// position is the same tile ty P + tx pixels further on: the two halo columns of a row
+// are computed as well and dropped (2 of P), instead of staging each tap's operand anew.
+struct ConvTile {
+  int TW, TH, P, npx;   // npx: pixels of a staged plane
+  int ncol, nrow, ntile;
+};
 struct ConvArgs {
-  const bf16* x;     // [n][H][W][KC]: forward input, or dY of the layer (dgrad)
-  const bf16* gate;  // dgrad: the layer's forward output [n][H][W][KC]
+  Input in;          // forward input, or (dgrad) dZ of the layer
   const bf16* w;     // forward: W [9][COUT][CIN]; dgrad: W^T [9][CIN][COUT]
   const float* bias; // forward: [COUT]
+  const bf16* mask;  // dgrad: the tensor whose ReLU masks the result, or null
   bf16* y;           // [n][H][W][NO]
-  int n, H, W, relu;
+  int n, H, W;
   int* err;
+  ConvTile t;
 };
 
+// accumulator blocks per tile: two where the weights leave room for two or more CTAs per SM
 template <int KC, int NO>
-__host__ __device__ constexpr int conv_smem() {
-  return 2 * (128 * KC * 2 + NO * KC * 2) + 64 + 1024;
+__host__ __device__ constexpr int conv_blocks() {
+  return KC * NO <= 64 * 32 ? 2 : 1;
+}
+// bytes between the 8-channel planes of one tap's weights (padded like plane_px)
+template <int KC, int NO>
+__host__ __device__ constexpr int conv_wplane() {
+  return plane_px(NO, KC) * 16;
+}
+template <int KC, int NO>
+__host__ __device__ constexpr int conv_wbytes() {
+  return 9 * (KC / 8) * conv_wplane<KC, NO>();
 }
 
+// Bound by the rate at which the tensor core takes K = 16 MMAs from unswizzled operands (about
+// 100 cycles each) and by the tile copies.  On 8 samples of 561 x 321 the 32 -> 32 layer takes
+// 92 us, the 64 -> 32 one 170 us (2 x 93 MB and 4 x 93 MB in and out); a kernel that gathered
+// its 128-pixel operand per tap, nine copies of the input through L2 with a barrier each, took
+// 274 and 892 us.
 template <int KC, int NO, bool DGRAD>
-__global__ void __launch_bounds__(128) k_conv3x3(ConvArgs a) {
-  static_assert(KC % 16 == 0 && NO % 16 == 0 && NO <= 128, "tile shape");
-  constexpr int A_BYTES = 128 * KC * 2, B_BYTES = NO * KC * 2, STAGE = A_BYTES + B_BYTES;
-  constexpr int NCOL = tmem_cols<NO>();
+__global__ void __launch_bounds__(kConvThreads) k_conv3x3(ConvArgs a) {
+  static_assert(KC % 16 == 0 && NO % 32 == 0 && NO <= 128, "tile shape");
+  constexpr int C8 = KC / 8, NB = conv_blocks<KC, NO>();
+  constexpr int WL = conv_wplane<KC, NO>(), WT = C8 * WL;
+  constexpr int NCOL = tmem_cols<NB * NO>();
   constexpr uint32_t IDESC = idesc_bf16(128, NO);
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = align1024(smem_raw);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + 2 * STAGE);
-  uint32_t* taddr_s = reinterpret_cast<uint32_t*>(bar + 2);
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ uint32_t taddr_s;
+  __shared__ __align__(16) float sbias[NO];
+  unsigned char* Ws = align128(smem_raw);
+  unsigned char* Xs = Ws + conv_wbytes<KC, NO>();
+  const uint32_t ws = smem_u32(Ws), xs = smem_u32(Xs);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int H = a.H, W = a.W, P = a.t.P, npx = a.t.npx;
 
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int H = a.H, W = a.W;
-  const long npix = (long)a.n * H * W;
-  const long p = (long)blockIdx.x * 128 + tid;  // this thread's row of D
-  const bool pin = p < npix;
-  int pb = 0, py = 0, px = 0;
-  if (pin) {
-    px = (int)(p % W);
-    const long q = p / W;
-    py = (int)(q % H);
-    pb = (int)(q / H);
-  }
   if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
+    mbar_init(&bar, 1);
     fence_mbar_init();
   }
-  if (warp == 0) tc_alloc(taddr_s, NCOL);
+  if (warp == 0) tc_alloc(&taddr_s, NCOL);
+  if (!DGRAD && tid < NO) sbias[tid] = a.bias[tid];
+  // the weights of all taps, once per CTA: B(n, k) of tap t at t WT + (k/8) WL + 16 n
+  for (int i = tid; i < 9 * NO * C8; i += kConvThreads) {
+    const int c8 = i % C8, r = i / C8;   // r = t NO + n
+    cp16(ws + (r / NO) * WT + c8 * WL + (r % NO) * 16, a.w + (long)r * KC + c8 * 8, true);
+  }
+  auto origin = [&](int tile, int& b, int& y0, int& x0) {
+    const int c = tile % a.t.ncol, q = tile / a.t.ncol;
+    x0 = c * a.t.TW;
+    y0 = (q % a.t.nrow) * a.t.TH;
+    b = q / a.t.nrow;
+  };
+  auto stage = [&](int tile) {
+    int b, y0, x0;
+    origin(tile, b, y0, x0);
+    stage_rows<KC>(xs, P * 16, npx * 16, a.in, H, W, b, y0 - 1, a.t.TH + 2, x0 - 1, P);
+  };
+  int tile = blockIdx.x;
+  if (tile < a.t.ntile) stage(tile);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *taddr_s;
-
+  const uint32_t tmem = taddr_s;
   bool ok = true;
-  for (int t = 0; t < 9; ++t) {
-    const int s = t & 1;
-    unsigned char* As = sm + s * STAGE;
-    unsigned char* Bs = As + A_BYTES;
-    if (t >= 2 && !mbar_wait(&bar[s], ((t - 2) >> 1) & 1)) ok = false;  // stage free again
-    int dy = t / 3 - 1, dx = t % 3 - 1;
-    if (DGRAD) { dy = -dy; dx = -dx; }
-    const int yy = py + dy, xx = px + dx;
-    const bool in = pin && yy >= 0 && yy < H && xx >= 0 && xx < W;
-    const long src = (((long)pb * H + yy) * W + xx) * KC;
-#pragma unroll 4
-    for (int kc = 0; kc < KC / 8; ++kc) {
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (in) {
-        v = *reinterpret_cast<const uint4*>(a.x + src + kc * 8);
-        if (DGRAD) v = relu_gate(v, *reinterpret_cast<const uint4*>(a.gate + src + kc * 8));
-      }
-      *reinterpret_cast<uint4*>(As + kc * 2048 + tid * 16) = v;
-    }
-    // B(n, k) = w[t][n][k]: forward, W[t][cout][cin]; dgrad, the transposed copy
-    // W^T[t][cin][cout] (k_transpose_w), so both stage contiguous 16-byte rows
-    for (int c = tid; c < NO * (KC / 8); c += 128) {
-      const int n = c % NO, kc = c / NO;
-      const uint4 v = *reinterpret_cast<const uint4*>(a.w + ((long)t * NO + n) * KC + kc * 8);
-      *reinterpret_cast<uint4*>(Bs + kc * (NO * 16) + n * 16) = v;
-    }
+  uint32_t phase = 0;
+  for (; tile < a.t.ntile; tile += gridDim.x) {
+    cp_wait_all();
     fence_async_smem();
-    tc_fence_before();
+    tc_fence_before();   // the previous tile's accumulator reads before this tile's MMAs
     __syncthreads();
     if (tid == 0) {
       tc_fence_after();
-#pragma unroll
-      for (int k = 0; k < KC / 16; ++k) {
-        const uint64_t da = sdesc(smem_u32(As) + 2 * k * 2048, 2048, 128);
-        const uint64_t db = sdesc(smem_u32(Bs) + 2 * k * (NO * 16), NO * 16, 128);
-        tc_mma(tmem, da, db, IDESC, (t > 0 || k > 0) ? 1u : 0u);
-      }
-      tc_commit(&bar[s]);
-    }
-  }
-  if (!mbar_wait(&bar[0], 0)) ok = false;  // tap 8: fifth phase of barrier 0
-  tc_fence_after();
-  ok = __syncthreads_and(ok);
-  if (ok) {
+      const uint64_t da0 = sdesc(xs, npx * 16, 128), db0 = sdesc(ws, WL, 128);
 #pragma unroll 1
-    for (int n0 = 0; n0 < NO; n0 += 16) {
+      for (int blk = 0; blk < NB; ++blk) {
+        const uint32_t d = tmem + blk * NO;
+        uint32_t ao = blk * 128 + (DGRAD ? 2 * P + 2 : 0), bo = 0;   // dgrad: the taps mirrored
+#pragma unroll 1
+        for (int ty = 0; ty < 3; ++ty) {
+#pragma unroll
+          for (int tx = 0; tx < 3; ++tx)
+#pragma unroll
+            for (int k = 0; k < KC / 16; ++k)
+              tc_mma(d, sdesc_at(da0, ao + 2 * k * npx + (DGRAD ? -tx : tx)),
+                     sdesc_at(db0, bo + (tx * WT + 2 * k * WL) / 16), IDESC, (ty > 0 || tx > 0 || k > 0) ? 1u : 0u);
+          ao += DGRAD ? -P : P;
+          bo += 3 * WT / 16;
+        }
+      }
+      tc_commit(&bar);
+    }
+    ok = mbar_wait(&bar, phase) && ok;
+    phase ^= 1;
+    tc_fence_after();
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
+    int b, y0, x0;
+    origin(tile, b, y0, x0);
+    if (tile + (int)gridDim.x < a.t.ntile) stage(tile + gridDim.x);   // overlaps the epilogue
+    // warps 4g..4g+3 read block g (two blocks) or column half g (one block)
+    const int g = warp >> 2, blk = NB == 2 ? g : 0;
+    constexpr int NC = NB == 2 ? NO : NO / 2;
+    const int c0 = NB == 2 ? 0 : g * NC;
+    const int pos = blk * 128 + (warp & 3) * 32 + lane, py = pos / P, px = pos % P;
+    const bool pin = py < a.t.TH && px < a.t.TW && y0 + py < H && x0 + px < W;
+    const long out = (((long)b * H + y0 + py) * W + x0 + px) * NO + c0;
+#pragma unroll
+    for (int n0 = 0; n0 < NC; n0 += 16) {
       float v[16];
-      tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)n0, v);
+      tc_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(blk * NO + c0 + n0), v);
       if (pin) {
         __align__(16) bf16 o[16];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          float f = v[q];
-          if (!DGRAD) {
-            f += a.bias[n0 + q];
-            if (a.relu) f = fmaxf(f, 0.0f);
+        for (int q4 = 0; q4 < 4; ++q4) {
+          float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (!DGRAD) b4 = *reinterpret_cast<const float4*>(sbias + c0 + n0 + 4 * q4);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float f = v[4 * q4 + q];
+            if (!DGRAD) f = fmaxf(f + (&b4.x)[q], 0.0f);
+            o[4 * q4 + q] = __float2bfloat16_rn(f);
           }
-          o[q] = __float2bfloat16_rn(f);
         }
-        uint4* dst = reinterpret_cast<uint4*>(a.y + p * NO + n0);
-        dst[0] = reinterpret_cast<const uint4*>(o)[0];
-        dst[1] = reinterpret_cast<const uint4*>(o)[1];
+        uint4 o0 = reinterpret_cast<const uint4*>(o)[0], o1 = reinterpret_cast<const uint4*>(o)[1];
+        if (DGRAD && a.mask) {
+          const uint4* m = reinterpret_cast<const uint4*>(a.mask + out + n0);
+          o0 = relu_gate(o0, m[0]);
+          o1 = relu_gate(o1, m[1]);
+        }
+        uint4* dst = reinterpret_cast<uint4*>(a.y + out + n0);
+        dst[0] = o0;
+        dst[1] = o1;
       }
     }
-  } else if (tid == 0) {
-    atomicExch(a.err, 1);
   }
+  if (!ok && tid == 0) atomicExch(a.err, 1);
+  cp_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -275,134 +374,152 @@ __global__ void __launch_bounds__(128) k_conv3x3(ConvArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// wgrad: D[cout (rows, padded to 128)][cin] over a slice of pixels, per tap
+// wgrad: every tap's D[cout][cin] over the pixels of the CTA's tiles, and the bias gradient
 // ---------------------------------------------------------------------------
-struct WgradArgs {
-  const bf16* x;     // the layer's input [n][H][W][CI]
-  const bf16* dy;    // gradient of the layer's output [n][H][W][CO]
-  const bf16* gate;  // the layer's output (ReLU mask)
-  float* part;       // [nsplit][9][CO][CI]
-  int n, H, W, nsplit;
-  int* err;
+// A tile is TH rows of X (TW + 2 pixels, halo columns included) and the TH + 2 rows of dZ
+// (TW pixels) that they meet.  K runs over 16 pixels of a row; both operands are MN-major
+// (8 channels contiguous), a tap's column shift is a start address one pixel further on.
+// dZ is staged [row][8-channel chunk][pixel], so the 16 chunk groups of a 128-row A operand
+// run on into the following dZ rows: one MMA forms 128 / COUT vertical taps at once
+// (COUT = 32: all three, the last 32 rows of D unused; 64: two and one; 128: one each).
+struct WgradTile {
+  int TW, TH, zp, xp;   // zp: pixels between dZ chunk groups; xp: of an X plane
+  int ncol, nrow, ntile;
+  int buf;              // bytes of one of the two tile buffers
 };
-
-template <int CI>
-__host__ __device__ constexpr int wgrad_smem() {
-  return 2 * (128 * kPixChunk * 2 + CI * kPixChunk * 2) + 64 + 1024;
+struct WgradArgs {
+  Input in;          // the layer's input
+  const bf16* dz;    // masked gradient of the layer's output [n][H][W][CO]
+  float* part;       // [nsplit][9 CO CI + CO]
+  int n, H, W;
+  int* err;
+  WgradTile t;
+};
+// Vertical tap sets of a layer; a CTA (blockIdx.y) takes one set and one horizontal tap.
+// The slices of the pixels (blockIdx.x) stay at 64 and the taps fill the GPU instead: the
+// tensor core truncates every addition to its FP32 accumulator, so the sum shrinks with the
+// length of the chain, and 64 slices give the chain lengths that the library has always had.
+template <int CO>
+__host__ __device__ constexpr int wgrad_sets() {
+  return CO == 32 ? 1 : CO == 64 ? 2 : 3;
 }
+constexpr int kWgradSlices = 64;
 
+// Bound by the copies of its tiles and the MMA issue of the 64 slices' CTAs (about 3000 and
+// 2700 cycles a tile).  436 us for the 32 -> 32 layer on 8 samples of 561 x 321 with its bias
+// gradient; one tap per CTA, with both operands transposed by 2-byte shared-memory stores, took
+// 958 us and 1 to 2 ms for the bias in a kernel of its own.
 template <int CI, int CO>
-__global__ void __launch_bounds__(128) k_conv3x3_wgrad(WgradArgs a) {
-  static_assert(CI % 16 == 0 && CO % 8 == 0 && CO <= 128 && CI <= 128, "tile shape");
-  constexpr int A_BYTES = 128 * kPixChunk * 2, B_BYTES = CI * kPixChunk * 2, STAGE = A_BYTES + B_BYTES;
+__global__ void __launch_bounds__(kConvThreads) k_conv3x3_wgrad(WgradArgs a) {
+  static_assert(CI % 16 == 0 && CI <= 128 && (CO == 32 || CO == 64 || CO == 128), "tile shape");
+  constexpr int I8 = CI / 8, O8 = CO / 8, NT = 128 / CO;   // NT: vertical taps per MMA
   constexpr int NCOL = tmem_cols<CI>();
-  constexpr uint32_t IDESC = idesc_bf16(128, CI);
+  constexpr uint32_t IDESC = idesc_bf16(128, CI) | (1u << 15) | (1u << 16);   // A and B MN-major
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = align1024(smem_raw);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + 2 * STAGE);
-  uint32_t* taddr_s = reinterpret_cast<uint32_t*>(bar + 2);
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ uint32_t taddr_s;
+  __shared__ float bsum[kConvThreads];
+  const int TW = a.t.TW, TH = a.t.TH, zp = a.t.zp, xp = a.t.xp, XW = TW + 2;
+  unsigned char* sm = align128(smem_raw);
+  const int xoff = (TH + 2) * O8 * zp * 16;   // X after dZ in each buffer
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int H = a.H, W = a.W, set = blockIdx.y / 3, dx = blockIdx.y % 3;
 
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int t = blockIdx.y, split = blockIdx.x;
-  const int dy = t / 3 - 1, dx = t % 3 - 1;
-  const int H = a.H, W = a.W;
-  const long npix = (long)a.n * H * W;
-  const long nchunk = (npix + kPixChunk - 1) / kPixChunk;
-  const long per = (nchunk + a.nsplit - 1) / a.nsplit;
-  const long c0 = split * per, c1 = c0 + per < nchunk ? c0 + per : nchunk;
-  const int nloc = c1 > c0 ? (int)(c1 - c0) : 0;
-
-  // rows CO..127 of A stay zero in both stages
-  if constexpr (CO < 128) {
-    constexpr int PAD = 128 - CO;
-    for (int i = tid; i < 2 * PAD * (kPixChunk / 8); i += 128) {
-      const int st = i / (PAD * (kPixChunk / 8));
-      const int r = i % (PAD * (kPixChunk / 8));
-      const int m = CO + r % PAD, kc = r / PAD;
-      *reinterpret_cast<uint4*>(sm + st * STAGE + kc * 2048 + m * 16) = make_uint4(0u, 0u, 0u, 0u);
-    }
-  }
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     fence_mbar_init();
   }
-  if (warp == 0) tc_alloc(taddr_s, NCOL);
+  if (warp == 0) tc_alloc(&taddr_s, NCOL);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *taddr_s;
-
-  bool ok = true;
-  for (int c = 0; c < nloc; ++c) {
-    const int s = c & 1;
-    unsigned char* As = sm + s * STAGE;
-    unsigned char* Bs = As + A_BYTES;
-    if (c >= 2 && !mbar_wait(&bar[s], ((c - 2) >> 1) & 1)) ok = false;
-    const long pbase = (c0 + c) * kPixChunk;
-    // A(m = cout, k = pixel) = dY * (gate > 0)
-    for (int i = tid; i < kPixChunk * (CO / 8); i += 128) {
-      const int kk = i % kPixChunk, mc = i / kPixChunk;
-      const long p = pbase + kk;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (p < npix)
-        v = relu_gate(*reinterpret_cast<const uint4*>(a.dy + p * CO + mc * 8),
-                      *reinterpret_cast<const uint4*>(a.gate + p * CO + mc * 8));
-      const bf16* e = reinterpret_cast<const bf16*>(&v);
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<bf16*>(As + (kk >> 3) * 2048 + (mc * 8 + q) * 16 + (kk & 7) * 2) = e[q];
-    }
-    // B(n = cin, k = pixel) = X[pixel + tap]
-    for (int i = tid; i < kPixChunk * (CI / 8); i += 128) {
-      const int kk = i % kPixChunk, nc = i / kPixChunk;
-      const long p = pbase + kk;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (p < npix) {
-        const int px = (int)(p % W);
-        const long q = p / W;
-        const int py = (int)(q % H), pb = (int)(q / H);
-        const int yy = py + dy, xx = px + dx;
-        if (yy >= 0 && yy < H && xx >= 0 && xx < W)
-          v = *reinterpret_cast<const uint4*>(a.x + (((long)pb * H + yy) * W + xx) * CI + nc * 8);
+  const uint32_t tmem = taddr_s;
+  auto stage = [&](int tile, int buf) {
+    const uint32_t zs = smem_u32(sm + buf * a.t.buf), xs = zs + xoff;
+    const int c = tile % a.t.ncol, q = tile / a.t.ncol;
+    const int x0 = c * TW, y0 = (q % a.t.nrow) * TH, b = q / a.t.nrow;
+    stage_rows<CO>(zs, O8 * zp * 16, zp * 16, Input{a.dz, nullptr, 0}, H, W, b, y0 - 1, TH + 2, x0, TW);
+    stage_rows<CI>(xs, XW * 16, xp * 16, a.in, H, W, b, y0, TH, x0 - 1, XW);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  bool ok = true, any = false;
+  uint32_t phase[2] = {0, 0};
+  float bias = 0.0f;   // channel tid % CO over the pixel slice tid / CO
+  int it = 0;
+  if ((int)blockIdx.x < a.t.ntile) stage(blockIdx.x, 0);
+  for (int tile = blockIdx.x; tile < a.t.ntile; tile += gridDim.x, ++it) {
+    const int buf = it & 1;
+    const bool more = tile + (int)gridDim.x < a.t.ntile;
+    if (more) {   // the next tile's copies run beside this tile's MMAs, once the last ones are done
+      if (it > 0) {
+        ok = mbar_wait(&bar[buf ^ 1], phase[buf ^ 1]) && ok;
+        phase[buf ^ 1] ^= 1;
+        __syncthreads();   // and the bias sums' reads of that buffer
       }
-      const bf16* e = reinterpret_cast<const bf16*>(&v);
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<bf16*>(Bs + (kk >> 3) * (CI * 16) + (nc * 8 + q) * 16 + (kk & 7) * 2) = e[q];
+      stage(tile + gridDim.x, buf ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      cp_wait_all();
     }
     fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
+    unsigned char* Zs = sm + buf * a.t.buf;
+    const uint32_t zs = smem_u32(Zs), xs = zs + xoff;
     if (tid == 0) {
       tc_fence_after();
-#pragma unroll
-      for (int k = 0; k < kPixChunk / 16; ++k) {
-        const uint64_t da = sdesc(smem_u32(As) + 2 * k * 2048, 2048, 128);
-        const uint64_t db = sdesc(smem_u32(Bs) + 2 * k * (CI * 16), CI * 16, 128);
-        tc_mma(tmem, da, db, IDESC, (c > 0 || k > 0) ? 1u : 0u);
-      }
-      tc_commit(&bar[s]);
+      const uint64_t da0 = sdesc(zs + set * NT * O8 * zp * 16, 128, zp * 16), db0 = sdesc(xs + dx * 16, 128, xp * 16);
+      uint32_t ao = 0, bo = 0, acc = any ? 1u : 0u;
+#pragma unroll 1
+      for (int r = 0; r < TH; ++r, ao += O8 * zp, bo += XW)
+#pragma unroll 1
+        for (int x = 0; x < TW; x += 16, acc = 1u) tc_mma(tmem, sdesc_at(da0, ao + x), sdesc_at(db0, bo + x), IDESC, acc);
+      tc_commit(&bar[buf]);
+    }
+    any = true;
+    if (blockIdx.y == 0) {   // the bias gradient: the tile's own rows of dZ (zeros outside the image)
+      const int co = tid % CO;
+      const unsigned char* z = Zs + (O8 + co / 8) * zp * 16 + (co % 8) * 2;
+      for (int r = 0; r < TH; ++r, z += O8 * zp * 16)
+        for (int xx = tid / CO; xx < TW; xx += kConvThreads / CO)
+          bias += __bfloat162float(*reinterpret_cast<const bf16*>(z + xx * 16));
     }
   }
-  if (nloc > 0 && !mbar_wait(&bar[(nloc - 1) & 1], ((nloc - 1) >> 1) & 1)) ok = false;
+  // the last one or two tiles' MMAs
+  if (ok && it > 1) ok = mbar_wait(&bar[it & 1], phase[it & 1]);
+  if (ok && it > 0) ok = mbar_wait(&bar[(it - 1) & 1], phase[(it - 1) & 1]) && ok;
   tc_fence_after();
+  cp_wait_all();
   ok = __syncthreads_and(ok);
-  const int m = warp * 32 + (tid & 31);
-  float* dst = a.part + (((long)split * 9 + t) * CO + m) * CI;
+  float* dst = a.part + (long)blockIdx.x * (9 * CO * CI + CO);
   if (ok) {
+    // row r of D: vertical tap (r / CO) of its set, cout r % CO; the dZ row above the X row
+    // (index 0) is the tap dy = +1
+    const int r = (warp & 3) * 32 + lane, g = warp >> 2;
 #pragma unroll 1
-    for (int n0 = 0; n0 < CI; n0 += 16) {
+    for (int n0 = g * 16; n0 < CI; n0 += 32) {
       float v[16];
-      if (nloc > 0) {
-        tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)n0, v);
+      if (any) {
+        tc_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)n0, v);
       } else {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) v[q] = 0.0f;
+        for (int k = 0; k < 16; ++k) v[k] = 0.0f;
       }
-      if (m < CO) {
+      const int dyi = set * NT + r / CO;
+      if (dyi < 3) {
+        float4* o = reinterpret_cast<float4*>(dst + ((long)(3 * (2 - dyi) + dx) * CO + r % CO) * CI + n0);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) dst[n0 + q] = v[q];
+        for (int k = 0; k < 4; ++k) o[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+      }
+    }
+    if (blockIdx.y == 0) {
+      bsum[tid] = bias;
+      __syncthreads();
+      if (tid < CO) {
+        float s = 0.0f;
+        for (int k = tid; k < kConvThreads; k += CO) s += bsum[k];
+        dst[9 * CO * CI + tid] = s;
       }
     }
   } else if (tid == 0) {
@@ -419,27 +536,36 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad(WgradArgs a) {
 // ---------------------------------------------------------------------------
 // reductions, elementwise layers, head + loss, Adam
 // ---------------------------------------------------------------------------
-// out[c] = sum over r of part[r][c], r in order (deterministic)
-__global__ void k_sum_rows(const float* part, int nrows, int ncols, float* out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncols) return;
+// out[c] = sum over r of part[r][c] in a fixed order: 8 threads per column take every eighth
+// row, their sums are added in turn (deterministic)
+__global__ void __launch_bounds__(256) k_sum_rows(const float* part, int nrows, int ncols, float* out) {
+  __shared__ float sh[8][32];
+  const int c = blockIdx.x * 32 + threadIdx.x;
   float s = 0.0f;
-  for (int r = 0; r < nrows; ++r) s += part[(long)r * ncols + c];
-  out[c] = s;
-}
-
-// per-block partial sums of dZ = dY * (Y > 0) over a slice of pixels, one thread per channel
-__global__ void k_bias_part(const bf16* dy, const bf16* gate, long npix, int C, int nblk, float* part) {
-  const int c = threadIdx.x;
-  if (c >= C) return;
-  const long per = (npix + nblk - 1) / nblk;
-  const long p0 = blockIdx.x * per, p1 = p0 + per < npix ? p0 + per : npix;
-  float s = 0.0f;
-  for (long p = p0; p < p1; ++p) {
-    const float g = __bfloat162float(gate[p * C + c]);
-    if (g > 0.0f) s += __bfloat162float(dy[p * C + c]);
+  if (c < ncols) {
+#pragma unroll 8
+    for (int r = threadIdx.y; r < nrows; r += 8) s += part[(long)r * ncols + c];
   }
-  part[(long)blockIdx.x * C + c] = s;
+  sh[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && c < ncols) {
+    for (int k = 1; k < 8; ++k) s += sh[k][threadIdx.x];
+    out[c] = s;
+  }
+}
+// out[0] = sum of part[0..n) by one block, in a fixed order
+__global__ void __launch_bounds__(1024) k_sum_all(const float* part, int n, float* out) {
+  __shared__ float sh[32];
+  float s = 0.0f;
+  for (int i = threadIdx.x; i < n; i += 1024) s += part[i];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = sh[threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) out[0] = s;
+  }
 }
 
 // 2x2 average pool, 8 channels per thread
@@ -466,8 +592,9 @@ __global__ void k_pool(const bf16* x, bf16* y, int n, int H, int W, int C) {
   *reinterpret_cast<uint4*>(y + (((long)b * H2 + Y) * W2 + X) * C + c8 * 8) = *reinterpret_cast<uint4*>(o);
 }
 
-// g_hi += 0.25 * g_lo (nearest), the adjoint of the 2x2 average pool
-__global__ void k_pool_bwd_add(const bf16* glo, bf16* ghi, int n, int H, int W, int C) {
+// g_hi = (g_hi + 0.25 g_lo) masked by the ReLU of act: the adjoint of the 2x2 average pool
+// added to the gradient from the skip connection, which completes that tensor's gradient
+__global__ void k_pool_bwd_add(const bf16* glo, const bf16* act, bf16* ghi, int n, int H, int W, int C) {
   const int C8 = C / 8;
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long)n * H * W * C8) return;
@@ -484,30 +611,12 @@ __global__ void k_pool_bwd_add(const bf16* glo, bf16* ghi, int n, int H, int W, 
   const bf16* el = reinterpret_cast<const bf16*>(&vl);
 #pragma unroll
   for (int k = 0; k < 8; ++k) eh[k] = __float2bfloat16_rn(__bfloat162float(eh[k]) + 0.25f * __bfloat162float(el[k]));
-  *reinterpret_cast<uint4*>(ghi + dst) = vh;
+  *reinterpret_cast<uint4*>(ghi + dst) = relu_gate(vh, *reinterpret_cast<const uint4*>(act + dst));
 }
 
-// out[..][0:C1] = lo (nearest x2), out[..][C1:C1+C2] = skip
-__global__ void k_upcat(const bf16* lo, const bf16* skip, bf16* out, int n, int H, int W, int C1, int C2) {
-  const int C = C1 + C2, C8 = C / 8;
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long)n * H * W * C8) return;
-  const int c8 = (int)(i % C8);
-  long q = i / C8;
-  const int x = (int)(q % W);
-  q /= W;
-  const int y = (int)(q % H), b = (int)(q / H);
-  const int c = c8 * 8;
-  uint4 v;
-  if (c < C1)
-    v = *reinterpret_cast<const uint4*>(lo + (((long)b * (H / 2) + y / 2) * (W / 2) + x / 2) * C1 + c);
-  else
-    v = *reinterpret_cast<const uint4*>(skip + (((long)b * H + y) * W + x) * C2 + (c - C1));
-  *reinterpret_cast<uint4*>(out + (((long)b * H + y) * W + x) * C + c) = v;
-}
-
-// adjoint of k_upcat: g_lo = sum of the 4 children, g_skip = its slice (written)
-__global__ void k_upcat_bwd(const bf16* gout, bf16* glo, bf16* gskip, int n, int H, int W, int C1, int C2) {
+// adjoint of the upsampling + concatenation [lo (nearest x2), skip]: g_lo = sum of the 4
+// children, masked by the ReLU of alo; g_skip = its slice (written, not yet masked)
+__global__ void k_upcat_bwd(const bf16* gout, const bf16* alo, bf16* glo, bf16* gskip, int n, int H, int W, int C1, int C2) {
   const int C = C1 + C2;
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const long nlo = (long)n * (H / 2) * (W / 2) * (C1 / 8);
@@ -529,8 +638,9 @@ __global__ void k_upcat_bwd(const bf16* gout, bf16* glo, bf16* gskip, int n, int
     __align__(16) bf16 o[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) o[k] = __float2bfloat16_rn(s[k]);
-    *reinterpret_cast<uint4*>(glo + (((long)b * (H / 2) + Y) * (W / 2) + X) * C1 + c8 * 8) =
-        *reinterpret_cast<uint4*>(o);
+    const long dst = (((long)b * (H / 2) + Y) * (W / 2) + X) * C1 + c8 * 8;
+    *reinterpret_cast<uint4*>(glo + dst) =
+        relu_gate(*reinterpret_cast<uint4*>(o), *reinterpret_cast<const uint4*>(alo + dst));
   } else if (i < nlo + nsk) {
     const long r = i - nlo;
     const int c8 = (int)(r % (C2 / 8));
@@ -557,10 +667,19 @@ struct LossWeights {
   float w[kOut];
 };
 
+// One thread per pixel.  The weights are read from shared memory four at a time (a broadcast:
+// every thread needs the same ones); read from global memory, one load per multiply-add made
+// the load unit the bound (326 us for 8 training samples of 561 x 321, whose tensors cross
+// HBM in 65 us).  With targets, gd1 is masked by the ReLU of d1.
 __global__ void __launch_bounds__(128) k_head(const bf16* d1, const float* wh, const float* bh, float* out,
                                               const float* tgt, float* dout, bf16* gd1, float* part, int n, int H,
                                               int W, int ny, int nx, int nz, float inv_count, LossWeights lw) {
   __shared__ float red[4];
+  __shared__ __align__(16) float sw[kOut * kHeadC];
+  __shared__ float sb[kOut];
+  for (int i = threadIdx.x; i < kOut * kHeadC; i += 128) sw[i] = wh[i];
+  if (threadIdx.x < kOut) sb[threadIdx.x] = bh[threadIdx.x];
+  __syncthreads();
   const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const long npix = (long)n * H * W;
   float se = 0.0f;
@@ -573,35 +692,50 @@ __global__ void __launch_bounds__(128) k_head(const bf16* d1, const float* wh, c
 #pragma unroll
       for (int k = 0; k < 8; ++k) f[c8 * 8 + k] = __bfloat162float(e[k]);
     }
-    float o[kOut];
+    float gd[kHeadC];
 #pragma unroll
-    for (int j = 0; j < kOut; ++j) {
-      float s = bh[j];
+    for (int c = 0; c < kHeadC; ++c) gd[c] = 0.0f;
+    const int x = (int)(p % W), y = (int)((p / W) % H);
 #pragma unroll
-      for (int c = 0; c < kHeadC; ++c) s = fmaf(wh[j * kHeadC + c], f[c], s);
-      o[j] = s;
-    }
-    if (out) {
+    for (int j4 = 0; j4 < kOut; j4 += 4) {
+      float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f), o4, g4;
+      if (tgt) t4 = *reinterpret_cast<const float4*>(tgt + p * kOut + j4);
 #pragma unroll
-      for (int j = 0; j < kOut; ++j) out[p * kOut + j] = o[j];
+      for (int jj = 0; jj < 4; ++jj) {
+        const int j = j4 + jj;
+        const float4* w4 = reinterpret_cast<const float4*>(sw + j * kHeadC);
+        float s = sb[j];
+#pragma unroll
+        for (int c4 = 0; c4 < kHeadC / 4; ++c4) {
+          const float4 w = w4[c4];
+          s = fmaf(w.x, f[4 * c4], s);
+          s = fmaf(w.y, f[4 * c4 + 1], s);
+          s = fmaf(w.z, f[4 * c4 + 2], s);
+          s = fmaf(w.w, f[4 * c4 + 3], s);
+        }
+        (&o4.x)[jj] = s;
+        if (tgt) {
+          const float e = out_valid(j, x, y, nx, ny, nz) ? s - (&t4.x)[jj] : 0.0f;
+          const float g = 2.0f * lw.w[j] * e * inv_count;
+          se += lw.w[j] * e * e;
+          (&g4.x)[jj] = g;
+#pragma unroll
+          for (int c4 = 0; c4 < kHeadC / 4; ++c4) {
+            const float4 w = w4[c4];
+            gd[4 * c4] = fmaf(g, w.x, gd[4 * c4]);
+            gd[4 * c4 + 1] = fmaf(g, w.y, gd[4 * c4 + 1]);
+            gd[4 * c4 + 2] = fmaf(g, w.z, gd[4 * c4 + 2]);
+            gd[4 * c4 + 3] = fmaf(g, w.w, gd[4 * c4 + 3]);
+          }
+        }
+      }
+      if (out) *reinterpret_cast<float4*>(out + p * kOut + j4) = o4;
+      if (tgt) *reinterpret_cast<float4*>(dout + p * kOut + j4) = g4;
     }
     if (tgt) {
-      const int x = (int)(p % W), y = (int)((p / W) % H);
-      float gd[kHeadC];
-#pragma unroll
-      for (int c = 0; c < kHeadC; ++c) gd[c] = 0.0f;
-#pragma unroll
-      for (int j = 0; j < kOut; ++j) {
-        const float e = out_valid(j, x, y, nx, ny, nz) ? o[j] - tgt[p * kOut + j] : 0.0f;
-        const float g = 2.0f * lw.w[j] * e * inv_count;
-        se += lw.w[j] * e * e;
-        dout[p * kOut + j] = g;
-#pragma unroll
-        for (int c = 0; c < kHeadC; ++c) gd[c] = fmaf(g, wh[j * kHeadC + c], gd[c]);
-      }
       __align__(16) bf16 gb[kHeadC];
 #pragma unroll
-      for (int c = 0; c < kHeadC; ++c) gb[c] = __float2bfloat16_rn(gd[c]);
+      for (int c = 0; c < kHeadC; ++c) gb[c] = __float2bfloat16_rn(f[c] > 0.0f ? gd[c] : 0.0f);
 #pragma unroll
       for (int c8 = 0; c8 < kHeadC / 8; ++c8)
         *reinterpret_cast<uint4*>(gd1 + p * kHeadC + c8 * 8) = reinterpret_cast<const uint4*>(gb)[c8];
@@ -614,23 +748,59 @@ __global__ void __launch_bounds__(128) k_head(const bf16* d1, const float* wh, c
   if (threadIdx.x == 0) part[blockIdx.x] = ((red[0] + red[1]) + red[2]) + red[3];
 }
 
-// per-block partial sums of the head's gradient: thread t < kOut*kHeadC sums
-// dout[p][t / kHeadC] * d1[p][t % kHeadC], thread kOut*kHeadC + o sums dout[p][o]
+// per-block partial sums of the head's gradient, out[o][c] = sum_p dout[p][o] d1[p][c], then
+// the bias gradient out[kOut kHeadC + o] = sum_p dout[p][o], all in FP32.  A block stages
+// kHwChunk pixels in shared memory; a thread owns a 4 x 4 tile of (o, c) over every fourth
+// pixel (two 16-byte reads for 16 multiply-adds; one output per thread took 1223 us on 8
+// samples of 561 x 321), and the four slices are added in turn at the end.
 constexpr int kHeadGrad = kOut * kHeadC + kOut;
-__global__ void __launch_bounds__(kHeadGrad) k_head_wgrad(const float* dout, const bf16* d1, long npix, int nblk,
-                                                          float* part) {
-  const int t = threadIdx.x;
+constexpr int kHwChunk = 64, kHwTiles = (kOut / 4) * (kHeadC / 4), kHwThreads = 4 * kHwTiles;
+__global__ void __launch_bounds__(kHwThreads) k_head_wgrad(const float* dout, const bf16* d1, long npix, int nblk,
+                                                           float* part) {
+  __shared__ __align__(16) float sd[kHwChunk * kOut];
+  __shared__ __align__(16) float sf[kHwChunk * kHeadC];
+  const int t = threadIdx.x, tile = t % kHwTiles, slice = t / kHwTiles;
+  const int o0 = tile % (kOut / 4) * 4, c0 = tile / (kOut / 4) * 4;
   const long per = (npix + nblk - 1) / nblk;
   const long p0 = blockIdx.x * per, p1 = p0 + per < npix ? p0 + per : npix;
-  float s = 0.0f;
-  if (t < kOut * kHeadC) {
-    const int o = t / kHeadC, c = t % kHeadC;
-    for (long p = p0; p < p1; ++p) s = fmaf(dout[p * kOut + o], __bfloat162float(d1[p * kHeadC + c]), s);
-  } else {
-    const int o = t - kOut * kHeadC;
-    for (long p = p0; p < p1; ++p) s += dout[p * kOut + o];
+  float acc[4][4] = {}, bs[4] = {};
+  for (long p = p0; p < p1; p += kHwChunk) {
+    const int m = (int)(p1 - p < kHwChunk ? p1 - p : kHwChunk);
+    __syncthreads();
+    for (int i = t; i < kHwChunk * kOut / 4; i += kHwThreads)
+      reinterpret_cast<float4*>(sd)[i] = i < m * (kOut / 4) ? reinterpret_cast<const float4*>(dout + p * kOut)[i]
+                                                            : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = t; i < kHwChunk * kHeadC / 8; i += kHwThreads) {
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (i < m * (kHeadC / 8)) v = reinterpret_cast<const uint4*>(d1 + p * kHeadC)[i];
+      const bf16* e = reinterpret_cast<const bf16*>(&v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sf[i * 8 + k] = __bfloat162float(e[k]);
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int q = slice; q < kHwChunk; q += 4) {
+      const float4 d = *reinterpret_cast<const float4*>(sd + q * kOut + o0);
+      const float4 f = *reinterpret_cast<const float4*>(sf + q * kHeadC + c0);
+      const float dv[4] = {d.x, d.y, d.z, d.w}, fv[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        bs[i] += dv[i];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[i][k] = fmaf(dv[i], fv[k], acc[i][k]);
+      }
+    }
   }
-  part[(long)blockIdx.x * kHeadGrad + t] = s;
+  float* dst = part + (long)blockIdx.x * kHeadGrad;
+  __shared__ float red[4][kHeadGrad];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) red[slice][(o0 + i) * kHeadC + c0 + k] = acc[i][k];
+    if (c0 == 0) red[slice][kOut * kHeadC + o0 + i] = bs[i];
+  }
+  __syncthreads();
+  for (int i = t; i < kHeadGrad; i += kHwThreads) dst[i] = ((red[0][i] + red[1][i]) + red[2][i]) + red[3][i];
 }
 
 __global__ void k_adam(float* w, const float* g, float* m, float* v, bf16* wb, long n, float lr, float c1,
@@ -750,36 +920,90 @@ __global__ void k_apply(Dims d, const float* pred, StatePtrs s, int Wp, int velo
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-template <int KC, int NO, bool DG>
-int launch_conv(const ConvArgs& a, cudaStream_t st) {
-  constexpr int need = conv_smem<KC, NO>();
-  constexpr int floor_ = smem_floor(tmem_cols<NO>());
-  constexpr int smem = need > floor_ ? need : floor_;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_conv3x3<KC, NO, DG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-        cudaSuccess)
-      return DIVA_CUDA_ERROR;
-    attr = true;
+constexpr int kSMs = 148;   // B200
+
+// CTAs of a persistent kernel that fit on the GPU: by its shared memory (228 KB per SM, 1 KB of
+// it per CTA) and by tensor memory (512 columns per SM)
+int resident_ctas(int smem, int ncols) {
+  const int by_smem = 228 * 1024 / (smem + 1024 + 2048), by_tmem = 512 / ncols;
+  const int k = std::min(std::min(by_smem, by_tmem), 8);
+  return kSMs * std::max(k, 1);
+}
+
+// The tile of a forward / dgrad convolution of H x W images: of all column splits the one with
+// the least work, counting the accumulator rows (128 per block, the halo columns and the
+// ragged ends among them) and the staged pixels of all tiles.
+ConvTile conv_tile(int n, int H, int W, int nb, int C) {
+  ConvTile best{};
+  double cost = 0.0;
+  for (int ncol = 1; ncol <= W; ++ncol) {
+    const int TW = (W + ncol - 1) / ncol, P = TW + 2;
+    if ((W + TW - 1) / TW != ncol || P > 128 * nb) continue;
+    if (best.TW && TW < 8) break;
+    const int TH = std::min(H, 128 * nb / P), nrow = (H + TH - 1) / TH;
+    const double c = (double)ncol * nrow * (128 * nb + (TH + 2) * P);
+    if (!best.TW || c < cost) {
+      cost = c;
+      best = ConvTile{TW, TH, P, plane_px(128 * nb + 2 * P + 2, C), ncol, nrow, n * ncol * nrow};
+    }
   }
-  const long npix = (long)a.n * a.H * a.W;
-  k_conv3x3<KC, NO, DG><<<(unsigned)((npix + 127) / 128), 128, smem, st>>>(a);
+  return best;
+}
+
+template <int KC, int NO, bool DG>
+int launch_conv(ConvArgs a, cudaStream_t st) {
+  constexpr int NB = conv_blocks<KC, NO>();
+  a.t = conv_tile(a.n, a.H, a.W, NB, KC);
+  const int smem = conv_wbytes<KC, NO>() + (KC / 8) * a.t.npx * 16 + 128;
+  if (cudaFuncSetAttribute(k_conv3x3<KC, NO, DG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return DIVA_CUDA_ERROR;
+  const int grid = std::min(a.t.ntile, resident_ctas(smem, tmem_cols<NB * NO>()));
+  k_conv3x3<KC, NO, DG><<<grid, kConvThreads, smem, st>>>(a);
   return DIVA_OK;
 }
 
+// The tile of a weight gradient: a multiple of 16 pixels wide (zeros beyond the image), the
+// width with the fewest staged pixels; rows so that two tile buffers take about 110 KB at
+// most (two CTAs per SM).
 template <int CI, int CO>
-int launch_wgrad(const WgradArgs& a, cudaStream_t st) {
-  constexpr int need = wgrad_smem<CI>();
-  constexpr int floor_ = smem_floor(tmem_cols<CI>());
-  constexpr int smem = need > floor_ ? need : floor_;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_conv3x3_wgrad<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-        cudaSuccess)
-      return DIVA_CUDA_ERROR;
-    attr = true;
+WgradTile wgrad_tile(int n, int H, int W) {
+  WgradTile t{};
+  long cost = 0;
+  for (int TW = 16; TW <= 64; TW += 16) {
+    const long c = (long)((W + TW - 1) / TW) * (TW * CO + (TW + 2) * CI);
+    if (!t.TW || c <= cost) {
+      cost = c;
+      t.TW = TW;
+    }
   }
-  k_conv3x3_wgrad<CI, CO><<<dim3(a.nsplit, 9), 128, smem, st>>>(a);
+  t.zp = plane_px(t.TW, CO);
+  for (t.TH = std::min(H, 8);; --t.TH) {
+    t.xp = plane_px(t.TH * (t.TW + 2), CI);
+    // dZ, then X; the last A operands run one or more dZ rows on (rows of D that nothing reads)
+    const int zrow = CO / 8 * t.zp * 16, xbytes = CI / 8 * t.xp * 16;
+    t.buf = ((t.TH + 2) * zrow + std::max(xbytes, 128 / CO * zrow) + 127) / 128 * 128;
+    if (2 * t.buf <= 110 * 1024 || t.TH <= 2) break;
+  }
+  t.ncol = (W + t.TW - 1) / t.TW;
+  t.nrow = (H + t.TH - 1) / t.TH;
+  t.ntile = n * t.ncol * t.nrow;
+  return t;
+}
+
+template <int CI, int CO>
+int launch_wgrad(WgradArgs a, long part_floats, int* nsplit, cudaStream_t st) {
+  constexpr int NCOL = tmem_cols<CI>();
+  a.t = wgrad_tile<CI, CO>(a.n, a.H, a.W);
+  int smem = 2 * a.t.buf + 128;
+  // no more CTAs on an SM than its tensor memory serves
+  smem = std::max(smem, 227 * 1024 / (512 / NCOL + 1));
+  if (cudaFuncSetAttribute(k_conv3x3_wgrad<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+      cudaSuccess)
+    return DIVA_CUDA_ERROR;
+  const int grid = std::min(a.t.ntile, kWgradSlices);
+  if ((long)grid * (9 * CI * CO + CO) > part_floats) return DIVA_BAD_INPUT;
+  *nsplit = grid;
+  k_conv3x3_wgrad<CI, CO><<<dim3(grid, 3 * wgrad_sets<CO>()), kConvThreads, smem, st>>>(a);
   return DIVA_OK;
 }
 
@@ -797,9 +1021,9 @@ int conv_dgrad(int cin, int cout, const ConvArgs& a, cudaStream_t st) {
 #undef DGR
   return DIVA_UNSUPPORTED;
 }
-int conv_wgrad(int cin, int cout, const WgradArgs& a, cudaStream_t st) {
+int conv_wgrad(int cin, int cout, const WgradArgs& a, long part_floats, int* nsplit, cudaStream_t st) {
 #define WGR(CI, CO) \
-  if (cin == CI && cout == CO) return launch_wgrad<CI, CO>(a, st);
+  if (cin == CI && cout == CO) return launch_wgrad<CI, CO>(a, part_floats, nsplit, st);
   WGR(16, 32) WGR(32, 32) WGR(32, 64) WGR(64, 64) WGR(64, 128) WGR(128, 64) WGR(64, 32)
 #undef WGR
   return DIVA_UNSUPPORTED;
@@ -860,11 +1084,6 @@ struct diva_cnn {
   int lvH(int l) const { return Hp >> l; }
   int lvW(int l) const { return Wp >> l; }
   long tsize(int t) const { return (long)lvH(kTLevel[t]) * lvW(kTLevel[t]) * kTChan[t]; }
-  int wgrad_split(long npix) const {
-    const long nchunk = (npix + kPixChunk - 1) / kPixChunk;
-    long s = nchunk < 64 ? nchunk : 64;
-    return (int)(s < 1 ? 1 : s);
-  }
 };
 
 namespace {
@@ -880,27 +1099,28 @@ namespace {
   } while (0)
 
 inline unsigned nblk(long n, int b) { return (unsigned)((n + b - 1) / b); }
-constexpr int kHeadBlocks = 148;
+constexpr int kHeadBlocks = 592;   // four per SM
+
+// the input of layer l: a stored tensor, or the concatenation [lo (upsampled), skip]
+Input layer_input(const diva_cnn_t* N, int l, const bf16* in) {
+  const int t = N->L[l].in;
+  if (t == T_U1) return Input{N->act[T_E1], N->act[T_D2], kTChan[T_D2]};
+  if (t == T_U2) return Input{N->act[T_E2], N->act[T_B2], kTChan[T_B2]};
+  return Input{t == T_IN ? in : N->act[t], nullptr, 0};
+}
 
 int forward(diva_cnn_t* N, const bf16* in, float* out, int n, cudaStream_t st) {
-  auto tens = [&](int t) -> const bf16* { return t == T_IN ? in : N->act[t]; };
   auto conv = [&](int l) {
     const Layer& ly = N->L[l];
     const int lv = kTLevel[ly.out];
-    ConvArgs a{tens(ly.in), nullptr, N->wb + ly.woff, N->w + ly.boff, N->act[ly.out], n, N->lvH(lv), N->lvW(lv),
-               1, N->err};
+    ConvArgs a{layer_input(N, l, in), N->wb + ly.woff, N->w + ly.boff, nullptr, N->act[ly.out], n, N->lvH(lv),
+               N->lvW(lv), N->err, {}};
     return conv_fwd(ly.cin, ly.cout, a, st);
   };
   auto pool = [&](int src, int dst) {
     const int lv = kTLevel[src];
     const long cnt = (long)n * (N->lvH(lv) / 2) * (N->lvW(lv) / 2) * (kTChan[src] / 8);
     k_pool<<<nblk(cnt, 256), 256, 0, st>>>(N->act[src], N->act[dst], n, N->lvH(lv), N->lvW(lv), kTChan[src]);
-  };
-  auto upcat = [&](int lo, int skip, int dst) {
-    const int lv = kTLevel[dst];
-    const long cnt = (long)n * N->lvH(lv) * N->lvW(lv) * (kTChan[dst] / 8);
-    k_upcat<<<nblk(cnt, 256), 256, 0, st>>>(N->act[lo], N->act[skip], N->act[dst], n, N->lvH(lv), N->lvW(lv),
-                                            kTChan[lo], kTChan[skip]);
   };
   RET(conv(0));
   RET(conv(1));
@@ -910,10 +1130,8 @@ int forward(diva_cnn_t* N, const bf16* in, float* out, int n, cudaStream_t st) {
   pool(T_E2, T_P2);
   RET(conv(4));
   RET(conv(5));
-  upcat(T_B2, T_E2, T_U2);
   RET(conv(6));
   RET(conv(7));
-  upcat(T_D2, T_E1, T_U1);
   RET(conv(8));
   RET(conv(9));
   if (out) {
@@ -931,30 +1149,30 @@ int backward(diva_cnn_t* N, const bf16* in, const float* tgt, int n, cudaStream_
   const long npix0 = (long)n * N->Hp * N->Wp;
   const unsigned hb = nblk(npix0, 128);
   if ((long)hb > N->part_floats - 128 || (long)kHeadBlocks * kHeadGrad > N->part_floats - 128) return DIVA_BAD_INPUT;
+  auto sum_rows = [&](int rows, long cols, float* dst) {
+    k_sum_rows<<<nblk(cols, 32), dim3(32, 8), 0, st>>>(N->part, rows, (int)cols, dst);
+  };
   k_head<<<hb, 128, 0, st>>>(N->act[T_D1], N->w + N->head_w, N->w + N->head_b, nullptr, tgt, N->dout,
                              N->grad[T_D1], N->part, n, N->Hp, N->Wp, N->ny, N->nx, N->nz,
                              1.0f / (float)N->valid(n), N->lw);
-  k_sum_rows<<<1, 32, 0, st>>>(N->part, (int)hb, 1, loss_dst);
-  k_head_wgrad<<<kHeadBlocks, kHeadGrad, 0, st>>>(N->dout, N->act[T_D1], npix0, kHeadBlocks, N->part);
-  k_sum_rows<<<nblk(kHeadGrad, 256), 256, 0, st>>>(N->part, kHeadBlocks, kHeadGrad, N->g + N->head_w);
+  k_sum_all<<<1, 1024, 0, st>>>(N->part, (int)hb, loss_dst);
+  k_head_wgrad<<<kHeadBlocks, kHwThreads, 0, st>>>(N->dout, N->act[T_D1], npix0, kHeadBlocks, N->part);
+  sum_rows(kHeadBlocks, kHeadGrad, N->g + N->head_w);
 
-  auto tens = [&](int t) -> const bf16* { return t == T_IN ? in : N->act[t]; };
   auto layer_bwd = [&](int l, bool dgrad) -> int {
     const Layer& ly = N->L[l];
     const int lv = kTLevel[ly.out];
     const int H = N->lvH(lv), W = N->lvW(lv);
-    const long npix = (long)n * H * W;
-    const int ns = N->wgrad_split(npix);
-    const long wn = 9L * ly.cout * ly.cin;
-    if ((long)ns * wn > N->part_floats - 128) return DIVA_BAD_INPUT;
-    WgradArgs wa{tens(ly.in), N->grad[ly.out], N->act[ly.out], N->part, n, H, W, ns, N->err};
-    RET(conv_wgrad(ly.cin, ly.cout, wa, st));
-    k_sum_rows<<<nblk(wn, 256), 256, 0, st>>>(N->part, ns, (int)wn, N->g + ly.woff);
-    const int nb = 128;
-    k_bias_part<<<nb, 128, 0, st>>>(N->grad[ly.out], N->act[ly.out], npix, ly.cout, nb, N->part);
-    k_sum_rows<<<1, 128, 0, st>>>(N->part, nb, ly.cout, N->g + ly.boff);
+    int ns = 0;
+    WgradArgs wa{layer_input(N, l, in), N->grad[ly.out], N->part, n, H, W, N->err, {}};
+    RET(conv_wgrad(ly.cin, ly.cout, wa, N->part_floats - 128, &ns, st));
+    sum_rows(ns, 9L * ly.cout * ly.cin + ly.cout, N->g + ly.woff);   // the bias follows the weights
     if (dgrad) {
-      ConvArgs a{N->grad[ly.out], N->act[ly.out], N->wbt + ly.woff, nullptr, N->grad[ly.in], n, H, W, 0, N->err};
+      // a tensor that one convolution writes and one reads has its whole gradient here: masked;
+      // pooled and concatenated ones pass through the adjoints below
+      const bool whole = ly.in == T_A1 || ly.in == T_A2 || ly.in == T_B1 || ly.in == T_C1 || ly.in == T_C2;
+      ConvArgs a{Input{N->grad[ly.out], nullptr, 0}, N->wbt + ly.woff, nullptr, whole ? N->act[ly.in] : nullptr,
+                 N->grad[ly.in], n, H, W, N->err, {}};
       RET(conv_dgrad(ly.cin, ly.cout, a, st));
     }
     return DIVA_OK;
@@ -963,13 +1181,13 @@ int backward(diva_cnn_t* N, const bf16* in, const float* tgt, int n, cudaStream_
     const int lv = kTLevel[dst];
     const int H = N->lvH(lv), W = N->lvW(lv);
     const long cnt = (long)n * (H / 2) * (W / 2) * (kTChan[lo] / 8) + (long)n * H * W * (kTChan[skip] / 8);
-    k_upcat_bwd<<<nblk(cnt, 256), 256, 0, st>>>(N->grad[dst], N->grad[lo], N->grad[skip], n, H, W, kTChan[lo],
-                                                kTChan[skip]);
+    k_upcat_bwd<<<nblk(cnt, 256), 256, 0, st>>>(N->grad[dst], N->act[lo], N->grad[lo], N->grad[skip], n, H, W,
+                                                kTChan[lo], kTChan[skip]);
   };
   auto pool_bwd = [&](int lo, int hi) {
     const int lv = kTLevel[hi];
     const long cnt = (long)n * N->lvH(lv) * N->lvW(lv) * (kTChan[hi] / 8);
-    k_pool_bwd_add<<<nblk(cnt, 256), 256, 0, st>>>(N->grad[lo], N->grad[hi], n, N->lvH(lv), N->lvW(lv),
+    k_pool_bwd_add<<<nblk(cnt, 256), 256, 0, st>>>(N->grad[lo], N->act[hi], N->grad[hi], n, N->lvH(lv), N->lvW(lv),
                                                    kTChan[hi]);
   };
   RET(layer_bwd(9, true));   // d1b -> g_c1
@@ -1068,12 +1286,11 @@ int32_t diva_cnn_create(diva_cnn_t** out, int32_t ny, int32_t nx, int32_t nz, in
   off += kOut;
   N->nw = off;
 
-  // wgrad partials: up to 64 slices of the largest layer; head partials
-  long part = 64L * 9 * 128 * 64;
+  // weight-gradient sums: up to 64 CTAs' of the largest layer (more of a smaller one); head sums
+  long part = 64L * (9 * 128 * 64 + 128);
   const long hb = (long)nblk((long)batch * N->Hp * N->Wp, 128);
   if (hb > part) part = hb;
   if ((long)kHeadBlocks * kHeadGrad > part) part = (long)kHeadBlocks * kHeadGrad;
-  if (128L * 128 > part) part = 128L * 128;
   N->part_floats = part + 128;
 
   const long img = (long)N->Hp * N->Wp;
@@ -1087,7 +1304,8 @@ int32_t diva_cnn_create(diva_cnn_t** out, int32_t ny, int32_t nx, int32_t nz, in
   const size_t o_wb = carve(N->nw * 2), o_wbt = carve(N->nw * 2);
   size_t o_act[T_N], o_grad[T_N];
   for (int t = 0; t < T_N; ++t) {
-    o_act[t] = carve((size_t)batch * N->tsize(t) * 2);
+    // the concatenated tensors are never stored: the convolutions read their two parts
+    o_act[t] = (t == T_U1 || t == T_U2) ? 0 : carve((size_t)batch * N->tsize(t) * 2);
     o_grad[t] = t == T_IN ? 0 : carve((size_t)batch * N->tsize(t) * 2);
   }
   const size_t o_out = carve((size_t)batch * img * kOut * 4), o_tgt = carve((size_t)batch * img * kOut * 4);
@@ -1107,7 +1325,7 @@ int32_t diva_cnn_create(diva_cnn_t** out, int32_t ny, int32_t nx, int32_t nz, in
   N->wb = reinterpret_cast<bf16*>(base + o_wb);
   N->wbt = reinterpret_cast<bf16*>(base + o_wbt);
   for (int t = 0; t < T_N; ++t) {
-    N->act[t] = reinterpret_cast<bf16*>(base + o_act[t]);
+    N->act[t] = (t == T_U1 || t == T_U2) ? nullptr : reinterpret_cast<bf16*>(base + o_act[t]);
     N->grad[t] = t == T_IN ? nullptr : reinterpret_cast<bf16*>(base + o_grad[t]);
   }
   N->out = reinterpret_cast<float*>(base + o_out);
@@ -1235,8 +1453,8 @@ int32_t diva_cnn_predict(diva_cnn_t* N, diva_ctx_t* ctx, int32_t complete_sweeps
   k_apply<<<img_grid(N->ny, N->nx), block2d(), 0, c->stream>>>(c->d, N->out, state_ptrs(c), N->Wp,
                                                                 complete_sweeps > 0, c->c.DIVA_vel_max);
   // the context's launch count includes the network's kernels run on its stream: features,
-  // 10 convolutions, 2 pools, 2 up-concatenations, the head and the state write
-  c->launches += 17;
+  // 10 convolutions, 2 pools, the head and the state write
+  c->launches += 15;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->stream));
   RET(check_err(N));
