@@ -201,6 +201,7 @@ size_t carve(Ctx* c, Carver& cv) {
   const dim3 g = grid2d(d.ny, d.nx);
   c->max_blocks = g.x * g.y;
   c->partials = (double*)cv.take(sizeof(double) * (kAAPartials > 4 ? kAAPartials : 4) * c->max_blocks);
+  c->red_count = (int*)cv.take(sizeof(int) * 4);
   for (int k = 0; k < KV_COUNT; ++k)
     for (int q = 0; q < 2; ++q) c->kv[k][q] = (double*)cv.take(sizeof(double) * d.plane);
   for (int q = 0; q < 2; ++q) {
@@ -376,6 +377,7 @@ int picard(Ctx* c, bool diva, double* u, double* v, diva_report_t* rep) {
                               stall_after(relres, &stall_best, &stall_since, C.picard_stall_its);
       if (relres <= C.picard_relres_tol || stop_stall) {
         stalled_exit = stop_stall;
+        if (it > 1 && (st = launch_commit_err(c))) return st;
         if (diva && (st = launch_basal_stress_velocities(c))) return st;
         break;
       }
@@ -392,9 +394,9 @@ int picard(Ctx* c, bool diva, double* u, double* v, diva_report_t* rep) {
     if (C.picard_anderson_m > 0) {
       // the mixing step reads this iteration's nonlinear residual from the device scalars
       DIVA_CUDA(c, cudaMemcpyAsync(c->scal + SC_RELRES, &relres, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-      if ((st = launch_anderson_prepare(c, u, v, c->kv[KV_X][0], c->kv[KV_X][1]))) return st;
+      if ((st = launch_anderson_prepare(c, u, v, c->kv[KV_XF][0], c->kv[KV_XF][1]))) return st;
     }
-    if ((st = launch_picard_update(c, u, v, c->kv[KV_X][0], c->kv[KV_X][1], diva))) return st;
+    if ((st = launch_picard_update(c, u, v, c->kv[KV_XF][0], c->kv[KV_XF][1], diva, it > 1 ? 1 : 0))) return st;
     DIVA_CUDA(c, cudaMemcpyAsync(c->h_scal + SC_RES1, c->scal + SC_RES1, 3 * sizeof(double), cudaMemcpyDeviceToHost,
                                  c->stream));
     DIVA_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -404,7 +406,6 @@ int picard(Ctx* c, bool diva, double* u, double* v, diva_report_t* rep) {
     bool converged = false;
     if (!relmode && resid < C.DIVA_visc_it_norm_dUV_tol) converged = true;
     else if (it >= C.DIVA_visc_it_nit) converged = true;
-    if (!converged) launch_commit_err(c);
     if (converged) break;
   }
   int status = DIVA_OK;

@@ -412,7 +412,7 @@ constexpr int kWgradSlices = 64;
 template <int CI, int CO>
 __global__ void __launch_bounds__(kConvThreads) k_conv3x3_wgrad(WgradArgs a) {
   static_assert(CI % 16 == 0 && CI <= 128 && (CO == 32 || CO == 64 || CO == 128), "tile shape");
-  constexpr int I8 = CI / 8, O8 = CO / 8, NT = 128 / CO;   // NT: vertical taps per MMA
+  constexpr int O8 = CO / 8, NT = 128 / CO;   // NT: vertical taps per MMA
   constexpr int NCOL = tmem_cols<CI>();
   constexpr uint32_t IDESC = idesc_bf16(128, CI) | (1u << 15) | (1u << 16);   // A and B MN-major
   extern __shared__ unsigned char smem_raw[];

@@ -90,4 +90,49 @@ __device__ __forceinline__ void block_sum(double (&v)[N]) {
   }
 }
 
+// ---- reductions finished by the kernel that starts them ---------------------------------
+// Blocks of 32 x 8 threads walk the points in 32 (j) x 8 (i) tiles, tile t, t + gridDim.x, ...;
+// at most kRedBlocks of them (six per SM), so that the last block's sum over the blocks'
+// partials stays at a few microseconds (one partial per tile: 23 us at 1501 x 1501).
+constexpr int kRedBlocks = 148 * 6;
+inline int red_blocks(const Dims& d) {
+  const int n = ((d.ny + kBX - 1) / kBX) * ((d.nx + kBY - 1) / kBY);
+  return n < kRedBlocks ? n : kRedBlocks;
+}
+#define FOR_TILES(d)                                                                                  \
+  for (int nbx_ = ((d).ny + kBX - 1) / kBX, nt_ = nbx_ * (((d).nx + kBY - 1) / kBY), t_ = blockIdx.x; \
+       t_ < nt_; t_ += gridDim.x)                                                                     \
+    if (const int j = (t_ % nbx_) * kBX + threadIdx.x, i = (t_ / nbx_) * kBY + threadIdx.y;           \
+        j < (d).ny && i < (d).nx)
+
+struct Reduction {
+  double* partials;   // the blocks' sums
+  int* count;         // blocks that have stored theirs: zero before and after every kernel
+};
+// The grid's sum of v: true in thread 0 of the block that finishes last, which has the totals
+// (block sums added in block order by a fixed tree: the same bits whichever block is last).
+template <int N>
+__device__ __forceinline__ bool reduce_all(double (&v)[N], const Reduction& red) {
+  __shared__ bool last;
+  const int t = threadIdx.x + threadIdx.y * blockDim.x, nt = blockDim.x * blockDim.y;
+  block_sum<N>(v);
+  if (t == 0) {
+#pragma unroll
+    for (int q = 0; q < N; ++q) __stcg(red.partials + (long long)N * blockIdx.x + q, v[q]);
+    __threadfence();
+    last = atomicAdd(red.count, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+#pragma unroll
+  for (int q = 0; q < N; ++q) v[q] = 0.0;
+  for (int b = t; b < (int)gridDim.x; b += nt)
+#pragma unroll
+    for (int q = 0; q < N; ++q) v[q] += __ldcg(red.partials + (long long)N * b + q);
+  block_sum<N>(v);
+  if (t == 0) *red.count = 0;
+  return t == 0;
+}
+
 }  // namespace diva

@@ -41,7 +41,9 @@ struct BCs {
 enum { F32_NA = 0, F32_NB, F32_BX, F32_BY, F32_IDU, F32_IDV };
 
 // Krylov vectors on the fine level, each a (u,v) pair of planes.
-enum { KV_X = 0, KV_R, KV_RHAT, KV_P, KV_PHAT, KV_V, KV_S, KV_SHAT, KV_T, KV_B, KV_COUNT };
+enum { KV_X = 0, KV_R, KV_RHAT, KV_P, KV_PHAT, KV_V, KV_S, KV_SHAT, KV_T, KV_B,
+       KV_XF,   // the solution: KV_X with the last half step and the boundary unknowns
+       KV_COUNT };
 
 // Device scalars of the linear solver and of the Picard bookkeeping.
 enum {
@@ -210,6 +212,7 @@ struct Ctx {
   double* scal = nullptr;             // device scalars (SC_*)
   double* h_scal = nullptr;           // pinned host mirror
   double* partials = nullptr;         // block partial sums
+  int* red_count = nullptr;           // blocks of the running reduction that have finished (reduce_all)
   int max_blocks = 0;
   double* kv[KV_COUNT][2] = {};       // Krylov vectors (u,v)
   // Anderson mixing history (u,v plane pairs): ring of residual differences dF and map
@@ -277,25 +280,36 @@ int launch_prepare_afac(Ctx* c);
 // viscosity loop) keeps what it needs to write them after the loop instead
 // (launch_visc_b_output); K1_COLUMNS_ONLY launches the column kernel alone (timing).
 enum { K1_WRITE_SHEAR = 0, K1_LOOP = 1, K1_COLUMNS_ONLY = 2 };
-int launch_diva_coefficients(Ctx* c, const double* u, const double* v, bool diva, int what = K1_WRITE_SHEAR);
-int launch_picard_update(Ctx* c, double* u, double* v, const double* xu, const double* xv, bool diva);
+// begin: also start the counters of a graph-launched viscosity iteration (SC_PIC_IT and on).
+int launch_diva_coefficients(Ctx* c, const double* u, const double* v, bool diva, int what = K1_WRITE_SHEAR,
+                             bool begin = false);
+// The end of a viscosity iteration.  graph: the device decides (0: host-driven loop); loop: the
+// caller also sets the loop's handles a (and b, if has_b) to whether it goes on.
+struct IterEnd {
+  int graph, loop, nit, has_b;
+  double tol;
+  cudaGraphConditionalHandle a, b;
+};
+// commit: whether the previous iteration's DIVA_err candidate becomes the field (it does unless
+// that iteration converged, ice_velocity_module.f90:353-355): 1, 0, or -1: when the device
+// counter says that this is not the first iteration.
+int launch_picard_update(Ctx* c, double* u, double* v, const double* xu, const double* xv, bool diva, int commit,
+                         const IterEnd* end = nullptr);
 // Anderson mixing step before launch_picard_update (picard_anderson_m > 0): the map value
 // g = velocity-limited linear solution, its residual f = g - u, the new history columns
 // and the mixing coefficients (device scalars); launch_picard_update then forms the
 // mixed iterate g - sum gamma_i dG_i in place of the relaxation.
 int launch_anderson_prepare(Ctx* c, const double* u, const double* v, const double* xu, const double* xv);
 int anderson_reset(Ctx* c);   // empty history at the start of a solve (zeroed columns)
-int launch_commit_err(Ctx* c);
+int launch_commit_err(Ctx* c);   // the last candidate, after a host-driven loop that the residual ended
 int launch_basal_stress_velocities(Ctx* c);
+int launch_relres_end(Ctx* c, bool diva, const IterEnd& end);   // post kernel of a rel-res iteration
 int launch_visc_b_output(Ctx* c);   // after the viscosity loop: visc_eff_3D_b and the shear strain rates
 int launch_3d_horizontal_velocities(Ctx* c);
 int launch_secondary_velocities(Ctx* c);
 int launch_sia(Ctx* c);
 int launch_ssa_beta_eff(Ctx* c);
 int launch_zero_velocities(Ctx* c, double* u, double* v);
-int launch_ctl_end(Ctx* c, bool relmode);
-int launch_err_commit_pred(Ctx* c);
-int launch_basal_pred(Ctx* c);
 int launch_any_sheet(Ctx* c, int* result);
 
 // solver.cu
@@ -325,7 +339,6 @@ __host__ __device__ inline bool stall_after(double relres, double* best, double*
 }
 int solver_solve(Ctx* c, const double* u0, const double* v0, double rtol, int maxit, int* iters, double* relres0);
 int solver_relres(Ctx* c, const double* u, const double* v, double* relres);
-int solver_fill_boundary(Ctx* c, double* u, double* v);
 int solver_row_types(Ctx* c);   // finest-level row types of choice_ice_margin 'BC' (after the SICO masks)
 int solver_smooth_fine(Ctx* c, int sweeps);
 int solver_smooth_fine_values(const Ctx* c);

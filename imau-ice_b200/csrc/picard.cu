@@ -48,6 +48,7 @@ struct CoefArgs {
   // rates of the viscosity loop's last iteration can be written after the loop
   int keep_seen;
   double *taub_seen_cx, *taub_seen_cy;
+  double* sc;   // device scalars of a graph-launched iteration that starts here, else null
 };
 
 // strain rates of the depth-averaged velocity on the a-grid,
@@ -158,6 +159,10 @@ __device__ __forceinline__ double stag_mode(int mode, double v0, double v1) {
 __global__ void __launch_bounds__(256) k_column_prep(CoefArgs a) {
   const Dims d = a.d;
   const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
+  if (j == 0 && i == 0 && a.sc) {   // the iteration's counters (nothing else here reads them)
+    a.sc[SC_PIC_IT] += 1.0;
+    a.sc[SC_EXIT_RELRES] = a.sc[SC_LIN_IT] = a.sc[SC_LIN_FULL] = a.sc[SC_SOLVED] = a.sc[SC_CONVERGED] = 0.0;
+  }
   if (j >= d.ny || i >= d.nx) return;
   const int nx = d.nx, ny = d.ny;
   const long long q = d.at(j, i);
@@ -469,28 +474,27 @@ __device__ __forceinline__ double limited_v(const Dims& d, const double* xu, con
 // last m iterations, the next iterate is g - sum_i gamma_i dG_i, gamma the least-squares
 // minimiser of |f - sum_i gamma_i dF_i| (u on the cx points and v on the cy points make
 // one vector).  k_aa_prepare writes g, f and the newest difference columns and reduces
-// the inner products of the newest dF and of f with every history column; k_aa_solve
+// the inner products of the newest dF and of f with every history column; its last block
 // updates the Gram matrix and solves for gamma on one thread; k_picard_update mixes.
 struct AAArgs {
   Dims d;
-  int m, nblk_x;
+  int m;
   double vmax;
   const double *u, *v, *xu, *xv;
   double *dFu[kAAMax], *dFv[kAAMax], *dGu[kAAMax], *dGv[kAAMax];
   double *fu, *fv, *gu, *gv;   // previous f, g on entry; this iteration's on exit
-  const double* sc;
-  double* partials;            // kAAPartials per block: dF_i . dF_new, then dF_i . f
+  double* sc;
+  Reduction red;               // kAAPartials sums: dF_i . dF_new, then dF_i . f
 };
 
 __global__ void __launch_bounds__(256) k_aa_prepare(AAArgs a) {
   const Dims d = a.d;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
   const bool have = a.sc[SC_AA_HAVE] != 0.0;
   const int s = (int)a.sc[SC_AA_HEAD];
   double acc[kAAPartials];
 #pragma unroll
   for (int k = 0; k < kAAPartials; ++k) acc[k] = 0.0;
-  if (j < d.ny && i < d.nx) {
+  FOR_TILES(d) {
     const long long q = d.at(j, i);
     auto point = [&](double g, double x, double* fp, double* gp, double* const* dF, double* const* dG) {
       const double f = g - x;
@@ -517,64 +521,48 @@ __global__ void __launch_bounds__(256) k_aa_prepare(AAArgs a) {
     if (i < d.nx - 1) point(limited_u(d, a.xu, a.xv, a.vmax, j, i), a.u[q], a.fu, a.gu, a.dFu, a.dGu);
     if (j < d.ny - 1) point(limited_v(d, a.xu, a.xv, a.vmax, j, i), a.v[q], a.fv, a.gv, a.dFv, a.dGv);
   }
-  // block sums in groups of at most four values (block_sum keeps one shared array per width)
-  double* out = a.partials + (long long)kAAPartials * (blockIdx.y * a.nblk_x + blockIdx.x);
-  for (int base = 0; base < kAAPartials; base += 4) {
-    double v4[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v4[k] = base + k < kAAPartials ? acc[base + k] : 0.0;
-    block_sum<4>(v4);
-    if (threadIdx.x == 0 && threadIdx.y == 0)
-      for (int k = 0; k < 4 && base + k < kAAPartials; ++k) out[base + k] = v4[k];
-    __syncthreads();
-  }
-}
-
-// One thread: fixed-order sums of the partials, the Gram matrix update and the mixing
-// coefficients.  Shared with the oracle's restatement (aa_coefficients).
-__global__ void k_aa_solve(const double* partials, int nblocks, int m, double* sc) {
-  __shared__ double sh[kAAPartials][256];
-  double t[kAAPartials];
-#pragma unroll
-  for (int k = 0; k < kAAPartials; ++k) t[k] = 0.0;
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-    for (int k = 0; k < kAAPartials; ++k) t[k] += partials[(long long)kAAPartials * b + k];
-  for (int k = 0; k < kAAPartials; ++k) sh[k][threadIdx.x] = t[k];
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int k = 0; k < kAAPartials; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x != 0) return;
-  double dots[kAAPartials];
-  for (int k = 0; k < kAAPartials; ++k) dots[k] = sh[k][0];
-  aa_coefficients(sc, m, dots);
+  // one thread: the Gram matrix update and the mixing coefficients (shared with the oracle's
+  // restatement)
+  if (reduce_all(acc, a.red)) aa_coefficients(a.sc, a.m, acc);
 }
 
 struct UpdArgs {
   Dims d;
-  int diva, sliding_none, basal_freezing, nblk_x;
+  int diva, sliding_none, basal_freezing;
   double vmax, rel, dT_freeze;
   const double *xu, *xv;           // linear solution
   double *u, *v, *up, *vp;         // velocities (relaxed in place) and the previous iterate
   // Anderson mixing (aa_m > 0): the iterate is g - sum gamma_i dG_i instead of the relaxation
   int aa_m;
-  const double* sc;
+  double* sc;
   const double *gu, *gv;
   const double *dGu[kAAMax], *dGv[kAAMax];
   const double *uchk, *vchk;       // fields tested by estimate_visc_iter_UV_errors
   double *errx, *erry;             // DIVA_err candidates
+  double *fex, *fey;               // DIVA_err: the previous iteration's candidate, if `commit`
+  int commit;
   const double *bex, *bey, *F2, *Hi, *Ti, *Tpmp;
   double *taubx, *tauby, *ubx, *vby;
-  double* partials;                // 3 per block
+  Reduction red;                   // 3 sums
+  IterEnd end;
 };
+
+// The loop's totals and whether it goes on (thread 0 of one block).
+__device__ __forceinline__ void loop_end(double* sc, const IterEnd& e) {
+  sc[SC_SUM_LIN] += sc[SC_LIN_IT];
+  sc[SC_SUM_FULL] += sc[SC_LIN_FULL];
+  sc[SC_N_SOLVED] += sc[SC_SOLVED];
+  const bool stop = sc[SC_CONVERGED] != 0.0 || sc[SC_EXIT_RELRES] != 0.0 || sc[SC_NAN] != 0.0 ||
+                    sc[SC_PIC_IT] > (double)e.nit;
+  cudaGraphSetConditional(e.a, stop ? 0u : 1u);
+  if (e.has_b) cudaGraphSetConditional(e.b, stop ? 0u : 1u);
+}
 
 __global__ void __launch_bounds__(256) k_picard_update(UpdArgs a) {
   const Dims d = a.d;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
   double sums[3] = {0.0, 0.0, 0.0};
-  if (j < d.ny && i < d.nx) {
+  const bool commit = a.commit < 0 ? a.sc[SC_PIC_IT] > 1.0 : a.commit != 0;
+  FOR_TILES(d) {
     const int nx = d.nx, ny = d.ny;
     const long long q = d.at(j, i);
     bool frozen = false;
@@ -602,6 +590,7 @@ __global__ void __launch_bounds__(256) k_picard_update(UpdArgs a) {
         sums[1] += (un + uo) * (un + uo);
       }
       const double chk = a.diva ? un : a.uchk[q];
+      if (commit) a.fex[q] = a.errx[q];
       a.errx[q] = (fabs(chk) > kVelTol) ? 2.0 * fabs(un - uo) / fabs(un + uo + 1E-5) : 0.0;
       if (a.diva) {
         const double tb = a.bex[q] * un;
@@ -634,6 +623,7 @@ __global__ void __launch_bounds__(256) k_picard_update(UpdArgs a) {
         sums[1] += (vn + vo) * (vn + vo);
       }
       const double chk = a.diva ? vn : a.vchk[q];
+      if (commit) a.fey[q] = a.erry[q];
       a.erry[q] = (fabs(chk) > kVelTol) ? 2.0 * fabs(vn - vo) / fabs(vn + vo + 1E-5) : 0.0;
       if (a.diva) {
         const double tb = a.bey[q] * vn;
@@ -647,41 +637,26 @@ __global__ void __launch_bounds__(256) k_picard_update(UpdArgs a) {
       }
     }
   }
-  block_sum<3>(sums);
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    const int b = blockIdx.y * a.nblk_x + blockIdx.x;
-    a.partials[3 * b + 0] = sums[0];
-    a.partials[3 * b + 1] = sums[1];
-    a.partials[3 * b + 2] = sums[2];
-  }
+  if (!reduce_all(sums, a.red)) return;
+  double* sc = a.sc;
+  sc[SC_RES1] = sums[0];
+  sc[SC_RES2] = sums[1];
+  sc[SC_RES1 + 2] = sums[2];
+  if (!a.end.graph) return;
+  // the step norm (calc_visc_iter_UV_resid :1588-1596) and the stop test (:346-351)
+  if (sc[SC_RNORM2] > sc[SC_TARGET2]) sc[SC_LIN_FAILED] += 1.0;
+  if (!isfinite(sums[0]) || !isfinite(sums[1])) sc[SC_NAN] = 1.0;
+  const double resid = (sums[2] > 0.0) ? 2.0 * sqrt(sums[0]) / max_ref(sqrt(sums[1]), 1E-8) : 0.0;
+  sc[SC_RESID] = resid;
+  sc[SC_CONVERGED] = ((a.end.loop && resid < a.end.tol) || sc[SC_PIC_IT] >= (double)a.end.nit) ? 1.0 : 0.0;
+  if (a.end.loop) loop_end(sc, a.end);
 }
 
-// fixed-order sum of block partials (deterministic)
-__global__ void k_sum_partials(const double* partials, int nblocks, int width, double* out) {
-  __shared__ double sh[256];
-  for (int w = 0; w < width; ++w) {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) s += partials[(long long)width * b + w];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-      if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[w] = sh[0];
-    __syncthreads();
-  }
-}
-
-// calc_basal_stress + calc_basal_velocities at the current velocities (used when
-// the viscosity iteration stops on the nonlinear residual before a linear solve)
-__global__ void k_basal_stress_velocities(Dims d, int sliding_none, int basal_freezing, double dT, const double* u,
-                                          const double* v, const double* bex, const double* bey, const double* F2,
-                                          const double* Hi, const double* Ti, const double* Tpmp, double* tbx,
-                                          double* tby, double* ubx, double* vby, const double* pred) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (j >= d.ny || i >= d.nx) return;
-  if (pred && *pred == 0.0) return;   // graph launch: only when the iteration stopped on the nonlinear residual
+// basal stress and velocity of the faces of point (j,i)
+__device__ __forceinline__ void basal_point(const Dims& d, int sliding_none, int basal_freezing, double dT,
+                                            const double* u, const double* v, const double* bex, const double* bey,
+                                            const double* F2, const double* Hi, const double* Ti, const double* Tpmp,
+                                            double* tbx, double* tby, double* ubx, double* vby, int j, int i) {
   const long long q = d.at(j, i);
   bool frozen = false;
   if (basal_freezing) {
@@ -700,6 +675,37 @@ __global__ void k_basal_stress_velocities(Dims d, int sliding_none, int basal_fr
     const double F2s = stag_margin(F2[q], F2[d.at(j + 1, i)], Hi[q], Hi[d.at(j + 1, i)]);
     vby[q] = sliding_none ? 0.0 : (frozen ? 0.0 : v[q] - tb * F2s);
   }
+}
+
+// calc_basal_stress + calc_basal_velocities at the current velocities (used when
+// the viscosity iteration stops on the nonlinear residual before a linear solve)
+__global__ void k_basal_stress_velocities(Dims d, int sliding_none, int basal_freezing, double dT, const double* u,
+                                          const double* v, const double* bex, const double* bey, const double* F2,
+                                          const double* Hi, const double* Ti, const double* Tpmp, double* tbx,
+                                          double* tby, double* ubx, double* vby) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
+  if (j >= d.ny || i >= d.nx) return;
+  basal_point(d, sliding_none, basal_freezing, dT, u, v, bex, bey, F2, Hi, Ti, Tpmp, tbx, tby, ubx, vby, j, i);
+}
+// The post kernel of a graph-launched iteration under the rel-res stop rule: when the nonlinear
+// residual ended it before a linear solve, the last DIVA_err candidate becomes the field and
+// [DIVA] the basal stress and velocities are formed at the current velocities; the loop's
+// handles are set either way.
+__global__ void k_relres_end(Dims d, int diva, int sliding_none, int basal_freezing, double dT, const double* u,
+                             const double* v, const double* bex, const double* bey, const double* F2,
+                             const double* Hi, const double* Ti, const double* Tpmp, double* tbx, double* tby,
+                             double* ubx, double* vby, const double* cx, const double* cy, double* fx, double* fy,
+                             double* sc, IterEnd end) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
+  const bool stopped = sc[SC_EXIT_RELRES] != 0.0;
+  if (j == 0 && i == 0) loop_end(sc, end);   // (writes nothing that the other threads read)
+  if (j >= d.ny || i >= d.nx || !stopped) return;
+  const long long q = d.at(j, i);
+  if (sc[SC_PIC_IT] > 1.0) {
+    fx[q] = cx[q];
+    fy[q] = cy[q];
+  }
+  if (diva) basal_point(d, sliding_none, basal_freezing, dT, u, v, bex, bey, F2, Hi, Ti, Tpmp, tbx, tby, ubx, vby, j, i);
 }
 
 // visc_eff_3D_b of the last viscosity iteration (:820-858), written once per solve
@@ -1047,7 +1053,7 @@ static void fill_coef_args(Ctx* c, CoefArgs& a, const double* u, const double* v
   a.taub_seen_cy = c->taub_seen[1];
 }
 
-int launch_diva_coefficients(Ctx* c, const double* u, const double* v, bool diva, int what) {
+int launch_diva_coefficients(Ctx* c, const double* u, const double* v, bool diva, int what, bool begin) {
   const diva_config_t& C = c->c;
   // Picard double buffering of visc_eff_3D_a: read the previous, write the new
   std::swap(c->f[DIVA_F_VISC_EFF_3D_A], *reinterpret_cast<void**>(&c->visc_prev));
@@ -1060,6 +1066,7 @@ int launch_diva_coefficients(Ctx* c, const double* u, const double* v, bool diva
                                  cudaMemcpyDeviceToDevice, c->stream));
   }
   a.keep_seen = what != K1_WRITE_SHEAR;
+  a.sc = begin ? c->scal : nullptr;
   k_column_prep<<<G2>>>(a); c->launches++;
   {
     const dim3 block(kColLanes, kColRows);
@@ -1104,15 +1111,14 @@ int launch_diva_coefficients(Ctx* c, const double* u, const double* v, bool diva
   return DIVA_OK;
 }
 
-int launch_picard_update(Ctx* c, double* u, double* v, const double* xu, const double* xv, bool diva) {
+int launch_picard_update(Ctx* c, double* u, double* v, const double* xu, const double* xv, bool diva, int commit,
+                         const IterEnd* end) {
   const diva_config_t& C = c->c;
   UpdArgs a{};
   a.d = c->d;
   a.diva = diva;
   a.sliding_none = C.choice_sliding_law == DIVA_SLIDING_NONE;
   a.basal_freezing = C.include_basal_freezing;
-  dim3 g = grid2d(c->d.ny, c->d.nx);
-  a.nblk_x = g.x;
   a.vmax = C.DIVA_vel_max;
   a.rel = C.DIVA_visc_it_relax;
   a.dT_freeze = C.deltaT_basal_freezing;
@@ -1120,19 +1126,20 @@ int launch_picard_update(Ctx* c, double* u, double* v, const double* xu, const d
   a.up = c->D(DIVA_F_U_CX_PREV); a.vp = c->D(DIVA_F_V_CY_PREV);
   a.uchk = c->D(DIVA_F_U_VAV_CX); a.vchk = c->D(DIVA_F_V_VAV_CY);
   a.errx = c->err_cand[0]; a.erry = c->err_cand[1];
+  a.fex = c->D(DIVA_F_DIVA_ERR_CX); a.fey = c->D(DIVA_F_DIVA_ERR_CY);
+  a.commit = commit;
   a.bex = c->D(DIVA_F_BETA_EFF_CX); a.bey = c->D(DIVA_F_BETA_EFF_CY); a.F2 = c->D(DIVA_F_F2_A);
   a.Hi = c->D(DIVA_F_HI_A); a.Ti = c->D(DIVA_F_TI_A); a.Tpmp = c->D(DIVA_F_TI_PMP_A);
   a.taubx = c->D(DIVA_F_TAUB_CX); a.tauby = c->D(DIVA_F_TAUB_CY);
   a.ubx = c->D(DIVA_F_U_BASE_CX); a.vby = c->D(DIVA_F_V_BASE_CY);
-  a.partials = c->partials;
+  a.red = Reduction{c->partials, c->red_count};
+  if (end) a.end = *end;
   a.aa_m = C.picard_anderson_m;
   a.sc = c->scal;
   a.gu = c->aa_g[0]; a.gv = c->aa_g[1];
   for (int k = 0; k < kAAMax; ++k) { a.dGu[k] = c->aa_dG[k][0]; a.dGv[k] = c->aa_dG[k][1]; }
-  k_picard_update<<<g, block2d(), 0, c->stream>>>(a); c->launches++;
+  k_picard_update<<<red_blocks(c->d), block2d(), 0, c->stream>>>(a); c->launches++;
   DIVA_LAUNCHED(c, "k_picard_update");
-  k_sum_partials<<<1, 256, 0, c->stream>>>(c->partials, (int)(g.x * g.y), 3, c->scal + SC_RES1); c->launches++;
-  DIVA_LAUNCHED(c, "k_sum_partials");
   return DIVA_OK;
 }
 
@@ -1141,8 +1148,6 @@ int launch_anderson_prepare(Ctx* c, const double* u, const double* v, const doub
   AAArgs a{};
   a.d = c->d;
   a.m = C.picard_anderson_m;
-  const dim3 g = grid2d(c->d.ny, c->d.nx);
-  a.nblk_x = g.x;
   a.vmax = C.DIVA_vel_max;
   a.u = u; a.v = v; a.xu = xu; a.xv = xv;
   for (int k = 0; k < kAAMax; ++k) {
@@ -1151,11 +1156,9 @@ int launch_anderson_prepare(Ctx* c, const double* u, const double* v, const doub
   }
   a.fu = c->aa_f[0]; a.fv = c->aa_f[1]; a.gu = c->aa_g[0]; a.gv = c->aa_g[1];
   a.sc = c->scal;
-  a.partials = c->partials;
-  k_aa_prepare<<<g, block2d(), 0, c->stream>>>(a); c->launches++;
+  a.red = Reduction{c->partials, c->red_count};
+  k_aa_prepare<<<red_blocks(c->d), block2d(), 0, c->stream>>>(a); c->launches++;
   DIVA_LAUNCHED(c, "k_aa_prepare");
-  k_aa_solve<<<1, 256, 0, c->stream>>>(c->partials, (int)(g.x * g.y), a.m, c->scal); c->launches++;
-  DIVA_LAUNCHED(c, "k_aa_solve");
   return DIVA_OK;
 }
 
@@ -1171,8 +1174,9 @@ int anderson_reset(Ctx* c) {
 }
 
 int launch_commit_err(Ctx* c) {
-  std::swap(c->f[DIVA_F_DIVA_ERR_CX], *reinterpret_cast<void**>(&c->err_cand[0]));
-  std::swap(c->f[DIVA_F_DIVA_ERR_CY], *reinterpret_cast<void**>(&c->err_cand[1]));
+  const size_t nb = sizeof(double) * c->d.plane;
+  DIVA_CUDA(c, cudaMemcpyAsync(c->D(DIVA_F_DIVA_ERR_CX), c->err_cand[0], nb, cudaMemcpyDeviceToDevice, c->stream));
+  DIVA_CUDA(c, cudaMemcpyAsync(c->D(DIVA_F_DIVA_ERR_CY), c->err_cand[1], nb, cudaMemcpyDeviceToDevice, c->stream));
   return DIVA_OK;
 }
 
@@ -1183,56 +1187,20 @@ int launch_basal_stress_velocities(Ctx* c) {
                                     c->D(DIVA_F_BETA_EFF_CX), c->D(DIVA_F_BETA_EFF_CY), c->D(DIVA_F_F2_A),
                                     c->D(DIVA_F_HI_A), c->D(DIVA_F_TI_A), c->D(DIVA_F_TI_PMP_A),
                                     c->D(DIVA_F_TAUB_CX), c->D(DIVA_F_TAUB_CY), c->D(DIVA_F_U_BASE_CX),
-                                    c->D(DIVA_F_V_BASE_CY), nullptr); c->launches++;
+                                    c->D(DIVA_F_V_BASE_CY)); c->launches++;
   DIVA_LAUNCHED(c, "k_basal_stress_velocities");
   return DIVA_OK;
 }
 
-int launch_basal_pred(Ctx* c) {
+int launch_relres_end(Ctx* c, bool diva, const IterEnd& end) {
   const diva_config_t& C = c->c;
-  k_basal_stress_velocities<<<G2>>>(c->d, C.choice_sliding_law == DIVA_SLIDING_NONE, C.include_basal_freezing,
-                                    C.deltaT_basal_freezing, c->D(DIVA_F_U_VAV_CX), c->D(DIVA_F_V_VAV_CY),
-                                    c->D(DIVA_F_BETA_EFF_CX), c->D(DIVA_F_BETA_EFF_CY), c->D(DIVA_F_F2_A),
-                                    c->D(DIVA_F_HI_A), c->D(DIVA_F_TI_A), c->D(DIVA_F_TI_PMP_A),
-                                    c->D(DIVA_F_TAUB_CX), c->D(DIVA_F_TAUB_CY), c->D(DIVA_F_U_BASE_CX),
-                                    c->D(DIVA_F_V_BASE_CY), c->scal + SC_EXIT_RELRES); c->launches++;
-  DIVA_LAUNCHED(c, "k_basal_stress_velocities");
-  return DIVA_OK;
-}
-
-// end of a graph-launched viscosity iteration: the step norm from the summed
-// partials (calc_visc_iter_UV_resid :1588-1596) and the stop test (:346-351)
-__global__ void k_ctl_end(double* sc, int relmode, double tol, int nit) {
-  const double r1 = sc[SC_RES1], r2 = sc[SC_RES2], cnt = sc[SC_RES1 + 2];
-  if (!isfinite(r1) || !isfinite(r2)) sc[SC_NAN] = 1.0;
-  const double resid = (cnt > 0.0) ? 2.0 * sqrt(r1) / max_ref(sqrt(r2), 1E-8) : 0.0;
-  sc[SC_RESID] = resid;
-  bool conv = false;
-  if (!relmode && resid < tol) conv = true;
-  else if (sc[SC_PIC_IT] >= (double)nit) conv = true;
-  sc[SC_CONVERGED] = conv ? 1.0 : 0.0;
-}
-
-// DIVA_err of this iteration becomes the field unless the iteration converged (:353-355)
-__global__ void k_err_commit(Dims d, const double* sc, const double* cx, const double* cy, double* fx, double* fy) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (j >= d.ny || i >= d.nx) return;
-  if (sc[SC_CONVERGED] != 0.0) return;
-  const long long q = d.at(j, i);
-  fx[q] = cx[q];
-  fy[q] = cy[q];
-}
-
-int launch_ctl_end(Ctx* c, bool relmode) {
-  k_ctl_end<<<1, 1, 0, c->stream>>>(c->scal, relmode, c->c.DIVA_visc_it_norm_dUV_tol, c->c.DIVA_visc_it_nit); c->launches++;
-  DIVA_LAUNCHED(c, "k_ctl_end");
-  return DIVA_OK;
-}
-
-int launch_err_commit_pred(Ctx* c) {
-  k_err_commit<<<G2>>>(c->d, c->scal, c->err_cand[0], c->err_cand[1], c->D(DIVA_F_DIVA_ERR_CX),
-                       c->D(DIVA_F_DIVA_ERR_CY)); c->launches++;
-  DIVA_LAUNCHED(c, "k_err_commit");
+  k_relres_end<<<G2>>>(c->d, diva, C.choice_sliding_law == DIVA_SLIDING_NONE, C.include_basal_freezing,
+                       C.deltaT_basal_freezing, c->D(DIVA_F_U_VAV_CX), c->D(DIVA_F_V_VAV_CY),
+                       c->D(DIVA_F_BETA_EFF_CX), c->D(DIVA_F_BETA_EFF_CY), c->D(DIVA_F_F2_A), c->D(DIVA_F_HI_A),
+                       c->D(DIVA_F_TI_A), c->D(DIVA_F_TI_PMP_A), c->D(DIVA_F_TAUB_CX), c->D(DIVA_F_TAUB_CY),
+                       c->D(DIVA_F_U_BASE_CX), c->D(DIVA_F_V_BASE_CY), c->err_cand[0], c->err_cand[1],
+                       c->D(DIVA_F_DIVA_ERR_CX), c->D(DIVA_F_DIVA_ERR_CY), c->scal, end); c->launches++;
+  DIVA_LAUNCHED(c, "k_relres_end");
   return DIVA_OK;
 }
 

@@ -1534,97 +1534,168 @@ __global__ void __launch_bounds__(kInvThreads) k_small_setup(SmallSetup a) {
 }
 
 // ---- Krylov kernels (fine level) --------------------------------------------------
-constexpr int kPW = 4;   // partial sums per block
+// Every kernel with an inner product walks the points in 32 x 8 tiles with at most
+// kRedBlocks blocks and finishes its reductions and the scalar step that follows itself
+// (reduce_all): a reduction kernel and a one-thread control kernel of their own cost two
+// launches of a few microseconds each, several times per Krylov half step (561 x 321: one
+// viscosity iteration of 41 launches in 383 us).
 
-__device__ __forceinline__ void store_partials(double (&v)[kPW], double* partials, int nbx) {
-  block_sum<kPW>(v);
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    const int b = blockIdx.y * nbx + blockIdx.x;
-#pragma unroll
-    for (int q = 0; q < kPW; ++q) partials[kPW * b + q] = v[q];
-  }
+constexpr int kPW = 3;   // inner products per kernel
+
+// whether every value the u and v rows at (j,i) read is interior, so stored reads suffice
+__device__ __forceinline__ bool rows_deep(const Dims& d, int j, int i) {
+  return i >= 2 && i <= d.nx - 4 && j >= 2 && j <= d.ny - 4;
+}
+// (A x) of the interior u (v) row at (j,i): stored reads inside, the boundary mapping only
+// next to it (the mapping's index selection for nine reads made the operator's kernels
+// instruction-bound: k_matvec took 82 us on 1501 x 1501 for 22 us worth of bytes)
+__device__ __forceinline__ double Au_any(const Op& o, const double* xu, const double* xv, int j, int i, bool deep) {
+  return deep ? Au<true>(o, xu, xv, j, i) : Au(o, xu, xv, j, i);
+}
+__device__ __forceinline__ double Av_any(const Op& o, const double* xu, const double* xv, int j, int i, bool deep) {
+  return deep ? Av<true>(o, xu, xv, j, i) : Av(o, xu, xv, j, i);
 }
 
-// out = A x ; partial dots: [0] = w1.out, [1] = w2.out, [2] = out.out
-__global__ void k_matvec(Op o, const double* xu, const double* xv, double* ou, double* ov, const double* w1u,
-                         const double* w1v, const double* w2u, const double* w2v, double* partials, int nbx) {
-  IDX2D
-  double acc[kPW] = {0.0, 0.0, 0.0, 0.0};
-  if (j < o.d.ny && i < o.d.nx) {
+// out = A x ; dots [0] w.out, [1] out.out ; then the scalar step
+enum { ST_NONE = 0, ST_ALPHA, ST_OMEGA };
+__global__ void __launch_bounds__(256) k_matvec(Op o, const double* xu, const double* xv, double* ou, double* ov,
+                                                const double* wu, const double* wv, Reduction red, double* sc,
+                                                int stage) {
+  double acc[kPW] = {};
+  FOR_TILES(o.d) {
     const long long q = o.d.at(j, i);
+    const bool deep = rows_deep(o.d, j, i);
+    double a = 0.0, b = 0.0;
     if (u_int(o.d, j, i)) {
-      const double a = Au(o, xu, xv, j, i);
-      ou[q] = a;
-      if (w1u) acc[0] += w1u[q] * a;
-      if (w2u) acc[1] += w2u[q] * a;
-      acc[2] += a * a;
-    } else {
-      ou[q] = 0.0;
+      a = Au_any(o, xu, xv, j, i, deep);
+      acc[0] += wu[q] * a;
+      acc[1] += a * a;
     }
     if (v_int(o.d, j, i)) {
-      const double a = Av(o, xu, xv, j, i);
-      ov[q] = a;
-      if (w1v) acc[0] += w1v[q] * a;
-      if (w2v) acc[1] += w2v[q] * a;
-      acc[2] += a * a;
-    } else {
-      ov[q] = 0.0;
+      b = Av_any(o, xu, xv, j, i, deep);
+      acc[0] += wv[q] * b;
+      acc[1] += b * b;
     }
+    ou[q] = a;
+    ov[q] = b;
   }
-  store_partials(acc, partials, nbx);
+  if (!reduce_all(acc, red)) return;
+  if (stage == ST_ALPHA) sc[SC_ALPHA] = acc[0] != 0.0 ? sc[SC_RHO] / acc[0] : 0.0;
+  if (stage == ST_OMEGA) sc[SC_OMEGA] = acc[1] != 0.0 ? acc[0] / acc[1] : 0.0;
 }
 
-// r = b - A x; rhat = r; partials: [0] r.r, [1] b.b
-__global__ void k_init_residual(Op o, const double* xu, const double* xv, const double* bu, const double* bv,
-                                double* ru, double* rv, double* hu, double* hv, double* pu, double* pv,
-                                double* partials, int nbx) {
-  IDX2D
-  double acc[kPW] = {0.0, 0.0, 0.0, 0.0};
-  if (j < o.d.ny && i < o.d.nx) {
+// The start of a viscosity iteration's linear solve: x <- (u, v), r = rhat = p = b - A x on
+// the interior, and (raw) the nonlinear residual over all rows of the reference matrix, whose
+// interior rows read stored values and whose boundary rows are u_src - u_b (or -u_b for zero).
+// Dots: [0] raw r.r, [1] b.b, [2] r.r.
+struct RelresTest {   // the stop test of a graph-launched iteration (h: IF(solve)), on = 0: none
+  int on, stall_its;
+  double tol;
+  cudaGraphConditionalHandle h;
+};
+__global__ void __launch_bounds__(256) k_init_residual(Op o, const double* u, const double* v, const double* bu,
+                                                       const double* bv, double* xu, double* xv, double* ru,
+                                                       double* rv, double* hu, double* hv, double* pu, double* pv,
+                                                       int raw, Reduction red, double* sc, RelresTest test) {
+  double acc[kPW] = {};
+  FOR_TILES(o.d) {
     const long long q = o.d.at(j, i);
-    double r = 0.0;
+    const bool deep = rows_deep(o.d, j, i);
+    xu[q] = u[q];
+    xv[q] = v[q];
+    double r = 0.0, w = 0.0;
     if (u_int(o.d, j, i)) {
-      r = bu[q] - Au(o, xu, xv, j, i);
-      acc[0] += r * r;
-      acc[1] += bu[q] * bu[q];
+      const double b = bu[q];
+      r = b - Au_any(o, u, v, j, i, deep);
+      w = (deep || !raw) ? r : b - Au<true>(o, u, v, j, i);
+      acc[1] += b * b;
+    } else if (raw && i < o.d.nx - 1) {
+      w = LU(o, u, j, i) - u[q];
     }
+    acc[0] += w * w;
+    acc[2] += r * r;
     ru[q] = r; hu[q] = r; pu[q] = r;
-    r = 0.0;
+    r = w = 0.0;
     if (v_int(o.d, j, i)) {
-      r = bv[q] - Av(o, xu, xv, j, i);
-      acc[0] += r * r;
-      acc[1] += bv[q] * bv[q];
+      const double b = bv[q];
+      r = b - Av_any(o, u, v, j, i, deep);
+      w = (deep || !raw) ? r : b - Av<true>(o, u, v, j, i);
+      acc[1] += b * b;
+    } else if (raw && j < o.d.ny - 1) {
+      w = LV(o, v, j, i) - v[q];
     }
+    acc[0] += w * w;
+    acc[2] += r * r;
     rv[q] = r; hv[q] = r; pv[q] = r;
   }
-  store_partials(acc, partials, nbx);
-}
-
-// s = r - alpha v ; partial [0] s.s
-__global__ void k_update_s(Dims d, const double* sc, const double* ru, const double* rv, const double* vu,
-                           const double* vv, double* su, double* sv, double* partials, int nbx) {
-  IDX2D
-  double acc[kPW] = {0.0, 0.0, 0.0, 0.0};
-  if (j < d.ny && i < d.nx) {
-    const long long q = d.at(j, i);
-    const double alpha = sc[SC_ALPHA];
-    const double a = ru[q] - alpha * vu[q], b = rv[q] - alpha * vv[q];
-    su[q] = a; sv[q] = b;
-    acc[0] = a * a + b * b;
+  if (!reduce_all(acc, red)) return;
+  const double rr = acc[0], bb = acc[1];
+  sc[SC_RR] = rr;
+  sc[SC_BNORM2] = bb;
+  sc[SC_RNORM2] = acc[2];
+  sc[SC_RHO] = acc[2];
+  if (!test.on) return;
+  // nonlinear residual of the current iterate; skip the solve when it meets the tolerance
+  const double relres = bb > 0.0 ? sqrt(rr / bb) : sqrt(rr);
+  sc[SC_RELRES] = relres;
+  sc[SC_ETA] = eta_after(sc[SC_ETA], relres, sc[SC_RELRES_PREV], test.tol);
+  sc[SC_RELRES_PREV] = relres;
+  bool stop = false;
+  if (!isfinite(relres)) { sc[SC_NAN] = 1.0; stop = true; }
+  else if (relres <= test.tol) { sc[SC_EXIT_RELRES] = 1.0; stop = true; }
+  else if (stall_after(relres, sc + SC_STALL_BEST, sc + SC_STALL_SINCE, test.stall_its)) {
+    sc[SC_EXIT_RELRES] = 1.0;   // ends like a converged one (basal stress at this state), flagged
+    sc[SC_STALLED] = 1.0;
+    stop = true;
   }
-  store_partials(acc, partials, nbx);
+  cudaGraphSetConditional(test.h, stop ? 0u : 1u);
 }
 
-// x += alpha phat + omega shat ; r = s - omega t ; partials [0] rhat.r, [1] r.r
-__global__ void k_update_xr(Dims d, const double* sc, double* xu, double* xv, const double* phu, const double* phv,
-                            const double* shu, const double* shv, const double* su, const double* sv,
-                            const double* tu, const double* tv, double* ru, double* rv, const double* hu,
-                            const double* hv, double* partials, int nbx) {
-  IDX2D
-  double acc[kPW] = {0.0, 0.0, 0.0, 0.0};
-  if (j < d.ny && i < d.nx) {
+// Handles a kernel sets when it runs inside a graph-launched loop (on = 0: host-driven).
+struct LoopHandles {
+  int on;
+  cudaGraphConditionalHandle a, b;
+};
+
+// s = r - alpha v ; dot [0] s.s ; then the half-step test: stop there if |s| meets the target
+__global__ void __launch_bounds__(256) k_update_s(Dims d, double* sc, const double* ru, const double* rv,
+                                                  const double* vu, const double* vv, double* su, double* sv,
+                                                  Reduction red, LoopHandles h) {   // h.a: WHILE(krylov), h.b: IF(second)
+  double acc[kPW] = {};
+  const double alpha = sc[SC_ALPHA];
+  FOR_TILES(d) {
     const long long q = d.at(j, i);
-    const double alpha = sc[SC_ALPHA], omega = sc[SC_OMEGA];
+    const double a = ru[q] - alpha * vu[q], b = rv[q] - alpha * vv[q];
+    su[q] = a;
+    sv[q] = b;
+    acc[0] += a * a;
+    acc[0] += b * b;
+  }
+  if (!reduce_all(acc, red)) return;
+  const double ss = acc[0];
+  sc[SC_SNORM2] = ss;
+  if (!h.on) return;
+  sc[SC_LIN_IT] += 1.0;
+  const bool fin = isfinite(ss), done = fin && ss <= sc[SC_TARGET2];
+  if (!fin) sc[SC_NAN] = 1.0;
+  sc[SC_HALFDONE] = done ? 1.0 : 0.0;
+  if (done) sc[SC_RNORM2] = ss;
+  const bool go = fin && !done;
+  cudaGraphSetConditional(h.b, go ? 1u : 0u);
+  if (!go) cudaGraphSetConditional(h.a, 0u);
+}
+
+// x += alpha phat + omega shat ; r = s - omega t ; dots [0] rhat.r, [1] r.r ; then rho, beta
+// and the continue test
+__global__ void __launch_bounds__(256) k_update_xr(Dims d, double* sc, double* xu, double* xv, const double* phu,
+                                                   const double* phv, const double* shu, const double* shv,
+                                                   const double* su, const double* sv, const double* tu,
+                                                   const double* tv, double* ru, double* rv, const double* hu,
+                                                   const double* hv, Reduction red, int maxit, LoopHandles h) {
+  double acc[kPW] = {};
+  const double alpha = sc[SC_ALPHA], omega = sc[SC_OMEGA];
+  FOR_TILES(d) {
+    const long long q = d.at(j, i);
     if (u_int(d, j, i)) {
       xu[q] += alpha * phu[q] + omega * shu[q];
       const double r = su[q] - omega * tu[q];
@@ -1640,18 +1711,16 @@ __global__ void k_update_xr(Dims d, const double* sc, double* xu, double* xv, co
       acc[1] += r * r;
     }
   }
-  store_partials(acc, partials, nbx);
-}
-
-// x += alpha phat (early exit on small s)
-__global__ void k_update_x_half(Dims d, const double* sc, double* xu, double* xv, const double* phu,
-                                const double* phv) {
-  IDX2D
-  if (j >= d.ny || i >= d.nx) return;
-  const long long q = d.at(j, i);
-  const double alpha = sc[SC_ALPHA];
-  if (u_int(d, j, i)) xu[q] += alpha * phu[q];
-  if (v_int(d, j, i)) xv[q] += alpha * phv[q];
+  if (!reduce_all(acc, red)) return;
+  const double rho_new = acc[0], rr = acc[1], rho = sc[SC_RHO];
+  sc[SC_BETA] = (rho != 0.0 && omega != 0.0) ? (rho_new / rho) * (alpha / omega) : 0.0;
+  sc[SC_RHO] = rho_new;
+  sc[SC_RNORM2] = rr;
+  if (!h.on) return;
+  sc[SC_LIN_FULL] += 1.0;
+  const bool fin = isfinite(rr);
+  if (!fin) sc[SC_NAN] = 1.0;
+  cudaGraphSetConditional(h.a, (fin && rr > sc[SC_TARGET2] && sc[SC_LIN_IT] < (double)maxit) ? 1u : 0u);
 }
 
 // p = r + beta (p - omega v)
@@ -1665,201 +1734,43 @@ __global__ void k_update_p(Dims d, const double* sc, const double* ru, const dou
   pv[q] = rv[q] + beta * (pv[q] - omega * vv[q]);
 }
 
-// fixed-order reduction of block partials into sc[dst..dst+3], then the scalar step
-enum { ST_INIT = 0, ST_ALPHA, ST_SNORM, ST_OMEGA, ST_RHO };
-__global__ void k_reduce(const double* partials, int nblocks, double* sc, int stage) {
-  __shared__ double sh[kPW][256];
-  double s[kPW] = {0.0, 0.0, 0.0, 0.0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-    for (int q = 0; q < kPW; ++q) s[q] += partials[kPW * b + q];
-  for (int q = 0; q < kPW; ++q) sh[q][threadIdx.x] = s[q];
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int q = 0; q < kPW; ++q) sh[q][threadIdx.x] += sh[q][threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x != 0) return;
-  const double r0 = sh[0][0], r1 = sh[1][0];
-  switch (stage) {
-    case ST_INIT:   // [0] r.r, [1] b.b
-      sc[SC_RNORM2] = r0; sc[SC_BNORM2] = r1; sc[SC_RHO] = r0; break;
-    case ST_ALPHA:  // [0] rhat.v
-      sc[SC_TMP0] = r0;
-      sc[SC_ALPHA] = (r0 != 0.0) ? sc[SC_RHO] / r0 : 0.0; break;
-    case ST_SNORM:  // [0] s.s
-      sc[SC_SNORM2] = r0; break;
-    case ST_OMEGA:  // [0] s.t, [2] t.t  (k_matvec with w1 = s)
-      sc[SC_OMEGA] = (sh[2][0] != 0.0) ? r0 / sh[2][0] : 0.0; break;
-    case ST_RHO: {  // [0] rhat.r, [1] r.r
-      const double rho_new = r0;
-      const double om = sc[SC_OMEGA], al = sc[SC_ALPHA], rho = sc[SC_RHO];
-      sc[SC_BETA] = (rho != 0.0 && om != 0.0) ? (rho_new / rho) * (al / om) : 0.0;
-      sc[SC_RHO] = rho_new;
-      sc[SC_RNORM2] = r1;
-      break;
-    }
-  }
-}
-
-// boundary unknowns = their sources (after a solve)
-__global__ void k_fill_boundary(Dims d, BCs bc, double* xu, double* xv) {
+// The solution of a linear solve: x, plus alpha phat when it ended at a half step (half 1; 0:
+// not; -1: as the device scalar says), boundary unknowns from their sources.
+__global__ void k_finish_x(Dims d, BCs bc, const double* sc, int half, const double* xu, const double* xv,
+                           const double* phu, const double* phv, double* fu, double* fv) {
   IDX2D
   if (j >= d.ny || i >= d.nx) return;
-  Op o;
-  o.d = d; o.bc = bc;
+  const bool add = half < 0 ? sc[SC_HALFDONE] != 0.0 : half != 0;
+  const double alpha = sc[SC_ALPHA];
   const long long q = d.at(j, i);
-  if (i < d.nx - 1 && !u_int(d, j, i)) xu[q] = LU(o, xu, j, i);
-  if (j < d.ny - 1 && !v_int(d, j, i)) xv[q] = LV(o, xv, j, i);
-}
-
-// nonlinear residual over all rows of the reference matrix: interior rows
-// b - A u, boundary rows -(u_b - u_src) (or -u_b for zero); partials [0] r.r, [1] b.b
-__global__ void k_relres(Op o, const double* u, const double* v, const double* bu, const double* bv,
-                         double* partials, int nbx) {
-  IDX2D
-  double acc[kPW] = {0.0, 0.0, 0.0, 0.0};
-  if (j < o.d.ny && i < o.d.nx) {
-    const long long q = o.d.at(j, i);
-    if (i < o.d.nx - 1) {
-      double r;
-      if (u_int(o.d, j, i)) { r = bu[q] - Au<true>(o, u, v, j, i); acc[1] += bu[q] * bu[q]; }
-      else r = LU(o, u, j, i) - u[q];
-      acc[0] += r * r;
-    }
-    if (j < o.d.ny - 1) {
-      double r;
-      if (v_int(o.d, j, i)) { r = bv[q] - Av<true>(o, u, v, j, i); acc[1] += bv[q] * bv[q]; }
-      else r = LV(o, v, j, i) - v[q];
-      acc[0] += r * r;
-    }
+  int js, is;
+  double a = 0.0, b = 0.0;
+  if (i < d.nx - 1 && u_src(d, bc, j, i, js, is)) {
+    const long long p = d.at(js, is);
+    a = xu[p];
+    if (add) a += alpha * phu[p];
   }
-  store_partials(acc, partials, nbx);
-}
-
-// ---- device-side control of a graph-launched viscosity iteration ------------------
-// Single-thread kernels that finish a reduction and set the conditional-node
-// handles, so the Krylov loop and the skip of a converged iteration are
-// decided on the device without a host round trip.
-__device__ __forceinline__ void sum_partials4(const double* partials, int nblocks, double (&out)[kPW]) {
-  __shared__ double sh[kPW][256];
-  double s[kPW] = {0.0, 0.0, 0.0, 0.0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-    for (int q = 0; q < kPW; ++q) s[q] += partials[kPW * b + q];
-  for (int q = 0; q < kPW; ++q) sh[q][threadIdx.x] = s[q];
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int q = 0; q < kPW; ++q) sh[q][threadIdx.x] += sh[q][threadIdx.x + o];
-    __syncthreads();
+  if (j < d.ny - 1 && v_src(d, bc, j, i, js, is)) {
+    const long long p = d.at(js, is);
+    b = xv[p];
+    if (add) b += alpha * phv[p];
   }
-  for (int q = 0; q < kPW; ++q) out[q] = sh[q][0];
+  fu[q] = a;
+  fv[q] = b;
 }
 
-__global__ void k_ctl_begin(double* sc) {
-  sc[SC_PIC_IT] += 1.0;
-  sc[SC_EXIT_RELRES] = 0.0;
-  sc[SC_LIN_IT] = 0.0;
-  sc[SC_LIN_FULL] = 0.0;
-  sc[SC_SOLVED] = 0.0;
-  sc[SC_CONVERGED] = 0.0;
-}
-
-// nonlinear residual of the current iterate; skip the solve when it meets the tolerance
-__global__ void k_ctl_relres(const double* partials, int nblocks, double* sc, cudaGraphConditionalHandle h_solve,
-                             double tol, int stall_its) {
-  double v[kPW];
-  sum_partials4(partials, nblocks, v);
-  if (threadIdx.x != 0) return;
-  const double rr = v[0], bb = v[1];
-  const double relres = bb > 0.0 ? sqrt(rr / bb) : sqrt(rr);
-  sc[SC_RELRES] = relres;
-  sc[SC_ETA] = eta_after(sc[SC_ETA], relres, sc[SC_RELRES_PREV], tol);
-  sc[SC_RELRES_PREV] = relres;
-  bool stop = false;
-  if (!isfinite(relres)) { sc[SC_NAN] = 1.0; stop = true; }
-  else if (relres <= tol) { sc[SC_EXIT_RELRES] = 1.0; stop = true; }
-  else if (stall_after(relres, sc + SC_STALL_BEST, sc + SC_STALL_SINCE, stall_its)) {
-    sc[SC_EXIT_RELRES] = 1.0;   // ends like a converged one (basal stress at this state), flagged
-    sc[SC_STALLED] = 1.0;
-    stop = true;
-  }
-  cudaGraphSetConditional(h_solve, stop ? 0u : 1u);
-}
-
-// initial Krylov residual and the target of this linear solve
-__global__ void k_ctl_lin_init(const double* partials, int nblocks, double* sc, cudaGraphConditionalHandle h_while,
-                               int adaptive, double lin_rtol, int maxit) {
-  double v[kPW];
-  sum_partials4(partials, nblocks, v);
-  if (threadIdx.x != 0) return;
-  const double rr = v[0], bb = v[1];
-  sc[SC_RNORM2] = rr;
-  sc[SC_BNORM2] = bb;
-  sc[SC_RHO] = rr;
+// the target of this linear solve, and whether it needs any iteration
+__global__ void k_ctl_lin_init(double* sc, cudaGraphConditionalHandle h_while, int adaptive, double lin_rtol,
+                               int maxit) {
+  const double rr = sc[SC_RNORM2], bb = sc[SC_BNORM2];
   double rtol = lin_rtol;
   if (adaptive) rtol = max_ref(lin_rtol, sc[SC_ETA] * min_ref(1.0, sc[SC_RELRES]));
   const double t = rtol * (bb > 0.0 ? sqrt(bb) : 1.0);
   sc[SC_TARGET2] = t * t;
   sc[SC_SOLVED] = 1.0;
+  sc[SC_HALFDONE] = 0.0;
   if (!isfinite(rr)) sc[SC_NAN] = 1.0;
   cudaGraphSetConditional(h_while, (isfinite(rr) && rr > t * t && maxit > 0) ? 1u : 0u);
-}
-
-// after s = r - alpha v: stop at the half step if |s| meets the target
-__global__ void k_ctl_half(const double* partials, int nblocks, double* sc, cudaGraphConditionalHandle h_while,
-                           cudaGraphConditionalHandle h_half) {
-  double v[kPW];
-  sum_partials4(partials, nblocks, v);
-  if (threadIdx.x != 0) return;
-  const double ss = v[0];
-  sc[SC_SNORM2] = ss;
-  sc[SC_LIN_IT] += 1.0;
-  if (!isfinite(ss)) {
-    sc[SC_NAN] = 1.0;
-    sc[SC_HALFDONE] = 0.0;
-    cudaGraphSetConditional(h_half, 0u);
-    cudaGraphSetConditional(h_while, 0u);
-  } else if (ss <= sc[SC_TARGET2]) {
-    sc[SC_HALFDONE] = 1.0;
-    sc[SC_RNORM2] = ss;
-    cudaGraphSetConditional(h_half, 0u);
-    cudaGraphSetConditional(h_while, 0u);
-  } else {
-    sc[SC_HALFDONE] = 0.0;
-    cudaGraphSetConditional(h_half, 1u);
-  }
-}
-
-__global__ void k_x_half_pred(Dims d, const double* sc, double* xu, double* xv, const double* phu, const double* phv) {
-  IDX2D
-  if (j >= d.ny || i >= d.nx) return;
-  if (sc[SC_HALFDONE] == 0.0) return;
-  const long long q = d.at(j, i);
-  const double alpha = sc[SC_ALPHA];
-  if (u_int(d, j, i)) xu[q] += alpha * phu[q];
-  if (v_int(d, j, i)) xv[q] += alpha * phv[q];
-}
-
-// after the full step: rho, beta and the continue test
-__global__ void k_ctl_full(const double* partials, int nblocks, double* sc, cudaGraphConditionalHandle h_while,
-                           int maxit) {
-  double v[kPW];
-  sum_partials4(partials, nblocks, v);
-  if (threadIdx.x != 0) return;
-  const double rho_new = v[0], rr = v[1];
-  const double om = sc[SC_OMEGA], al = sc[SC_ALPHA], rho = sc[SC_RHO];
-  sc[SC_BETA] = (rho != 0.0 && om != 0.0) ? (rho_new / rho) * (al / om) : 0.0;
-  sc[SC_RHO] = rho_new;
-  sc[SC_RNORM2] = rr;
-  sc[SC_LIN_FULL] += 1.0;
-  const bool fin = isfinite(rr);
-  if (!fin) sc[SC_NAN] = 1.0;
-  cudaGraphSetConditional(h_while, (fin && rr > sc[SC_TARGET2] && sc[SC_LIN_IT] < (double)maxit) ? 1u : 0u);
-}
-
-__global__ void k_ctl_lin_finish(double* sc) {
-  if (sc[SC_RNORM2] > sc[SC_TARGET2]) sc[SC_LIN_FAILED] += 1.0;
 }
 
 // ---- host side --------------------------------------------------------------------
@@ -2412,65 +2323,83 @@ static int read_scalars(Ctx* c) {
   return DIVA_OK;
 }
 
+static Reduction reduction(Ctx* c) { return Reduction{c->partials, c->red_count}; }
+
+// x <- (u, v), the initial residual, its norms and (raw) the nonlinear residual's
+static void launch_init_residual(Ctx* c, const double* u, const double* v, int raw, const RelresTest& test) {
+  auto K = c->kv;
+  k_init_residual<<<red_blocks(c->d), block2d(), 0, c->stream>>>(
+      make_op(c, 0), u, v, K[KV_B][0], K[KV_B][1], K[KV_X][0], K[KV_X][1], K[KV_R][0], K[KV_R][1], K[KV_RHAT][0],
+      K[KV_RHAT][1], K[KV_P][0], K[KV_P][1], raw, reduction(c), c->scal, test); c->launches++;
+  c->fine_passes += 1.0;
+}
+// v = A phat and alpha, then s = r - alpha v and the half-step test (after the V-cycle p -> phat)
+static void launch_first_half(Ctx* c, const LoopHandles& h) {
+  auto K = c->kv;
+  const int nb = red_blocks(c->d);
+  k_matvec<<<nb, block2d(), 0, c->stream>>>(make_op(c, 0), K[KV_PHAT][0], K[KV_PHAT][1], K[KV_V][0], K[KV_V][1],
+                                            K[KV_RHAT][0], K[KV_RHAT][1], reduction(c), c->scal, ST_ALPHA); c->launches++;
+  k_update_s<<<nb, block2d(), 0, c->stream>>>(c->d, c->scal, K[KV_R][0], K[KV_R][1], K[KV_V][0], K[KV_V][1],
+                                              K[KV_S][0], K[KV_S][1], reduction(c), h); c->launches++;
+  c->fine_passes += 3.0;
+}
+// t = A shat and omega, x and r, rho and beta, p (after the V-cycle s -> shat)
+static void launch_second_half(Ctx* c, const LoopHandles& h) {
+  auto K = c->kv;
+  const int nb = red_blocks(c->d);
+  k_matvec<<<nb, block2d(), 0, c->stream>>>(make_op(c, 0), K[KV_SHAT][0], K[KV_SHAT][1], K[KV_T][0], K[KV_T][1],
+                                            K[KV_S][0], K[KV_S][1], reduction(c), c->scal, ST_OMEGA); c->launches++;
+  k_update_xr<<<nb, block2d(), 0, c->stream>>>(c->d, c->scal, K[KV_X][0], K[KV_X][1], K[KV_PHAT][0], K[KV_PHAT][1],
+                                               K[KV_SHAT][0], K[KV_SHAT][1], K[KV_S][0], K[KV_S][1], K[KV_T][0],
+                                               K[KV_T][1], K[KV_R][0], K[KV_R][1], K[KV_RHAT][0], K[KV_RHAT][1],
+                                               reduction(c), c->c.lin_maxit, h); c->launches++;
+  k_update_p<<<grid2d(c->d.ny, c->d.nx), block2d(), 0, c->stream>>>(c->d, c->scal, K[KV_R][0], K[KV_R][1], K[KV_V][0],
+                                                                    K[KV_V][1], K[KV_P][0], K[KV_P][1]); c->launches++;
+  c->fine_passes += 3.0;
+}
+// the solution (KV_XF)
+static void launch_finish_x(Ctx* c, int half) {
+  auto K = c->kv;
+  k_finish_x<<<grid2d(c->d.ny, c->d.nx), block2d(), 0, c->stream>>>(c->d, c->bc, c->scal, half, K[KV_X][0], K[KV_X][1],
+                                                                    K[KV_PHAT][0], K[KV_PHAT][1], K[KV_XF][0],
+                                                                    K[KV_XF][1]); c->launches++;
+}
+
 int solver_solve(Ctx* c, const double* u0, const double* v0, double rtol, int maxit, int* iters, double* relres0) {
-  const Dims d = c->d;
-  const Op o = make_op(c, 0);
   auto U_ = [&](int k) { return c->kv[k][0]; };
   auto V_ = [&](int k) { return c->kv[k][1]; };
-  dim3 g = grid2d(d.ny, d.nx);
-  const int nb = g.x * g.y;
-  DIVA_CUDA(c, cudaMemcpyAsync(U_(KV_X), u0, sizeof(double) * d.plane, cudaMemcpyDeviceToDevice, c->stream));
-  DIVA_CUDA(c, cudaMemcpyAsync(V_(KV_X), v0, sizeof(double) * d.plane, cudaMemcpyDeviceToDevice, c->stream));
-  k_init_residual<<<g, block2d(), 0, c->stream>>>(o, U_(KV_X), V_(KV_X), U_(KV_B), V_(KV_B), U_(KV_R), V_(KV_R),
-                                                  U_(KV_RHAT), V_(KV_RHAT), U_(KV_P), V_(KV_P), c->partials, g.x); c->launches++;
-  k_reduce<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, ST_INIT); c->launches++;
+  launch_init_residual(c, u0, v0, 0, RelresTest{});
   DIVA_LAUNCHED(c, "k_init_residual");
-  c->fine_passes += 1.0;
   int st = read_scalars(c);
   if (st) return st;
   const double bnorm = sqrt(c->h_scal[SC_BNORM2]);
   double rnorm = sqrt(c->h_scal[SC_RNORM2]);
   if (relres0) *relres0 = bnorm > 0.0 ? rnorm / bnorm : rnorm;
   const double target = rtol * (bnorm > 0.0 ? bnorm : 1.0);
-  int it = 0;
+  int it = 0, half = 0;
   bool done = rnorm <= target;
   while (!done && it < maxit) {
     ++it;
     if ((st = precond(c, U_(KV_P), V_(KV_P), U_(KV_PHAT), V_(KV_PHAT)))) return st;
-    k_matvec<<<g, block2d(), 0, c->stream>>>(o, U_(KV_PHAT), V_(KV_PHAT), U_(KV_V), V_(KV_V), U_(KV_RHAT),
-                                             V_(KV_RHAT), nullptr, nullptr, c->partials, g.x); c->launches++;
-    k_reduce<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, ST_ALPHA); c->launches++;
-    k_update_s<<<g, block2d(), 0, c->stream>>>(d, c->scal, U_(KV_R), V_(KV_R), U_(KV_V), V_(KV_V), U_(KV_S),
-                                               V_(KV_S), c->partials, g.x); c->launches++;
-    k_reduce<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, ST_SNORM); c->launches++;
+    launch_first_half(c, LoopHandles{});
     DIVA_LAUNCHED(c, "bicgstab half step");
     if ((st = read_scalars(c))) return st;
     if (sqrt(c->h_scal[SC_SNORM2]) <= target) {
-      k_update_x_half<<<g, block2d(), 0, c->stream>>>(d, c->scal, U_(KV_X), V_(KV_X), U_(KV_PHAT), V_(KV_PHAT)); c->launches++;
-      DIVA_LAUNCHED(c, "k_update_x_half");
+      half = 1;
       rnorm = sqrt(c->h_scal[SC_SNORM2]);
       done = true;
       break;
     }
     if ((st = precond(c, U_(KV_S), V_(KV_S), U_(KV_SHAT), V_(KV_SHAT)))) return st;
-    k_matvec<<<g, block2d(), 0, c->stream>>>(o, U_(KV_SHAT), V_(KV_SHAT), U_(KV_T), V_(KV_T), U_(KV_S), V_(KV_S),
-                                             nullptr, nullptr, c->partials, g.x); c->launches++;
-    k_reduce<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, ST_OMEGA); c->launches++;
-    k_update_xr<<<g, block2d(), 0, c->stream>>>(d, c->scal, U_(KV_X), V_(KV_X), U_(KV_PHAT), V_(KV_PHAT),
-                                                U_(KV_SHAT), V_(KV_SHAT), U_(KV_S), V_(KV_S), U_(KV_T), V_(KV_T),
-                                                U_(KV_R), V_(KV_R), U_(KV_RHAT), V_(KV_RHAT), c->partials, g.x); c->launches++;
-    k_reduce<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, ST_RHO); c->launches++;
-    k_update_p<<<g, block2d(), 0, c->stream>>>(d, c->scal, U_(KV_R), V_(KV_R), U_(KV_V), V_(KV_V), U_(KV_P),
-                                               V_(KV_P)); c->launches++;
+    launch_second_half(c, LoopHandles{});
     DIVA_LAUNCHED(c, "bicgstab full step");
-    c->fine_passes += 6.0;
     if ((st = read_scalars(c))) return st;
     rnorm = sqrt(c->h_scal[SC_RNORM2]);
     if (!std::isfinite(rnorm)) return set_error(c, DIVA_NAN_DETECTED, "NaN in the linear solve");
     done = rnorm <= target;
   }
-  k_fill_boundary<<<g, block2d(), 0, c->stream>>>(d, c->bc, U_(KV_X), V_(KV_X)); c->launches++;
-  DIVA_LAUNCHED(c, "k_fill_boundary");
+  launch_finish_x(c, half);
+  DIVA_LAUNCHED(c, "k_finish_x");
   *iters = it;
   c->lin_iters += it;
   if (!done) {
@@ -2484,15 +2413,11 @@ int solver_solve(Ctx* c, const double* u0, const double* v0, double rtol, int ma
 }
 
 int solver_relres(Ctx* c, const double* u, const double* v, double* relres) {
-  const Dims d = c->d;
-  dim3 g = grid2d(d.ny, d.nx);
-  k_relres<<<g, block2d(), 0, c->stream>>>(make_op(c, 0), u, v, c->kv[KV_B][0], c->kv[KV_B][1], c->partials, g.x); c->launches++;
-  k_reduce<<<1, 256, 0, c->stream>>>(c->partials, g.x * g.y, c->scal, ST_INIT); c->launches++;
-  DIVA_LAUNCHED(c, "k_relres");
-  c->fine_passes += 1.0;
+  launch_init_residual(c, u, v, 1, RelresTest{});
+  DIVA_LAUNCHED(c, "k_init_residual");
   int st = read_scalars(c);
   if (st) return st;
-  const double bb = c->h_scal[SC_BNORM2], rr = c->h_scal[SC_RNORM2];
+  const double bb = c->h_scal[SC_BNORM2], rr = c->h_scal[SC_RR];
   *relres = bb > 0.0 ? sqrt(rr / bb) : sqrt(rr);
   return DIVA_OK;
 }
@@ -2528,12 +2453,11 @@ int solver_smooth_fine_values(const Ctx* c) {
 }
 
 int solver_matvec_fine(Ctx* c, int reps) {
-  const Dims d = c->d;
-  dim3 g = grid2d(d.ny, d.nx);
-  const Op o = make_op(c, 0);
+  auto K = c->kv;
   for (int r = 0; r < reps; ++r) {
-    k_matvec<<<g, block2d(), 0, c->stream>>>(o, c->kv[KV_X][0], c->kv[KV_X][1], c->kv[KV_T][0], c->kv[KV_T][1],
-                                             c->kv[KV_RHAT][0], c->kv[KV_RHAT][1], nullptr, nullptr, c->partials, g.x); c->launches++;
+    k_matvec<<<red_blocks(c->d), block2d(), 0, c->stream>>>(make_op(c, 0), K[KV_X][0], K[KV_X][1], K[KV_T][0], K[KV_T][1],
+                                                            K[KV_RHAT][0], K[KV_RHAT][1], reduction(c), c->scal,
+                                                            ST_NONE); c->launches++;
   }
   DIVA_LAUNCHED(c, "k_matvec");
   return DIVA_OK;
@@ -2577,29 +2501,25 @@ int solver_row_types(Ctx* c) {
   return DIVA_OK;
 }
 
-int solver_fill_boundary(Ctx* c, double* u, double* v) {
-  k_fill_boundary<<<grid2d(c->d.ny, c->d.nx), block2d(), 0, c->stream>>>(c->d, c->bc, u, v); c->launches++;
-  DIVA_LAUNCHED(c, "k_fill_boundary");
-  return DIVA_OK;
-}
-
 // ---- the viscosity iteration loop as one CUDA graph -------------------------------
 //
 // One viscosity iteration (ITER):
-//   pre   : k_ctl_begin, coefficients (K1 + faces), operator set-up of all levels,
-//           [relres stop rule] nonlinear residual -> k_ctl_relres sets IF(solve)
+//   pre   : coefficients (K1 + faces; K1 also starts the iteration's counters), operator
+//           set-up of all levels, x <- (u,v) and the initial residual with the nonlinear
+//           one, which [relres stop rule] sets IF(solve)
 //   IF(solve):
-//     head  : x <- (u,v), initial residual, k_ctl_lin_init sets WHILE(krylov)
+//     head  : k_ctl_lin_init sets WHILE(krylov)
 //     WHILE(krylov):
-//       first : V-cycle p -> phat, v = A phat, alpha, s, k_ctl_half sets IF(second)
-//               and may end the loop; x += alpha phat if it did
-//       IF(second): V-cycle s -> shat, t = A shat, omega, x and r, k_ctl_full
-//                   sets WHILE(krylov), p update
-//     tail  : boundary fill, Picard update (limits, relaxation, step norm, basal
-//             stress and velocity), stop test, DIVA_err commit
-//   post  : [DIVA] basal stress/velocity when the residual stopped the iteration;
-//           k_ctl_loop: continue unless the iteration converged, the residual met
-//           its tolerance, a NaN appeared or the iteration budget is spent
+//       first : V-cycle p -> phat, v = A phat, alpha, s, whose norm sets IF(second)
+//               and may end the loop
+//       IF(second): V-cycle s -> shat, t = A shat, omega, x and r, whose norm sets
+//                   WHILE(krylov), p update
+//     tail  : the solution (half step, boundary), Picard update (limits, relaxation, step
+//             norm, basal stress and velocity, DIVA_err), stop test
+//   the loop goes on unless the iteration converged, the residual met its tolerance, a NaN
+//   appeared or the iteration budget is spent: decided by the Picard update (step-norm rule)
+//   or [relres stop rule] by the post kernel, which also forms the basal stress and velocity
+//   of an iteration the residual stopped
 //
 // The whole loop: WHILE(picard) { ITER(parity p); IF(odd) { ITER(parity 1 - p) } }.
 // The viscosity is double-buffered (each iteration reads one buffer and writes the
@@ -2648,28 +2568,12 @@ int capture_graph(Ctx* c, cudaStream_t s, cudaGraph_t* g) {
   return DIVA_OK;
 }
 
-// end of an iteration: totals of the loop, and whether it goes on (sets h_a, and h_b if given)
-__global__ void k_ctl_loop(double* sc, cudaGraphConditionalHandle h_a, cudaGraphConditionalHandle h_b, int has_b,
-                           int nit) {
-  sc[SC_SUM_LIN] += sc[SC_LIN_IT];
-  sc[SC_SUM_FULL] += sc[SC_LIN_FULL];
-  sc[SC_N_SOLVED] += sc[SC_SOLVED];
-  const bool stop = sc[SC_CONVERGED] != 0.0 || sc[SC_EXIT_RELRES] != 0.0 || sc[SC_NAN] != 0.0 ||
-                    sc[SC_PIC_IT] > (double)nit;
-  cudaGraphSetConditional(h_a, stop ? 0u : 1u);
-  if (has_b) cudaGraphSetConditional(h_b, stop ? 0u : 1u);
-}
-
 // One viscosity iteration recorded into the graph that stream `top` is capturing; its
 // conditional bodies use cc.s[3..5].  `count`: record the launches and passes of its parts.
 int capture_iteration(Ctx* c, CaptureCtx& cc, cudaStream_t top, bool diva, PicardGraphs& G, bool count,
                       cudaGraphConditionalHandle h_a, cudaGraphConditionalHandle h_b, int has_b) {
   const diva_config_t& C = c->c;
   const bool relmode = C.picard_stop == DIVA_STOP_RELRES;
-  const Dims d = c->d;
-  const Op o = make_op(c, 0);
-  dim3 g2 = grid2d(d.ny, d.nx);
-  const int nb = g2.x * g2.y;
   auto U_ = [&](int k) { return c->kv[k][0]; };
   auto V_ = [&](int k) { return c->kv[k][1]; };
   double* u = c->D(diva ? DIVA_F_U_VAV_CX : DIVA_F_U_SSA_CX);
@@ -2680,17 +2584,13 @@ int capture_iteration(Ctx* c, CaptureCtx& cc, cudaStream_t top, bool diva, Picar
   cudaGraphConditionalHandle h_solve;
   DIVA_CUDA(c, cudaGraphConditionalHandleCreate(&h_solve, graph, 1, cudaGraphCondAssignDefault));
   c->stream = top;
+  const IterEnd end{1, relmode ? 0 : 1, C.DIVA_visc_it_nit, has_b, C.DIVA_visc_it_norm_dUV_tol, h_a, h_b};
   // ---- pre
   cc.mark();
-  k_ctl_begin<<<1, 1, 0, c->stream>>>(c->scal); c->launches++;
-  if ((st = launch_diva_coefficients(c, u, v, diva, K1_LOOP))) return st;   // swaps the viscosity buffers
+  if ((st = launch_diva_coefficients(c, u, v, diva, K1_LOOP, true))) return st;   // swaps the viscosity buffers
   if ((st = solver_setup(c, 1))) return st;
-  if (relmode) {
-    k_relres<<<g2, block2d(), 0, c->stream>>>(o, u, v, U_(KV_B), V_(KV_B), c->partials, g2.x); c->launches++;
-    k_ctl_relres<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, h_solve, C.picard_relres_tol,
-                                           C.picard_stall_its); c->launches++;
-    c->fine_passes += 1.0;
-  }
+  launch_init_residual(c, u, v, relmode ? 1 : 0,
+                       RelresTest{relmode ? 1 : 0, C.picard_stall_its, C.picard_relres_tol, h_solve});
   DIVA_LAUNCHED(c, "graph pre");
   if (count) { G.n_pre = cc.dl(); G.p_pre = cc.dp(); }
   // ---- IF(solve)
@@ -2703,13 +2603,7 @@ int capture_iteration(Ctx* c, CaptureCtx& cc, cudaStream_t top, bool diva, Picar
   cc.capturing[3] = true;
   c->stream = cc.s[3];
   cc.mark();
-  DIVA_CUDA(c, cudaMemcpyAsync(U_(KV_X), u, sizeof(double) * d.plane, cudaMemcpyDeviceToDevice, c->stream));
-  DIVA_CUDA(c, cudaMemcpyAsync(V_(KV_X), v, sizeof(double) * d.plane, cudaMemcpyDeviceToDevice, c->stream));
-  k_init_residual<<<g2, block2d(), 0, c->stream>>>(o, U_(KV_X), V_(KV_X), U_(KV_B), V_(KV_B), U_(KV_R), V_(KV_R),
-                                                   U_(KV_RHAT), V_(KV_RHAT), U_(KV_P), V_(KV_P), c->partials, g2.x); c->launches++;
-  k_ctl_lin_init<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, h_while, relmode && C.lin_adaptive, C.lin_rtol,
-                                           C.lin_maxit); c->launches++;
-  c->fine_passes += 1.0;
+  k_ctl_lin_init<<<1, 1, 0, c->stream>>>(c->scal, h_while, relmode && C.lin_adaptive, C.lin_rtol, C.lin_maxit); c->launches++;
   DIVA_LAUNCHED(c, "graph head");
   if (count) { G.n_head = cc.dl(); G.p_head = cc.dp(); }
   // ---- WHILE(krylov)
@@ -2723,14 +2617,7 @@ int capture_iteration(Ctx* c, CaptureCtx& cc, cudaStream_t top, bool diva, Picar
   c->stream = cc.s[4];
   cc.mark();
   if ((st = precond(c, U_(KV_P), V_(KV_P), U_(KV_PHAT), V_(KV_PHAT)))) return st;
-  k_matvec<<<g2, block2d(), 0, c->stream>>>(o, U_(KV_PHAT), V_(KV_PHAT), U_(KV_V), V_(KV_V), U_(KV_RHAT), V_(KV_RHAT),
-                                            nullptr, nullptr, c->partials, g2.x); c->launches++;
-  k_reduce<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, ST_ALPHA); c->launches++;
-  k_update_s<<<g2, block2d(), 0, c->stream>>>(d, c->scal, U_(KV_R), V_(KV_R), U_(KV_V), V_(KV_V), U_(KV_S), V_(KV_S),
-                                              c->partials, g2.x); c->launches++;
-  k_ctl_half<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, h_while, h_half); c->launches++;
-  k_x_half_pred<<<g2, block2d(), 0, c->stream>>>(d, c->scal, U_(KV_X), V_(KV_X), U_(KV_PHAT), V_(KV_PHAT)); c->launches++;
-  c->fine_passes += 3.0;
+  launch_first_half(c, LoopHandles{1, h_while, h_half});
   DIVA_LAUNCHED(c, "graph first half");
   if (count) { G.n_first = cc.dl(); G.p_first = cc.dp(); }
   // ---- IF(second half)
@@ -2742,15 +2629,7 @@ int capture_iteration(Ctx* c, CaptureCtx& cc, cudaStream_t top, bool diva, Picar
   c->stream = cc.s[5];
   cc.mark();
   if ((st = precond(c, U_(KV_S), V_(KV_S), U_(KV_SHAT), V_(KV_SHAT)))) return st;
-  k_matvec<<<g2, block2d(), 0, c->stream>>>(o, U_(KV_SHAT), V_(KV_SHAT), U_(KV_T), V_(KV_T), U_(KV_S), V_(KV_S),
-                                            nullptr, nullptr, c->partials, g2.x); c->launches++;
-  k_reduce<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, ST_OMEGA); c->launches++;
-  k_update_xr<<<g2, block2d(), 0, c->stream>>>(d, c->scal, U_(KV_X), V_(KV_X), U_(KV_PHAT), V_(KV_PHAT), U_(KV_SHAT),
-                                               V_(KV_SHAT), U_(KV_S), V_(KV_S), U_(KV_T), V_(KV_T), U_(KV_R),
-                                               V_(KV_R), U_(KV_RHAT), V_(KV_RHAT), c->partials, g2.x); c->launches++;
-  k_ctl_full<<<1, 256, 0, c->stream>>>(c->partials, nb, c->scal, h_while, C.lin_maxit); c->launches++;
-  k_update_p<<<g2, block2d(), 0, c->stream>>>(d, c->scal, U_(KV_R), V_(KV_R), U_(KV_V), V_(KV_V), U_(KV_P), V_(KV_P)); c->launches++;
-  c->fine_passes += 3.0;
+  launch_second_half(c, LoopHandles{1, h_while, h_while});
   DIVA_LAUNCHED(c, "graph second half");
   if (count) { G.n_second = cc.dl(); G.p_second = cc.dp(); }
   DIVA_CUDA(c, cudaStreamEndCapture(cc.s[5], &body_half));
@@ -2760,22 +2639,17 @@ int capture_iteration(Ctx* c, CaptureCtx& cc, cudaStream_t top, bool diva, Picar
   // ---- tail
   c->stream = cc.s[3];
   cc.mark();
-  k_ctl_lin_finish<<<1, 1, 0, c->stream>>>(c->scal); c->launches++;
-  k_fill_boundary<<<g2, block2d(), 0, c->stream>>>(d, c->bc, U_(KV_X), V_(KV_X)); c->launches++;
+  launch_finish_x(c, -1);
   DIVA_LAUNCHED(c, "graph tail");
-  if (C.picard_anderson_m > 0 && (st = launch_anderson_prepare(c, u, v, U_(KV_X), V_(KV_X)))) return st;
-  if ((st = launch_picard_update(c, u, v, U_(KV_X), V_(KV_X), diva))) return st;
-  if ((st = launch_ctl_end(c, relmode))) return st;
-  if ((st = launch_err_commit_pred(c))) return st;
+  if (C.picard_anderson_m > 0 && (st = launch_anderson_prepare(c, u, v, U_(KV_XF), V_(KV_XF)))) return st;
+  if ((st = launch_picard_update(c, u, v, U_(KV_XF), V_(KV_XF), diva, -1, &end))) return st;
   if (count) { G.n_tail = cc.dl(); G.p_tail = cc.dp(); }
   DIVA_CUDA(c, cudaStreamEndCapture(cc.s[3], &body_solve));
   cc.capturing[3] = false;
   // ---- post
   c->stream = top;
   cc.mark();
-  if (diva && relmode && (st = launch_basal_pred(c))) return st;
-  k_ctl_loop<<<1, 1, 0, c->stream>>>(c->scal, h_a, h_b, has_b, C.DIVA_visc_it_nit); c->launches++;
-  DIVA_LAUNCHED(c, "k_ctl_loop");
+  if (relmode && (st = launch_relres_end(c, diva, end))) return st;
   if (count) G.n_post = cc.dl();
   return DIVA_OK;
 }
