@@ -930,6 +930,409 @@ __global__ void __launch_bounds__(kTileThreads) k_smooth_up(OpT<R> o, Op oc, int
   }
 }
 
+// ---- streamed smoothing of the large levels --------------------------------------------
+// One block owns a strip of rows (j) and a chunk of columns (i) of a level and sweeps over the
+// chunk two columns a step.  A ring of columns in shared memory holds x, b and the operator's
+// coefficients of the columns in flight; colour pass q of a smoothing phase runs 3 q columns
+// behind the first, each pass in a warp of its own, so that in every step all passes (and the
+// copies of the columns ahead, the prolongation and the output) work on different columns and
+// one barrier separates the steps:
+//   step s: copy the pair s + kWavePre, prolong columns 2 s and 2 s + 1, pass q on columns
+//           2 s - 3 - 3 q and the next, output columns 2 s - 3 - 3 NP and the next.
+// A pass reads its columns and the two beside them.  With three columns between consecutive
+// passes every value it reads has been through exactly the passes of the level-wide colour
+// sweeps: pass q - 1 left the column beyond one step ago, pass q + 1 reaches the column before
+// one step from now (the two columns' points of one colour do not read each other).  The halo
+// (H = NP + 1 points: one per pass and one for the residual) is recomputed by the neighbouring
+// blocks instead of exchanged, at the ends of the chunk and along the strip's sides, pass q
+// updating the points within H - 1 - q of the tile.  The columns arrive by bulk copies (one
+// per plane and column) that complete on mbarriers.
+//
+// Bound by shared-memory bandwidth: about 16 reads per point update.  A colour's points in one
+// column lie two rows apart, which alone is a 2-way bank conflict; half of a half-warp takes
+// the column's points and the other half the next column's, whose rows have the other parity,
+// so the 16 values fill all banks.
+// Against the square tiles (k_smooth_down/up), which recompute 9 points on every side and keep
+// no more than 32 x 32 points and no coefficients beside them: a strip's halo along i is paid
+// once per chunk, and the coefficients come from the ring.  Pre- and post-smoothing of the
+// 1501 x 1501 sheet 312 us (tiles 408), of the 321 x 561 cap 48 us (tiles 53); a step of two
+// columns takes 0.7 us, most of it the latency of one point update after the other.  Issuing
+// the columns as tensor copies of two columns by one thread was slower (379 us).
+//
+// Boundary unknowns ("ghosts"): a u or v value outside its component's interior is read, by
+// the rows next to it, as its source's value or as zero (u_src, v_src).  The ring keeps each
+// such value in its own slot; the thread that updates a source point writes its ghosts as
+// well, so every row reads its whole stencil as stored.  (Corner ghosts are read by no
+// interior row.  Periodic sides, whose sources lie across the domain, use the per-colour
+// kernels.)
+constexpr int kWavePre = 3;       // pairs of columns the copies run ahead
+constexpr int kWaveBars = 8;      // mbarriers: more than the pairs in flight
+constexpr int kWaveCopy = 5;      // copying warps: five of a pair's 20 plane columns each (a bulk copy takes about
+                                  // 110 cycles to issue), the last the coarse columns
+constexpr int kWaveCoarse = 8;    // coarse columns held (2 (kWavePre + 1) of a level not coarsened along i)
+constexpr long kWaveSpin = 1L << 22;
+
+struct WaveGeom {
+  static constexpr int NU = 2;   // sweeps per phase
+  static constexpr int NP = 4 * NU, H = NP + 1;
+  static constexpr int TJ = 64 - 2 * NP;              // largest tile height: pass 0's rows of a colour fill a warp
+  static constexpr int HB = (H + 3) / 4 * 4;          // ring rows before the tile (even: 16-byte aligned)
+  static constexpr int RP = (HB + TJ + H + 3) / 4 * 4;   // ring rows
+  static constexpr int NC = 2 * kWavePre + 3 * NP + 6;   // ring columns: from the copies' to the output's left neighbour
+  static constexpr int CP = RP + 8;                   // rows of a coarse column (a level not coarsened along j)
+  static constexpr size_t xk = (size_t)NC * 8 * RP * sizeof(double), b = (size_t)NC * 2 * RP * sizeof(double);
+  static constexpr size_t coarse = (size_t)kWaveCoarse * 2 * CP * sizeof(double);
+  static constexpr size_t smem_down = xk + b + 128, smem_up = xk + b + coarse + 128;
+  // two per pass (rows below and above the middle); output (descent: a warp per component, half
+  // of the rows and column, ascent: per half of the rows); copies; prolongation (ascent: a lane
+  // per row, component and column)
+  static_assert(NC % 2 == 0 && (8 * RP * sizeof(double)) % 128 == 0 && (2 * RP) % 16 == 0, "pairs of slots, whole banks");
+  static constexpr int passes = 2 * NP, out_down = 8, out_up = 2, pro = RP * 4 / 32;
+  static constexpr int warps_down = passes + out_down + kWaveCopy, warps_up = passes + out_up + kWaveCopy + pro;
+  static_assert(RP * 4 % 32 == 0 && warps_up <= 32 && warps_down <= 32, "warps of a block");
+};
+
+struct WaveArgs {
+  Op o;
+  const double *idu, *idv;
+  const double *bu, *bv;
+  double *xu, *xv;            // pre-smoothed x: written by the descent, read by the ascent
+  double *ru, *rv;            // descent: the residual
+  double *ou, *ov;       // ascent: the result
+  Op oc;                 // ascent: the coarser level and its correction
+  const double *xcu, *xcv;
+  int fx, fy;
+  int rows, chunk;       // tile height and width
+  double* fail;          // set when a wait ran out
+};
+
+// ring offsets of the three columns a row reads
+struct RIx {
+  int w, c, e, i, j0;
+  __device__ __forceinline__ int operator()(int jj, int ii) const {
+    return (ii == i ? c : (ii > i ? e : w)) + (jj - j0);
+  }
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool wave_wait(uint32_t bar, uint32_t parity) {
+  for (long it = 0; it < kWaveSpin; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
+// Where a coarse column position is read from along i: clamped, then through the boundary rule
+// (u: cx points, v: cy points); rows are mapped by the reader.  -1: zero everywhere.
+__device__ __forceinline__ int coarse_col(const Op& oc, int C, bool ucomp) {
+  const int last = ucomp ? oc.d.nx - 2 : oc.d.nx - 1;
+  const int I = min(max(C, 0), last);
+  const int west = ucomp ? oc.bc.uW : oc.bc.vW, east = ucomp ? oc.bc.uE : oc.bc.vE;
+  if (I == 0) return west == DIVA_BC_INFINITE ? 1 : -1;
+  if (I == last) return east == DIVA_BC_INFINITE ? last - 1 : -1;
+  return I;
+}
+
+// Two taps of the prolongation along one direction, C and weight (the second weight 0 where
+// there is one tap: adding 0 x keeps the sum's bits).
+__device__ __forceinline__ void two_taps(int f, int fac, bool cell, int (&C)[2], double (&w)[2]) {
+  const int n = cell ? scatter_cell_n(f, fac) : scatter_node_n(f, fac);
+  if (cell) scatter_cell(f, fac, 0, C[0], w[0]);
+  else scatter_node(f, fac, 0, C[0], w[0]);
+  C[1] = C[0];
+  w[1] = 0.0;
+  if (n == 2) {
+    if (cell) scatter_cell(f, fac, 1, C[1], w[1]);
+    else scatter_node(f, fac, 1, C[1], w[1]);
+  }
+}
+
+// Every role runs its own loop over the steps, with ring offsets that move on by one column a
+// step: the step lasts as long as its slowest warp, so each warp's instructions count.
+template <bool FRONT, bool UP>
+__global__ void __launch_bounds__(32 * (UP ? WaveGeom::warps_up : WaveGeom::warps_down))
+    k_wave(const __grid_constant__ WaveArgs a) {
+  using G = WaveGeom;
+  constexpr int NP = G::NP, H = G::H, RP = G::RP, NC = G::NC, CP = G::CP, COL = 8 * RP;
+  constexpr int NPW = G::passes, NOUT = UP ? G::out_up : G::out_down;
+  extern __shared__ __align__(128) unsigned char wsm[];
+  __shared__ __align__(8) uint64_t bars[kWaveBars];
+  double* ring = reinterpret_cast<double*>(wsm);                          // [NC][8: xu xv Na Nb Bx By idu idv][RP]
+  double* bring = reinterpret_cast<double*>(wsm + G::xk);        // [NC][2][RP]
+  double* cring = reinterpret_cast<double*>(wsm + G::xk + G::b); // [kWaveCoarse][2][CP]
+  const Dims& d = a.o.d;
+  const BCs& bc = a.o.bc;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tj0 = blockIdx.x * a.rows, ti0 = blockIdx.y * a.chunk;
+  const int j0 = tj0 - G::HB, i0 = ti0 - H;                      // the ring's first row, the region's first column
+  const int tw = min(a.chunk, d.nx - ti0), ncols = tw + 2 * H;   // tile width here, region columns
+  const int CJ0 = a.fy == 2 ? ((j0 >> 1) - 2) & ~1 : j0 - 2;     // first coarse row held (even)
+  const int last = (tw + H + 3 * NP + 2) / 2;   // the step that puts out the tile's last column
+  constexpr int kINF = DIVA_BC_INFINITE;
+
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < kWaveBars; ++k)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&bars[k])), "r"(kWaveCopy) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+
+  // the operator reading from the ring
+  Op os = a.o;
+  os.Na = ring + 2 * RP; os.Nb = ring + 3 * RP; os.Bx = ring + 4 * RP; os.By = ring + 5 * RP;
+  auto slot_of = [](int cc) { return ((cc % NC) + NC) % NC * COL; };
+  auto next2 = [](int off) { return off >= (NC - 2) * COL ? off - (NC - 2) * COL : off + 2 * COL; };
+  auto beside = [&](int off, int i) {   // the three columns around ring offset off
+    return RIx{off == 0 ? (NC - 1) * COL : off - COL, off, off == (NC - 1) * COL ? 0 : off + COL, i, j0};
+  };
+  // a new value of the interior point (j,i) into the ghosts whose source it is (x: its plane;
+  // il, jl: the last interior column and row)
+  auto ghosts = [&](double* x, const RIx& ix, int j, int i, int il, int jl, int gW, int gE, int gS, int gN, double val) {
+    if (gS == kINF && j == 1) x[ix.c - j0] = val;
+    if (gN == kINF && j == jl) x[ix.c + jl + 1 - j0] = val;
+    if (gW == kINF && i == 1) x[ix.w + j - j0] = val;
+    if (gE == kINF && i == il) x[ix.e + j - j0] = val;
+  };
+
+  if (warp < NPW) {
+    // ---- pass q: lanes 0-7, 16-23 the first column's points, 8-15, 24-31 the second's
+    const int q = warp >> 1, p4 = q & 3, p = UP ? 3 - p4 : p4, comp = p >> 1, color = p & 1, reach = H - 1 - q;
+    const int il = comp == 0 ? d.nx - 3 : d.nx - 2, jl = comp == 0 ? d.ny - 2 : d.ny - 3;   // interior 1 .. il, 1 .. jl
+    const int jlo = tj0 - reach, jmin = max(jlo, 1), jmax = min(tj0 + a.rows + reach - 1, jl);
+    const int c0 = max(H - reach, 1 - i0), c1 = min(H + tw + reach - 1, il - i0);           // region columns updated
+    const int gW = comp == 0 ? bc.uW : bc.vW, gE = comp == 0 ? bc.uE : bc.vE;
+    const int gS = comp == 0 ? bc.uS : bc.vS, gN = comp == 0 ? bc.uN : bc.vN;
+    double* x = ring + comp * RP;
+    const double* xu = ring;
+    const double* xv = ring + RP;
+    const double* id = ring + (6 + comp) * RP;
+    const double* bb = bring + comp * RP;
+    int cc = -3 - 3 * q + ((lane >> 3) & 1), off = slot_of(cc);
+    // (i + j) & 1 == color: a lane's column keeps its parity
+    const int j = jlo + ((color + i0 + cc + jlo) & 1) + 2 * ((lane & 7) | ((lane >> 4) << 3)) + 32 * (warp & 1);
+    const bool row = j >= jmin && j <= jmax, jghost = j == 1 || j == jl;
+    __syncthreads();   // the first columns are there
+#pragma unroll 1
+    for (int s = 0; s <= last; ++s, cc += 2, off = next2(off)) {
+      if (row && cc >= c0 && cc <= c1) {
+        const int i = i0 + cc;
+        const RIx ix = beside(off, i);
+        const int k = off + j - j0;
+        const double b = bb[(off >> 2) + j - j0];   // (the b ring has a quarter of the planes)
+        const double Ax = comp == 0 ? AuXC<true, FRONT>(os, xu, xv, ix, ix, j, i) : AvXC<true, FRONT>(os, xu, xv, ix, ix, j, i);
+        const double val = fma_r(b - Ax, id[k], x[k]);
+        x[k] = val;
+        if (jghost || i == 1 || i == il) ghosts(x, ix, j, i, il, jl, gW, gE, gS, gN, val);
+      }
+      __syncthreads();
+    }
+  } else if (warp < NPW + NOUT) {
+    // ---- the tile's values
+    const int w = warp - NPW, comp = UP ? 0 : w >> 2, h0 = UP ? 0 : (w >> 1) & 1, jj = (w & 1) * 32 + lane, j = tj0 + jj;
+    const bool row = jj < a.rows && j < d.ny;
+    const double* xu = ring;
+    const double* xv = ring + RP;
+    int cc = -3 - 3 * NP + h0, off = slot_of(cc);
+    __syncthreads();
+#pragma unroll 1
+    for (int s = 0; s <= last; ++s, cc += 2, off = next2(off)) {
+      int o = off;
+#pragma unroll
+      for (int h = 0; h < (UP ? 2 : 1); ++h) {
+        const int c = cc + h, i = i0 + c, k = o + j - j0;
+        if (c >= H && c < H + tw && row) {
+          const long long g = d.at(j, i);
+          if (UP) {   // no ghost values out
+            a.ou[g] = u_int(d, j, i) ? xu[k] : 0.0;
+            a.ov[g] = v_int(d, j, i) ? xv[k] : 0.0;
+          } else {
+            const RIx ix = beside(o, i);
+            const double b = bring[(o >> 2) + comp * RP + j - j0];
+            if (comp == 0) {
+              a.xu[g] = xu[k];
+              a.ru[g] = u_int(d, j, i) ? b - AuXC<true, FRONT>(os, xu, xv, ix, ix, j, i) : 0.0;
+            } else {
+              a.xv[g] = xv[k];
+              a.rv[g] = v_int(d, j, i) ? b - AvXC<true, FRONT>(os, xu, xv, ix, ix, j, i) : 0.0;
+            }
+          }
+        }
+        o = o == (NC - 1) * COL ? 0 : o + COL;
+      }
+      __syncthreads();
+    }
+  } else if (warp < NPW + NOUT + kWaveCopy) {
+    // ---- copies of pair s + kWavePre: copy c = 5 w + lane of 20 is plane c / 2 of column c % 2; the
+    // last warp moves the coarse columns (lane 0: u, 1: v), or zeroes x for the descent
+    const int w = warp - NPW - NOUT, copy = min(5 * w + lane, 19), pl = copy >> 1, hc = copy & 1;
+    const bool mover = w < kWaveCopy - 1;
+    const int r0 = max(0, -j0), r1 = min(RP, d.ld - j0);           // ring rows inside the planes (even numbers)
+    const int cr0 = max(0, -CJ0), cr1 = UP ? min(CP, a.oc.d.ld - CJ0) : 0;
+    constexpr uint32_t es = sizeof(double);
+    const uint32_t bytes = mover && lane < 5 && (UP || pl >= 2) && r1 > r0 ? (r1 - r0) * es : 0;
+    uint32_t sum[2] = {hc == 0 ? bytes : 0, hc == 1 ? bytes : 0};  // the warp's bytes of either column
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      sum[0] += __shfl_down_sync(0xffffffffu, sum[0], o);          // (lanes 0-7 to lane 0)
+      sum[1] += __shfl_down_sync(0xffffffffu, sum[1], o);
+    }
+    const void* plane = pl == 0 ? (const void*)a.xu : pl == 1 ? (const void*)a.xv : pl == 2 ? (const void*)a.o.Na
+                        : pl == 3 ? (const void*)a.o.Nb : pl == 4 ? (const void*)a.o.Bx : pl == 5 ? (const void*)a.o.By
+                        : pl == 6 ? (const void*)a.idu : pl == 7 ? (const void*)a.idv
+                        : pl == 8 ? (const void*)a.bu : (const void*)a.bv;
+    const char* src = static_cast<const char*>(plane) + ((long long)(i0 + hc) * d.ld + j0 + r0) * (long long)es;
+    const uint32_t pitch = 2 * d.ld * es;
+    const uint32_t dcol = (pl < 8 ? COL : 2 * RP) * es;
+    const uint32_t dst0 = (pl < 8 ? smem_addr(ring + pl * RP + r0) : smem_addr(bring + (pl - 8) * RP + r0)) + hc * dcol;
+    const uint32_t cbytes = cr1 > cr0 ? (cr1 - cr0) * sizeof(double) : 0;
+    const uint32_t bar0 = smem_addr(&bars[0]);
+    const int npair = tw / 2 + H + (tw & 1);   // pairs of the region (an odd width's last column is beyond it)
+    int slot = 0;
+    auto coarse_total = [&](int C) {
+      return ((coarse_col(a.oc, C, true) >= 0 ? 1u : 0u) + (coarse_col(a.oc, C, false) >= 0 ? 1u : 0u)) * cbytes;
+    };
+    auto issue = [&](int t) {
+      const int i = i0 + 2 * t;
+      const uint32_t bar = bar0 + (t & (kWaveBars - 1)) * 8;
+      if (mover) {
+        const bool in0 = i >= 0 && i < d.nx, in1 = i + 1 >= 0 && i + 1 < d.nx;
+        if (lane == 0) {
+          // x has been written by other threads since its last copy
+          if (UP && w == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                       "r"((in0 ? sum[0] : 0u) + (in1 ? sum[1] : 0u))
+                       : "memory");
+        }
+        __syncwarp();
+        if (bytes && (hc ? in1 : in0)) bulk_copy(dst0 + slot * dcol, src, bytes, bar);
+      } else if (UP) {
+        // coarse columns that arrive with the pair: fx = 2, the one beyond that of its even column
+        // (with the first pair also those before it); fx = 1, the pair's own
+        const int Cb = a.fx == 1 ? i + 1 : ((i + 1) >> 1) + 1, Ca = a.fx == 1 ? i : t == 0 ? Cb - 3 : Cb;
+        if (lane == 0) {
+          uint32_t total = 0;
+          for (int C = Ca; C <= Cb; ++C) total += coarse_total(C);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(total) : "memory");
+        }
+        __syncwarp();
+        if (lane < 2 && cbytes)
+          for (int C = Ca; C <= Cb; ++C) {
+            const int I = coarse_col(a.oc, C, lane == 0);
+            if (I >= 0)
+              bulk_copy(smem_addr(cring + ((C & (kWaveCoarse - 1)) * 2 + lane) * CP + cr0),
+                        (lane == 0 ? a.xcu : a.xcv) + (long long)I * a.oc.d.ld + CJ0 + cr0, cbytes, bar);
+          }
+      } else {   // the descent enters a level with x = 0
+        constexpr int n16 = 2 * RP * sizeof(double) / 16;
+        for (int t2 = lane; t2 < 2 * n16; t2 += 32)
+          reinterpret_cast<uint4*>(ring + (slot + t2 / n16) * COL)[t2 % n16] = make_uint4(0u, 0u, 0u, 0u);
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+      }
+      src += pitch;
+      slot = slot == NC - 2 ? 0 : slot + 2;
+    };
+    auto arrived = [&](int t) { return wave_wait(bar0 + (t & (kWaveBars - 1)) * 8, (t / kWaveBars) & 1); };
+    int issued = 0, waited = 0;   // pairs issued and waited for
+    for (; issued < kWavePre && issued < npair; ++issued) issue(issued);
+    bool ok = arrived(0) && arrived(1);
+    waited = 2;
+    __syncthreads();
+#pragma unroll 1
+    for (int s = 0; s <= last; ++s) {
+      if (issued < npair) issue(issued++);
+      // the next step reads up to pair s + 2; a wait that runs out fails the solve, and the
+      // block goes on without waiting
+      if (ok && waited < npair) ok = arrived(waited++);
+      __syncthreads();
+    }
+    for (; waited < issued; ++waited) ok = arrived(waited) && ok;   // no copy in flight when the block ends
+    if (!ok && lane == 0) *a.fail = 1.0;
+  } else {
+    // ---- x += P x_c (prolong_delta's taps, weights and order)
+    const int t0 = (warp - NPW - NOUT - kWaveCopy) * 32 + lane, r = t0 % RP, comp = (t0 / RP) & 1, h = t0 / (2 * RP);
+    const int j = j0 + r;
+    const Dims& dc = a.oc.d;
+    const int il = comp == 0 ? d.nx - 3 : d.nx - 2, jl = comp == 0 ? d.ny - 2 : d.ny - 3;
+    const int lj = comp == 0 ? dc.ny - 1 : dc.ny - 2, li = comp == 0 ? dc.nx - 2 : dc.nx - 1;   // coarse: last row, column
+    const int gW = comp == 0 ? bc.uW : bc.vW, gE = comp == 0 ? bc.uE : bc.vE;
+    const int gS = comp == 0 ? bc.uS : bc.vS, gN = comp == 0 ? bc.uN : bc.vN;
+    const bool row = r < RP - 1 && j >= 1 && j <= jl;   // (the ring's last row is no halo row)
+    int Cj[2];
+    double wj[2];
+    two_taps(j, a.fy, comp == 1, Cj, wj);
+    // the taps' coarse rows, clamped and through the boundary rule of an interior column (-1: zero)
+    const int cS = comp == 0 ? a.oc.bc.uS : a.oc.bc.vS, cN = comp == 0 ? a.oc.bc.uN : a.oc.bc.vN;
+    int J[2], Jr[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      J[e] = min(max(Cj[e], 0), lj);
+      Jr[e] = J[e] == 0 ? (cS == kINF ? 1 : -1) : J[e] == lj ? (cN == kINF ? lj - 1 : -1) : J[e];
+    }
+    const double* cp = cring + comp * CP;
+    double* x = ring + comp * RP;
+    const int c0 = 1 - i0, c1 = min(ncols - 1, il - i0);
+    int cc = 0, off = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int s = 0; s <= last; ++s, cc += 2, off = next2(off)) {
+      const int c = cc + h, o = off + h * COL;   // (a pair's slots are neighbours)
+      if (row && c >= c0 && c <= c1) {
+        const int i = i0 + c;
+        int Ci[2];
+        double wi[2];
+        two_taps(i, a.fx, comp == 0, Ci, wi);
+        const int I0 = min(max(Ci[0], 0), li), I1 = min(max(Ci[1], 0), li);
+        double v[2][2];
+        const bool iedge = I0 == 0 || I0 == li || I1 == 0 || I1 == li;
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int f = 0; f < 2; ++f) {
+            int jr = Jr[e], js, is;
+            if (iedge)   // the corners' rule (the column is mapped already)
+              jr = (comp == 0 ? u_src(dc, a.oc.bc, J[e], f ? I1 : I0, js, is)
+                              : v_src(dc, a.oc.bc, J[e], f ? I1 : I0, js, is)) ? js : -1;
+            v[e][f] = jr >= 0 ? cp[(Ci[f] & (kWaveCoarse - 1)) * 2 * CP + jr - CJ0] : 0.0;
+          }
+        double t = (wj[0] * wi[0]) * v[0][0];
+        t = fma(wj[0] * wi[1], v[0][1], t);
+        t = fma(wj[1] * wi[0], v[1][0], t);
+        t = fma(wj[1] * wi[1], v[1][1], t);
+        const RIx ix = beside(o, i);
+        const double val = x[o + r] + t;
+        x[o + r] = val;
+        if (j == 1 || j == jl || i == 1 || i == il) ghosts(x, ix, j, i, il, jl, gW, gE, gS, gN, val);
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// the restricted residual of the finer level as this level's right-hand side
+__global__ void k_restrict_b(Dims df, Dims dc, int fx, int fy, const double* ru, const double* rv, double* bu, double* bv) {
+  IDX2D
+  if (j >= dc.ny || i >= dc.nx) return;
+  const long long q = dc.at(j, i);
+  double b0, b1;
+  restrict_values(df, dc, fx, fy, ru, rv, j, i, b0, b1);
+  bu[q] = b0;
+  bv[q] = b1;
+}
+
 // ---- direct solve of the coarsest level ------------------------------------------------
 // The coarsest level has at most kCoarseDirectMax interior unknowns, numbered u first,
 // then v, each in plane order (i outer, j inner).  Once per viscosity iteration its
@@ -2081,6 +2484,84 @@ static int tile_up(Ctx* c, int l, int fx, int fy, const double* bu, const double
   return DIVA_OK;
 }
 
+// Whether level l is smoothed by the streamed kernel: double, two sweeps per phase, and more
+// points than one round of 16 x 16 tiles covers (two per SM).  Smoothing pair, tiles against
+// the streamed kernel: 24.7 / 30.8 us at 129 x 17, 33.1 / 37.6 at 201 x 351 (286 tiles: one
+// round), 49.6 / 39.0 at 229 x 401 (390 tiles: a second one), 53.3 / 48.2 at 321 x 561, 57.8 /
+// 57.4 at 501 x 501, 107.5 / 92.1 at 751 x 751, 408 / 312 at 1501 x 1501.  Float levels keep
+// the tiles, which hold the coefficients of a 32 x 32 tile in shared memory: 41 / 46 us at
+// 321 x 561.
+constexpr long long kWavePoints = 2LL * kSMs * 16 * 16;
+static int level_nu(const Ctx* c, int l);
+static bool level_streamed(const Ctx* c, int l) {
+  const Dims& d = c->lv[l].d;
+  return !level_fp32(c, l) && level_nu(c, l) == WaveGeom::NU && (long long)d.nx * d.ny >= kWavePoints;
+}
+// Strips and chunks of a streamed level: strips as high as two warps per pass allow (fewer halo
+// rows), or 16 rows where the caller chose that edge, evened out over the level; then the number of chunks with the
+// fewest steps in turn, each block (one per SM) taking half its chunk, halo and lag, and some to
+// start, over as many rounds as needed.
+static void wave_shape(const Ctx* c, int l, int* rows, int* chunk, dim3* grid) {
+  using G = WaveGeom;
+  const Dims& d = c->lv[l].d;
+  const int top = c->tile_override[l] == 16 ? 16 : G::TJ;
+  const int ns = (d.ny + top - 1) / top;
+  *rows = ((d.ny + ns - 1) / ns + 1) / 2 * 2;
+  const int nstrip = (d.ny + *rows - 1) / *rows;
+  long best = 0;
+  for (int n = 1; n <= d.nx; ++n) {
+    const int w = (d.nx + n - 1) / n, nc = (d.nx + w - 1) / w;
+    if (w < 4 && n > 1) break;
+    const long rounds = ((long)nstrip * nc + kSMs - 1) / kSMs;
+    const long cost = rounds * ((w + G::H + 3 * G::NP + 2) / 2 + 5);
+    if (best == 0 || cost < best) {
+      best = cost;
+      *chunk = w;
+      *grid = dim3(nstrip, nc);
+    }
+  }
+}
+template <bool UP>
+static void launch_wave(Ctx* c, int l, const double* bu, const double* bv, double* ou, double* ov) {
+  using G = WaveGeom;
+  const Level& L = c->lv[l];
+  WaveArgs a{};
+  a.o = make_op(c, l);
+  a.idu = L.idu; a.idv = L.idv; a.bu = bu; a.bv = bv;
+  a.xu = L.tu; a.xv = L.tv; a.ru = L.ru; a.rv = L.rv;
+  a.fail = c->scal + SC_NAN;
+  if (UP) {
+    a.ou = ou; a.ov = ov;
+    a.oc = make_op(c, l + 1);
+    a.xcu = c->lv[l + 1].xu; a.xcv = c->lv[l + 1].xv;
+    factors(c, l, &a.fx, &a.fy);
+  }
+  dim3 grid;
+  wave_shape(c, l, &a.rows, &a.chunk, &grid);
+  const auto kern = a.o.rtu ? k_wave<true, UP> : k_wave<false, UP>;   // 'BC' rows: the finest level
+  kern<<<grid, 32 * (UP ? G::warps_up : G::warps_down), UP ? G::smem_up : G::smem_down, c->stream>>>(a);
+  c->launches++;
+}
+// pre-smoothing from x = 0 (the descent of a V-cycle enters every level with x = 0): two forward
+// sweeps (u0 u1 v0 v1), x and r = b - A x written; b first, where it is the finer level's residual
+static int wave_down(Ctx* c, int l, const Restriction& rs, const double* bu, const double* bv) {
+  if (rs.on) {
+    k_restrict_b<<<GL(l)>>>(rs.df, c->lv[l].d, rs.fx, rs.fy, static_cast<const double*>(rs.ru),
+                            static_cast<const double*>(rs.rv), const_cast<double*>(bu), const_cast<double*>(bv));
+    c->launches++;
+    DIVA_LAUNCHED(c, "k_restrict_b");
+  }
+  launch_wave<false>(c, l, bu, bv, nullptr, nullptr);
+  DIVA_LAUNCHED(c, "k_wave (descent)");
+  return DIVA_OK;
+}
+// post-smoothing: x += P x_c, then two backward sweeps (v1 v0 u1 u0)
+static int wave_up(Ctx* c, int l, const double* bu, const double* bv, double* xu, double* xv) {
+  launch_wave<true>(c, l, bu, bv, xu, xv);
+  DIVA_LAUNCHED(c, "k_wave (ascent)");
+  return DIVA_OK;
+}
+
 // V-cycle step of a tiled level: 2 launches for the smoothing, the residual and the
 // restriction instead of 4 per sweep and 2 more
 static int vcycle_tiled(Ctx* c, int l, double* xu, double* xv, const double* bu, const double* bv,
@@ -2089,7 +2570,8 @@ static int vcycle_tiled(Ctx* c, int l, double* xu, double* xv, const double* bu,
     return set_error(c, DIVA_UNSUPPORTED, "tiled smoothing depth");
   const Level& L = c->lv[l];
   const Level& K = c->lv[l + 1];
-  int st = tile_down(c, l, rs, bu, bv, xu, xv, nu1);
+  const bool wave = level_streamed(c, l);
+  int st = wave ? wave_down(c, l, rs, bu, bv) : tile_down(c, l, rs, bu, bv, xu, xv, nu1);
   if (st) return st;
   Restriction next{};
   next.on = 1;
@@ -2099,7 +2581,7 @@ static int vcycle_tiled(Ctx* c, int l, double* xu, double* xv, const double* bu,
   next.rv = L.rv;
   next.rfloat = level_fp32(c, l) ? 1 : 0;   // the float residual of a mixed-precision level
   if ((st = vcycle(c, l + 1, K.xu, K.xv, K.bu, K.bv, next))) return st;
-  if ((st = tile_up(c, l, next.fx, next.fy, bu, bv, xu, xv, nu2))) return st;
+  if ((st = wave ? wave_up(c, l, bu, bv, xu, xv) : tile_up(c, l, next.fx, next.fy, bu, bv, xu, xv, nu2))) return st;
   c->fine_passes += (nu1 + nu2 + 1) * (double)L.d.plane / (double)c->d.plane;
   return DIVA_OK;
 }
@@ -2216,6 +2698,11 @@ int solver_init(Ctx* c) {
   if (int st = tile_attrs_shape<16, 16>(c)) return st;
   if (int st = tile_attrs_shape<32, 48>(c)) return st;
   if (int st = tile_attrs_shape<16, 24>(c)) return st;
+  const void* wave[4] = {(const void*)k_wave<false, false>, (const void*)k_wave<true, false>,
+                         (const void*)k_wave<false, true>, (const void*)k_wave<true, true>};
+  for (int q = 0; q < 4; ++q)
+    DIVA_CUDA(c, cudaFuncSetAttribute(wave[q], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(q < 2 ? WaveGeom::smem_down : WaveGeom::smem_up)));
   const BCs& b = c->bc;
   const int all[8] = {b.uW, b.uE, b.uS, b.uN, b.vW, b.vE, b.vS, b.vN};
   bool periodic = false;
@@ -2433,8 +2920,9 @@ int solver_smooth_fine(Ctx* c, int sweeps) {
     factors(c, 0, &fx, &fy);
     double *xu = c->kv[KV_X][0], *xv = c->kv[KV_X][1];
     double *bu = c->kv[KV_B][0], *bv = c->kv[KV_B][1];   // not written: the restriction is off
-    int st = tile_down(c, 0, Restriction{}, bu, bv, xu, xv, nu);
-    if (!st) st = tile_up(c, 0, fx, fy, bu, bv, xu, xv, nu);
+    const bool wave = level_streamed(c, 0);
+    int st = wave ? wave_down(c, 0, Restriction{}, bu, bv) : tile_down(c, 0, Restriction{}, bu, bv, xu, xv, nu);
+    if (!st) st = wave ? wave_up(c, 0, bu, bv, xu, xv) : tile_up(c, 0, fx, fy, bu, bv, xu, xv, nu);
     return st;
   }
   for (int s = 0; s < sweeps; ++s) {
