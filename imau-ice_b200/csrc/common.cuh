@@ -60,6 +60,23 @@ __device__ __forceinline__ double stag_margin(double v0, double v1, double H0, d
 constexpr int kBX = 32, kBY = 8;
 inline dim3 grid2d(int nj, int ni) { return dim3((nj + kBX - 1) / kBX, (ni + kBY - 1) / kBY); }
 inline dim3 block2d() { return dim3(kBX, kBY); }
+// Kernels over 3D fields.  A thread loads kLayers layers of its column before it uses or stores
+// any: a loop that loads, computes and stores layer by layer waits for memory once per layer,
+// the compiler not being able to move a load over a store.  Where the layers are independent
+// the grid has a block per kLayers of them (grid_layers), which also fills the GPU on small grids.
+// 1001 x 1001 x 15: staggering of one field 82 -> 58 us, k_secondary 688 -> 260 us, SIA velocities
+// 157 -> 95 us, rate factor 71 -> 60 us; staggering on 161 x 281 15.2 -> 4.9 us.
+constexpr int kLayers = 5;
+inline dim3 grid_layers(int nj, int ni, int nz) {
+  dim3 g = grid2d(nj, ni);
+  g.z = (nz + kLayers - 1) / kLayers;
+  return g;
+}
+// (loads: of the last layer again instead of behind a branch, where there are fewer left)
+#define FOR_LAYERS(e, k0, nz) _Pragma("unroll") for (int e = 0; e < kLayers; ++e) if ((k0) + e < (nz))
+#define LOAD_LAYERS(e, k, k0, nz)                      \
+  _Pragma("unroll") for (int e = 0; e < kLayers; ++e)  \
+    if (const int k = (k0) + e < (nz) ? (k0) + e : (nz) - 1; true)
 
 __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);

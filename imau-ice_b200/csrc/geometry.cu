@@ -128,10 +128,14 @@ __global__ void k_masks_transitions(Dims d, const int* land, const int* ocean, c
 
 // staggering and slopes of update_general_ice_model_data :60-79
 // (map_a_to_cx/cy/b_2D, ddx/ddy_a_to_a/cx/cy_2D of derivatives_and_grids_module.f90)
-__global__ void k_stagger_slopes(Dims d, const double* Hi, const double* Hs, const double* Avav, double* Hi_cx,
-                                 double* Hi_cy, double* Hi_b, double* Avav_cx, double* Avav_cy, double* dHi_dx,
-                                 double* dHi_dy, double* dHs_dx, double* dHs_dy, double* dHs_dx_cx, double* dHs_dy_cx,
-                                 double* dHs_dx_cy, double* dHs_dy_cy) {
+__global__ void k_stagger_slopes(Dims d, const double* __restrict__ Hi, const double* __restrict__ Hs,
+                                 const double* __restrict__ Avav, double* __restrict__ Hi_cx,
+                                 double* __restrict__ Hi_cy, double* __restrict__ Hi_b, double* __restrict__ Avav_cx,
+                                 double* __restrict__ Avav_cy, double* __restrict__ dHi_dx,
+                                 double* __restrict__ dHi_dy, double* __restrict__ dHs_dx,
+                                 double* __restrict__ dHs_dy, double* __restrict__ dHs_dx_cx,
+                                 double* __restrict__ dHs_dy_cx, double* __restrict__ dHs_dx_cy,
+                                 double* __restrict__ dHs_dy_cy) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
   const int nx = d.nx, ny = d.ny;
   if (j >= ny || i >= nx) return;
@@ -185,14 +189,22 @@ __global__ void k_stagger_slopes(Dims d, const double* Hi, const double* Hs, con
   }
 }
 
-// map_a_to_cx_3D / map_a_to_cy_3D :1513-1578
+// map_a_to_cx_3D / map_a_to_cy_3D :1513-1578.  Bound by memory (one field read, two written).
 __global__ void k_stagger3d(Dims d, const double* A, double* Acx, double* Acy) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y, k0 = blockIdx.z * kLayers;
   if (j >= d.ny || i >= d.nx) return;
-  for (int k = 0; k < d.nz; ++k) {
-    const long long o = (long long)k * d.plane;
-    if (i < d.nx - 1) Acx[o + d.at(j, i)] = (A[o + d.at(j, i)] + A[o + d.at(j, i + 1)]) / 2.0;
-    if (j < d.ny - 1) Acy[o + d.at(j, i)] = (A[o + d.at(j, i)] + A[o + d.at(j + 1, i)]) / 2.0;
+  const bool cx = i < d.nx - 1, cy = j < d.ny - 1;
+  const long long q = d.at(j, i), qe = cx ? q + d.ld : q, qn = cy ? q + 1 : q;
+  double a[kLayers], ae[kLayers], an[kLayers];
+  LOAD_LAYERS(e, k, k0, d.nz) {
+    a[e] = A[k * d.plane + q];
+    ae[e] = A[k * d.plane + qe];
+    an[e] = A[k * d.plane + qn];
+  }
+  FOR_LAYERS(e, k0, d.nz) {
+    const long long o = (k0 + e) * d.plane + q;
+    if (cx) Acx[o] = (a[e] + ae[e]) / 2.0;
+    if (cy) Acy[o] = (a[e] + an[e]) / 2.0;
   }
 }
 
@@ -213,21 +225,25 @@ __global__ void k_rheology(Dims d, Zeta zt, int choice, int bc_margin, double un
   const double A_low = 1.14E-05, A_high = 5.47E+10, Q_low = 6.0E+04, Q_high = 13.9E+04;
   const double m = sheet[q] == 1 ? m_sheet : (shelf[q] == 1 ? m_shelf : 1.0);
   const bool apply = sheet[q] == 1 || shelf[q] == 1;
+  const bool arrhenius = choice != DIVA_RHEO_UNIFORM && ice[q] == 1;
+  // the same in every layer where it does not depend on the temperature
+  const double a0 = choice == DIVA_RHEO_UNIFORM ? uniform_A : bc_margin ? 0.0 : A_low * exp(-Q_low / (kRGas * 263.15));
   double prev = 0.0, avg = 0.0;
-  for (int k = 0; k < d.nz; ++k) {
-    double a;
-    if (choice == DIVA_RHEO_UNIFORM) {
-      a = uniform_A;
-    } else if (ice[q] == 1) {
-      const double T = Ti[k * d.plane + q];
-      a = (T < 263.15) ? A_low * exp(-Q_low / (kRGas * T)) : A_high * exp(-Q_high / (kRGas * T));
-    } else {
-      a = bc_margin ? 0.0 : A_low * exp(-Q_low / (kRGas * 263.15));
+  for (int k0 = 0; k0 < d.nz; k0 += kLayers) {
+    double T[kLayers];
+    LOAD_LAYERS(e, k, k0, d.nz) T[e] = arrhenius ? Ti[k * d.plane + q] : 0.0;
+    FOR_LAYERS(e, k0, d.nz) {
+      const int k = k0 + e;
+      double a = a0;
+      if (arrhenius) {   // (one exponential for the warp's cold and warm ice)
+        const bool cold = T[e] < 263.15;
+        a = (cold ? A_low : A_high) * exp(-(cold ? Q_low : Q_high) / (kRGas * T[e]));
+      }
+      if (apply) a = a * m;
+      A[k * d.plane + q] = a;
+      if (k > 0) avg = avg + 0.5 * (a + prev) * (zt.z[k] - zt.z[k - 1]);  // vertical_average
+      prev = a;
     }
-    if (apply) a = a * m;
-    A[k * d.plane + q] = a;
-    if (k > 0) avg = avg + 0.5 * (a + prev) * (zt.z[k] - zt.z[k - 1]);  // vertical_average
-    prev = a;
   }
   Avav[q] = avg;
 }
@@ -407,6 +423,7 @@ __global__ void k_sico_masks(Dims d, const double* TAF, const double* Hi, int* c
 }  // namespace
 
 #define G2 grid2d(c->d.ny, c->d.nx), block2d(), 0, c->stream
+#define G3 grid_layers(c->d.ny, c->d.nx, c->d.nz), block2d(), 0, c->stream
 
 int launch_update_general_ice_model_data(Ctx* c) {
   const Dims d = c->d;
@@ -444,7 +461,7 @@ int launch_update_general_ice_model_data(Ctx* c) {
                            c->D(DIVA_F_DHS_DX_CX), c->D(DIVA_F_DHS_DY_CX), c->D(DIVA_F_DHS_DX_CY),
                            c->D(DIVA_F_DHS_DY_CY)); c->launches++;
   DIVA_LAUNCHED(c, "k_stagger_slopes");
-  k_stagger3d<<<G2>>>(d, c->D(DIVA_F_A_FLOW_3D_A), c->D(DIVA_F_A_FLOW_3D_CX), c->D(DIVA_F_A_FLOW_3D_CY)); c->launches++;
+  k_stagger3d<<<G3>>>(d, c->D(DIVA_F_A_FLOW_3D_A), c->D(DIVA_F_A_FLOW_3D_CX), c->D(DIVA_F_A_FLOW_3D_CY)); c->launches++;
   DIVA_LAUNCHED(c, "k_stagger3d");
   return DIVA_OK;
 }
@@ -463,7 +480,7 @@ int launch_ice_rheology(Ctx* c) {
                      c->I(DIVA_F_MASK_ICE_A), c->I(DIVA_F_MASK_SHEET_A), c->I(DIVA_F_MASK_SHELF_A),
                      c->D(DIVA_F_A_FLOW_3D_A), c->D(DIVA_F_A_FLOW_VAV_A)); c->launches++;
   DIVA_LAUNCHED(c, "k_rheology");
-  k_stagger3d<<<G2>>>(c->d, c->D(DIVA_F_A_FLOW_3D_A), c->D(DIVA_F_A_FLOW_3D_CX), c->D(DIVA_F_A_FLOW_3D_CY)); c->launches++;
+  k_stagger3d<<<G3>>>(c->d, c->D(DIVA_F_A_FLOW_3D_A), c->D(DIVA_F_A_FLOW_3D_CX), c->D(DIVA_F_A_FLOW_3D_CY)); c->launches++;
   DIVA_LAUNCHED(c, "k_stagger3d");
   k_stagger2d<<<G2>>>(c->d, c->D(DIVA_F_A_FLOW_VAV_A), c->D(DIVA_F_A_FLOW_VAV_CX), c->D(DIVA_F_A_FLOW_VAV_CY)); c->launches++;
   DIVA_LAUNCHED(c, "k_stagger2d");

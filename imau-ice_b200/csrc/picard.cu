@@ -428,13 +428,13 @@ __global__ void __launch_bounds__(256) k_face_coefficients(FaceArgs a) {
 
 // 0.5 * A^(-1/n): constant over one solve, so the pow of A is taken once per solve
 __global__ void k_afac(Dims d, double n_flow, const double* A, double* afac) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y, k0 = blockIdx.z * kLayers;
   if (j >= d.ny || i >= d.nx) return;
-  const double e = -1.0 / n_flow;
-  for (int k = 0; k < d.nz; ++k) {
-    const long long o = (long long)k * d.plane + d.at(j, i);
-    afac[o] = 0.5 * pow(A[o], e);
-  }
+  const double p = -1.0 / n_flow;
+  const long long q = d.at(j, i);
+  double f[kLayers];
+  LOAD_LAYERS(e, k, k0, d.nz) f[e] = A[k * d.plane + q];
+  FOR_LAYERS(e, k0, d.nz) afac[(k0 + e) * d.plane + q] = 0.5 * pow(f[e], p);
 }
 
 // apply_velocity_limits (:1432-1498) of the linear solution at a cx point: |u| with v mapped
@@ -710,7 +710,7 @@ __global__ void k_relres_end(Dims d, int diva, int sliding_none, int basal_freez
 
 // visc_eff_3D_b of the last viscosity iteration (:820-858), written once per solve
 __global__ void k_visc_b(Dims d, int bc_margin, const double* visc, const int* mask_ice, double* vb) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y, k0 = blockIdx.z * kLayers;
   if (j >= d.ny - 1 || i >= d.nx - 1) return;
   const long long q = d.at(j, i), q1 = d.at(j, i + 1), q2 = d.at(j + 1, i), q3 = d.at(j + 1, i + 1);
   int m0 = 1, m1 = 1, m2 = 1, m3 = 1;
@@ -719,20 +719,24 @@ __global__ void k_visc_b(Dims d, int bc_margin, const double* visc, const int* m
     m0 = mask_ice[q] == 1; m1 = mask_ice[q1] == 1; m2 = mask_ice[q2] == 1; m3 = mask_ice[q3] == 1;
     w = (double)m0 + (double)m1 + (double)m2 + (double)m3;
   }
-  for (int k = 0; k < d.nz; ++k) {
-    const long long o = (long long)k * d.plane;
+  double f0[kLayers], f1[kLayers], f2[kLayers], f3[kLayers];
+  LOAD_LAYERS(e, k, k0, d.nz) {
+    const double* f = visc + k * d.plane;
+    f0[e] = f[q]; f1[e] = f[q1]; f2[e] = f[q2]; f3[e] = f[q3];
+  }
+  FOR_LAYERS(e, k0, d.nz) {
     double s;
     if (bc_margin) {
       s = 0.0;
-      if (m0) s = s + visc[o + q];
-      if (m1) s = s + visc[o + q1];
-      if (m2) s = s + visc[o + q2];
-      if (m3) s = s + visc[o + q3];
+      if (m0) s = s + f0[e];
+      if (m1) s = s + f1[e];
+      if (m2) s = s + f2[e];
+      if (m3) s = s + f3[e];
       if (w > 0.0) s = s / w;
     } else {
-      s = (visc[o + q] + visc[o + q1] + visc[o + q2] + visc[o + q3]) / 4.0;
+      s = (f0[e] + f1[e] + f2[e] + f3[e]) / 4.0;
     }
-    vb[o + q] = s;
+    vb[(k0 + e) * d.plane + q] = s;
   }
 }
 
@@ -743,58 +747,45 @@ __global__ void k_f1(Dims d, Zeta zt, const double* Hi, const double* visc, doub
   const long long q = d.at(j, i);
   const double H = Hi[q];
   const int nz = d.nz;
-  double acc = 0.0;
-  double fk1 = (-H / visc[(long long)(nz - 1) * d.plane + q]) * zt.z[nz - 1];
-  F1[(long long)(nz - 1) * d.plane + q] = 0.0;
-  for (int k = nz - 2; k >= 0; --k) {
-    const double fk = (-H / visc[(long long)k * d.plane + q]) * zt.z[k];
-    acc = acc - 0.5 * (fk1 + fk) * (zt.z[k + 1] - zt.z[k]);
-    F1[(long long)k * d.plane + q] = acc;
-    fk1 = fk;
+  double acc = 0.0, fk1 = 0.0;
+  for (int k0 = 0; k0 < nz; k0 += kLayers) {   // from the base up
+    double f[kLayers];
+    LOAD_LAYERS(e, k, k0, nz) f[e] = visc[(nz - 1 - k) * d.plane + q];
+    FOR_LAYERS(e, k0, nz) {
+      const int k = nz - 1 - k0 - e;
+      const double fk = (-H / f[e]) * zt.z[k];
+      if (k < nz - 1) acc = acc - 0.5 * (fk1 + fk) * (zt.z[k + 1] - zt.z[k]);
+      F1[(long long)k * d.plane + q] = acc;
+      fk1 = fk;
+    }
   }
 }
 
 // u_3D = u_base + taub * F1_stag (:1229-1289)
 __global__ void k_u3d(Dims d, int bc_margin, const double* Hi, const double* F1, const double* ubx, const double* vby,
                       const double* tbx, const double* tby, double* u3, double* v3) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y, k0 = blockIdx.z * kLayers;
   if (j >= d.ny || i >= d.nx) return;
   const long long q = d.at(j, i);
-  if (i < d.nx - 1) {
-    const long long q1 = d.at(j, i + 1);
-    const double H0 = Hi[q], H1 = Hi[q1];
-    for (int k = 0; k < d.nz; ++k) {
-      const long long o = (long long)k * d.plane;
-      const double f0 = F1[o + q], f1 = F1[o + q1];
-      double s;
-      if (bc_margin) {
-        if (H0 > 0.0 && H1 == 0.0) s = f0;
-        else if (H0 == 0.0 && H1 > 0.0) s = f1;
-        else if (H0 > 0.0 && H1 > 0.0) s = 0.5 * (f0 + f1);
-        else s = 0.0;
-      } else {
-        s = 0.5 * (f0 + f1);
-      }
-      u3[o + q] = ubx[q] + tbx[q] * s;
-    }
+  const bool cx = i < d.nx - 1, cy = j < d.ny - 1;
+  const double H0 = Hi[q], He = cx ? Hi[q + d.ld] : 0.0, Hn = cy ? Hi[q + 1] : 0.0;
+  const double ub = cx ? ubx[q] : 0.0, tx = cx ? tbx[q] : 0.0, vb = cy ? vby[q] : 0.0, ty = cy ? tby[q] : 0.0;
+  const long long qe = cx ? q + d.ld : q, qn = cy ? q + 1 : q;
+  double f[kLayers], fe[kLayers], fn[kLayers];
+  LOAD_LAYERS(e, k, k0, d.nz) {
+    const double* F = F1 + k * d.plane;
+    f[e] = F[q]; fe[e] = F[qe]; fn[e] = F[qn];
   }
-  if (j < d.ny - 1) {
-    const long long q1 = d.at(j + 1, i);
-    const double H0 = Hi[q], H1 = Hi[q1];
-    for (int k = 0; k < d.nz; ++k) {
-      const long long o = (long long)k * d.plane;
-      const double f0 = F1[o + q], f1 = F1[o + q1];
-      double s;
-      if (bc_margin) {
-        if (H0 > 0.0 && H1 == 0.0) s = f0;
-        else if (H0 == 0.0 && H1 > 0.0) s = f1;
-        else if (H0 > 0.0 && H1 > 0.0) s = 0.5 * (f0 + f1);
-        else s = 0.0;
-      } else {
-        s = 0.5 * (f0 + f1);
-      }
-      v3[o + q] = vby[q] + tby[q] * s;
-    }
+  auto staggered = [&](double H1, double f0, double f1) {
+    if (!bc_margin) return 0.5 * (f0 + f1);
+    if (H0 > 0.0 && H1 == 0.0) return f0;
+    if (H0 == 0.0 && H1 > 0.0) return f1;
+    return H0 > 0.0 && H1 > 0.0 ? 0.5 * (f0 + f1) : 0.0;
+  };
+  FOR_LAYERS(e, k0, d.nz) {
+    const long long o = (k0 + e) * d.plane + q;
+    if (cx) u3[o] = ub + tx * staggered(He, f[e], fe[e]);
+    if (cy) v3[o] = vb + ty * staggered(Hn, f[e], fn[e]);
   }
 }
 
@@ -815,67 +806,71 @@ __global__ void k_faces_prelude(Dims d, Zeta zt, int dyn, double* u3, double* v3
     double* base = face == 0 ? ub : vb;
     double* surf = face == 0 ? us : vs;
     double* vav = face == 0 ? uv : vv;
-    if (dyn == DIVA_DYN_SIA) {
-      for (int k = 0; k < d.nz; ++k) f3[(long long)k * d.plane + q] = s3[(long long)k * d.plane + q];
-      base[q] = 0.0;
-    } else if (dyn == DIVA_DYN_SSA) {
-      base[q] = sS;
-      vav[q] = sS;
-      for (int k = 0; k < d.nz; ++k) f3[(long long)k * d.plane + q] = sS;
-    } else if (dyn == DIVA_DYN_SIA_SSA) {
-      for (int k = 0; k < d.nz; ++k) f3[(long long)k * d.plane + q] = s3[(long long)k * d.plane + q] + sS;
-      base[q] = sS;
+    // the layers this face has: its own, or made here
+    const bool own = dyn != DIVA_DYN_SIA && dyn != DIVA_DYN_SSA && dyn != DIVA_DYN_SIA_SSA;
+    const bool mean = dyn == DIVA_DYN_SIA || dyn == DIVA_DYN_SIA_SSA;
+    if (own) {
+      surf[q] = f3[q];
+      continue;
     }
-    surf[q] = f3[q];
-    if (dyn == DIVA_DYN_SIA || dyn == DIVA_DYN_SIA_SSA) {
-      double avg = 0.0;
-      for (int k = 0; k < d.nz - 1; ++k)
-        avg = avg + 0.5 * (f3[(long long)(k + 1) * d.plane + q] + f3[(long long)k * d.plane + q]) *
-                        (zt.z[k + 1] - zt.z[k]);
-      vav[q] = avg;
+    base[q] = dyn == DIVA_DYN_SIA ? 0.0 : sS;
+    if (dyn == DIVA_DYN_SSA) vav[q] = sS;
+    double avg = 0.0, prev = 0.0;
+    for (int k0 = 0; k0 < d.nz; k0 += kLayers) {
+      double f[kLayers];
+      LOAD_LAYERS(e, k, k0, d.nz) f[e] = dyn == DIVA_DYN_SSA ? sS : s3[k * d.plane + q];
+      FOR_LAYERS(e, k0, d.nz) {
+        const int k = k0 + e;
+        if (dyn == DIVA_DYN_SIA_SSA) f[e] = f[e] + sS;
+        f3[k * d.plane + q] = f[e];
+        if (k == 0) surf[q] = f[e];
+        else avg = avg + 0.5 * (f[e] + prev) * (zt.z[k] - zt.z[k - 1]);
+        prev = f[e];
+      }
     }
+    if (mean) vav[q] = avg;
   }
 }
 
 struct SecArgs {
   Dims d;
   Zeta zt;
-  int dyn, do_w;
+  int dyn;
   const double *u3, *v3, *Hs, *Hi, *dHs_dx, *dHs_dy, *dHi_dx, *dHi_dy, *dHb_dt;
   const double *uv, *vv, *us, *vs, *ub, *vb;
   const int *sheet, *ice;
   double *w, *ws, *wb, *u3a, *v3a, *uva, *vva, *usa, *vsa, *uba, *vba, *abv, *abs_, *abb, *Rs;
 };
 
-// map_velocity_from_cx_to_a (:2592-2701) for one value, mask_ice along x
-__device__ __forceinline__ double map_cx_a(const Dims& d, const int* ice, const double* f, long long off, int j, int i) {
-  if (i == 0) return ice[d.at(j, 0)] == 1 ? f[off + d.at(j, 0)] : 0.0;
-  if (i == d.nx - 1) return ice[d.at(j, i)] == 1 ? f[off + d.at(j, i - 1)] : 0.0;
-  const int m0 = ice[d.at(j, i - 1)], m1 = ice[d.at(j, i)], m2 = ice[d.at(j, i + 1)];
-  if (m0 == 1 && m1 == 1 && m2 == 1) return 0.5 * (f[off + d.at(j, i - 1)] + f[off + d.at(j, i)]);
-  if (m0 == 0 && m1 == 1 && m2 == 1) return f[off + d.at(j, i)];
-  if (m0 == 1 && m1 == 1 && m2 == 0) return f[off + d.at(j, i - 1)];
-  return 0.0;
+// map_velocity_from_cx_to_a, ..cy_to_a (:2592-2811) at a point: which of the two neighbouring
+// faces its value comes from, by the ice mask along the direction: 0 none, 1 the first (west or
+// south), 2 the second, 3 their mean.  At the grid's ends the one face there is: the first of
+// the pair (0, 1) at the start, the second of the last pair at the end.
+__device__ __forceinline__ int map_mode(const int* ice, long long q, long long step, bool start, bool end) {
+  const bool m1 = ice[q] == 1;
+  const int m0 = ice[start ? q : q - step], m2 = ice[end ? q : q + step];
+  if (!m1) return 0;
+  if (start) return 1;
+  if (end) return 2;
+  if (m0 == 1) return m2 == 1 ? 3 : (m2 == 0 ? 1 : 0);
+  return m0 == 0 && m2 == 1 ? 2 : 0;
 }
-// map_velocity_from_cy_to_a (:2702-2811), mask_ice along y
-__device__ __forceinline__ double map_cy_a(const Dims& d, const int* ice, const double* f, long long off, int j, int i) {
-  if (j == 0) return ice[d.at(0, i)] == 1 ? f[off + d.at(0, i)] : 0.0;
-  if (j == d.ny - 1) return ice[d.at(j, i)] == 1 ? f[off + d.at(j - 1, i)] : 0.0;
-  const int m0 = ice[d.at(j - 1, i)], m1 = ice[d.at(j, i)], m2 = ice[d.at(j + 1, i)];
-  if (m0 == 1 && m1 == 1 && m2 == 1) return 0.5 * (f[off + d.at(j - 1, i)] + f[off + d.at(j, i)]);
-  if (m0 == 0 && m1 == 1 && m2 == 1) return f[off + d.at(j, i)];
-  if (m0 == 1 && m1 == 1 && m2 == 0) return f[off + d.at(j - 1, i)];
-  return 0.0;
+__device__ __forceinline__ double map_faces(int mode, double f0, double f1) {
+  return mode == 3 ? 0.5 * (f0 + f1) : mode == 2 ? f1 : mode == 1 ? f0 : 0.0;
 }
 
-__global__ void __launch_bounds__(256) k_secondary(SecArgs a) {
+// W: the vertical velocities too (not in SSA).  Bound by memory: with them five 3D fields are read
+// and three written.
+template <bool W>
+__global__ void __launch_bounds__(256, 2) k_secondary(SecArgs a) {
   const Dims d = a.d;
   const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
   if (j >= d.ny || i >= d.nx) return;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const long long q = d.at(j, i), P = d.plane;
   const double dx = d.dx;
-  if (a.do_w) {
+  double dHbase_dx = 0.0, dHbase_dy = 0.0;
+  if (W) {
     // calc_3D_vertical_velocities :562-650; surface/thickness slopes recomputed from Hs, Hi (:563-566)
     auto A = [&](const double* f, int jj, int ii) { return f[d.at(jj, ii)]; };
     double sx, sy, hx, hy;
@@ -885,52 +880,59 @@ __global__ void __launch_bounds__(256) k_secondary(SecArgs a) {
     if (j > 0 && j < ny - 1) { sy = (A(a.Hs, j + 1, i) - A(a.Hs, j - 1, i)) / (2 * dx); hy = (A(a.Hi, j + 1, i) - A(a.Hi, j - 1, i)) / (2 * dx); }
     else if (j == 0) { sy = (A(a.Hs, 1, i) - A(a.Hs, 0, i)) / dx; hy = (A(a.Hi, 1, i) - A(a.Hi, 0, i)) / dx; }
     else { sy = (A(a.Hs, ny - 1, i) - A(a.Hs, ny - 2, i)) / dx; hy = (A(a.Hi, ny - 1, i) - A(a.Hi, ny - 2, i)) / dx; }
-    const double dHbase_dx = sx - hx, dHbase_dy = sy - hy;
-    const long long ob = (long long)(nz - 1) * P;
-    double ubase, vbase;
-    if (i == 0) ubase = a.u3[ob + d.at(j, 0)];
-    else if (i == nx - 1) ubase = a.u3[ob + d.at(j, nx - 2)];
-    else ubase = 0.5 * (a.u3[ob + d.at(j, i - 1)] + a.u3[ob + d.at(j, i)]);
-    if (j == 0) vbase = a.v3[ob + d.at(0, i)];
-    else if (j == ny - 1) vbase = a.v3[ob + d.at(ny - 2, i)];
-    else vbase = 0.5 * (a.v3[ob + d.at(j - 1, i)] + a.v3[ob + d.at(j, i)]);
-    double wk1 = (ubase * dHbase_dx) + (vbase * dHbase_dy);
-    if (a.sheet[q] == 1) wk1 = wk1 + a.dHb_dt[q];
-    a.w[ob + q] = wk1;
-    // x and y index pairs of the divergence stencil (:603-622)
-    const int ia = (i == 0) ? 1 : (i == nx - 1 ? nx - 2 : i), ib = ia - 1;
-    const int ja = (j == 0) ? 1 : (j == ny - 1 ? ny - 2 : j), jb = ja - 1;
-    const double H = a.Hi[q], Hm = max_ref(0.1, H);
-    const double gsx = a.dHs_dx[q], gsy = a.dHs_dy[q], gix = a.dHi_dx[q], giy = a.dHi_dy[q];
-    double du_kp1 = (a.u3[ob + d.at(j, ia)] - a.u3[ob + d.at(j, ib)]) / dx;
-    double dv_kp1 = (a.v3[ob + d.at(ja, i)] - a.v3[ob + d.at(jb, i)]) / dx;
-    double ua_kp1 = a.u3a[ob + q], va_kp1 = a.v3a[ob + q];   // stale a-grid velocities (read before refresh)
-    for (int k = nz - 2; k >= 0; --k) {
-      const long long o = (long long)k * P;
-      const double du_k = (a.u3[o + d.at(j, ia)] - a.u3[o + d.at(j, ib)]) / dx;
-      const double dv_k = (a.v3[o + d.at(ja, i)] - a.v3[o + d.at(jb, i)]) / dx;
-      const double ua_k = a.u3a[o + q], va_k = a.v3a[o + q];
-      const double w1 = (du_k + du_kp1) / 2.0, w2 = (dv_k + dv_kp1) / 2.0;
-      const double dz = a.zt.z[k + 1] - a.zt.z[k], zm = 0.5 * (a.zt.z[k + 1] + a.zt.z[k]);
-      const double w3 = ((gsx - zm * gix) / Hm) * ((ua_kp1 - ua_k) / dz);
-      const double w4 = ((gsy - zm * giy) / Hm) * ((va_kp1 - va_k) / dz);
-      const double wk = wk1 - H * (w1 + w2 + w3 + w4) * dz;
-      a.w[o + q] = wk;
-      wk1 = wk;
-      du_kp1 = du_k; dv_kp1 = dv_k; ua_kp1 = ua_k; va_kp1 = va_k;
+    dHbase_dx = sx - hx;
+    dHbase_dy = sy - hy;
+  }
+  // the faces of the divergence stencil in x and y (:603-622), which the a-grid maps read as well
+  const int ia = (i == 0) ? 1 : (i == nx - 1 ? nx - 2 : i), ja = (j == 0) ? 1 : (j == ny - 1 ? ny - 2 : j);
+  const long long qe = d.at(j, ia), qw = d.at(j, ia - 1), qn = d.at(ja, i), qs = d.at(ja - 1, i);
+  const int mx = map_mode(a.ice, q, d.ld, i == 0, i == nx - 1), my = map_mode(a.ice, q, 1, j == 0, j == ny - 1);
+  double Hdx = 0.0, Hr = 0.0, gsx = 0.0, gsy = 0.0, gix = 0.0, giy = 0.0;
+  if (W) {
+    const double H = a.Hi[q];
+    Hdx = H / (2.0 * dx); Hr = H / max_ref(0.1, H);
+    gsx = a.dHs_dx[q]; gsy = a.dHs_dy[q]; gix = a.dHi_dx[q]; giy = a.dHi_dy[q];
+  }
+  // From the base up; a layer's a-grid velocities are read (stale) for w before they are replaced.
+  // w_k = w_k+1 - H ((du/dx + dv/dy) + (dHs/dx - zm dHi/dx) / H du/dz + ..) dz with the means of
+  // both layers, dx, H and dz taken out of the sums: no division in a layer (six cost 500
+  // instructions a layer, 3/4 of the kernel).
+  double wk1 = 0.0, div_kp1 = 0.0, ua_kp1 = 0.0, va_kp1 = 0.0;
+  for (int k0 = 0; k0 < nz; k0 += kLayers) {
+    double ue[kLayers], uw[kLayers], vn[kLayers], vs[kLayers], ua[kLayers], va[kLayers];
+    LOAD_LAYERS(e, kb, k0, nz) {
+      const long long o = (nz - 1 - kb) * P;
+      ue[e] = a.u3[o + qe]; uw[e] = a.u3[o + qw]; vn[e] = a.v3[o + qn]; vs[e] = a.v3[o + qs];
+      if (W) { ua[e] = a.u3a[o + q]; va[e] = a.v3a[o + q]; }
     }
-    a.ws[q] = a.w[q];
-    a.wb[q] = a.w[ob + q];
+    FOR_LAYERS(e, k0, nz) {
+      const int k = nz - 1 - k0 - e;
+      const long long o = k * P;
+      if (W) {
+        const double div = (ue[e] - uw[e]) + (vn[e] - vs[e]);
+        if (k == nz - 1) {
+          const double ubase = i == 0 ? uw[e] : i == nx - 1 ? ue[e] : 0.5 * (uw[e] + ue[e]);
+          const double vbase = j == 0 ? vs[e] : j == ny - 1 ? vn[e] : 0.5 * (vs[e] + vn[e]);
+          wk1 = (ubase * dHbase_dx) + (vbase * dHbase_dy);
+          if (a.sheet[q] == 1) wk1 = wk1 + a.dHb_dt[q];
+          a.wb[q] = wk1;
+        } else {
+          const double dz = a.zt.z[k + 1] - a.zt.z[k], zm = 0.5 * (a.zt.z[k + 1] + a.zt.z[k]);
+          const double tilt = (gsx - zm * gix) * (ua_kp1 - ua[e]) + (gsy - zm * giy) * (va_kp1 - va[e]);
+          wk1 = wk1 - (Hdx * dz * (div + div_kp1) + Hr * tilt);
+        }
+        a.w[o + q] = wk1;
+        if (k == 0) a.ws[q] = wk1;
+        div_kp1 = div; ua_kp1 = ua[e]; va_kp1 = va[e];
+      }
+      a.u3a[o + q] = map_faces(mx, uw[e], ue[e]);
+      a.v3a[o + q] = map_faces(my, vs[e], vn[e]);
+    }
   }
-  // a-grid maps of the 3D field (own column only: safe after the stale reads above)
-  for (int k = 0; k < nz; ++k) {
-    const long long o = (long long)k * P;
-    a.u3a[o + q] = map_cx_a(d, a.ice, a.u3, o, j, i);
-    a.v3a[o + q] = map_cy_a(d, a.ice, a.v3, o, j, i);
-  }
-  const double uva = map_cx_a(d, a.ice, a.uv, 0, j, i), vva = map_cy_a(d, a.ice, a.vv, 0, j, i);
-  const double usa = map_cx_a(d, a.ice, a.us, 0, j, i), vsa = map_cy_a(d, a.ice, a.vs, 0, j, i);
-  const double uba = map_cx_a(d, a.ice, a.ub, 0, j, i), vba = map_cy_a(d, a.ice, a.vb, 0, j, i);
+  auto map_x = [&](const double* f) { return map_faces(mx, f[qw], f[qe]); };
+  auto map_y = [&](const double* f) { return map_faces(my, f[qs], f[qn]); };
+  const double uva = map_x(a.uv), vva = map_y(a.vv), usa = map_x(a.us), vsa = map_y(a.vs);
+  const double uba = map_x(a.ub), vba = map_y(a.vb);
   a.uva[q] = uva; a.vva[q] = vva; a.usa[q] = usa; a.vsa[q] = vsa; a.uba[q] = uba; a.vba[q] = vba;
   const double av = sqrt(uva * uva + vva * vva), as = sqrt(usa * usa + vsa * vsa), ab = sqrt(uba * uba + vba * vba);
   a.abv[q] = av; a.abs_[q] = as; a.abb[q] = ab;
@@ -964,13 +966,17 @@ __global__ void k_sia(Dims d, Zeta zt, double n, const int* sheet, const double*
     const double slope = face == 0 ? sx : sy;
     const double D0 = pow(kRhoI * kGrav * H, n) * pow((sx * sx + sy * sy), (n - 1.0) / 2.0);
     // D(zeta) = 2 H int_base^zeta A zeta^n (vertical_integration_from_bottom_to_zeta)
-    double acc = 0.0, fk1 = A[(long long)(nz - 1) * P + q] * zt.zn[nz - 1];
-    out[(long long)(nz - 1) * P + q] = max_ref(D0 * (2.0 * H * 0.0), -1E5) * slope;
-    for (int k = nz - 2; k >= 0; --k) {
-      const double fk = A[(long long)k * P + q] * zt.zn[k];
-      acc = acc - 0.5 * (fk1 + fk) * (zt.z[k + 1] - zt.z[k]);
-      out[(long long)k * P + q] = max_ref(D0 * (2.0 * H * acc), -1E5) * slope;
-      fk1 = fk;
+    double acc = 0.0, fk1 = 0.0;
+    for (int k0 = 0; k0 < nz; k0 += kLayers) {   // from the base up
+      double f[kLayers];
+      LOAD_LAYERS(e, k, k0, nz) f[e] = A[(nz - 1 - k) * P + q];
+      FOR_LAYERS(e, k0, nz) {
+        const int k = nz - 1 - k0 - e;
+        const double fk = f[e] * zt.zn[k];
+        if (k < nz - 1) acc = acc - 0.5 * (fk1 + fk) * (zt.z[k + 1] - zt.z[k]);
+        out[k * P + q] = max_ref(D0 * (2.0 * H * acc), -1E5) * slope;
+        fk1 = fk;
+      }
     }
   }
 }
@@ -991,6 +997,7 @@ __global__ void k_zero_uv(Dims d, double* u, double* v) {
 }  // namespace
 
 #define G2 grid2d(c->d.ny, c->d.nx), block2d(), 0, c->stream
+#define G3 grid_layers(c->d.ny, c->d.nx, c->d.nz), block2d(), 0, c->stream
 
 // Whether K1 computes the viscosity of the linearisation in FP32 (precision 'mixed').
 #ifndef DIVA_K1_FP32
@@ -999,7 +1006,7 @@ __global__ void k_zero_uv(Dims d, double* u, double* v) {
 static bool k1_fp32(const diva_config_t& C) { return DIVA_K1_FP32 && C.precision == DIVA_PREC_MIXED; }
 
 int launch_prepare_afac(Ctx* c) {
-  k_afac<<<G2>>>(c->d, c->c.n_flow, c->D(DIVA_F_A_FLOW_3D_A), c->afac); c->launches++;
+  k_afac<<<G3>>>(c->d, c->c.n_flow, c->D(DIVA_F_A_FLOW_3D_A), c->afac); c->launches++;
   DIVA_LAUNCHED(c, "k_afac");
   return DIVA_OK;
 }
@@ -1220,7 +1227,7 @@ int launch_visc_b_output(Ctx* c) {
   // the shear strain rates the last viscosity iteration's K1 saw (the loop does not write them)
   int st;
   if ((st = launch_shear_rates(c))) return st;
-  k_visc_b<<<G2>>>(c->d, c->c.choice_ice_margin == DIVA_MARGIN_BC, c->D(DIVA_F_VISC_EFF_3D_A),
+  k_visc_b<<<G3>>>(c->d, c->c.choice_ice_margin == DIVA_MARGIN_BC, c->D(DIVA_F_VISC_EFF_3D_A),
                    c->I(DIVA_F_MASK_ICE_A), c->D(DIVA_F_VISC_EFF_3D_B)); c->launches++;
   DIVA_LAUNCHED(c, "k_visc_b");
   return DIVA_OK;
@@ -1229,7 +1236,7 @@ int launch_visc_b_output(Ctx* c) {
 int launch_3d_horizontal_velocities(Ctx* c) {
   k_f1<<<G2>>>(c->d, c->zt, c->D(DIVA_F_HI_A), c->D(DIVA_F_VISC_EFF_3D_A), c->D(DIVA_F_F1_3D_A)); c->launches++;
   DIVA_LAUNCHED(c, "k_f1");
-  k_u3d<<<G2>>>(c->d, c->c.choice_ice_margin == DIVA_MARGIN_BC, c->D(DIVA_F_HI_A), c->D(DIVA_F_F1_3D_A),
+  k_u3d<<<G3>>>(c->d, c->c.choice_ice_margin == DIVA_MARGIN_BC, c->D(DIVA_F_HI_A), c->D(DIVA_F_F1_3D_A),
                 c->D(DIVA_F_U_BASE_CX), c->D(DIVA_F_V_BASE_CY), c->D(DIVA_F_TAUB_CX), c->D(DIVA_F_TAUB_CY),
                 c->D(DIVA_F_U_3D_CX), c->D(DIVA_F_V_3D_CY)); c->launches++;
   DIVA_LAUNCHED(c, "k_u3d");
@@ -1244,7 +1251,7 @@ int launch_secondary_velocities(Ctx* c) {
                           c->D(DIVA_F_V_SURF_CY), c->D(DIVA_F_U_VAV_CX), c->D(DIVA_F_V_VAV_CY)); c->launches++;
   DIVA_LAUNCHED(c, "k_faces_prelude");
   SecArgs a{};
-  a.d = c->d; a.zt = c->zt; a.dyn = dyn; a.do_w = dyn != DIVA_DYN_SSA;
+  a.d = c->d; a.zt = c->zt; a.dyn = dyn;
   a.u3 = c->D(DIVA_F_U_3D_CX); a.v3 = c->D(DIVA_F_V_3D_CY); a.Hs = c->D(DIVA_F_HS_A); a.Hi = c->D(DIVA_F_HI_A);
   a.dHs_dx = c->D(DIVA_F_DHS_DX_A); a.dHs_dy = c->D(DIVA_F_DHS_DY_A);
   a.dHi_dx = c->D(DIVA_F_DHI_DX_A); a.dHi_dy = c->D(DIVA_F_DHI_DY_A); a.dHb_dt = c->D(DIVA_F_DHB_DT_A);
@@ -1257,7 +1264,9 @@ int launch_secondary_velocities(Ctx* c) {
   a.vsa = c->D(DIVA_F_V_SURF_A); a.uba = c->D(DIVA_F_U_BASE_A); a.vba = c->D(DIVA_F_V_BASE_A);
   a.abv = c->D(DIVA_F_UABS_VAV_A); a.abs_ = c->D(DIVA_F_UABS_SURF_A); a.abb = c->D(DIVA_F_UABS_BASE_A);
   a.Rs = c->D(DIVA_F_R_SHEAR);
-  k_secondary<<<G2>>>(a); c->launches++;
+  if (dyn != DIVA_DYN_SSA) k_secondary<true><<<G2>>>(a);
+  else k_secondary<false><<<G2>>>(a);
+  c->launches++;
   DIVA_LAUNCHED(c, "k_secondary");
   return DIVA_OK;
 }
