@@ -29,6 +29,7 @@
 // results are bit-reproducible from run to run.
 #include <cmath>
 #include <cstdio>
+#include <algorithm>
 #include <utility>
 #include <vector>
 #include "ctx.hpp"
@@ -365,13 +366,13 @@ __global__ void k_residual(Op o, const double* xu, const double* xv, const doubl
 // along that direction (f2 = 1).  The taps are formed in registers, one at a time, and
 // summed with explicit fused multiply-adds (the weights' products are exact), so every
 // kernel that restricts or prolongs rounds alike.
-__device__ __forceinline__ int gather_cell_n(int f2) { return f2 == 1 ? 1 : 4; }
-__device__ __forceinline__ int gather_node_n(int f2) { return f2 == 1 ? 1 : 3; }
-__device__ __forceinline__ void gather_cell(int C, int f2, int k, int& f, double& w) {
+__host__ __device__ __forceinline__ int gather_cell_n(int f2) { return f2 == 1 ? 1 : 4; }
+__host__ __device__ __forceinline__ int gather_node_n(int f2) { return f2 == 1 ? 1 : 3; }
+__host__ __device__ __forceinline__ void gather_cell(int C, int f2, int k, int& f, double& w) {
   if (f2 == 1) { f = C; w = 1.0; return; }
   f = 2 * C - 1 + k; w = (k == 0 || k == 3) ? 0.25 : 0.75;
 }
-__device__ __forceinline__ void gather_node(int C, int f2, int k, int& f, double& w) {
+__host__ __device__ __forceinline__ void gather_node(int C, int f2, int k, int& f, double& w) {
   if (f2 == 1) { f = C; w = 1.0; return; }
   f = 2 * C - 1 + k; w = k == 1 ? 1.0 : 0.5;
 }
@@ -1346,15 +1347,11 @@ __global__ void k_restrict_b(Dims df, Dims dc, int fx, int fy, const double* ru,
 struct CoarseMap {
   int ny, nu, nv;
   __host__ __device__ __forceinline__ int n() const { return nu + nv; }
-  __device__ __forceinline__ void point(int r, int& comp, int& j, int& i) const {
-    if (r < nu) { comp = 0; i = 1 + r / (ny - 2); j = 1 + r % (ny - 2); }
-    else { const int q = r - nu; comp = 1; i = 1 + q / (ny - 3); j = 1 + q % (ny - 3); }
-  }
 };
 
 // Assembly and inversion of the coarsest level's matrix by one block.  tab is the level's
-// row table (kTabCols columns of R = n rows: plane position, 4 same-component and 4
-// cross-component mapped reads; the zero element P = nx*ny stands for 'zero' sides).
+// row table (of R = n rows: 4 same-component and 4 cross-component mapped reads of each, then
+// their own positions; the zero element P = nx*ny stands for 'zero' sides).
 // Gauss-Jordan step k maps the matrix of step k-1 (buffer k&1) to the next one in one
 // pass with one barrier: every warp finds the pivot row p of column k itself, and every
 // element takes its value from the old matrix with rows k and p exchanged.
@@ -1378,9 +1375,9 @@ __device__ __forceinline__ void coarse_setup_block(const Op& o, const CoarseMap&
     return ucomp ? (i - 1) * (ny - 2) + (j - 1) : m.nu + (i - 1) * (ny - 3) + (j - 1);
   };
   for (int r = tid; r < n; r += blockDim.x) {
-    const int pos = tab[r], i = pos / ny, j = pos % ny;
+    const int pos = tab[8 * n + r], i = pos / ny, j = pos % ny;   // (tab_pos)
     int src[8];
-    for (int t = 0; t < 8; ++t) src[t] = tab[(1 + t) * n + r];
+    for (int t = 0; t < 8; ++t) src[t] = tab[8 * r + t];
     double cf[9];
     if (r < m.nu) {
       const double Ae = o.Na[d.at(j, i + 1)], Aw = o.Na[d.at(j, i)], Bn = o.Nb[d.at(j, i)], Bs = o.Nb[d.at(j - 1, i)];
@@ -1470,58 +1467,50 @@ __device__ __forceinline__ void coarse_setup_block(const Op& o, const CoarseMap&
 }
 
 
-// x = Ainv b on the coarsest level, by one block (the caller synchronises).  The descent
-// enters the coarsest level with x = 0, so its residual is b itself.  AinvT is the
-// inverse transposed (AinvT[c * n + r] = Ainv[r][c]), in shared memory, so the threads of
-// a warp read consecutive elements; the sums run over c in ascending order.
-__device__ __forceinline__ void block_coarse_direct(const Op& o, const CoarseMap& m, const double* AinvT, double* xu,
-                                                    double* xv, const double* bu, const double* bv) {
-  __shared__ double sr[kCoarseDirectMax];
-  const int n = m.n();
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
-    int comp, j, i;
-    m.point(r, comp, j, i);
-    const long long q = o.d.at(j, i);
-    sr[r] = comp == 0 ? bu[q] : bv[q];
-  }
-  __syncthreads();
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
-    double s = 0.0;
-    for (int c = 0; c < n; ++c) s += AinvT[c * n + r] * sr[c];
-    int comp, j, i;
-    m.point(r, comp, j, i);
-    (comp == 0 ? xu : xv)[o.d.at(j, i)] = s;
-  }
-}
-
-// The levels from `first` down, run by one thread block out of shared memory with
-// barriers between the phases: the same per-point operations in the same order
-// as the per-level kernels of vcycle(), without a launch per phase and without a
-// global-memory round trip per phase.  Each level keeps kSubArrays compact planes
-// (row length ny, one extra element that stays 0) in the block's dynamic shared
-// memory; the coefficients of every level and b of the first are staged in at the
-// start, x of the first level is written back at the end.
+// The levels from `first` down, run by one thread block out of shared memory with barriers
+// between the phases (colour passes, residual, transfers), without a launch and a global-memory
+// round trip per phase.  Each level keeps kSubArrays compact planes (row length ny, one extra
+// element that stays 0) in the block's dynamic shared memory; the coefficients of every level
+// are copied in at the start, x of the first level is written back at the end.
 //
-// The Gauss-Seidel passes and residuals run from row tables built once on the host
-// (they depend on the grid and the boundary conditions only): for each level the
-// interior rows grouped by (component, colour), each with its plane position and the
-// positions its eight off-diagonal stencil reads map to (boundary unknowns resolved
-// to their sources, 'zero' sides to the zero element).  A row update is then table
-// reads and the operator's arithmetic, without per-read boundary logic.
-enum { SA_NA, SA_NB, SA_BX, SA_BY, SA_IDU, SA_IDV, SA_XU, SA_XV, SA_BU, SA_BV, SA_RU, SA_RV, kSubArrays };
-constexpr size_t kSubSmemBudget = 200 * 1024;   // dynamic shared memory of the sub-cycle
-constexpr int kTabCols = 9;                      // a row's position and its eight mapped reads
-constexpr int kTabProlong = 4;                   // then the row's prolongation taps (coarse positions)
+// Bound by the latency of a phase, not by its points (a coarse level has a handful), so a phase
+// keeps only what depends on the phase before it.  The interior rows of a level are grouped by
+// (component, colour); a quarter of the block (kSubQuarter threads) belongs to each of the four
+// groups.  On the levels of at most kSubQuarter rows a group a thread has one row ("resident"):
+// it loads the row's coefficients, its neighbours' addresses and b when it comes to the level,
+// ahead of the passes that need them, and a pass is nine reads of x, three chains of three
+// multiply-adds and a write; the levels' phases are separated by named barriers of the threads
+// that have rows there, while the others wait at the level above.  Larger levels load a row's
+// operands in the pass, every thread on every class.  (With every thread at every barrier and
+// all operands loaded in every pass, a pass over three rows a group took 650 cycles, now 400;
+// the kernel 27.3 -> 22.7 us from 65 x 9 points, 30 -> 24.7 us from 40 x 23.  Launching the next
+// kernel ahead of the end of the last saved 0.2 us a launch in a graph, not worth its waits.)
+//
+// The row tables are built once on the host (they depend on the grid and the boundary
+// conditions only), per level of R rows: the positions of each row's eight off-diagonal reads
+// (boundary unknowns resolved to their sources, 'zero' sides to the zero element), its own
+// position, its prolongation taps from the next level and, below the first level, its
+// restriction taps from the level above, each a position and a weight in sixteenths.
+enum { SA_NA, SA_NB, SA_BX, SA_BY, SA_IDU, SA_IDV, SA_XU, SA_XV, SA_BU, SA_BV, kSubArrays };
+constexpr size_t kSubSmemBudget = 200 * 1024;   // of a level and those below it (sub_bytes)
+constexpr size_t kSubSmemMax = 224 * 1024;      // with the restriction taps and the residual
+constexpr int kSubQuarter = kSubThreads / 4;
+constexpr int kTabReads = 8, kTabProlong = 4, kTabRestrict = 12;   // entries per row
+constexpr int kTapBits = 12;   // a tap: position, and above it 16 x weight - 1
+// where a level's blocks of the table start: reads, positions (padded to 4), prolongation, restriction
+__host__ __device__ __forceinline__ int tab_pos(int R) { return kTabReads * R; }
+__host__ __device__ __forceinline__ int tab_prolong(int R) { return tab_pos(R) + (R + 3) / 4 * 4; }
+__host__ __device__ __forceinline__ int tab_restrict(int R) { return tab_prolong(R) + kTabProlong * R; }
 
 struct SubLevel {
   Op o;                      // global-memory operator of the level
   const double *idu, *idv;   // global inverse diagonals
-  int fx, fy;                // coarsening factors to the next level
   int soff;                  // offset of the level's planes in shared memory (doubles)
   int rows;                  // interior rows (u then v)
   int cls[5];                // row ranges of the classes u colour 0, u 1, v 0, v 1
+  int most;                  // rows of the largest class
   int toff;                  // offset of the level's row table in the shared table area (uint16)
-  const uint16_t* gtab;      // the table in global memory: kTabCols columns of `rows` entries
+  const uint16_t* gtab;      // the table in global memory
 };
 struct SubCycle {
   int first, last, nu1, nu2, coarse_sweeps;
@@ -1531,228 +1520,327 @@ struct SubCycle {
   const int* singular;
   Restriction rs;              // b of the first level: given, or restricted from the finer residual
   int dbl;                     // doubles of all levels' planes (the table area follows)
-  int ainv_off;                // offset (doubles) of the staged, transposed inverse, after the tables
+  int ainv_off;                // offset (doubles) of the staged inverse, after the tables
+  int res_off;                 // the residual of the level being left: u, v (a zero element before each)
   int tab16;                   // 16-byte vectors of all levels' row tables
   SubLevel L[kMaxLevels];
 };
 
-template <class F>
-__device__ __forceinline__ void block_for_points(const Dims& d, F f) {
-  const int n = d.nx * d.ny;
-  for (int t = threadIdx.x; t < n; t += blockDim.x) f(t % d.ny, t / d.ny);
+__device__ __forceinline__ void copy8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 
-// (A x) of table row r: same terms in the same order as AuX / AvX
-__device__ __forceinline__ double table_row_apply(const uint16_t* tab, int R, int r, bool urow, int ny, double ax,
-                                                  double ay, const double* Na, const double* Nb, const double* Bx,
-                                                  const double* By, const double* xu, const double* xv, int& q) {
-  q = tab[r];
-  const int s0 = tab[R + r], s1 = tab[2 * R + r], s2 = tab[3 * R + r], s3 = tab[4 * R + r];
-  const int s4 = tab[5 * R + r], s5 = tab[6 * R + r], s6 = tab[7 * R + r], s7 = tab[8 * R + r];
-  if (urow) {
-    const double Ae = Na[q + ny], Aw = Na[q], Bn = Nb[q], Bs = Nb[q - 1];
-    const double cE = 4.0 * ax * Ae, cW = 4.0 * ax * Aw, cN = ay * Bn, cS = ay * Bs;
-    const double diag = -(cE + cW + cN + cS) - Bx[q];
-    return stencil9(cE, xu[s0], cW, xu[s1], cN, xu[s2], cS, xu[s3], diag, xu[q], -2.0 * Aw - Bn, xv[s4],
-                    2.0 * Ae + Bn, xv[s5], 2.0 * Aw + Bs, xv[s6], -2.0 * Ae - Bs, xv[s7]);
+__device__ __forceinline__ double lds(uint32_t at) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(at));
+  return v;
+}
+__device__ __forceinline__ void sts(uint32_t at, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(at), "d"(v)); }
+
+// A level of the sub-cycle in shared memory: its planes, its row table and the operator's scale.
+struct SubMem {
+  double* a;
+  const uint16_t* tab;
+  int P1, ny, R;
+  double ax, ay;
+  __device__ __forceinline__ SubMem(const SubCycle& sc, double* sm, const uint16_t* tabs, int l) {
+    const SubLevel& L = sc.L[l];
+    a = sm + L.soff;
+    tab = tabs + L.toff;
+    ny = L.o.d.ny;
+    P1 = L.o.d.nx * ny + 1;
+    R = L.rows;
+    ax = L.o.ax;
+    ay = L.o.ay;
   }
-  const double An = Na[q + 1], As = Na[q], Be = Nb[q], Bw = Nb[q - ny];
-  const double cN = 4.0 * ay * An, cS = 4.0 * ay * As, cE = ax * Be, cW = ax * Bw;
-  const double diag = -(cN + cS + cE + cW) - By[q];
-  return stencil9(cN, xv[s0], cS, xv[s1], cE, xv[s2], cW, xv[s3], diag, xv[q], -2.0 * An - Bw, xu[s4],
-                  2.0 * An + Be, xu[s5], 2.0 * As + Bw, xu[s6], -2.0 * As - Be, xu[s7]);
+  __device__ __forceinline__ double* plane(int k) const { return a + k * P1; }
+  __device__ __forceinline__ int pos(int r) const { return tab[tab_pos(R) + r]; }
+};
+// N_a and N_b a row takes, in the order A1 A0 B1 B0 of row_terms, and its diagonal
+template <bool U>
+__device__ __forceinline__ void row_coefficients(const SubMem& m, int q, double (&c)[5]) {
+  const double *Na = m.plane(SA_NA), *Nb = m.plane(SA_NB), pa = U ? m.ax : m.ay, pb = U ? m.ay : m.ax;
+  c[0] = U ? Na[q + m.ny] : Na[q + 1];
+  c[1] = Na[q];
+  c[2] = Nb[q];
+  c[3] = U ? Nb[q - 1] : Nb[q - m.ny];
+  c[4] = -(4.0 * pa * c[0] + 4.0 * pa * c[1] + pb * c[2] + pb * c[3]) - m.plane(U ? SA_BX : SA_BY)[q];
+}
+// (A x) of a u (v) row: the operator's nine terms (AuXC, AvXC) in three chains.  x: the row's own
+// value, then its four neighbours of the same component and the four of the other.
+template <bool U>
+__device__ __forceinline__ double row_terms(const double (&c)[5], double ax, double ay, const double (&x)[9]) {
+  const double A1 = c[0], A0 = c[1], B1 = c[2], B0 = c[3], pa = U ? ax : ay, pb = U ? ay : ax;
+  double s0 = 4.0 * pa * A1 * x[1], s1 = 4.0 * pa * A0 * x[2], s2 = pb * B1 * x[3];
+  s0 = fma(pb * B0, x[4], s0);
+  s1 = fma(c[4], x[0], s1);
+  s2 = fma(U ? -2.0 * A0 - B1 : -2.0 * A1 - B0, x[5], s2);
+  s0 = fma(2.0 * A1 + B1, x[6], s0);
+  s1 = fma(2.0 * A0 + B0, x[7], s1);
+  s2 = fma(U ? -2.0 * A1 - B0 : -2.0 * A0 - B1, x[8], s2);
+  return (s0 + s1) + s2;
+}
+// the same from the tables (x, y: the planes of the row's component and of the other)
+template <bool U>
+__device__ __forceinline__ double row_apply(const SubMem& m, int r, int& q, const double* x, const double* y) {
+  const uint4 at = reinterpret_cast<const uint4*>(m.tab)[r];
+  q = m.pos(r);
+  double c[5];
+  row_coefficients<U>(m, q, c);
+  const double v[9] = {x[q], x[at.x & 0xffffu], x[at.x >> 16], x[at.y & 0xffffu], x[at.y >> 16],
+                       y[at.z & 0xffffu], y[at.z >> 16], y[at.w & 0xffffu], y[at.w >> 16]};
+  return row_terms<U>(c, m.ax, m.ay, v);
 }
 
-__global__ void __launch_bounds__(kSubThreads) k_subcycle(SubCycle sc, double* xu0, double* xv0,
-                                                          const double* bu0, const double* bv0) {
+__global__ void __launch_bounds__(kSubThreads) k_subcycle(const __grid_constant__ SubCycle sc, double* xu0,
+                                                          double* xv0, const double* bu0, const double* bv0) {
   extern __shared__ double sm[];
-  __shared__ Op so[kMaxLevels];   // operators of the staged levels
+  __shared__ double weight[16], sr[kCoarseDirectMax];
+  __shared__ uint16_t number[kCoarseDirectMax], place[kCoarseDirectMax];   // unknown of a coarsest row; its position
   uint16_t* tabs = reinterpret_cast<uint16_t*>(sm + sc.dbl);
-  double* AinvT = sm + sc.ainv_off;
-  // whether the coarsest level is solved with its inverse (read before the staging, so
-  // that the flag's load overlaps it)
+  double* Ainv = sm + sc.ainv_off;
+  const int tid = threadIdx.x, quarter = tid / kSubQuarter, t = tid % kSubQuarter;
+  const bool urow = quarter < 2;   // (of a resident row)
+  // whether the coarsest level is solved with its inverse (the flag's load overlaps the copies)
   const bool direct = sc.direct && *sc.singular == 0;
-  if (threadIdx.x == 0)
-    for (int l = sc.first; l <= sc.last; ++l) {
-      Op o = sc.L[l].o;
-      const int P1 = o.d.nx * o.d.ny + 1;
-      o.d.ld = o.d.ny;
-      o.d.plane = P1 - 1;
-      double* a = sm + sc.L[l].soff;
-      o.Na = a + SA_NA * P1;
-      o.Nb = a + SA_NB * P1;
-      o.Bx = a + SA_BX * P1;
-      o.By = a + SA_BY * P1;
-      so[l] = o;
-    }
-  // the staging: one pass over the points of all levels (their loads independent of one
-  // another), then the row tables and the coarsest level's inverse
+  if (tid < 16) weight[tid] = 0.0625 * (tid + 1);
   {
     int total = 0;
     for (int l = sc.first; l <= sc.last; ++l) total += sc.L[l].o.d.nx * sc.L[l].o.d.ny + 1;
-    for (int t0 = threadIdx.x; t0 < total; t0 += blockDim.x) {
-      int l = sc.first, t = t0;
-      while (t >= sc.L[l].o.d.nx * sc.L[l].o.d.ny + 1) { t -= sc.L[l].o.d.nx * sc.L[l].o.d.ny + 1; ++l; }
+    for (int t0 = tid; t0 < total; t0 += kSubThreads) {
+      int l = sc.first, e = t0;
+      while (e >= sc.L[l].o.d.nx * sc.L[l].o.d.ny + 1) { e -= sc.L[l].o.d.nx * sc.L[l].o.d.ny + 1; ++l; }
       const SubLevel& L = sc.L[l];
-      const Dims& g = L.o.d;
-      const int P = g.nx * g.ny, P1 = P + 1;
+      const Dims& d = L.o.d;
+      const int P = d.nx * d.ny, P1 = P + 1;
       double* a = sm + L.soff;
-      if (t == P) {   // the zero element read by 'zero' boundary sides
-        a[SA_XU * P1 + t] = 0.0;
-        a[SA_XV * P1 + t] = 0.0;
+      a[SA_XU * P1 + e] = 0.0;   // every level is entered with x = 0
+      a[SA_XV * P1 + e] = 0.0;
+      if (e == P) continue;
+      const long long q = d.at(e % d.ny, e / d.ny);
+      copy8(a + SA_NA * P1 + e, L.o.Na + q);
+      copy8(a + SA_NB * P1 + e, L.o.Nb + q);
+      copy8(a + SA_BX * P1 + e, L.o.Bx + q);
+      copy8(a + SA_BY * P1 + e, L.o.By + q);
+      copy8(a + SA_IDU * P1 + e, L.idu + q);
+      copy8(a + SA_IDV * P1 + e, L.idv + q);
+    }
+    // the levels' tables are contiguous and padded to 16 bytes in both places
+    const uint4* g = reinterpret_cast<const uint4*>(sc.L[sc.first].gtab);
+    for (int e = tid; e < sc.tab16; e += kSubThreads) copy16(reinterpret_cast<uint4*>(tabs) + e, g + e);
+    if (direct)
+      for (int e = tid, n = sc.map.n(); e < n * n; e += kSubThreads) copy8(Ainv + e, sc.Ainv + e);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (direct && tid >= kSubThreads - kCoarseDirectMax && tid - (kSubThreads - kCoarseDirectMax) < sc.map.n()) {
+      const SubLevel& L = sc.L[sc.last];
+      const int r = tid - (kSubThreads - kCoarseDirectMax), ny = sc.map.ny, q = L.gtab[tab_pos(L.rows) + r];
+      const int i = q / ny, j = q % ny, k = r < L.cls[2] ? (i - 1) * (ny - 2) + j - 1 : sc.map.nu + (i - 1) * (ny - 3) + j - 1;
+      number[r] = (uint16_t)k;
+      place[k] = (uint16_t)q;
+    }
+    const SubLevel& L = sc.L[sc.first];
+    const Dims& d = L.o.d;
+    const int P = d.nx * d.ny, P1 = P + 1;
+    double* a = sm + L.soff;
+    for (int e = tid; e < P; e += kSubThreads) {
+      const int j = e % d.ny, i = e / d.ny;
+      double b0, b1;
+      if (sc.rs.on) {
+        restrict_from(sc.rs, d, j, i, b0, b1);
+      } else {
+        const long long q = d.at(j, i);
+        b0 = bu0[q];
+        b1 = bv0[q];
+      }
+      a[SA_BU * P1 + e] = b0;
+      a[SA_BV * P1 + e] = b1;
+    }
+    if (tid == 0) sm[sc.res_off] = sm[sc.res_off + P1] = 0.0;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+  }
+  __syncthreads();
+  double* ru = sm + sc.res_off + 1;
+  double* rv = ru + sc.L[sc.first].o.d.nx * sc.L[sc.first].o.d.ny + 1;
+  auto tap = [&](const double* x, uint32_t e, double s) {
+    return fma(weight[e >> kTapBits], x[e & ((1u << kTapBits) - 1)], s);
+  };
+  // b of a row from the residual of the level above (restrict_values' taps and order)
+  auto restricted = [&](const SubMem& m, int r, bool u) {
+    const uint2* e = reinterpret_cast<const uint2*>(m.tab + tab_restrict(m.R)) + 3 * r;
+    const double* f = (u ? ru : rv) - 1;
+    const uint2 v0 = e[0], v1 = e[1], v2 = e[2];
+    double s = tap(f, v0.x & 0xffffu, 0.0);
+    s = tap(f, v0.x >> 16, s); s = tap(f, v0.y & 0xffffu, s); s = tap(f, v0.y >> 16, s);
+    s = tap(f, v1.x & 0xffffu, s); s = tap(f, v1.x >> 16, s); s = tap(f, v1.y & 0xffffu, s); s = tap(f, v1.y >> 16, s);
+    s = tap(f, v2.x & 0xffffu, s); s = tap(f, v2.x >> 16, s); s = tap(f, v2.y & 0xffffu, s); s = tap(f, v2.y >> 16, s);
+    return s;
+  };
+  // (P x_c) of a row (prolong_delta's taps and order)
+  auto prolonged = [&](const SubMem& m, const SubMem& k, int r, bool u) {
+    const uint2 e = reinterpret_cast<const uint2*>(m.tab + tab_prolong(m.R))[r];
+    const double* f = k.plane(u ? SA_XU : SA_XV);
+    double s = tap(f, e.x & 0xffffu, 0.0);
+    s = tap(f, e.x >> 16, s);
+    s = tap(f, e.y & 0xffffu, s);
+    return tap(f, e.y >> 16, s);
+  };
+  // ---- the levels with more rows than the block has threads for them: every thread on every row
+  auto gs_pass = [&](const SubMem& m, int l, int p) {
+    double *xu = m.plane(SA_XU), *xv = m.plane(SA_XV);
+    for (int r = sc.L[l].cls[p] + tid; r < sc.L[l].cls[p + 1]; r += kSubThreads) {
+      int q;
+      if (p < 2) {
+        const double Ax = row_apply<true>(m, r, q, xu, xv);
+        xu[q] = fma(m.plane(SA_BU)[q] - Ax, m.plane(SA_IDU)[q], xu[q]);
+      } else {
+        const double Ax = row_apply<false>(m, r, q, xv, xu);
+        xv[q] = fma(m.plane(SA_BV)[q] - Ax, m.plane(SA_IDV)[q], xv[q]);
+      }
+    }
+    __syncthreads();
+  };
+  int tail = sc.first;   // the first level of resident rows; none where the coarsest level is relaxed
+  while (direct ? sc.L[tail].most > kSubQuarter : tail <= sc.last) ++tail;
+  for (int l = sc.first; l < tail; ++l) {
+    const SubMem m(sc, sm, tabs, l);
+    double *xu = m.plane(SA_XU), *xv = m.plane(SA_XV);
+    if (l > sc.first) {
+      for (int r = tid; r < m.R; r += kSubThreads) {
+        const bool u = r < sc.L[l].cls[2];
+        m.plane(u ? SA_BU : SA_BV)[m.pos(r)] = restricted(m, r, u);
+      }
+      __syncthreads();
+    }
+    if (l == sc.last) {
+      Op o = sc.L[l].o;
+      o.d.ld = m.ny;
+      o.d.plane = m.P1 - 1;
+      o.Na = m.plane(SA_NA); o.Nb = m.plane(SA_NB); o.Bx = m.plane(SA_BX); o.By = m.plane(SA_BY);
+      block_coarse_relax(o, xu, xv, m.plane(SA_BU), m.plane(SA_BV), m.plane(SA_IDU), m.plane(SA_IDV), sc.coarse_sweeps);
+      break;
+    }
+    for (int s = 0; s < 4 * sc.nu1; ++s) gs_pass(m, l, s & 3);
+    // residual of the interior rows (the restriction reads interior rows only)
+    for (int r = tid; r < m.R; r += kSubThreads) {
+      int q;
+      if (r < sc.L[l].cls[2]) {
+        const double Ax = row_apply<true>(m, r, q, xu, xv);
+        ru[q] = m.plane(SA_BU)[q] - Ax;
+      } else {
+        const double Ax = row_apply<false>(m, r, q, xv, xu);
+        rv[q] = m.plane(SA_BV)[q] - Ax;
+      }
+    }
+    __syncthreads();
+  }
+  // ---- the levels of resident rows: a quarter's first `width` threads (whole warps) have the
+  // rows of its class (`most` does not grow from a level to the next)
+  auto width_of = [&](int l) { return max(1, (sc.L[l].most + 31) / 32) * 32; };
+  if (tail <= sc.last && t < width_of(tail)) {
+    int l = tail;
+    bool up = false;
+    while (true) {
+      const SubMem m(sc, sm, tabs, l);
+      const int width = width_of(l), bar = 1 + l - tail;
+      auto barrier = [&] {   // of the level's threads
+        __syncwarp();
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(4 * width) : "memory");
+      };
+      if (!up && l == sc.last) {   // x = Ainv b, eight threads to a row
+        const int flat = quarter * width + t, n = sc.map.n();
+        for (int r = flat; r < m.R; r += 4 * width) {
+          const bool u = r < sc.L[l].cls[2];
+          sr[number[r]] = l > sc.first ? restricted(m, r, u) : m.plane(u ? SA_BU : SA_BV)[m.pos(r)];
+        }
+        barrier();
+        for (int r0 = 0; r0 < n; r0 += width / 2) {
+          const int r = r0 + flat / 8;
+          double s = 0.0;
+          if (r < n)
+            for (int c = flat % 8; c < n; c += 8) s += Ainv[r * n + c] * sr[c];
+          s += __shfl_xor_sync(0xffffffffu, s, 4);
+          s += __shfl_xor_sync(0xffffffffu, s, 2);
+          s += __shfl_xor_sync(0xffffffffu, s, 1);
+          if (r < n && flat % 8 == 0) m.plane(r < sc.map.nu ? SA_XU : SA_XV)[place[r]] = s;
+        }
+        if (l == tail) break;
+        up = true;
+        --l;
         continue;
       }
-      const int jj = t % g.ny, ii = t / g.ny;
-      const long long q = g.at(jj, ii);
-      a[SA_NA * P1 + t] = L.o.Na[q];
-      a[SA_NB * P1 + t] = L.o.Nb[q];
-      a[SA_BX * P1 + t] = L.o.Bx[q];
-      a[SA_BY * P1 + t] = L.o.By[q];
-      a[SA_IDU * P1 + t] = L.idu[q];
-      a[SA_IDV * P1 + t] = L.idv[q];
-      if (l == sc.first) {   // entered with x = 0
-        double b0, b1;
-        if (sc.rs.on) {
-          restrict_from(sc.rs, g, jj, ii, b0, b1);
-        } else {
-          b0 = bu0[q];
-          b1 = bv0[q];
-        }
-        a[SA_XU * P1 + t] = 0.0;
-        a[SA_XV * P1 + t] = 0.0;
-        a[SA_BU * P1 + t] = b0;
-        a[SA_BV * P1 + t] = b1;
+      const int r = sc.L[l].cls[quarter] + t;
+      const bool on = r < sc.L[l].cls[quarter + 1];
+      // the row's neighbours (shared-memory addresses), coefficients, inverse diagonal and b
+      uint32_t at[9], atb = 0;
+      double c[5] = {}, id = 0.0, b = 0.0;
+      int q = 0;
+      if (on) {
+        const uint4 e = reinterpret_cast<const uint4*>(m.tab)[r];
+        const uint32_t x = smem_addr(m.plane(urow ? SA_XU : SA_XV)), y = smem_addr(m.plane(urow ? SA_XV : SA_XU));
+        q = m.pos(r);
+        at[0] = x + 8 * q;
+        at[1] = x + 8 * (e.x & 0xffffu); at[2] = x + 8 * (e.x >> 16);
+        at[3] = x + 8 * (e.y & 0xffffu); at[4] = x + 8 * (e.y >> 16);
+        at[5] = y + 8 * (e.z & 0xffffu); at[6] = y + 8 * (e.z >> 16);
+        at[7] = y + 8 * (e.w & 0xffffu); at[8] = y + 8 * (e.w >> 16);
+        atb = smem_addr(m.plane(urow ? SA_BU : SA_BV) + q);
+        if (urow) row_coefficients<true>(m, q, c);
+        else row_coefficients<false>(m, q, c);
+        id = m.plane(urow ? SA_IDU : SA_IDV)[q];
       }
-    }
-    {   // the levels' tables are contiguous and padded to 16 bytes in both places
-      const uint4* g = reinterpret_cast<const uint4*>(sc.L[sc.first].gtab);
-      uint4* t = reinterpret_cast<uint4*>(tabs);
-      for (int e = threadIdx.x; e < sc.tab16; e += blockDim.x) t[e] = g[e];
-    }
-    if (direct) {
-      const int n = sc.map.n();
-      for (int e = threadIdx.x; e < n * n; e += blockDim.x) AinvT[(e % n) * n + e / n] = sc.Ainv[e];
+      if (up) {   // x += P x_c, once the level below is done
+        barrier();
+        if (on) sts(at[0], lds(at[0]) + prolonged(m, SubMem(sc, sm, tabs, l + 1), r, urow));
+        barrier();
+      } else if (l > sc.first && on) {
+        sts(atb, restricted(m, r, urow));
+      }
+      if (on) b = lds(atb);
+      auto rest = [&] {   // b - A x of the row; its x
+        double v[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) v[k] = lds(at[k]);
+        const double Ax = urow ? row_terms<true>(c, m.ax, m.ay, v) : row_terms<false>(c, m.ax, m.ay, v);
+        return make_double2(b - Ax, v[0]);
+      };
+      for (int s = 4 * (up ? sc.nu2 : sc.nu1); s > 0; --s) {   // in the ascent the other way round
+        if (on && quarter == (up ? (s - 1) & 3 : -s & 3)) {
+          const double2 f = rest();
+          sts(at[0], fma(f.x, id, f.y));
+        }
+        barrier();
+      }
+      if (up) {
+        if (l == tail) break;
+        --l;
+        continue;
+      }
+      if (on) (urow ? ru : rv)[q] = rest().x;
+      barrier();
+      if (t < width_of(l + 1)) ++l;
+      else up = true;   // no rows below: on to this level's ascent
     }
   }
   __syncthreads();
-  auto arr = [&](int l, int k) { return sm + sc.L[l].soff + k * (sc.L[l].o.d.nx * sc.L[l].o.d.ny + 1); };
-  // one Gauss-Seidel pass over the rows of class p (0/1: u colours, 2/3: v colours)
-  auto gs_pass = [&](int l, int p) {
-    const SubLevel& L = sc.L[l];
-    const Op& o = so[l];
-    const int P1 = L.o.d.nx * L.o.d.ny + 1, ny = L.o.d.ny;
-    const double* a = sm + L.soff;
-    double* xu = sm + L.soff + SA_XU * P1;
-    double* xv = sm + L.soff + SA_XV * P1;
-    const uint16_t* tab = tabs + L.toff;
-    const bool urow = p < 2;
-    for (int r = L.cls[p] + threadIdx.x; r < L.cls[p + 1]; r += blockDim.x) {
-      int q;
-      const double Ax = table_row_apply(tab, L.rows, r, urow, ny, o.ax, o.ay, a + SA_NA * P1, a + SA_NB * P1,
-                                        a + SA_BX * P1, a + SA_BY * P1, xu, xv, q);
-      if (urow) xu[q] = fma(a[SA_BU * P1 + q] - Ax, a[SA_IDU * P1 + q], xu[q]);
-      else xv[q] = fma(a[SA_BV * P1 + q] - Ax, a[SA_IDV * P1 + q], xv[q]);
-    }
-  };
-  // descend
-  for (int l = sc.first; l <= sc.last; ++l) {
-    const Op& o = so[l];
-    double *xu = arr(l, SA_XU), *xv = arr(l, SA_XV), *bu = arr(l, SA_BU), *bv = arr(l, SA_BV);
-    const double *idu = arr(l, SA_IDU), *idv = arr(l, SA_IDV);
-    if (l == sc.last) {
-      if (direct) {
-        block_coarse_direct(o, sc.map, AinvT, xu, xv, bu, bv);
-        __syncthreads();
-      } else {
-        block_coarse_relax(o, xu, xv, bu, bv, idu, idv, sc.coarse_sweeps);
-      }
-      break;
-    }
-    for (int s = 0; s < sc.nu1; ++s)
-      for (int p = 0; p < 4; ++p) {
-        gs_pass(l, p);
-        __syncthreads();
-      }
-    // residual of the interior rows (the restriction reads interior rows only)
-    double *ru = arr(l, SA_RU), *rv = arr(l, SA_RV);
-    {
-      const SubLevel& L = sc.L[l];
-      const int P1 = L.o.d.nx * L.o.d.ny + 1;
-      const double* a = sm + L.soff;
-      const uint16_t* tab = tabs + L.toff;
-      for (int r = threadIdx.x; r < L.rows; r += blockDim.x) {
-        const bool urow = r < L.cls[2];
-        int q;
-        const double Ax = table_row_apply(tab, L.rows, r, urow, L.o.d.ny, o.ax, o.ay, a + SA_NA * P1,
-                                          a + SA_NB * P1, a + SA_BX * P1, a + SA_BY * P1, xu, xv, q);
-        if (urow) ru[q] = bu[q] - Ax;
-        else rv[q] = bv[q] - Ax;
-      }
+  for (int l = min(tail, sc.last) - 1; l >= sc.first; --l) {
+    const SubMem m(sc, sm, tabs, l), k(sc, sm, tabs, l + 1);
+    for (int r = tid; r < m.R; r += kSubThreads) {
+      const bool u = r < sc.L[l].cls[2];
+      m.plane(u ? SA_XU : SA_XV)[m.pos(r)] += prolonged(m, k, r, u);
     }
     __syncthreads();
-    const Op& k = so[l + 1];
-    double *kxu = arr(l + 1, SA_XU), *kxv = arr(l + 1, SA_XV), *kbu = arr(l + 1, SA_BU), *kbv = arr(l + 1, SA_BV);
-    const int fx = sc.L[l].fx, fy = sc.L[l].fy;
-    // the two levels' dimensions in registers for the transfer (not re-read from shared
-    // memory for every tap)
-    const Dims df = o.d, dc = k.d;
-    block_for_points(dc, [&](int j, int i) {
-      restrict_point(df, dc, fx, fy, ru, rv, kbu, kbv, kxu, kxv, j, i);
-    });
-    __syncthreads();
-  }
-  // ascend
-  for (int l = sc.last - 1; l >= sc.first; --l) {
-    double *xu = arr(l, SA_XU), *xv = arr(l, SA_XV);
-    const double *kxu = arr(l + 1, SA_XU), *kxv = arr(l + 1, SA_XV);
-    {   // x += P x_c on the interior rows, from the rows' prolongation taps (coarse positions
-        // mapped on the host; the weights formed here, in prolong_delta's order)
-      const SubLevel& L = sc.L[l];
-      const int fx = L.fx, fy = L.fy, ny = L.o.d.ny, R = L.rows;
-      const uint16_t* tab = tabs + L.toff;
-      const uint16_t* ptab = tab + kTabCols * R;
-      for (int r = threadIdx.x; r < R; r += blockDim.x) {
-        const int q = tab[r], j = q % ny, i = q / ny;
-        double s = 0.0, wj, wi;
-        int k = 0, C;
-        if (r < L.cls[2]) {
-          const int nj = scatter_node_n(j, fy), ni = scatter_cell_n(i, fx);
-          for (int a = 0; a < nj; ++a) {
-            scatter_node(j, fy, a, C, wj);
-            for (int b = 0; b < ni; ++b, ++k) {
-              scatter_cell(i, fx, b, C, wi);
-              s = fma(wj * wi, kxu[ptab[k * R + r]], s);
-            }
-          }
-          xu[q] += s;
-        } else {
-          const int nj = scatter_cell_n(j, fy), ni = scatter_node_n(i, fx);
-          for (int a = 0; a < nj; ++a) {
-            scatter_cell(j, fy, a, C, wj);
-            for (int b = 0; b < ni; ++b, ++k) {
-              scatter_node(i, fx, b, C, wi);
-              s = fma(wj * wi, kxv[ptab[k * R + r]], s);
-            }
-          }
-          xv[q] += s;
-        }
-      }
-    }
-    __syncthreads();
-    for (int s = 0; s < sc.nu2; ++s)
-      for (int p = 3; p >= 0; --p) {
-        gs_pass(l, p);
-        __syncthreads();
-      }
+    for (int s = 4 * sc.nu2 - 1; s >= 0; --s) gs_pass(m, l, s & 3);
   }
   {
-    const Dims& g = sc.L[sc.first].o.d;
-    const int P = g.nx * g.ny;
-    const double *xu = arr(sc.first, SA_XU), *xv = arr(sc.first, SA_XV);
-    for (int t = threadIdx.x; t < P; t += blockDim.x) {
-      const long long q = g.at(t % g.ny, t / g.ny);
-      xu0[q] = xu[t];
-      xv0[q] = xv[t];
+    const SubMem m(sc, sm, tabs, sc.first);
+    const double *xu = m.plane(SA_XU), *xv = m.plane(SA_XV);
+    for (int e = tid; e < m.P1 - 1; e += kSubThreads) {
+      const long long q = sc.L[sc.first].o.d.at(e % m.ny, e / m.ny);
+      xu0[q] = xu[e];
+      xv0[q] = xv[e];
     }
   }
 }
@@ -2335,35 +2423,54 @@ static int level_rows(const Dims& d) {
   return nu + nv;
 }
 
-// shared memory the sub-cycle needs from level l down: the planes, then the row tables
-static size_t sub_dbl(const Ctx* c, int l) {
+// Shared memory of the sub-cycle from level l down: the planes, the row tables, the inverse, the
+// residual.  The level it starts from is the first whose planes, residual planes, reads and
+// prolongation taps, and those of the levels below, fit in kSubSmemBudget (sub_bytes).
+static size_t sub_points(const Ctx* c, int l) {
   size_t n = 0;
-  for (int q = l; q < c->nlev; ++q) n += (size_t)kSubArrays * ((size_t)c->lv[q].d.nx * c->lv[q].d.ny + 1);
+  for (int q = l; q < c->nlev; ++q) n += (size_t)c->lv[q].d.nx * c->lv[q].d.ny + 1;
   return n;
 }
-// entries of one level's row table, padded to 8 (16 bytes) so that every level's table
-// starts 16-byte aligned and the sub-cycle copies the tables as 16-byte vectors
-static size_t level_tab_entries(const Dims& d) { return ((size_t)(kTabCols + kTabProlong) * level_rows(d) + 7) / 8 * 8; }
+static size_t sub_rows(const Ctx* c, int l) {
+  size_t n = 0;
+  for (int q = l; q < c->nlev; ++q) n += ((size_t)13 * level_rows(c->lv[q].d) + 7) / 8 * 8;
+  return n;
+}
+static int sub_first_fit(const Ctx* c);
+// entries of a level's row table, padded to 8 (16 bytes) so that every level's table starts
+// 16-byte aligned and the sub-cycle copies the tables as 16-byte vectors; the restriction
+// taps only below the first level that may start the sub-cycle
+static size_t level_tab_entries(const Ctx* c, int l) {
+  const int R = level_rows(c->lv[l].d);
+  return ((size_t)tab_restrict(R) + (l > sub_first_fit(c) ? kTabRestrict * R : 0) + 7) / 8 * 8;
+}
 static size_t sub_tab_entries(const Ctx* c, int l) {
   size_t n = 0;
-  for (int q = l; q < c->nlev; ++q) n += level_tab_entries(c->lv[q].d);
+  for (int q = l; q < c->nlev; ++q) n += level_tab_entries(c, q);
   return n;
 }
 // the coarsest level's unknowns when it is solved with its inverse, else 0
 static int coarse_direct_n(const Ctx* c);
 // doubles of the sub-cycle's table area (16-byte aligned), between the planes and the inverse
 static size_t sub_tab_dbl(const Ctx* c, int l) { return ((sub_tab_entries(c, l) * sizeof(uint16_t) + 15) / 16) * 2; }
-// dynamic shared memory of the sub-cycle from level l: planes, row tables, the inverse
+// doubles of the planes from level l down (an even number: the tables follow, 16-byte aligned)
+static size_t sub_dbl(const Ctx* c, int l) { return (kSubArrays * sub_points(c, l) + 1) / 2 * 2; }
 static size_t sub_bytes(const Ctx* c, int l) {
   const size_t n = (size_t)coarse_direct_n(c);
-  return (sub_dbl(c, l) + sub_tab_dbl(c, l) + n * n) * sizeof(double);
+  return ((kSubArrays + 2) * sub_points(c, l) + (sub_rows(c, l) * sizeof(uint16_t) + 15) / 16 * 2 + n * n) * sizeof(double);
+}
+// what is allocated
+static size_t sub_alloc(const Ctx* c, int l) {
+  const size_t n = (size_t)coarse_direct_n(c);
+  const Dims& d = c->lv[l].d;
+  return (sub_dbl(c, l) + sub_tab_dbl(c, l) + n * n + 2 * ((size_t)d.nx * d.ny + 1)) * sizeof(double);
 }
 
 // the largest level whose levels all fit in the sub-cycle's shared memory (the row
 // tables are built from there down, whatever the configuration)
 static int sub_first_fit(const Ctx* c) {
   for (int l = 0; l < c->nlev; ++l)
-    if (sub_bytes(c, l) <= kSubSmemBudget) return l;
+    if (sub_bytes(c, l) <= kSubSmemBudget) return l;   // (then sub_alloc is at most kSubSmemMax)
   return c->nlev - 1;
 }
 // first level of the one-block sub-cycle
@@ -2598,21 +2705,24 @@ static int build_sub_tables(Ctx* c) {
     Dims d = c->lv[l].d;
     d.ld = d.ny;   // compact planes in shared memory
     const int P = d.nx * d.ny, R = level_rows(d);
-    if (P >= 65535) return set_error(c, DIVA_UNSUPPORTED, "sub-cycle level too large for 16-bit row tables");
+    if (P + 1 >= 1 << kTapBits) return set_error(c, DIVA_UNSUPPORTED, "sub-cycle level too large for its row tables");
     c->sub_tab_off[l] = off;
+    uint16_t *reads = tab.data() + off, *pos = reads + tab_pos(R), *prolong = reads + tab_prolong(R),
+             *restricted = reads + tab_restrict(R);
+    auto tap = [](size_t at, double w) { return (uint16_t)(at | (size_t)(16.0 * w - 1.0) << kTapBits); };
     int r = 0;
     auto put = [&](int j, int i, bool urow) {
       const int js_[4] = {urow ? j : j + 1, urow ? j : j - 1, urow ? j + 1 : j, urow ? j - 1 : j};
       const int is_[4] = {urow ? i + 1 : i, urow ? i - 1 : i, urow ? i : i + 1, urow ? i : i - 1};
       const int jc_[4] = {urow ? j : j + 1, urow ? j : j + 1, urow ? j - 1 : j, urow ? j - 1 : j};
       const int ic_[4] = {urow ? i : i - 1, urow ? i + 1 : i, urow ? i : i - 1, urow ? i + 1 : i};
-      tab[off + r] = (uint16_t)d.at(j, i);
+      pos[r] = (uint16_t)d.at(j, i);
       for (int k = 0; k < 4; ++k) {   // same-component neighbours, then the cross-coupled reads
         int js, is;
         const bool on = urow ? u_src(d, c->bc, js_[k], is_[k], js, is) : v_src(d, c->bc, js_[k], is_[k], js, is);
-        tab[off + (size_t)(1 + k) * R + r] = on ? (uint16_t)d.at(js, is) : (uint16_t)P;
+        reads[8 * r + k] = on ? (uint16_t)d.at(js, is) : (uint16_t)P;
         const bool on2 = urow ? v_src(d, c->bc, jc_[k], ic_[k], js, is) : u_src(d, c->bc, jc_[k], ic_[k], js, is);
-        tab[off + (size_t)(5 + k) * R + r] = on2 ? (uint16_t)d.at(js, is) : (uint16_t)P;
+        reads[8 * r + 4 + k] = on2 ? (uint16_t)d.at(js, is) : (uint16_t)P;
       }
       // the prolongation taps of the row from the next level (prolong_delta's taps in its
       // order, each clamped and read through the coarse level's boundary mapping; the
@@ -2624,26 +2734,43 @@ static int build_sub_tables(Ctx* c) {
         int fx, fy;
         factors(c, l, &fx, &fy);
         int k = 0, js, is, Cj, Ci;
-        double w;
+        double wj, wi;
         auto clampi = [](int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); };
         if (urow) {
           for (int a = 0; a < scatter_node_n(j, fy); ++a)
             for (int b = 0; b < scatter_cell_n(i, fx); ++b, ++k) {
-              scatter_node(j, fy, a, Cj, w);
-              scatter_cell(i, fx, b, Ci, w);
+              scatter_node(j, fy, a, Cj, wj);
+              scatter_cell(i, fx, b, Ci, wi);
               const bool on = u_src(dc, c->bc, clampi(Cj, 0, dc.ny - 1), clampi(Ci, 0, dc.nx - 2), js, is);
-              tab[off + (size_t)(kTabCols + k) * R + r] = on ? (uint16_t)dc.at(js, is) : (uint16_t)Pc;
+              prolong[kTabProlong * r + k] = tap(on ? dc.at(js, is) : Pc, wj * wi);
             }
         } else {
           for (int a = 0; a < scatter_cell_n(j, fy); ++a)
             for (int b = 0; b < scatter_node_n(i, fx); ++b, ++k) {
-              scatter_cell(j, fy, a, Cj, w);
-              scatter_node(i, fx, b, Ci, w);
+              scatter_cell(j, fy, a, Cj, wj);
+              scatter_node(i, fx, b, Ci, wi);
               const bool on = v_src(dc, c->bc, clampi(Cj, 0, dc.ny - 2), clampi(Ci, 0, dc.nx - 1), js, is);
-              tab[off + (size_t)(kTabCols + k) * R + r] = on ? (uint16_t)dc.at(js, is) : (uint16_t)Pc;
+              prolong[kTabProlong * r + k] = tap(on ? dc.at(js, is) : Pc, wj * wi);
             }
         }
-        for (; k < kTabProlong; ++k) tab[off + (size_t)(kTabCols + k) * R + r] = (uint16_t)Pc;
+        for (; k < kTabProlong; ++k) prolong[kTabProlong * r + k] = tap(Pc, 1.0);
+      }
+      // the restriction taps of the row from the level above (restrict_values' taps in its order),
+      // one beyond the position; 0 for none
+      if (l > first) {
+        Dims df = c->lv[l - 1].d;
+        df.ld = df.ny;
+        int fx, fy, fj, fi, k = 0;
+        double wj, wi;
+        factors(c, l - 1, &fx, &fy);
+        const int nj = urow ? gather_node_n(fy) : gather_cell_n(fy), ni = urow ? gather_cell_n(fx) : gather_node_n(fx);
+        for (int a = 0; a < nj; ++a)
+          for (int b = 0; b < ni; ++b) {
+            if (urow) { gather_node(j, fy, a, fj, wj); gather_cell(i, fx, b, fi, wi); }
+            else { gather_cell(j, fy, a, fj, wj); gather_node(i, fx, b, fi, wi); }
+            if (urow ? u_int(df, fj, fi) : v_int(df, fj, fi))
+              restricted[kTabRestrict * r + k++] = tap(df.at(fj, fi) + 1, wj * wi);
+          }
       }
       ++r;
     };
@@ -2656,7 +2783,7 @@ static int build_sub_tables(Ctx* c) {
     }
     c->sub_cls[l][4] = r;
     if (r != R) return set_error(c, DIVA_CUDA_ERROR, "sub-cycle row table size");
-    off += level_tab_entries(c->lv[l].d);
+    off += level_tab_entries(c, l);
   }
   if (!tab.empty())
     DIVA_CUDA(c, cudaMemcpy(c->sub_tab, tab.data(), tab.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
@@ -2692,8 +2819,7 @@ int solver_init(Ctx* c) {
     return set_error(c, DIVA_UNSUPPORTED, "coarsest multigrid level too large for the one-block sub-cycle");
   if (int st = build_sub_tables(c)) return st;
   DIVA_CUDA(c, cudaFuncSetAttribute(k_small_setup, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem));
-  DIVA_CUDA(c, cudaFuncSetAttribute(k_subcycle, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kSubSmemBudget));
+  DIVA_CUDA(c, cudaFuncSetAttribute(k_subcycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSubSmemMax));
   if (int st = tile_attrs_shape<32, 32>(c)) return st;
   if (int st = tile_attrs_shape<16, 16>(c)) return st;
   if (int st = tile_attrs_shape<32, 48>(c)) return st;
@@ -2731,7 +2857,7 @@ static int vcycle(Ctx* c, int l, double* xu, double* xv, const double* bu, const
                   const Restriction& rs) {
   const int nu1 = level_nu(c, l), nu2 = nu1, coarse_sweeps = 64;
   if (l == sub_first_level(c)) {
-    SubCycle sc;
+    SubCycle sc{};
     sc.first = l;
     sc.last = c->nlev - 1;
     sc.nu1 = nu1;
@@ -2747,21 +2873,21 @@ static int vcycle(Ctx* c, int l, double* xu, double* xv, const double* bu, const
       SubLevel& S = sc.L[q];
       S.o = make_op(c, q);
       S.idu = L.idu; S.idv = L.idv;
-      S.fx = 1; S.fy = 1;
-      if (q + 1 < c->nlev) factors(c, q, &S.fx, &S.fy);
       S.soff = soff;
       soff += kSubArrays * (L.d.nx * L.d.ny + 1);
       S.rows = level_rows(L.d);
       for (int k = 0; k < 5; ++k) S.cls[k] = c->sub_cls[q][k];
+      for (int k = 0; k < 4; ++k) S.most = std::max(S.most, S.cls[k + 1] - S.cls[k]);
       S.toff = toff;
       S.gtab = c->sub_tab + c->sub_tab_off[q];
-      toff += (int)level_tab_entries(L.d);
+      toff += (int)level_tab_entries(c, q);
     }
-    sc.dbl = soff;
-    sc.ainv_off = soff + (int)sub_tab_dbl(c, l);
+    sc.dbl = (int)sub_dbl(c, l);
+    sc.ainv_off = sc.dbl + (int)sub_tab_dbl(c, l);
+    sc.res_off = sc.ainv_off + coarse_direct_n(c) * coarse_direct_n(c);
     sc.tab16 = toff / 8;
     sc.rs = rs;
-    k_subcycle<<<1, kSubThreads, sub_bytes(c, l), c->stream>>>(sc, xu, xv, bu, bv); c->launches++;
+    k_subcycle<<<1, kSubThreads, sub_alloc(c, l), c->stream>>>(sc, xu, xv, bu, bv); c->launches++;
     DIVA_LAUNCHED(c, "k_subcycle");
     for (int q = l; q < c->nlev; ++q) c->fine_passes += 8.0 * (double)c->lv[q].d.plane / (double)c->d.plane;
     return DIVA_OK;
