@@ -1349,32 +1349,42 @@ struct CoarseMap {
   __host__ __device__ __forceinline__ int n() const { return nu + nv; }
 };
 
-// Assembly and inversion of the coarsest level's matrix by one block.  tab is the level's
-// row table (of R = n rows: 4 same-component and 4 cross-component mapped reads of each, then
-// their own positions; the zero element P = nx*ny stands for 'zero' sides).
-// Gauss-Jordan step k maps the matrix of step k-1 (buffer k&1) to the next one in one
-// pass with one barrier: every warp finds the pivot row p of column k itself, and every
-// element takes its value from the old matrix with rows k and p exchanged.
-constexpr int kInvThreads = 1024;
-constexpr size_t kInvSmem = 2 * kCoarseDirectMax * (kCoarseDirectMax + 1) * sizeof(double);
+// Assembly and inversion of the coarsest level's matrix by the first threads of a block.  tab is the
+// level's row table (of R = n rows: 4 same-component and 4 cross-component mapped reads of each,
+// then their own positions; the zero element P = nx*ny stands for 'zero' sides); o reads
+// compact planes (row length ny).  Gauss-Jordan step k maps the matrix of step k-1 (buffer k&1)
+// to the next one in one pass with one barrier: every warp finds the pivot row p of column k
+// itself, and every element takes its value from the old matrix with rows k and p exchanged.
+// Bound by the latency of the n steps (pivot search, division, barrier): eight warps, a lane to a
+// column (two at most), so that a step takes one division per column and warp and the
+// redundant search stays cheap (a step takes 1100 cycles at n = 12, 1500 at 31; a thread per
+// element was no faster).
+constexpr int kInvThreads = 1024;   // of the set-up kernel
+constexpr int kInvWarps = 8;
+constexpr size_t kInvDbl = 2 * kCoarseDirectMax * (kCoarseDirectMax + 1);
 
 __device__ __forceinline__ void coarse_setup_block(const Op& o, const CoarseMap& m, const uint16_t* tab,
-                                                   double* Ainv, int* singular) {
+                                                   double* inv_buf, double* Ainv, int* singular) {
   constexpr int M = kCoarseDirectMax, LD = M + 1;
-  extern __shared__ double inv_buf[];   // two n x n matrices, row stride LD
   __shared__ int perm[M];
-  __shared__ double wmax[kInvThreads / 32];
+  __shared__ double wmax[kInvWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = m.n(), ny = m.ny, P = o.d.nx * ny;
+  constexpr int threads = 32 * kInvWarps;
+  if (tid >= threads) return;
+  auto barrier = [&] {
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"n"(threads) : "memory");
+  };
   const Dims& d = o.d;
-  for (int e = tid; e < n * n; e += blockDim.x) inv_buf[(e / n) * LD + e % n] = 0.0;
-  __syncthreads();
+  for (int e = tid; e < n * n; e += threads) inv_buf[(e / n) * LD + e % n] = 0.0;
+  barrier();
   // the unknown of a plane position (compact rows of length ny) of a u or v point
   auto unknown = [&](int pos, bool ucomp) {
     const int i = pos / ny, j = pos % ny;
     return ucomp ? (i - 1) * (ny - 2) + (j - 1) : m.nu + (i - 1) * (ny - 3) + (j - 1);
   };
-  for (int r = tid; r < n; r += blockDim.x) {
+  for (int r = tid; r < n; r += threads) {
     const int pos = tab[8 * n + r], i = pos / ny, j = pos % ny;   // (tab_pos)
     int src[8];
     for (int t = 0; t < 8; ++t) src[t] = tab[8 * r + t];
@@ -1402,9 +1412,9 @@ __device__ __forceinline__ void coarse_setup_block(const Op& o, const CoarseMap&
     for (int t = 4; t < 8; ++t)
       if (src[t] != P) a[unknown(src[t], !u)] += cf[t + 1];
   }
-  __syncthreads();
+  barrier();
   double amax = 0.0;
-  for (int e = tid; e < n * n; e += blockDim.x) {
+  for (int e = tid; e < n * n; e += threads) {
     const double v = inv_buf[(e / n) * LD + e % n];
     amax = (fabs(v) > amax || v != v) ? fabs(v) : amax;
   }
@@ -1413,55 +1423,59 @@ __device__ __forceinline__ void coarse_setup_block(const Op& o, const CoarseMap&
     amax = (w > amax || w != w) ? w : amax;
   }
   if (lane == 0) wmax[warp] = amax;
-  __syncthreads();
+  barrier();
   amax = wmax[0];
-  for (int w = 1; w < (int)(blockDim.x >> 5); ++w) amax = (wmax[w] > amax || wmax[w] != wmax[w]) ? wmax[w] : amax;
+  for (int w = 1; w < kInvWarps; ++w) amax = (wmax[w] > amax || wmax[w] != wmax[w]) ? wmax[w] : amax;
   const double tiny = 1e-13 * amax;
   bool bad = !(amax > 0.0) || amax != amax;
+  static_assert(M <= 64, "two columns per lane");
   int cur = 0;
   for (int k = 0; k < n && !bad; ++k) {
     const double* a = inv_buf + cur * M * LD;
     double* b = inv_buf + (cur ^ 1) * M * LD;
-    // pivot: largest |a[r][k]|, r >= k, lowest r on ties (the same in every warp)
-    double best = -1.0;
-    int br = k;
-    for (int r = k + lane; r < n; r += 32)
-      if (fabs(a[r * LD + k]) > best) { best = fabs(a[r * LD + k]); br = r; }
-    for (int o2 = 16; o2 > 0; o2 >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, o2);
-      const int orr = __shfl_xor_sync(0xffffffffu, br, o2);
-      if (ob > best || (ob == best && orr < br)) { best = ob; br = orr; }
-    }
-    if (!(best > tiny)) { bad = true; break; }
-    const int p = br;
+    // pivot: largest |a[r][k]|, r >= k, lowest r on ties (the same in every warp; magnitudes
+    // compare like their bits, a NaN counts as zero)
+    int br = k + lane;
+    double best = br < n ? fabs(a[br * LD + k]) : 0.0;
+    const double second = br + 32 < n ? fabs(a[(br + 32) * LD + k]) : 0.0;
+    if (best != best) best = 0.0;
+    if (second > best) { best = second; br += 32; }
+    const unsigned hi = (unsigned)__double2hiint(best), top = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = hi == top ? (unsigned)__double2loint(best) : 0u, low = __reduce_max_sync(0xffffffffu, lo);
+    const bool wins = br < n && hi == top && (unsigned)__double2loint(best) == low;
+    const int p = __reduce_min_sync(0xffffffffu, wins ? br : n);
+    if (!(__hiloint2double((int)top, (int)low) > tiny)) { bad = true; break; }
     if (tid == 0) perm[k] = p;
     const double piv = a[p * LD + k];
-    for (int e = tid; e < n * n; e += blockDim.x) {
-      const int r = e / n, c = e % n;
-      const double pk = (c == k ? 1.0 : a[p * LD + c]) / piv;   // normalised pivot row
-      if (r == k) {
-        b[r * LD + c] = pk;
-      } else {
-        const int src = r == p ? k : r;   // the row that sits at r after the exchange
-        b[r * LD + c] = (c == k ? 0.0 : a[src * LD + c]) - a[src * LD + k] * pk;
+    double pk[2];   // the normalised pivot row at this lane's columns
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = lane + 32 * h;
+      if (c >= n) continue;
+      pk[h] = (c == k ? 1.0 : a[p * LD + c]) / piv;
+    }
+    for (int r = warp; r < n; r += kInvWarps) {
+      const int src = r == p ? k : r;   // the row that sits at r after the exchange
+      const double f = a[src * LD + k];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = lane + 32 * h;
+        if (c < n) b[r * LD + c] = r == k ? pk[h] : (c == k ? 0.0 : a[src * LD + c]) - f * pk[h];
       }
     }
     cur ^= 1;
-    __syncthreads();
+    barrier();
   }
-  if (!bad) {
-    double* a = inv_buf + cur * M * LD;
-    for (int k = n - 1; k >= 0; --k) {
-      const int p = perm[k];
-      if (p != k)
-        for (int r = tid; r < n; r += blockDim.x) {
-          const double t = a[r * LD + k];
-          a[r * LD + k] = a[r * LD + p];
-          a[r * LD + p] = t;
-        }
-      __syncthreads();
+  if (!bad) {   // columns back in order: the row exchanges undone from the last to the first
+    const double* a = inv_buf + cur * M * LD;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = lane + 32 * h;
+      if (c >= n) continue;
+      int from = c;
+      for (int k = 0; k < n; ++k) from = from == k ? perm[k] : (from == perm[k] ? k : from);
+      for (int r = warp; r < n; r += kInvWarps) Ainv[r * n + c] = a[r * LD + from];
     }
-    for (int e = tid; e < n * n; e += blockDim.x) Ainv[e] = a[(e / n) * LD + e % n];
   }
   if (tid == 0) *singular = bad ? 1 : 0;
 }
@@ -1846,52 +1860,62 @@ __global__ void __launch_bounds__(kSubThreads) k_subcycle(const __grid_constant_
 }
 
 // rediscretised coarse coefficients (averages of the fine ones; B scales with the cell area)
+__device__ __forceinline__ int clamp_index(int v, int hi) { return v < 0 ? 0 : (v > hi ? hi : v); }
+// weights of the full weighting, offsets -1, 0, 1 (the middle alone in a direction not coarsened)
+__device__ __forceinline__ double full_weight(int a, int f) { return f == 2 ? (a == 0 ? 0.5 : 0.25) : (a == 0 ? 1.0 : 0.0); }
+__device__ __forceinline__ double coarsen_Na(const Dims& df, int fx, int fy, const double* Na, int j, int i) {
+  double s = 0.0;   // around fine a (fy*j, fx*i)
+#pragma unroll
+  for (int a = -1; a <= 1; ++a)
+#pragma unroll
+    for (int b = -1; b <= 1; ++b) {
+      const double w = full_weight(a, fy) * full_weight(b, fx);
+      if (w != 0.0) s += w * Na[df.at(clamp_index(fy * j + a, df.ny - 1), clamp_index(fx * i + b, df.nx - 1))];
+    }
+  return s;
+}
+__device__ __forceinline__ double coarsen_Nb(const Dims& df, int fx, int fy, const double* Nb, int j, int i) {
+  double s = 0.0;   // fine b cells inside the coarse b cell
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+      if (a < fy && b < fx) s += Nb[df.at(clamp_index(fy * j + a, df.ny - 2), clamp_index(fx * i + b, df.nx - 2))];
+  return s / (double)(fy * fx);
+}
+__device__ __forceinline__ double coarsen_Bx(const Dims& df, int fx, int fy, const double* Bx, int j, int i) {
+  double s = 0.0;   // cell along x, node along y
+#pragma unroll
+  for (int a = -1; a <= 1; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const double w = full_weight(a, fy) * (1.0 / fx);
+      if (w != 0.0 && b < fx) s += w * Bx[df.at(clamp_index(fy * j + a, df.ny - 1), clamp_index(fx * i + b, df.nx - 2))];
+    }
+  return (double)(fx * fy) * s;
+}
+__device__ __forceinline__ double coarsen_By(const Dims& df, int fx, int fy, const double* By, int j, int i) {
+  double s = 0.0;   // cell along y, node along x
+#pragma unroll
+  for (int b = -1; b <= 1; ++b)
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      const double w = full_weight(b, fx) * (1.0 / fy);
+      if (w != 0.0 && a < fy) s += w * By[df.at(clamp_index(fy * j + a, df.ny - 2), clamp_index(fx * i + b, df.nx - 1))];
+    }
+  return (double)(fx * fy) * s;
+}
 __device__ __forceinline__ void coarsen_point(const Dims& df, const Dims& dc, int fx, int fy, const double* Na,
                                               const double* Nb, const double* Bx, const double* By, double* cNa,
                                               double* cNb, double* cBx, double* cBy, int j, int i) {
   const long long q = dc.at(j, i);
-  auto cl = [](int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); };
-  const double w3[3] = {0.25, 0.5, 0.25};
-  {  // N_a: full weighting around fine a (fy*j, fx*i)
-    double s = 0.0;
-    for (int a = -1; a <= 1; ++a)
-      for (int b = -1; b <= 1; ++b) {
-        const double wa = fy == 2 ? w3[a + 1] : (a == 0 ? 1.0 : 0.0);
-        const double wb = fx == 2 ? w3[b + 1] : (b == 0 ? 1.0 : 0.0);
-        if (wa == 0.0 || wb == 0.0) continue;
-        s += wa * wb * Na[df.at(cl(fy * j + a, 0, df.ny - 1), cl(fx * i + b, 0, df.nx - 1))];
-      }
-    cNa[q] = s;
-  }
-  if (j < dc.ny - 1 && i < dc.nx - 1) {  // N_b: fine b cells inside the coarse b cell
-    double s = 0.0;
-    const int na = fy, nb = fx;
-    for (int a = 0; a < na; ++a)
-      for (int b = 0; b < nb; ++b)
-        s += Nb[df.at(cl(fy * j + a, 0, df.ny - 2), cl(fx * i + b, 0, df.nx - 2))];
-    cNb[q] = s / (double)(na * nb);
-  }
-  const double area = (double)(fx * fy);
-  if (i < dc.nx - 1) {  // Bx: cell along x, node along y
-    double s = 0.0;
-    for (int a = -1; a <= 1; ++a) {
-      const double wa = fy == 2 ? w3[a + 1] : (a == 0 ? 1.0 : 0.0);
-      if (wa == 0.0) continue;
-      for (int b = 0; b < fx; ++b)
-        s += wa * (1.0 / fx) * Bx[df.at(cl(fy * j + a, 0, df.ny - 1), cl(fx * i + b, 0, df.nx - 2))];
-    }
-    cBx[q] = area * s;
-  }
-  if (j < dc.ny - 1) {  // By: cell along y, node along x
-    double s = 0.0;
-    for (int b = -1; b <= 1; ++b) {
-      const double wb = fx == 2 ? w3[b + 1] : (b == 0 ? 1.0 : 0.0);
-      if (wb == 0.0) continue;
-      for (int a = 0; a < fy; ++a)
-        s += wb * (1.0 / fy) * By[df.at(cl(fy * j + a, 0, df.ny - 2), cl(fx * i + b, 0, df.nx - 1))];
-    }
-    cBy[q] = area * s;
-  }
+  const bool jn = j < dc.ny - 1, in = i < dc.nx - 1;
+  const double na = coarsen_Na(df, fx, fy, Na, j, i), nb = jn && in ? coarsen_Nb(df, fx, fy, Nb, j, i) : 0.0;
+  const double bx = in ? coarsen_Bx(df, fx, fy, Bx, j, i) : 0.0, by = jn ? coarsen_By(df, fx, fy, By, j, i) : 0.0;
+  cNa[q] = na;
+  if (jn && in) cNb[q] = nb;
+  if (in) cBx[q] = bx;
+  if (jn) cBy[q] = by;
 }
 
 // the row types of the finest level from the SICO masks (assembly loop :1683-1727)
@@ -1983,10 +2007,12 @@ __global__ void k_level_setup(Op o, int coarsen, Dims dc, int fx, int fy, double
   }
 }
 
-// Operator set-up of the sub-cycle levels in one block: per level (one barrier each) the
-// inverse diagonals and the coefficients of the next level, then the coarsest level's
-// matrix and its inverse.  The same per-point operations as k_level_setup and
-// k_coarse_setup.
+// Operator set-up of the sub-cycle levels in one block: the first level's coefficients copied
+// to shared memory, the coarser ones' formed there level by level (a thread per point and
+// plane, one barrier per level), then every level's inverse diagonals at once, and the coarsest
+// level's matrix and its inverse.  The same per-point operations as k_level_setup.  Bound by the
+// latency of its phases: with each level's coefficients and diagonals read back from L2 level
+// by level it took 41 us on 65 x 9 points and 52 us on 36 x 21, now 21 and 28 us.
 struct SmallSetup {
   int first, last;           // the levels handled
   int direct;                // assemble and invert the coarsest level's matrix
@@ -2003,25 +2029,68 @@ struct SmallSetup {
   int fx[kMaxLevels], fy[kMaxLevels];
 };
 
-__global__ void __launch_bounds__(kInvThreads) k_small_setup(SmallSetup a) {
-  for (int l = a.first; l <= a.last; ++l) {
-    const Op& o = a.o[l];
-    const bool coarsen = l < a.last;
-    const Op& k = a.o[coarsen ? l + 1 : l];
-    const int n = o.d.nx * o.d.ny;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-      const int j = t % o.d.ny, i = t / o.d.ny;
-      const long long q = o.d.at(j, i);
-      a.idu[l][q] = u_int(o.d, j, i) ? 1.0 / diag_u(o, j, i) : 0.0;
-      a.idv[l][q] = v_int(o.d, j, i) ? 1.0 / diag_v(o, j, i) : 0.0;
-      if (coarsen && j < k.d.ny && i < k.d.nx)
-        coarsen_point(o.d, k.d, a.fx[l], a.fy[l], o.Na, o.Nb, o.Bx, o.By, const_cast<double*>(k.Na),
-                      const_cast<double*>(k.Nb), const_cast<double*>(k.Bx), const_cast<double*>(k.By), j, i);
+__global__ void __launch_bounds__(kInvThreads) k_small_setup(const __grid_constant__ SmallSetup a) {
+  extern __shared__ double sm[];   // per level compact planes of N_a, N_b, B_x, B_y; two matrices of the inverse
+  const int tid = threadIdx.x, lo = min(a.first, a.last);
+  auto points = [&](int l) { return a.o[l].d.nx * a.o[l].d.ny; };
+  auto compact = [&](int l, double* p) {   // level l's operator reading its planes at p
+    Op o = a.o[l];
+    o.d.ld = o.d.ny;
+    const int n = points(l);
+    o.Na = p; o.Nb = p + n; o.Bx = p + 2 * n; o.By = p + 3 * n;
+    return o;
+  };
+  const int n0 = points(lo);
+  for (int t = tid; t < n0; t += kInvThreads) {
+    const Op& o = a.o[lo];
+    const long long q = o.d.at(t % o.d.ny, t / o.d.ny);
+    copy8(sm + t, o.Na + q);
+    copy8(sm + n0 + t, o.Nb + q);
+    copy8(sm + 2 * n0 + t, o.Bx + q);
+    copy8(sm + 3 * n0 + t, o.By + q);
+  }
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  double* p = sm;
+  for (int l = lo; l < a.last; ++l) {   // a thread per coarse point and plane
+    const Op f = compact(l, p);
+    const int n = points(l), m = points(l + 1), ny = a.o[l + 1].d.ny, nx = a.o[l + 1].d.nx, fx = a.fx[l], fy = a.fy[l];
+    double* k = p + 4 * n;
+    for (int e = tid; e < 4 * m; e += kInvThreads) {
+      const int plane = e / m, t = e - plane * m, j = t % ny, i = t / ny;
+      const bool jn = j < ny - 1, in = i < nx - 1;
+      double v = 0.0;
+      if (plane == 0) v = coarsen_Na(f.d, fx, fy, f.Na, j, i);
+      else if (plane == 1) { if (jn && in) v = coarsen_Nb(f.d, fx, fy, f.Nb, j, i); }
+      else if (plane == 2) { if (in) v = coarsen_Bx(f.d, fx, fy, f.Bx, j, i); }
+      else if (jn) v = coarsen_By(f.d, fx, fy, f.By, j, i);
+      k[e] = v;
+      if (plane == 0 || (plane == 1 ? jn && in : plane == 2 ? in : jn)) {
+        const Op& o = a.o[l + 1];
+        const_cast<double*>(plane == 0 ? o.Na : plane == 1 ? o.Nb : plane == 2 ? o.Bx : o.By)[o.d.at(j, i)] = v;
+      }
     }
     __syncthreads();
+    p = k;
+  }
+  // inverse diagonals of all levels
+  int total = 0;
+  for (int l = a.first; l <= a.last; ++l) total += 2 * points(l);
+  for (int e = tid; e < total; e += kInvThreads) {
+    int l = a.first, t = e;
+    double* q = sm;
+    while (t >= 2 * points(l)) { t -= 2 * points(l); q += 4 * points(l); ++l; }
+    const Op o = compact(l, q);
+    const int n = points(l);
+    const bool u = t < n;
+    if (!u) t -= n;
+    const int j = t % o.d.ny, i = t / o.d.ny;
+    const long long at = a.o[l].d.at(j, i);
+    if (u) a.idu[l][at] = u_int(o.d, j, i) ? 1.0 / diag_u(o, j, i) : 0.0;
+    else a.idv[l][at] = v_int(o.d, j, i) ? 1.0 / diag_v(o, j, i) : 0.0;
   }
   const bool inv = a.inv_when == 0 || (a.inv_when == 1 && coarse_inverse_due((int)a.sc[SC_PIC_IT]));
-  if (a.direct && inv) coarse_setup_block(a.o[a.last], a.map, a.tab, a.Ainv, a.singular);
+  if (a.direct && inv) coarse_setup_block(compact(a.last, p), a.map, a.tab, p + 4 * points(a.last), a.Ainv, a.singular);
 }
 
 // ---- Krylov kernels (fine level) --------------------------------------------------
@@ -2381,7 +2450,7 @@ int solver_setup(Ctx* c, int inv_when) {
   const CoarseMap m = coarse_map(c);
   c->coarse_n = m.nu + m.nv;
   c->coarse_direct = c->coarse_n > 0 && c->coarse_n <= kCoarseDirectMax;
-  SmallSetup a;
+  SmallSetup a{};
   a.first = first_small;
   a.last = c->nlev - 1;
   a.direct = c->coarse_direct ? 1 : 0;
@@ -2398,7 +2467,9 @@ int solver_setup(Ctx* c, int inv_when) {
     a.fx[l] = a.fy[l] = 1;
     if (l < a.last) factors(c, l, &a.fx[l], &a.fy[l]);
   }
-  k_small_setup<<<1, kInvThreads, kInvSmem, c->stream>>>(a); c->launches++;
+  size_t dbl = kInvDbl;
+  for (int l = a.first < a.last ? a.first : a.last; l <= a.last; ++l) dbl += 4 * (size_t)c->lv[l].d.nx * c->lv[l].d.ny;
+  k_small_setup<<<1, kInvThreads, dbl * sizeof(double), c->stream>>>(a); c->launches++;
   DIVA_LAUNCHED(c, "k_small_setup");
   return DIVA_OK;
 }
@@ -2818,7 +2889,7 @@ int solver_init(Ctx* c) {
   if (sub_bytes(c, c->nlev - 1) > kSubSmemBudget)
     return set_error(c, DIVA_UNSUPPORTED, "coarsest multigrid level too large for the one-block sub-cycle");
   if (int st = build_sub_tables(c)) return st;
-  DIVA_CUDA(c, cudaFuncSetAttribute(k_small_setup, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem));
+  DIVA_CUDA(c, cudaFuncSetAttribute(k_small_setup, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSubSmemBudget));
   DIVA_CUDA(c, cudaFuncSetAttribute(k_subcycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSubSmemMax));
   if (int st = tile_attrs_shape<32, 32>(c)) return st;
   if (int st = tile_attrs_shape<16, 16>(c)) return st;
