@@ -109,9 +109,10 @@ __device__ __forceinline__ void block_sum(double (&v)[N]) {
 
 // ---- reductions finished by the kernel that starts them ---------------------------------
 // Blocks of 32 x 8 threads walk the points in 32 (j) x 8 (i) tiles, tile t, t + gridDim.x, ...;
-// at most kRedBlocks of them (six per SM), so that the last block's sum over the blocks'
-// partials stays at a few microseconds (one partial per tile: 23 us at 1501 x 1501).
-constexpr int kRedBlocks = 148 * 6;
+// at most kRedBlocks of them (the four that k_matvec's registers let an SM hold: with six a second
+// round starts half empty), so that the last block's sum over the blocks' partials stays at a
+// few microseconds (one partial per tile: 23 us at 1501 x 1501).
+constexpr int kRedBlocks = 148 * 4;
 inline int red_blocks(const Dims& d) {
   const int n = ((d.ny + kBX - 1) / kBX) * ((d.nx + kBY - 1) / kBY);
   return n < kRedBlocks ? n : kRedBlocks;

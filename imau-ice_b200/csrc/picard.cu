@@ -287,10 +287,29 @@ __global__ void __launch_bounds__(256) k_column_integrals(CoefArgs a) {
   const bool ice = a.mask_ice[q] == 1;
   const bool skip_visc = a.bc_margin && !ice;
   const double* __restrict__ visc = a.visc;
+  // every load ahead of the sliding law's arithmetic and of the stores
+  double etas[NZ > 0 ? NZ : 1];
+#pragma unroll
+  for (int k = 0; k < NZ; ++k) etas[k] = visc[(long long)k * d.plane + q];
+  bool frozen = false;
+  if (a.diva && a.basal_freezing) {
+    const long long ob = (long long)(nz - 1) * d.plane + q;
+    frozen = a.Tpmp[ob] - a.Ti[ob] > a.dT_freeze;
+  }
+  // sliding (calc_sliding_term_beta :924-951)
+  double ua, va;
+  if (i == 0) ua = a.u[d.at(j, 0)];
+  else if (i == nx - 1) ua = a.u[d.at(j, nx - 2)];
+  else ua = (a.u[d.at(j, i - 1)] + a.u[q]) / 2.0;
+  if (j == 0) va = a.v[d.at(0, i)];
+  else if (j == ny - 1) va = a.v[d.at(ny - 2, i)];
+  else va = (a.v[d.at(j - 1, i)] + a.v[q]) / 2.0;
+  double beta = min_ref(sliding_beta(a, q, ua, va), a.beta_max);
+  if (!a.gl_subgrid && a.mask_ocean[q] == 1) beta = 0.0;
   double vint = 0.0, fint = 0.0, vprev = 0.0, fprev = 0.0;
 #pragma unroll
   for (int k = 0; k < nz; ++k) {
-    const double eta = visc[(long long)k * d.plane + q];
+    const double eta = NZ > 0 ? etas[NZ > 0 ? k : 0] : visc[(long long)k * d.plane + q];
     const double zk = a.zt.z[k];
     if (k > 0) vint = vint + 0.5 * (eta + vprev) * (zk - a.zt.z[k - 1]);
     vprev = eta;
@@ -304,16 +323,6 @@ __global__ void __launch_bounds__(256) k_column_integrals(CoefArgs a) {
     a.visc_int[q] = vint;
     a.Na[q] = a.bc_margin ? vint * H : vint * max_ref(0.1, H);
   }
-  // sliding (calc_sliding_term_beta :924-951)
-  double ua, va;
-  if (i == 0) ua = a.u[d.at(j, 0)];
-  else if (i == nx - 1) ua = a.u[d.at(j, nx - 2)];
-  else ua = (a.u[d.at(j, i - 1)] + a.u[q]) / 2.0;
-  if (j == 0) va = a.v[d.at(0, i)];
-  else if (j == ny - 1) va = a.v[d.at(ny - 2, i)];
-  else va = (a.v[d.at(j - 1, i)] + a.v[q]) / 2.0;
-  double beta = min_ref(sliding_beta(a, q, ua, va), a.beta_max);
-  if (!a.gl_subgrid && a.mask_ocean[q] == 1) beta = 0.0;
   a.beta[q] = beta;
   if (a.diva) {
     double F2;
@@ -324,11 +333,7 @@ __global__ void __launch_bounds__(256) k_column_integrals(CoefArgs a) {
     if (a.sliding == DIVA_SLIDING_NONE) {
       be = 1.0 / F2;
     } else {
-      be = beta / (1.0 + beta * F2);
-      if (a.basal_freezing) {
-        const long long ob = (long long)(nz - 1) * d.plane + q;
-        if (a.Tpmp[ob] - a.Ti[ob] > a.dT_freeze) be = 1.0 / F2;
-      }
+      be = frozen ? 1.0 / F2 : beta / (1.0 + beta * F2);
     }
     a.beta_eff[q] = be;
   } else {
@@ -375,55 +380,64 @@ __global__ void __launch_bounds__(256) k_face_coefficients(FaceArgs a) {
   if (j >= d.ny || i >= d.nx) return;
   const long long q = d.at(j, i);
   const double dx2 = d.dx * d.dx;
-  if (i < d.nx - 1 && j < d.ny - 1) {
+  const bool cx = i < d.nx - 1, cy = j < d.ny - 1;
+  // every load before the first store
+  const long long q1 = cx ? d.at(j, i + 1) : q, q2 = cy ? d.at(j + 1, i) : q, q3 = cx && cy ? d.at(j + 1, i + 1) : q;
+  const double v0 = a.vint[q], v1 = a.vint[q1], v2 = a.vint[q2], v3 = a.vint[q3], Hb = cx && cy ? a.Hb_i[q] : 0.0;
+  const double e0 = a.beta_eff[q], e1 = a.beta_eff[q1], e2 = a.beta_eff[q2];
+  const double n0 = a.Na[q], n1 = a.Na[q1], n2 = a.Na[q2];
+  const double fx = cx && a.apply_fgrnd ? a.fcx[q] : 0.0, fy = cy && a.apply_fgrnd ? a.fcy[q] : 0.0;
+  int m0 = 1, m1 = 1, m2 = 1, m3 = 1;
+  if (a.bc_margin) {
+    m0 = a.mask_ice[q] == 1; m1 = a.mask_ice[q1] == 1; m2 = a.mask_ice[q2] == 1; m3 = a.mask_ice[q3] == 1;
+  }
+  if (cx && cy) {
     // the 3D viscosity staggered to the b-grid and integrated over the column (:820-874).
     // The staggering is a fixed weighting of the four corner columns and the trapezoid rule
     // is linear, so the integral is the same weighting of the corners' integrals (equal up
     // to rounding): the 3D viscosity is not read again.
-    const long long q1 = d.at(j, i + 1), q2 = d.at(j + 1, i), q3 = d.at(j + 1, i + 1);
     double s;
     if (a.bc_margin) {
-      const int m0 = a.mask_ice[q] == 1, m1 = a.mask_ice[q1] == 1, m2 = a.mask_ice[q2] == 1, m3 = a.mask_ice[q3] == 1;
       const double w = (double)m0 + (double)m1 + (double)m2 + (double)m3;
       double vb = 0.0;
-      if (m0) vb = vb + a.vint[q];
-      if (m1) vb = vb + a.vint[q1];
-      if (m2) vb = vb + a.vint[q2];
-      if (m3) vb = vb + a.vint[q3];
+      if (m0) vb = vb + v0;
+      if (m1) vb = vb + v1;
+      if (m2) vb = vb + v2;
+      if (m3) vb = vb + v3;
       s = w > 0.0 ? vb / w : 0.0;
     } else {
-      s = (a.vint[q] + a.vint[q1] + a.vint[q2] + a.vint[q3]) / 4.0;
+      s = (v0 + v1 + v2 + v3) / 4.0;
     }
     a.visc_int_b[q] = s;
-    const double nb = a.bc_margin ? s * a.Hb_i[q] : s * max_ref(0.1, a.Hb_i[q]);
+    const double nb = a.bc_margin ? s * Hb : s * max_ref(0.1, Hb);
     a.Nb[q] = nb;
     a.lvNb[q] = a.crossterms ? nb : 1.0;
   }
-  if (i < d.nx - 1) {
-    double b = (a.beta_eff[q] + a.beta_eff[d.at(j, i + 1)]) / 2.0;
-    if (a.apply_fgrnd) b = b * (a.fcx[q] * a.fcx[q]);
+  if (cx) {
+    double b = (e0 + e1) / 2.0;
+    if (a.apply_fgrnd) b = b * (fx * fx);
     a.bex[q] = b;
     if (a.crossterms) {
       a.lvBx[q] = b * dx2;
     } else {
-      const double ncx = (a.Na[q] + a.Na[d.at(j, i + 1)]) / 2.0;
+      const double ncx = (n0 + n1) / 2.0;
       a.Ncx[q] = ncx;
       a.lvBx[q] = dx2 * b / ncx;
     }
   }
-  if (j < d.ny - 1) {
-    double b = (a.beta_eff[q] + a.beta_eff[d.at(j + 1, i)]) / 2.0;
-    if (a.apply_fgrnd) b = b * (a.fcy[q] * a.fcy[q]);
+  if (cy) {
+    double b = (e0 + e2) / 2.0;
+    if (a.apply_fgrnd) b = b * (fy * fy);
     a.bey[q] = b;
     if (a.crossterms) {
       a.lvBy[q] = b * dx2;
     } else {
-      const double ncy = (a.Na[q] + a.Na[d.at(j + 1, i)]) / 2.0;
+      const double ncy = (n0 + n2) / 2.0;
       a.Ncy[q] = ncy;
       a.lvBy[q] = dx2 * b / ncy;
     }
   }
-  a.lvNa[q] = a.crossterms ? a.Na[q] : 1.0;
+  a.lvNa[q] = a.crossterms ? n0 : 1.0;
 }
 
 // 0.5 * A^(-1/n): constant over one solve, so the pow of A is taken once per solve
@@ -563,79 +577,55 @@ __global__ void __launch_bounds__(256) k_picard_update(UpdArgs a) {
   double sums[3] = {0.0, 0.0, 0.0};
   const bool commit = a.commit < 0 ? a.sc[SC_PIC_IT] > 1.0 : a.commit != 0;
   FOR_TILES(d) {
-    const int nx = d.nx, ny = d.ny;
     const long long q = d.at(j, i);
+    const bool cx = i < d.nx - 1, cy = j < d.ny - 1, aa = a.aa_m > 0, off = aa && a.sc[SC_AA_OFF] != 0.0;
+    // every load of the point's two faces, then their stores
     bool frozen = false;
     if (a.diva && a.basal_freezing) {
       const long long ob = (long long)(d.nz - 1) * d.plane + q;
       frozen = a.Tpmp[ob] - a.Ti[ob] > a.dT_freeze;
     }
-    if (i < nx - 1) {
-      const double uo = a.u[q];
-      double un;
-      if (a.aa_m > 0 && a.sc[SC_AA_OFF] != 0.0) {
-        un = a.rel * a.gu[q] + (1.0 - a.rel) * uo;   // mixing given up: the relaxation of g
-      } else if (a.aa_m > 0) {
-        un = a.gu[q];
-        for (int k = 0; k < a.aa_m; ++k) un -= a.sc[SC_AA_GAMMA + k] * a.dGu[k][q];
-      } else {
-        un = limited_u(d, a.xu, a.xv, a.vmax, j, i);
-        un = a.rel * un + (1.0 - a.rel) * uo;
-      }
-      a.up[q] = uo;
-      a.u[q] = un;
-      if (fabs(un) > kVelTol) {
+    const bool base = a.diva && !a.sliding_none;
+    const double F20 = base ? a.F2[q] : 0.0, H0 = base ? a.Hi[q] : 0.0;
+    struct Face { double old, now, last, chk, be, F2; } f[2] = {};
+    auto read = [&](Face& f, const double* x, const double* g, const double* const* dG, const double* chk,
+                    const double* err, const double* be, long long q1, auto limited) {
+      f.old = x[q];
+      if (aa) f.now = g[q];
+      else f.now = limited();
+      if (aa && !off)
+        for (int k = 0; k < a.aa_m; ++k) f.now -= a.sc[SC_AA_GAMMA + k] * dG[k][q];
+      else
+        f.now = a.rel * f.now + (1.0 - a.rel) * f.old;   // (mixing given up: the relaxation of g)
+      f.last = commit ? err[q] : 0.0;
+      f.chk = a.diva ? f.now : chk[q];
+      f.be = a.diva ? be[q] : 0.0;
+      f.F2 = base ? stag_margin(F20, a.F2[q1], H0, a.Hi[q1]) : 0.0;
+    };
+    if (cx)
+      read(f[0], a.u, a.gu, a.dGu, a.uchk, a.errx, a.bex, d.at(j, i + 1),
+           [&] { return limited_u(d, a.xu, a.xv, a.vmax, j, i); });
+    if (cy)
+      read(f[1], a.v, a.gv, a.dGv, a.vchk, a.erry, a.bey, d.at(j + 1, i),
+           [&] { return limited_v(d, a.xu, a.xv, a.vmax, j, i); });
+    auto write = [&](const Face& f, double* x, double* prev, double* err, double* fe, double* taub, double* ub) {
+      prev[q] = f.old;
+      x[q] = f.now;
+      if (fabs(f.now) > kVelTol) {
         sums[2] += 1.0;
-        sums[0] += (un - uo) * (un - uo);
-        sums[1] += (un + uo) * (un + uo);
+        sums[0] += (f.now - f.old) * (f.now - f.old);
+        sums[1] += (f.now + f.old) * (f.now + f.old);
       }
-      const double chk = a.diva ? un : a.uchk[q];
-      if (commit) a.fex[q] = a.errx[q];
-      a.errx[q] = (fabs(chk) > kVelTol) ? 2.0 * fabs(un - uo) / fabs(un + uo + 1E-5) : 0.0;
+      if (commit) fe[q] = f.last;
+      err[q] = (fabs(f.chk) > kVelTol) ? 2.0 * fabs(f.now - f.old) / fabs(f.now + f.old + 1E-5) : 0.0;
       if (a.diva) {
-        const double tb = a.bex[q] * un;
-        a.taubx[q] = tb;
-        if (a.sliding_none) {
-          a.ubx[q] = 0.0;
-        } else {
-          const double F2s = stag_margin(a.F2[q], a.F2[d.at(j, i + 1)], a.Hi[q], a.Hi[d.at(j, i + 1)]);
-          a.ubx[q] = frozen ? 0.0 : un - tb * F2s;
-        }
+        const double tb = f.be * f.now;
+        taub[q] = tb;
+        ub[q] = a.sliding_none || frozen ? 0.0 : f.now - tb * f.F2;
       }
-    }
-    if (j < ny - 1) {
-      const double vo = a.v[q];
-      double vn;
-      if (a.aa_m > 0 && a.sc[SC_AA_OFF] != 0.0) {
-        vn = a.rel * a.gv[q] + (1.0 - a.rel) * vo;
-      } else if (a.aa_m > 0) {
-        vn = a.gv[q];
-        for (int k = 0; k < a.aa_m; ++k) vn -= a.sc[SC_AA_GAMMA + k] * a.dGv[k][q];
-      } else {
-        vn = limited_v(d, a.xu, a.xv, a.vmax, j, i);
-        vn = a.rel * vn + (1.0 - a.rel) * vo;
-      }
-      a.vp[q] = vo;
-      a.v[q] = vn;
-      if (fabs(vn) > kVelTol) {
-        sums[2] += 1.0;
-        sums[0] += (vn - vo) * (vn - vo);
-        sums[1] += (vn + vo) * (vn + vo);
-      }
-      const double chk = a.diva ? vn : a.vchk[q];
-      if (commit) a.fey[q] = a.erry[q];
-      a.erry[q] = (fabs(chk) > kVelTol) ? 2.0 * fabs(vn - vo) / fabs(vn + vo + 1E-5) : 0.0;
-      if (a.diva) {
-        const double tb = a.bey[q] * vn;
-        a.tauby[q] = tb;
-        if (a.sliding_none) {
-          a.vby[q] = 0.0;
-        } else {
-          const double F2s = stag_margin(a.F2[q], a.F2[d.at(j + 1, i)], a.Hi[q], a.Hi[d.at(j + 1, i)]);
-          a.vby[q] = frozen ? 0.0 : vn - tb * F2s;
-        }
-      }
-    }
+    };
+    if (cx) write(f[0], a.u, a.up, a.errx, a.fex, a.taubx, a.ubx);
+    if (cy) write(f[1], a.v, a.vp, a.erry, a.fey, a.tauby, a.vby);
   }
   if (!reduce_all(sums, a.red)) return;
   double* sc = a.sc;

@@ -1981,29 +1981,38 @@ __global__ void k_level_setup(Op o, int coarsen, Dims dc, int fx, int fy, double
   IDX2D
   if (j >= o.d.ny || i >= o.d.nx) return;
   const long long q = o.d.at(j, i);
-  idu[q] = u_int(o.d, j, i) ? 1.0 / diag_u(o, j, i) : 0.0;
-  idv[q] = v_int(o.d, j, i) ? 1.0 / diag_v(o, j, i) : 0.0;
-  if (f32.Na) {
-    f32.Na[q] = (float)o.Na[q];
-    f32.Nb[q] = (float)o.Nb[q];
-    f32.Bx[q] = (float)o.Bx[q];
-    f32.By[q] = (float)o.By[q];
-    f32.idu[q] = (float)idu[q];
-    f32.idv[q] = (float)idv[q];
-  }
-  if (coarsen && j < dc.ny && i < dc.nx)
-    coarsen_point(o.d, dc, fx, fy, o.Na, o.Nb, o.Bx, o.By, cNa, cNb, cBx, cBy, j, i);
+  // every load before the first store
+  const bool ui = u_int(o.d, j, i), vi = v_int(o.d, j, i);
+  const double iu = ui ? 1.0 / diag_u(o, j, i) : 0.0, iv = vi ? 1.0 / diag_v(o, j, i) : 0.0;
+  double b0 = 0.0, b1 = 0.0;
   if (rhs.on) {
     const double dx2 = o.d.dx * o.d.dx;
-    rhs.bu[q] = u_int(o.d, j, i) ? (rhs.crossterms ? -rhs.tdx[q] * dx2 : -rhs.tdx[q] * dx2 / rhs.Ncx[q]) : 0.0;
-    rhs.bv[q] = v_int(o.d, j, i) ? (rhs.crossterms ? -rhs.tdy[q] * dx2 : -rhs.tdy[q] * dx2 / rhs.Ncy[q]) : 0.0;
+    if (ui) b0 = rhs.crossterms ? -rhs.tdx[q] * dx2 : -rhs.tdx[q] * dx2 / rhs.Ncx[q];
+    if (vi) b1 = rhs.crossterms ? -rhs.tdy[q] * dx2 : -rhs.tdy[q] * dx2 / rhs.Ncy[q];
     if (rhs.rtu) {
       const int tu = rhs.rtu[q], tv = rhs.rtv[q];
-      if (tu == RT_IDENT) rhs.bu[q] = 0.0;
-      else if (tu != RT_FREE) rhs.bu[q] = front_stress(rhs, o.d.at(j, tu == RT_MARGIN_LO ? i : i + 1));
-      if (tv == RT_IDENT) rhs.bv[q] = 0.0;
-      else if (tv != RT_FREE) rhs.bv[q] = front_stress(rhs, o.d.at(tv == RT_MARGIN_LO ? j : j + 1, i));
+      if (tu == RT_IDENT) b0 = 0.0;
+      else if (tu != RT_FREE) b0 = front_stress(rhs, o.d.at(j, tu == RT_MARGIN_LO ? i : i + 1));
+      if (tv == RT_IDENT) b1 = 0.0;
+      else if (tv != RT_FREE) b1 = front_stress(rhs, o.d.at(tv == RT_MARGIN_LO ? j : j + 1, i));
     }
+  }
+  const double na = f32.Na ? o.Na[q] : 0.0, nb = f32.Na ? o.Nb[q] : 0.0, bx = f32.Na ? o.Bx[q] : 0.0, by = f32.Na ? o.By[q] : 0.0;
+  if (coarsen && j < dc.ny && i < dc.nx)   // (its loads, then its stores: other planes than those below)
+    coarsen_point(o.d, dc, fx, fy, o.Na, o.Nb, o.Bx, o.By, cNa, cNb, cBx, cBy, j, i);
+  idu[q] = iu;
+  idv[q] = iv;
+  if (f32.Na) {
+    f32.Na[q] = (float)na;
+    f32.Nb[q] = (float)nb;
+    f32.Bx[q] = (float)bx;
+    f32.By[q] = (float)by;
+    f32.idu[q] = (float)iu;
+    f32.idv[q] = (float)iv;
+  }
+  if (rhs.on) {
+    rhs.bu[q] = b0;
+    rhs.bv[q] = b1;
   }
 }
 
@@ -2118,7 +2127,9 @@ __device__ __forceinline__ double Av_any(const Op& o, const double* xu, const do
 
 // out = A x ; dots [0] w.out, [1] out.out ; then the scalar step
 enum { ST_NONE = 0, ST_ALPHA, ST_OMEGA };
-__global__ void __launch_bounds__(256) k_matvec(Op o, const double* xu, const double* xv, double* ou, double* ov,
+// (Four blocks per SM: at the compiler's own choice of 98 registers two fit, too few loads in
+// flight; with kRedBlocks 90 -> 55 us on 1501 x 1501, 14.5 -> 12.4 us on 321 x 561.)
+__global__ void __launch_bounds__(256, 4) k_matvec(Op o, const double* xu, const double* xv, double* ou, double* ov,
                                                 const double* wu, const double* wv, Reduction red, double* sc,
                                                 int stage) {
   double acc[kPW] = {};
@@ -2153,7 +2164,8 @@ struct RelresTest {   // the stop test of a graph-launched iteration (h: IF(solv
   double tol;
   cudaGraphConditionalHandle h;
 };
-__global__ void __launch_bounds__(256) k_init_residual(Op o, const double* u, const double* v, const double* bu,
+// (Every load of a point before its first store: the compiler moves none over a store.)
+__global__ void __launch_bounds__(256, 4) k_init_residual(Op o, const double* u, const double* v, const double* bu,
                                                        const double* bv, double* xu, double* xv, double* ru,
                                                        double* rv, double* hu, double* hv, double* pu, double* pv,
                                                        int raw, Reduction red, double* sc, RelresTest test) {
@@ -2161,32 +2173,30 @@ __global__ void __launch_bounds__(256) k_init_residual(Op o, const double* u, co
   FOR_TILES(o.d) {
     const long long q = o.d.at(j, i);
     const bool deep = rows_deep(o.d, j, i);
-    xu[q] = u[q];
-    xv[q] = v[q];
-    double r = 0.0, w = 0.0;
+    const double u0 = u[q], v0 = v[q];
+    double r0 = 0.0, w0 = 0.0, b0 = 0.0, r1 = 0.0, w1 = 0.0, b1 = 0.0;
     if (u_int(o.d, j, i)) {
-      const double b = bu[q];
-      r = b - Au_any(o, u, v, j, i, deep);
-      w = (deep || !raw) ? r : b - Au<true>(o, u, v, j, i);
-      acc[1] += b * b;
+      b0 = bu[q];
+      r0 = b0 - Au_any(o, u, v, j, i, deep);
+      w0 = (deep || !raw) ? r0 : b0 - Au<true>(o, u, v, j, i);
     } else if (raw && i < o.d.nx - 1) {
-      w = LU(o, u, j, i) - u[q];
+      w0 = LU(o, u, j, i) - u0;
     }
-    acc[0] += w * w;
-    acc[2] += r * r;
-    ru[q] = r; hu[q] = r; pu[q] = r;
-    r = w = 0.0;
     if (v_int(o.d, j, i)) {
-      const double b = bv[q];
-      r = b - Av_any(o, u, v, j, i, deep);
-      w = (deep || !raw) ? r : b - Av<true>(o, u, v, j, i);
-      acc[1] += b * b;
+      b1 = bv[q];
+      r1 = b1 - Av_any(o, u, v, j, i, deep);
+      w1 = (deep || !raw) ? r1 : b1 - Av<true>(o, u, v, j, i);
     } else if (raw && j < o.d.ny - 1) {
-      w = LV(o, v, j, i) - v[q];
+      w1 = LV(o, v, j, i) - v0;
     }
-    acc[0] += w * w;
-    acc[2] += r * r;
-    rv[q] = r; hv[q] = r; pv[q] = r;
+    acc[0] += w0 * w0;
+    acc[1] += b0 * b0;
+    acc[2] += r0 * r0;
+    acc[0] += w1 * w1;
+    acc[1] += b1 * b1;
+    acc[2] += r1 * r1;
+    xu[q] = u0; ru[q] = r0; hu[q] = r0; pu[q] = r0;
+    xv[q] = v0; rv[q] = r1; hv[q] = r1; pv[q] = r1;
   }
   if (!reduce_all(acc, red)) return;
   const double rr = acc[0], bb = acc[1];
@@ -2256,19 +2266,29 @@ __global__ void __launch_bounds__(256) k_update_xr(Dims d, double* sc, double* x
   const double alpha = sc[SC_ALPHA], omega = sc[SC_OMEGA];
   FOR_TILES(d) {
     const long long q = d.at(j, i);
-    if (u_int(d, j, i)) {
-      xu[q] += alpha * phu[q] + omega * shu[q];
-      const double r = su[q] - omega * tu[q];
-      ru[q] = r;
-      acc[0] += hu[q] * r;
-      acc[1] += r * r;
+    const bool ui = u_int(d, j, i), vi = v_int(d, j, i);
+    double x0 = 0.0, r0 = 0.0, h0 = 0.0, x1 = 0.0, r1 = 0.0, h1 = 0.0;   // (loads before stores)
+    if (ui) {
+      x0 = xu[q] + (alpha * phu[q] + omega * shu[q]);
+      r0 = su[q] - omega * tu[q];
+      h0 = hu[q];
     }
-    if (v_int(d, j, i)) {
-      xv[q] += alpha * phv[q] + omega * shv[q];
-      const double r = sv[q] - omega * tv[q];
-      rv[q] = r;
-      acc[0] += hv[q] * r;
-      acc[1] += r * r;
+    if (vi) {
+      x1 = xv[q] + (alpha * phv[q] + omega * shv[q]);
+      r1 = sv[q] - omega * tv[q];
+      h1 = hv[q];
+    }
+    if (ui) {
+      xu[q] = x0;
+      ru[q] = r0;
+      acc[0] += h0 * r0;
+      acc[1] += r0 * r0;
+    }
+    if (vi) {
+      xv[q] = x1;
+      rv[q] = r1;
+      acc[0] += h1 * r1;
+      acc[1] += r1 * r1;
     }
   }
   if (!reduce_all(acc, red)) return;
@@ -2290,8 +2310,9 @@ __global__ void k_update_p(Dims d, const double* sc, const double* ru, const dou
   if (j >= d.ny || i >= d.nx) return;
   const long long q = d.at(j, i);
   const double beta = sc[SC_BETA], omega = sc[SC_OMEGA];
-  pu[q] = ru[q] + beta * (pu[q] - omega * vu[q]);
-  pv[q] = rv[q] + beta * (pv[q] - omega * vv[q]);
+  const double a = ru[q] + beta * (pu[q] - omega * vu[q]), b = rv[q] + beta * (pv[q] - omega * vv[q]);
+  pu[q] = a;
+  pv[q] = b;
 }
 
 // The solution of a linear solve: x, plus alpha phat when it ended at a half step (half 1; 0:
