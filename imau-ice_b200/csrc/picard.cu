@@ -137,15 +137,10 @@ __device__ __forceinline__ int margin_mode(double H0, double H1) {
   if (H0 == 0.0 && H1 > 0.0) return 2;
   return 0;
 }
-// calc_staggered_margin with the side choice made beforehand (same values as stag_margin)
-__device__ __forceinline__ double stag_mode(int mode, double v0, double v1) {
-  return mode == 1 ? v0 : (mode == 2 ? v1 : 0.5 * (v0 + v1));
-}
-
 // K1 in three launches.  (a) k_column_prep, one thread per column: the strain rates
 // of the depth-averaged flow and which of the column's four shear faces have ice.
-// (b) k_layer_viscosity, one thread per (column, layer), a warp over 32 neighbouring
-// rows j of one grid column i and one layer: the shear of the column's own east and
+// (b) k_layer_viscosity, one thread per column and kViscLayers layers, a warp over 32
+// neighbouring rows j of one grid column i: the shear of the column's own east and
 // north faces, the west face, and the south face as the north face of the lane below
 // (shuffle), then the viscosity of the layer.  (c) k_column_integrals, one thread per
 // column: the vertical integrals in layer order (as the sequential quadrature does), N_a,
@@ -204,6 +199,7 @@ __global__ void __launch_bounds__(256) k_column_prep(CoefArgs a) {
 // The layer step's arithmetic type R: double, or float for precision 'mixed' (the
 // viscosity of the linearisation in FP32: face shears, strain rate, the rate factor's
 // power and the viscosity bound; inputs and the stored viscosity stay FP64 fields).
+// (calc_staggered_margin with the side choice made beforehand: same values as stag_margin)
 template <class R> __device__ __forceinline__ R stag_mode_t(int mode, R v0, R v1) {
   return mode == 1 ? v0 : (mode == 2 ? v1 : R(0.5) * (v0 + v1));
 }
@@ -213,65 +209,102 @@ __device__ __forceinline__ float rcbrt_t(float x) { return rcbrtf(x); }
 __device__ __forceinline__ double pow_t(double x, double y) { return pow(x, y); }
 __device__ __forceinline__ float pow_t(float x, float y) { return powf(x, y); }
 
+// A thread takes kViscLayers layers of its column, whose loads are in flight together and share
+// the column's flags and basal stress.  All of K1 in FP64, one
+// layer a thread against three: 76.8 / 72.5 us on 321 x 561, 780 / 687 us on 1501 x 1501, 23.5 /
+// 24.6 us on 129 x 17 (five layers: 84.9, 804, 27.8: too few warps for their registers).
+constexpr int kViscLayers = 3;
 template <bool WRITE_SHEAR, class R>
 __global__ void __launch_bounds__(kColLanes * kColRows) k_layer_viscosity(CoefArgs a) {
+  constexpr int L = kViscLayers;
   const Dims d = a.d;
-  const int lane = threadIdx.x;
-  // the layer is the fastest grid index: blocks running together share their columns'
+  const int lane = threadIdx.x, y = threadIdx.y;
+  // the layers are the fastest grid index: blocks running together share their columns'
   // 2D inputs in L1/L2 instead of streaming them once per layer
-  const int k = blockIdx.x, j = blockIdx.y * kColLanes + lane, i = blockIdx.z * kColRows + threadIdx.y;
+  const int k0 = blockIdx.x * L, j = blockIdx.y * kColLanes + lane, i = blockIdx.z * kColRows + y;
   const bool row = i < d.nx;   // whole warps: i is uniform across a warp; idle warps stay for the barrier
   const bool col = row && j < d.ny;   // lanes past the last row stay for the shuffle
   const int nx = d.nx, ny = d.ny, ld = d.ld;
   const int q = (row ? i : nx - 1) * ld + (j < ny ? j : ny - 1);   // plane index (planes hold < 2^31 points)
-  const long long off = (long long)k * d.plane;
-  const double* __restrict__ vp = a.visc_prev + off;
-  const R zk = (R)a.zt.z[k];
   const int flags = a.col_flags[q];
   const bool has_e = col && i < nx - 1, has_w = col && i > 0, has_n = col && j < ny - 1, has_s = col && j > 0;
+  const bool on_e = has_e && (flags & FACE_E), on_n = has_n && (flags & FACE_N);
+  const bool on_w = has_w && (flags & FACE_W), on_s = has_s && (flags & FACE_S);
+  const bool skip = flags & COL_SKIP;
   auto mode = [&](int f) { return (flags >> (kModeShift + 2 * f)) & 3; };
-  auto shear = [&](double tb, double v0, double v1, int m) { return ((R)tb / stag_mode_t<R>(m, (R)v0, (R)v1)) * zk; };
+  auto shear = [](double tb, double v0, double v1, int m, R zk) { return ((R)tb / stag_mode_t<R>(m, (R)v0, (R)v1)) * zk; };
+  auto layer = [&](int e) { return k0 + e < d.nz ? k0 + e : d.nz - 1; };   // (the last again where there are fewer)
+  const double eps = skip ? 0.0 : a.col_eps[q];
+  double af[L];
+#pragma unroll
+  for (int e = 0; e < L; ++e) af[e] = a.afac[layer(e) * d.plane + q];
   // the west face of column i is the east face of column i-1: the warp below in the block
-  // computed it (the same operands, so the same value), the block's first warp computes it
-  __shared__ R east[kColRows][kColLanes];
-  R dudz_e = R(0), dvdz_n = R(0), dvdz_s = R(0), dudz_w = R(0);
+  // computed it (the same operands, so the same value), the block's first warp computes it;
+  // the south face of row j is the north face of row j-1, the lane below's
+  __shared__ R east[L][kColRows][kColLanes];
+  R dudz_e[L] = {}, dvdz_n[L] = {}, dvdz_s[L] = {}, dudz_w[L] = {};
   if (a.diva) {
-    const double vq = vp[q];
-    if (has_e) {
-      if (flags & FACE_E) dudz_e = shear(a.taub_cx[q], vq, vp[q + ld], mode(0));
-      if (WRITE_SHEAR) a.dudz[off + q] = (double)dudz_e;
+    const double te = on_e ? a.taub_cx[q] : 0.0, tn = on_n ? a.taub_cy[q] : 0.0;
+    const bool edge_w = y == 0 && on_w, edge_s = lane == 0 && on_s;
+    const double tw = edge_w ? a.taub_cx[q - ld] : 0.0, ts = edge_s ? a.taub_cy[q - 1] : 0.0;
+    double vq[L], ve[L], vn[L], vw[L], vs[L];
+#pragma unroll
+    for (int e = 0; e < L; ++e) {
+      const double* __restrict__ vp = a.visc_prev + layer(e) * d.plane;
+      vq[e] = vp[q];
+      ve[e] = on_e ? vp[q + ld] : 0.0;
+      vn[e] = on_n ? vp[q + 1] : 0.0;
+      vw[e] = edge_w ? vp[q - ld] : 0.0;
+      vs[e] = edge_s ? vp[q - 1] : 0.0;
     }
-    east[threadIdx.y][lane] = dudz_e;
-    if (has_n) {
-      if (flags & FACE_N) dvdz_n = shear(a.taub_cy[q], vq, vp[q + 1], mode(2));
-      if (WRITE_SHEAR) a.dvdz[off + q] = (double)dvdz_n;
+#pragma unroll
+    for (int e = 0; e < L; ++e) {
+      const R zk = (R)a.zt.z[layer(e)];
+      if (on_e) dudz_e[e] = shear(te, vq[e], ve[e], mode(0), zk);
+      if (on_n) dvdz_n[e] = shear(tn, vq[e], vn[e], mode(2), zk);
+      if (edge_w) dudz_w[e] = shear(tw, vw[e], vq[e], mode(1), zk);
+      if (edge_s) dvdz_s[e] = shear(ts, vs[e], vq[e], mode(3), zk);
+      east[e][y][lane] = dudz_e[e];
+      if (WRITE_SHEAR && k0 + e < d.nz) {
+        const long long o = (k0 + e) * d.plane + q;
+        if (has_e) a.dudz[o] = (double)dudz_e[e];
+        if (has_n) a.dvdz[o] = (double)dvdz_n[e];
+      }
     }
-    dvdz_s = __shfl_up_sync(0xffffffffu, dvdz_n, 1);   // north face of row j-1
-    if (lane == 0 && has_s) dvdz_s = (flags & FACE_S) ? shear(a.taub_cy[q - 1], vp[q - 1], vq, mode(3)) : R(0);
     __syncthreads();
-    if (has_w && (flags & FACE_W))
-      dudz_w = threadIdx.y > 0 ? east[threadIdx.y - 1][lane] : shear(a.taub_cx[q - ld], vp[q - ld], vq, mode(1));
+#pragma unroll
+    for (int e = 0; e < L; ++e) {
+      const R below = __shfl_up_sync(0xffffffffu, dvdz_n[e], 1);
+      if (lane > 0) dvdz_s[e] = below;
+      if (y > 0 && on_w) dudz_w[e] = east[e][y - 1][lane];
+    }
   }
   if (!col) return;
-  R eta = R(0);
-  if (!(flags & COL_SKIP)) {
-    const int mx = (flags >> kStagXShift) & 3, my = (flags >> kStagYShift) & 3;
-    R du_dz_a, dv_dz_a;
-    if (a.diva) {
-      du_dz_a = stag_mode_t<R>(mx, dudz_w, dudz_e);
-      dv_dz_a = stag_mode_t<R>(my, dvdz_s, dvdz_n);
-    } else {
-      // solve_SSA calls calc_effective_viscosity without refreshing du/dz: use the stored fields
-      const double* dudz = a.dudz + off;
-      const double* dvdz = a.dvdz + off;
-      du_dz_a = stag_mode_t<R>(mx, (R)(i > 0 ? dudz[q - ld] : 0.0), (R)(i < nx - 1 ? dudz[q] : 0.0));
-      dv_dz_a = stag_mode_t<R>(my, (R)(j > 0 ? dvdz[q - 1] : 0.0), (R)(j < ny - 1 ? dvdz[q] : 0.0));
+  const int mx = (flags >> kStagXShift) & 3, my = (flags >> kStagYShift) & 3;
+  const R flow = a.n_is_3 ? R(0) : (R)((1.0 - a.n_flow) / (2.0 * a.n_flow));
+#pragma unroll
+  for (int e = 0; e < L; ++e) {
+    if (k0 + e >= d.nz) break;
+    const long long off = (k0 + e) * d.plane;
+    R eta = R(0);
+    if (!skip) {
+      R du_dz_a, dv_dz_a;
+      if (a.diva) {
+        du_dz_a = stag_mode_t<R>(mx, dudz_w[e], dudz_e[e]);
+        dv_dz_a = stag_mode_t<R>(my, dvdz_s[e], dvdz_n[e]);
+      } else {
+        // solve_SSA calls calc_effective_viscosity without refreshing du/dz: use the stored fields
+        const double* dudz = a.dudz + off;
+        const double* dvdz = a.dvdz + off;
+        du_dz_a = stag_mode_t<R>(mx, (R)(i > 0 ? dudz[q - ld] : 0.0), (R)(i < nx - 1 ? dudz[q] : 0.0));
+        dv_dz_a = stag_mode_t<R>(my, (R)(j > 0 ? dvdz[q - 1] : 0.0), (R)(j < ny - 1 ? dvdz[q] : 0.0));
+      }
+      const R eps_sq = (R)eps + R(0.25) * (du_dz_a * du_dz_a + dv_dz_a * dv_dz_a) + (R)a.eps0;
+      const R pe = a.n_is_3 ? rcbrt_t(eps_sq) : pow_t(eps_sq, flow);
+      eta = max_ref_t<R>((R)af[e] * pe, (R)a.visc_min);   // NaN (first cold iteration) -> visc_min
     }
-    const R eps_sq = (R)a.col_eps[q] + R(0.25) * (du_dz_a * du_dz_a + dv_dz_a * dv_dz_a) + (R)a.eps0;
-    const R pe = a.n_is_3 ? rcbrt_t(eps_sq) : pow_t(eps_sq, (R)((1.0 - a.n_flow) / (2.0 * a.n_flow)));
-    eta = max_ref_t<R>((R)a.afac[off + q] * pe, (R)a.visc_min);   // NaN (first cold iteration) -> visc_min
+    a.visc[off + q] = (double)eta;
   }
-  a.visc[off + q] = (double)eta;
 }
 
 // NZ > 0: the layer count known at compile time (the default 15 layers), so the loop is
@@ -1067,7 +1100,8 @@ int launch_diva_coefficients(Ctx* c, const double* u, const double* v, bool diva
   k_column_prep<<<G2>>>(a); c->launches++;
   {
     const dim3 block(kColLanes, kColRows);
-    const dim3 grid(c->d.nz, (c->d.ny + kColLanes - 1) / kColLanes, (c->d.nx + kColRows - 1) / kColRows);
+    const dim3 grid((c->d.nz + kViscLayers - 1) / kViscLayers, (c->d.ny + kColLanes - 1) / kColLanes,
+                    (c->d.nx + kColRows - 1) / kColRows);
     const bool f32 = k1_fp32(C);
     if (what == K1_WRITE_SHEAR) {
       if (f32) k_layer_viscosity<true, float><<<grid, block, 0, c->stream>>>(a);
