@@ -370,7 +370,7 @@ int picard(Ctx* c, bool diva, double* u, double* v, diva_report_t* rep) {
     if ((st = solver_setup(c, coarse_inverse_due(it) ? 0 : 2))) return st;
     if (relmode) {
       if ((st = solver_relres(c, u, v, &relres))) return st;
-      eta = eta_after(eta, relres, relres_prev, C.picard_relres_tol);   // as the graph's k_ctl_relres does
+      eta = eta_after(eta, relres, relres_prev, C.picard_relres_tol);   // as the graph's k_init_residual does
       relres_prev = relres;
       if (!std::isfinite(relres)) return set_error(c, DIVA_NAN_DETECTED, "NaN in the nonlinear residual");
       const bool stop_stall = relres > C.picard_relres_tol &&

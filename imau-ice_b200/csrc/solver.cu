@@ -20,8 +20,8 @@
 //     restriction = transpose of prolongation;
 //   * smoothing is 4-colour Gauss-Seidel (u red/black, v red/black), with the
 //     exact diagonal of the reduced system;
-//   * the larger levels are smoothed by tile kernels (two launches per level and
-//     V-cycle, halo recomputed instead of exchanged), the coarse levels whose
+//   * the larger levels are smoothed by tile kernels, the largest of them in streamed strips
+//     (two launches per level and V-cycle, halo recomputed instead of exchanged), the coarse levels whose
 //     data fit in 200 KB run out of one thread block's shared memory (one launch
 //     per V-cycle), and the coarsest level is solved directly with its inverse,
 //     formed once per viscosity iteration.
@@ -146,8 +146,8 @@ __device__ __forceinline__ double LV(const Op& o, const double* x, int j, int i)
 }
 
 // Sum of the nine stencil terms, accumulated with explicit fused multiply-adds in a
-// fixed order, so every code path (boundary-mapped reads, plain reads, the row
-// tables of the sub-cycle) rounds identically whatever the compiler would contract.
+// fixed order, so every code path of a level (boundary-mapped reads, plain reads, tiles, the
+// ring) rounds identically whatever the compiler would contract.
 __device__ __forceinline__ double fma_r(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float fma_r(float a, float b, float c) { return fmaf(a, b, c); }
 
@@ -295,8 +295,9 @@ __device__ __forceinline__ double diag_v(const Op& o, int j, int i) {
   const int i = blockIdx.y * blockDim.y + threadIdx.y;
 
 // Gauss-Seidel update of one point of one component (comp 0 = u, 1 = v).  Every smoother
-// (these per-colour kernels, the tiles, the sub-cycle) forms x + (b - A x) / diag as one
-// explicit fused multiply-add, so all of them round alike.
+// (these per-colour kernels, the tiles, the streamed kernel, the sub-cycle) forms x + (b - A x) / diag as one
+// explicit fused multiply-add; those of one level also sum a row's terms in one order, so they
+// round alike.
 __device__ __forceinline__ void gs_point(const Op& o, double* xu, double* xv, const double* bu, const double* bv,
                                          const double* idu, const double* idv, int comp, int j, int i) {
   const long long q = o.d.at(j, i);
