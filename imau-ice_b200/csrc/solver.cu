@@ -950,10 +950,11 @@ __global__ void __launch_bounds__(kTileThreads) k_smooth_up(OpT<R> o, Op oc, int
 // updating the points within H - 1 - q of the tile.  The columns arrive by bulk copies (one
 // per plane and column) that complete on mbarriers.
 //
-// Bound by shared-memory bandwidth: about 16 reads per point update.  A colour's points in one
-// column lie two rows apart, which alone is a 2-way bank conflict; half of a half-warp takes
-// the column's points and the other half the next column's, whose rows have the other parity,
-// so the 16 values fill all banks.
+// Bound by latency: a step lasts as long as one point update (nine reads, 30 dependent operations,
+// a write) and its barrier; the schedulers issue in half of the cycles, shared memory is busy in a
+// fifth (counters at 321 x 561).  A colour's points in one column lie two rows apart, a 2-way bank
+// conflict; half of a half-warp takes the column's points and the other half the next column's,
+// whose rows have the other parity, so the 16 values fill all banks.
 // Against the square tiles (k_smooth_down/up), which recompute 9 points on every side and keep
 // no more than 32 x 32 points and no coefficients beside them: a strip's halo along i is paid
 // once per chunk, and the coefficients come from the ring.  Pre- and post-smoothing of the
