@@ -670,7 +670,9 @@ struct LossWeights {
 // One thread per pixel.  The weights are read from shared memory four at a time (a broadcast:
 // every thread needs the same ones); read from global memory, one load per multiply-add made
 // the load unit the bound (326 us for 8 training samples of 561 x 321, whose tensors cross
-// HBM in 65 us).  With targets, gd1 is masked by the ReLU of d1.
+// HBM in 65 us).  With targets, gd1 is masked by the ReLU of d1.  out and tgt may be a caller's
+// buffers at any float's address: four floats at a time where both lie on 16 bytes, else one by
+// one.
 __global__ void __launch_bounds__(128) k_head(const bf16* d1, const float* wh, const float* bh, float* out,
                                               const float* tgt, float* dout, bf16* gd1, float* part, int n, int H,
                                               int W, int ny, int nx, int nz, float inv_count, LossWeights lw) {
@@ -696,10 +698,14 @@ __global__ void __launch_bounds__(128) k_head(const bf16* d1, const float* wh, c
 #pragma unroll
     for (int c = 0; c < kHeadC; ++c) gd[c] = 0.0f;
     const int x = (int)(p % W), y = (int)((p / W) % H);
+    const bool wide = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(tgt)) & 15) == 0;
 #pragma unroll
     for (int j4 = 0; j4 < kOut; j4 += 4) {
       float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f), o4, g4;
-      if (tgt) t4 = *reinterpret_cast<const float4*>(tgt + p * kOut + j4);
+      if (tgt) {
+        const float* t = tgt + p * kOut + j4;
+        t4 = wide ? *reinterpret_cast<const float4*>(t) : make_float4(t[0], t[1], t[2], t[3]);
+      }
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
         const int j = j4 + jj;
@@ -729,7 +735,11 @@ __global__ void __launch_bounds__(128) k_head(const bf16* d1, const float* wh, c
           }
         }
       }
-      if (out) *reinterpret_cast<float4*>(out + p * kOut + j4) = o4;
+      if (out) {
+        float* o = out + p * kOut + j4;
+        if (wide) *reinterpret_cast<float4*>(o) = o4;
+        else o[0] = o4.x, o[1] = o4.y, o[2] = o4.z, o[3] = o4.w;
+      }
       if (tgt) *reinterpret_cast<float4*>(dout + p * kOut + j4) = g4;
     }
     if (tgt) {
