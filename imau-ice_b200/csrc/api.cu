@@ -307,7 +307,13 @@ int graph_loop_collect(Ctx* c, GraphLoop& L) {
   c->fine_passes += L.it * G.p_pre + solved * (G.p_head + G.p_tail) + lin * G.p_first + full * G.p_second;
   L.relres = h[SC_RELRES];
   L.done = true;
-  if (h[SC_NAN] != 0.0) return set_error(c, DIVA_NAN_DETECTED, "NaN in the viscosity iteration");
+  if (h[SC_NAN] != 0.0) {
+    // no later iteration makes the last candidate the DIVA_err field: this iteration's if it
+    // solved (and did not count as converged), else the previous one's
+    if (h[SC_CONVERGED] == 0.0 && (L.it > 1 || h[SC_SOLVED] != 0.0))
+      if (int st = launch_commit_err(c)) return st;
+    return set_error(c, DIVA_NAN_DETECTED, "NaN in the viscosity iteration");
+  }
   if (h[SC_EXIT_RELRES] != 0.0) {
     L.by_relres = true;
     return DIVA_OK;
@@ -364,6 +370,11 @@ int picard(Ctx* c, bool diva, double* u, double* v, diva_report_t* rep) {
     DIVA_CUDA(c, cudaMemcpyAsync(c->scal + SC_AA_N, init, sizeof(init), cudaMemcpyHostToDevice, c->stream));
     if ((st = anderson_reset(c))) return st;
   }
+  // an iteration that fails before its update: the previous one's candidate becomes DIVA_err
+  auto failed = [&](int status) {
+    const int e = it > 1 ? launch_commit_err(c) : DIVA_OK;
+    return e ? e : status;
+  };
   for (;;) {
     ++it;
     if ((st = launch_diva_coefficients(c, u, v, diva, K1_LOOP))) return st;
@@ -372,7 +383,7 @@ int picard(Ctx* c, bool diva, double* u, double* v, diva_report_t* rep) {
       if ((st = solver_relres(c, u, v, &relres))) return st;
       eta = eta_after(eta, relres, relres_prev, C.picard_relres_tol);   // as the graph's k_init_residual does
       relres_prev = relres;
-      if (!std::isfinite(relres)) return set_error(c, DIVA_NAN_DETECTED, "NaN in the nonlinear residual");
+      if (!std::isfinite(relres)) return failed(set_error(c, DIVA_NAN_DETECTED, "NaN in the nonlinear residual"));
       const bool stop_stall = relres > C.picard_relres_tol &&
                               stall_after(relres, &stall_best, &stall_since, C.picard_stall_its);
       if (relres <= C.picard_relres_tol || stop_stall) {
@@ -389,7 +400,7 @@ int picard(Ctx* c, bool diva, double* u, double* v, diva_report_t* rep) {
     if (st == DIVA_LINEAR_NOT_CONVERGED) {
       ++lin_fail;   // the reference does not check PETSc/SOR convergence either; keep iterating
     } else if (st) {
-      return st;
+      return failed(st);
     }
     if (C.picard_anderson_m > 0) {
       // the mixing step reads this iteration's nonlinear residual from the device scalars

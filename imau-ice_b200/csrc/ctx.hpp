@@ -301,7 +301,7 @@ int launch_picard_update(Ctx* c, double* u, double* v, const double* xu, const d
 // mixed iterate g - sum gamma_i dG_i in place of the relaxation.
 int launch_anderson_prepare(Ctx* c, const double* u, const double* v, const double* xu, const double* xv);
 int anderson_reset(Ctx* c);   // empty history at the start of a solve (zeroed columns)
-int launch_commit_err(Ctx* c);   // the last candidate, after a host-driven loop that the residual ended
+int launch_commit_err(Ctx* c);   // the last candidate, where no further update makes it the field
 int launch_basal_stress_velocities(Ctx* c);
 int launch_relres_end(Ctx* c, bool diva, const IterEnd& end);   // post kernel of a rel-res iteration
 int launch_visc_b_output(Ctx* c);   // after the viscosity loop: visc_eff_3D_b and the shear strain rates
