@@ -29,6 +29,7 @@
 #include <cstring>
 #include <new>
 #include <vector>
+#include "cnn_tiles.hpp"
 #include "ctx.hpp"
 #include "../../include/diva_cnn.h"
 
@@ -160,14 +161,6 @@ struct Input {
   const bf16 *x, *lo;
   int c1;   // channels from lo (0: none)
 };
-// Planes of 16-byte chunks are `px` pixels long; a warp stores chunks c8 = 0.. of one or more
-// consecutive pixels, so px is rounded up to the residue mod 8 that puts those 8 stores of a
-// phase into different banks (C = 16: 2 chunks x 4 pixels, 32: 4 x 2, 64 and more: 8 x 1).
-__host__ __device__ constexpr int plane_px(int px, int C) {
-  const int r = C == 16 ? 4 : C == 32 ? 2 : 1;
-  return px + ((r - px % 8) + 8) % 8;
-}
-
 constexpr int kConvThreads = 256;
 
 // Stage `rows` image rows from y0 (possibly -1) and `cols` pixels from x0 (possibly -1) of the
@@ -211,10 +204,6 @@ __device__ __forceinline__ void stage_rows(uint32_t dst, int rpitch, int cpitch,
 // that pitch-P order (row m of D = position 128 blk + m), so that tap (ty, tx) of every
 // position is the same tile ty P + tx pixels further on: the two halo columns of a row
 // are computed as well and dropped (2 of P), instead of staging each tap's operand anew.
-struct ConvTile {
-  int TW, TH, P, npx;   // npx: pixels of a staged plane
-  int ncol, nrow, ntile;
-};
 struct ConvArgs {
   Input in;          // forward input, or (dgrad) dZ of the layer
   const bf16* w;     // forward: W [9][COUT][CIN]; dgrad: W^T [9][CIN][COUT]
@@ -226,21 +215,6 @@ struct ConvArgs {
   ConvTile t;
 };
 
-// accumulator blocks per tile: two where the weights leave room for two or more CTAs per SM
-template <int KC, int NO>
-__host__ __device__ constexpr int conv_blocks() {
-  return KC * NO <= 64 * 32 ? 2 : 1;
-}
-// bytes between the 8-channel planes of one tap's weights (padded like plane_px)
-template <int KC, int NO>
-__host__ __device__ constexpr int conv_wplane() {
-  return plane_px(NO, KC) * 16;
-}
-template <int KC, int NO>
-__host__ __device__ constexpr int conv_wbytes() {
-  return 9 * (KC / 8) * conv_wplane<KC, NO>();
-}
-
 // Bound by the rate at which the tensor core takes K = 16 MMAs from unswizzled operands (about
 // 100 cycles each) and by the tile copies.  On 8 samples of 561 x 321 the 32 -> 32 layer takes
 // 92 us, the 64 -> 32 one 170 us (2 x 93 MB and 4 x 93 MB in and out); a kernel that gathered
@@ -249,8 +223,8 @@ __host__ __device__ constexpr int conv_wbytes() {
 template <int KC, int NO, bool DGRAD>
 __global__ void __launch_bounds__(kConvThreads) k_conv3x3(ConvArgs a) {
   static_assert(KC % 16 == 0 && NO % 32 == 0 && NO <= 128, "tile shape");
-  constexpr int C8 = KC / 8, NB = conv_blocks<KC, NO>();
-  constexpr int WL = conv_wplane<KC, NO>(), WT = C8 * WL;
+  constexpr int C8 = KC / 8, NB = conv_blocks(KC, NO);
+  constexpr int WL = conv_wplane(KC, NO), WT = C8 * WL;
   constexpr int NCOL = tmem_cols<NB * NO>();
   constexpr uint32_t IDESC = idesc_bf16(128, NO);
   extern __shared__ unsigned char smem_raw[];
@@ -258,7 +232,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3(ConvArgs a) {
   __shared__ uint32_t taddr_s;
   __shared__ __align__(16) float sbias[NO];
   unsigned char* Ws = align128(smem_raw);
-  unsigned char* Xs = Ws + conv_wbytes<KC, NO>();
+  unsigned char* Xs = Ws + conv_wbytes(KC, NO);
   const uint32_t ws = smem_u32(Ws), xs = smem_u32(Xs);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int H = a.H, W = a.W, P = a.t.P, npx = a.t.npx;
@@ -940,31 +914,11 @@ int resident_ctas(int smem, int ncols) {
   return kSMs * std::max(k, 1);
 }
 
-// The tile of a forward / dgrad convolution of H x W images: of all column splits the one with
-// the least work, counting the accumulator rows (128 per block, the halo columns and the
-// ragged ends among them) and the staged pixels of all tiles.
-ConvTile conv_tile(int n, int H, int W, int nb, int C) {
-  ConvTile best{};
-  double cost = 0.0;
-  for (int ncol = 1; ncol <= W; ++ncol) {
-    const int TW = (W + ncol - 1) / ncol, P = TW + 2;
-    if ((W + TW - 1) / TW != ncol || P > 128 * nb) continue;
-    if (best.TW && TW < 8) break;
-    const int TH = std::min(H, 128 * nb / P), nrow = (H + TH - 1) / TH;
-    const double c = (double)ncol * nrow * (128 * nb + (TH + 2) * P);
-    if (!best.TW || c < cost) {
-      cost = c;
-      best = ConvTile{TW, TH, P, plane_px(128 * nb + 2 * P + 2, C), ncol, nrow, n * ncol * nrow};
-    }
-  }
-  return best;
-}
-
 template <int KC, int NO, bool DG>
 int launch_conv(ConvArgs a, cudaStream_t st) {
-  constexpr int NB = conv_blocks<KC, NO>();
-  a.t = conv_tile(a.n, a.H, a.W, NB, KC);
-  const int smem = conv_wbytes<KC, NO>() + (KC / 8) * a.t.npx * 16 + 128;
+  constexpr int NB = conv_blocks(KC, NO);
+  a.t = conv_tile(a.n, a.H, a.W, KC, NO);
+  const int smem = conv_smem(KC, NO, a.t.npx);
   if (cudaFuncSetAttribute(k_conv3x3<KC, NO, DG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return DIVA_CUDA_ERROR;
   const int grid = std::min(a.t.ntile, resident_ctas(smem, tmem_cols<NB * NO>()));

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from imau_ice_b200 import diva, learned
+import cnn_reference as ref
 
 pytestmark = [pytest.mark.gpu,
               pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU (B200)")]
@@ -32,3 +33,31 @@ def test_outputs_and_targets_at_any_float(shift):
     net.close()
     (o0, g0, l0), (o1, g1, l1) = res
     assert np.array_equal(o0, o1) and np.array_equal(g0, g1) and l0 == l1
+
+
+@pytest.mark.parametrize("ny, nx", [(2, 400), (4, 372), (3, 1001)])
+def test_images_of_one_row_at_the_coarsest_level(ny, nx):
+    """Forward pass and gradients of a strip four rows high (one at a quarter of the resolution)
+    against the PyTorch reference, within the bounds of the network's other tests."""
+    g = diva.Grid(nx, ny, 10e3)
+    net = learned.WarmStartNet(g, batch=1, capacity=0, seed=nx)
+    Hp, Wp = net.padded_shape
+    rng = np.random.default_rng(nx)
+    feat = torch.as_tensor(rng.normal(0, 1, (1, Hp, Wp, learned.IN_C))).to(torch.bfloat16)
+    tgt = rng.normal(0, 1, (1, Hp, Wp, learned.N_OUT)).astype(np.float32)
+    w = torch.as_tensor(net.get_weights()).requires_grad_(True)
+    want = ref.forward(feat.float().numpy(), w, bf16=True)
+    mask = np.broadcast_to(ref.valid_mask(Hp, Wp, ny, nx, g.nz), tgt.shape)
+    ref.loss(want, torch.as_tensor(tgt), mask).backward()
+    gref = w.grad.numpy()
+    f, t = feat.cuda().contiguous(), torch.as_tensor(tgt).cuda()
+    out = torch.zeros(1, Hp, Wp, learned.N_OUT, device="cuda")
+    net.forward(f.data_ptr(), out.data_ptr(), 1)
+    assert (out.cpu() - want.detach()).abs().max() < 2e-2 * want.detach().abs().max()
+    net.train_step(f.data_ptr(), t.data_ptr(), 1, 0.0)
+    gdev = net.grads()
+    for name, (wo, shape, bo, nb) in learned.weight_layout()[0].items():
+        m = int(np.prod(shape))
+        for a, b, what in ((gdev[wo:wo + m], gref[wo:wo + m], "w"), (gdev[bo:bo + nb], gref[bo:bo + nb], "b")):
+            assert np.linalg.norm(a - b) <= 5e-2 * max(np.linalg.norm(b), 1e-30), (name, what)
+    net.close()
