@@ -919,8 +919,6 @@ int launch_conv(ConvArgs a, cudaStream_t st) {
   constexpr int NB = conv_blocks(KC, NO);
   a.t = conv_tile(a.n, a.H, a.W, KC, NO);
   const int smem = conv_smem(KC, NO, a.t.npx);
-  if (cudaFuncSetAttribute(k_conv3x3<KC, NO, DG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return DIVA_CUDA_ERROR;
   const int grid = std::min(a.t.ntile, resident_ctas(smem, tmem_cols<NB * NO>()));
   k_conv3x3<KC, NO, DG><<<grid, kConvThreads, smem, st>>>(a);
   return DIVA_OK;
@@ -961,9 +959,6 @@ int launch_wgrad(WgradArgs a, long part_floats, int* nsplit, cudaStream_t st) {
   int smem = 2 * a.t.buf + 128;
   // no more CTAs on an SM than its tensor memory serves
   smem = std::max(smem, 227 * 1024 / (512 / NCOL + 1));
-  if (cudaFuncSetAttribute(k_conv3x3_wgrad<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-      cudaSuccess)
-    return DIVA_CUDA_ERROR;
   const int grid = std::min(a.t.ntile, kWgradSlices);
   if ((long)grid * (9 * CI * CO + CO) > part_floats) return DIVA_BAD_INPUT;
   *nsplit = grid;
@@ -971,26 +966,51 @@ int launch_wgrad(WgradArgs a, long part_floats, int* nsplit, cudaStream_t st) {
   return DIVA_OK;
 }
 
+// the channel counts there are kernels for: (read, written) of a forward layer and of an input
+// gradient, (cin, cout) of a weight gradient
+#define FOR_FWD(X) X(16, 32) X(32, 32) X(32, 64) X(64, 64) X(64, 128) X(128, 64) X(64, 32)
+#define FOR_DGRAD(X) X(32, 32) X(32, 64) X(64, 128) X(128, 64) X(64, 64) X(64, 32)
+#define FOR_WGRAD(X) X(16, 32) X(32, 32) X(32, 64) X(64, 64) X(64, 128) X(128, 64) X(64, 32)
+
 int conv_fwd(int cin, int cout, const ConvArgs& a, cudaStream_t st) {
 #define FWD(KC, NO) \
   if (cin == KC && cout == NO) return launch_conv<KC, NO, false>(a, st);
-  FWD(16, 32) FWD(32, 32) FWD(32, 64) FWD(64, 64) FWD(64, 128) FWD(128, 64) FWD(64, 32)
+  FOR_FWD(FWD)
 #undef FWD
   return DIVA_UNSUPPORTED;
 }
 int conv_dgrad(int cin, int cout, const ConvArgs& a, cudaStream_t st) {
 #define DGR(KC, NO) \
   if (cout == KC && cin == NO) return launch_conv<KC, NO, true>(a, st);
-  DGR(32, 32) DGR(32, 64) DGR(64, 128) DGR(128, 64) DGR(64, 64) DGR(64, 32)
+  FOR_DGRAD(DGR)
 #undef DGR
   return DIVA_UNSUPPORTED;
 }
 int conv_wgrad(int cin, int cout, const WgradArgs& a, long part_floats, int* nsplit, cudaStream_t st) {
 #define WGR(CI, CO) \
   if (cin == CI && cout == CO) return launch_wgrad<CI, CO>(a, part_floats, nsplit, st);
-  WGR(16, 32) WGR(32, 32) WGR(32, 64) WGR(64, 64) WGR(64, 128) WGR(128, 64) WGR(64, 32)
+  FOR_WGRAD(WGR)
 #undef WGR
   return DIVA_UNSUPPORTED;
+}
+// The current device's limit of every kernel's dynamic shared memory, the same for every network
+// and never lowered: the limit belongs to the kernel, so a launch's own size set as the limit
+// would refuse a larger one that another thread's network is about to make.
+bool allow_shared_memory() {
+  bool ok = true;
+  auto allow = [&](const void* kernel) {
+    ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynSmemMax) == cudaSuccess && ok;
+  };
+#define ALLOW(KC, NO) allow((const void*)k_conv3x3<KC, NO, false>);
+  FOR_FWD(ALLOW)
+#undef ALLOW
+#define ALLOW(KC, NO) allow((const void*)k_conv3x3<KC, NO, true>);
+  FOR_DGRAD(ALLOW)
+#undef ALLOW
+#define ALLOW(CI, CO) allow((const void*)k_conv3x3_wgrad<CI, CO>);
+  FOR_WGRAD(ALLOW)
+#undef ALLOW
+  return ok;
 }
 
 // tensors of the network (index, level, channels)
@@ -1301,7 +1321,7 @@ int32_t diva_cnn_create(diva_cnn_t** out, int32_t ny, int32_t nx, int32_t nz, in
   N->loss_hist = reinterpret_cast<float*>(base + o_lh);
   N->ds_feat = reinterpret_cast<bf16*>(base + o_dsf);
   N->ds_tgt = reinterpret_cast<float*>(base + o_dst);
-  if (cudaStreamCreateWithFlags(&N->stream, cudaStreamNonBlocking) != cudaSuccess ||
+  if (cudaStreamCreateWithFlags(&N->stream, cudaStreamNonBlocking) != cudaSuccess || !allow_shared_memory() ||
       cudaMemset(N->arena, 0, bytes) != cudaSuccess) {
     diva_cnn_destroy(N);
     return DIVA_CUDA_ERROR;

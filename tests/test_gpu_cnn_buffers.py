@@ -1,11 +1,14 @@
 """The network's device-buffer forms on the caller's own buffers: outputs and targets at any
 float's address give the same bits as on 16-byte boundaries, and nothing beside them is written."""
+import threading
+
 import numpy as np
 import pytest
 import torch
 
 from imau_ice_b200 import diva, learned
 import cnn_reference as ref
+import helpers
 
 pytestmark = [pytest.mark.gpu,
               pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU (B200)")]
@@ -61,3 +64,40 @@ def test_images_of_one_row_at_the_coarsest_level(ny, nx):
         for a, b, what in ((gdev[wo:wo + m], gref[wo:wo + m], "w"), (gdev[bo:bo + nb], gref[bo:bo + nb], "b")):
             assert np.linalg.norm(a - b) <= 5e-2 * max(np.linalg.norm(b), 1e-30), (name, what)
     net.close()
+
+
+def test_networks_of_different_sizes_in_two_threads():
+    """Each network trains from its own host thread; every call succeeds and the weights are those
+    of the same training alone."""
+    cases = []
+    for dx in (200e3, 40e3):            # 9 x 15 and 41 x 71 cells
+        g, cfg, f = helpers.make_case(2, dx=dx)
+        ctx = diva.Context(g, cfg)
+        helpers.prepare(ctx, f)
+        net = learned.WarmStartNet(g, batch=1, capacity=8, seed=1)
+        for _ in range(8):
+            net.add_sample(ctx)
+        ctx.close()
+        w0 = net.get_weights()
+        net.train(150, lr=1e-3, seed=2)
+        cases.append((net, w0, net.get_weights()))
+        net.set_weights(w0)
+    failed = []
+
+    def drive(net, w0, want):
+        try:
+            for _ in range(3):
+                net.set_weights(w0)
+                net.train(150, lr=1e-3, seed=2)
+                if not np.array_equal(net.get_weights(), want):
+                    failed.append("weights")
+        except Exception as e:
+            failed.append(e)
+    threads = [threading.Thread(target=drive, args=c) for c in cases]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not failed, failed
+    for c in cases:
+        c[0].close()
