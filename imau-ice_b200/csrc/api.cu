@@ -307,6 +307,7 @@ int graph_loop_collect(Ctx* c, GraphLoop& L) {
   c->fine_passes += L.it * G.p_pre + solved * (G.p_head + G.p_tail) + lin * G.p_first + full * G.p_second;
   L.relres = h[SC_RELRES];
   L.done = true;
+  if (h[SC_TIMEOUT] != 0.0) return set_error(c, DIVA_TIMEOUT, kTimeoutMessage);
   if (h[SC_NAN] != 0.0) {
     // no later iteration makes the last candidate the DIVA_err field: this iteration's if it
     // solved (and did not count as converged), else the previous one's
@@ -365,6 +366,7 @@ int picard(Ctx* c, bool diva, double* u, double* v, diva_report_t* rep) {
   bool stalled_exit = false;
   double stall_best = 0.0, stall_since = 0.0;
   double resid = 0.0, relres = -1.0, eta = C.lin_adaptive_eta, relres_prev = 0.0;
+  DIVA_CUDA(c, cudaMemsetAsync(c->scal + SC_TIMEOUT, 0, sizeof(double), c->stream));
   if (C.picard_anderson_m > 0) {
     double init[SC_COUNT - SC_AA_N] = {};
     DIVA_CUDA(c, cudaMemcpyAsync(c->scal + SC_AA_N, init, sizeof(init), cudaMemcpyHostToDevice, c->stream));
@@ -508,6 +510,8 @@ int diva_create(diva_ctx_t** out, const diva_grid_t* g, const diva_config_t* cfg
   if (const char* e = getenv("DIVA_NO_GRAPHS")) c->graphs_disabled = (e[0] == '1');
   // DIVA_NO_TILES=1 smooths every level with the per-colour kernels (same results)
   if (const char* e = getenv("DIVA_NO_TILES")) c->tiles_disabled = (e[0] == '1');
+  // DIVA_WAVE_DROP=1: the streamed smoother issues no copies, so that its waits run out (tests)
+  if (const char* e = getenv("DIVA_WAVE_DROP")) c->wave_drop = (e[0] == '1');
   Carver dry{nullptr, 0, true};
   const size_t bytes = carve(c, dry);
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { delete h; return DIVA_CUDA_ERROR; }
@@ -1020,6 +1024,7 @@ int diva_profile_kernel(diva_ctx_t* h, int32_t which, int32_t reps, double* ms, 
   Ctx* c = &h->c;
   const double nc = (double)c->d.nx * c->d.ny, w = sizeof(double), nz = c->d.nz;
   int st = DIVA_OK;
+  DIVA_CUDA(c, cudaMemsetAsync(c->scal + SC_TIMEOUT, 0, sizeof(double), c->stream));
   DIVA_CUDA(c, cudaEventRecord(c->ev0, c->stream));
   for (int r = 0; r < reps && !st; ++r) {
     switch (which) {
@@ -1036,6 +1041,8 @@ int diva_profile_kernel(diva_ctx_t* h, int32_t which, int32_t reps, double* ms, 
   DIVA_CUDA(c, cudaEventSynchronize(c->ev1));
   float t = 0.f;
   DIVA_CUDA(c, cudaEventElapsedTime(&t, c->ev0, c->ev1));
+  DIVA_CUDA(c, cudaMemcpy(c->h_scal + SC_TIMEOUT, c->scal + SC_TIMEOUT, sizeof(double), cudaMemcpyDeviceToHost));
+  if (c->h_scal[SC_TIMEOUT] != 0.0) return set_error(c, DIVA_TIMEOUT, kTimeoutMessage);
   *ms = t / reps;
   // algorithmic bytes per launch (compulsory traffic per column, FP64):
   //  0: read A-factor and the previous viscosity, write the new one (3 nz) + 15 2D fields

@@ -52,6 +52,7 @@ enum {
   // device-side control of a graph-launched viscosity iteration
   SC_TARGET2, SC_LIN_IT, SC_LIN_FULL, SC_LIN_FAILED, SC_PIC_IT, SC_EXIT_RELRES, SC_CONVERGED, SC_RESID,
   SC_RELRES, SC_NAN, SC_SOLVED, SC_HALFDONE,
+  SC_TIMEOUT,               // a smoother's wait for its copies ran out: the solve fails
   SC_ETA, SC_RELRES_PREV,   // adaptive linear tolerance factor and the previous nonlinear residual
   SC_SUM_LIN, SC_SUM_FULL, SC_N_SOLVED,   // totals of a graph-launched viscosity loop
   // Anderson mixing of the viscosity iteration (picard_anderson_m > 0): history columns held,
@@ -64,6 +65,7 @@ enum {
   SC_AA_G, SC_AA_RHS = SC_AA_G + 25, SC_AA_GAMMA = SC_AA_RHS + 5,
   SC_COUNT = SC_AA_GAMMA + 5
 };
+constexpr const char* kTimeoutMessage = "a copy of the multigrid smoother did not arrive in time";
 constexpr int kAAMax = 5;             // largest Anderson depth
 constexpr int kAAPartials = 2 * kAAMax;   // block partials of one mixing step
 constexpr double kAAGammaMax = 20.0;      // largest sum of |gamma_i| a mixing step accepts
@@ -238,6 +240,7 @@ struct Ctx {
   bool graphs_disabled = false;         // set if graph construction failed: host-driven loop
   bool tiled = false;                   // large levels smoothed by the tiled kernels
   bool tiles_disabled = false;          // per-colour kernels on every level
+  bool wave_drop = false;               // the streamed smoother issues no copies (tests of its waits)
   int tile_override[kMaxLevels] = {};   // tile edge of a tiled level: 0 by its size, else 16 or 32
   // counters of the last solve
   long lin_iters = 0, mg_cycles = 0;

@@ -600,7 +600,7 @@ __device__ __forceinline__ void loop_end(double* sc, const IterEnd& e) {
   sc[SC_SUM_FULL] += sc[SC_LIN_FULL];
   sc[SC_N_SOLVED] += sc[SC_SOLVED];
   const bool stop = sc[SC_CONVERGED] != 0.0 || sc[SC_EXIT_RELRES] != 0.0 || sc[SC_NAN] != 0.0 ||
-                    sc[SC_PIC_IT] > (double)e.nit;
+                    sc[SC_TIMEOUT] != 0.0 || sc[SC_PIC_IT] > (double)e.nit;
   cudaGraphSetConditional(e.a, stop ? 0u : 1u);
   if (e.has_b) cudaGraphSetConditional(e.b, stop ? 0u : 1u);
 }

@@ -973,7 +973,8 @@ constexpr int kWaveBars = 8;      // mbarriers: more than the pairs in flight
 constexpr int kWaveCopy = 5;      // copying warps: five of a pair's 20 plane columns each (a bulk copy takes about
                                   // 110 cycles to issue), the last the coarse columns
 constexpr int kWaveCoarse = 8;    // coarse columns held (2 (kWavePre + 1) of a level not coarsened along i)
-constexpr long kWaveSpin = 1L << 22;
+constexpr int kWaveSpin = 1 << 16;   // polls before a wait gives up: 0.26 s, a poll lasting up to 4 us (a copy
+                                     // takes a few)
 
 struct WaveGeom {
   static constexpr int NU = 2;   // sweeps per phase
@@ -1007,6 +1008,7 @@ struct WaveArgs {
   int fx, fy;
   int rows, chunk;       // tile height and width
   double* fail;          // set when a wait ran out
+  int drop;              // issue no copies, so that the waits run out (tests)
 };
 
 // ring offsets of the three columns a row reads
@@ -1019,7 +1021,7 @@ struct RIx {
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool wave_wait(uint32_t bar, uint32_t parity) {
-  for (long it = 0; it < kWaveSpin; ++it) {
+  for (int it = 0; it < kWaveSpin; ++it) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -1204,6 +1206,9 @@ __global__ void __launch_bounds__(32 * (UP ? WaveGeom::warps_up : WaveGeom::warp
     const uint32_t bar0 = smem_addr(&bars[0]);
     const int npair = tw / 2 + H + (tw & 1);   // pairs of the region (an odd width's last column is beyond it)
     int slot = 0;
+    // A wait that runs out fails the solve: the lane issues nothing more, so that soon the waits of all
+    // run out, and the block goes on over what there is, its barriers unchanged.
+    bool ok = !a.drop;
     auto coarse_total = [&](int C) {
       return ((coarse_col(a.oc, C, true) >= 0 ? 1u : 0u) + (coarse_col(a.oc, C, false) >= 0 ? 1u : 0u)) * cbytes;
     };
@@ -1212,7 +1217,7 @@ __global__ void __launch_bounds__(32 * (UP ? WaveGeom::warps_up : WaveGeom::warp
       const uint32_t bar = bar0 + (t & (kWaveBars - 1)) * 8;
       if (mover) {
         const bool in0 = i >= 0 && i < d.nx, in1 = i + 1 >= 0 && i + 1 < d.nx;
-        if (lane == 0) {
+        if (lane == 0 && ok) {
           // x has been written by other threads since its last copy
           if (UP && w == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
@@ -1220,18 +1225,18 @@ __global__ void __launch_bounds__(32 * (UP ? WaveGeom::warps_up : WaveGeom::warp
                        : "memory");
         }
         __syncwarp();
-        if (bytes && (hc ? in1 : in0)) bulk_copy(dst0 + slot * dcol, src, bytes, bar);
+        if (bytes && ok && (hc ? in1 : in0)) bulk_copy(dst0 + slot * dcol, src, bytes, bar);
       } else if (UP) {
         // coarse columns that arrive with the pair: fx = 2, the one beyond that of its even column
         // (with the first pair also those before it); fx = 1, the pair's own
         const int Cb = a.fx == 1 ? i + 1 : ((i + 1) >> 1) + 1, Ca = a.fx == 1 ? i : t == 0 ? Cb - 3 : Cb;
-        if (lane == 0) {
+        if (lane == 0 && ok) {
           uint32_t total = 0;
           for (int C = Ca; C <= Cb; ++C) total += coarse_total(C);
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(total) : "memory");
         }
         __syncwarp();
-        if (lane < 2 && cbytes)
+        if (lane < 2 && cbytes && ok)
           for (int C = Ca; C <= Cb; ++C) {
             const int I = coarse_col(a.oc, C, lane == 0);
             if (I >= 0)
@@ -1242,28 +1247,31 @@ __global__ void __launch_bounds__(32 * (UP ? WaveGeom::warps_up : WaveGeom::warp
         constexpr int n16 = 2 * RP * sizeof(double) / 16;
         for (int t2 = lane; t2 < 2 * n16; t2 += 32)
           reinterpret_cast<uint4*>(ring + (slot + t2 / n16) * COL)[t2 % n16] = make_uint4(0u, 0u, 0u, 0u);
-        if (lane == 0)
+        if (lane == 0 && ok)
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
       }
       src += pitch;
       slot = slot == NC - 2 ? 0 : slot + 2;
     };
     auto arrived = [&](int t) { return wave_wait(bar0 + (t & (kWaveBars - 1)) * 8, (t / kWaveBars) & 1); };
-    int issued = 0, waited = 0;   // pairs issued and waited for
-    for (; issued < kWavePre && issued < npair; ++issued) issue(issued);
-    bool ok = arrived(0) && arrived(1);
-    waited = 2;
+    int next = 0, waited = 0, issued = npair;   // the pair to issue, those that have arrived, those a lane issued
+    auto wait_next = [&] {
+      ok = arrived(waited);
+      if (ok) ++waited;
+      else issued = a.drop ? 0 : next;
+    };
+    while (next < kWavePre && next < npair) issue(next++);
+    wait_next();
+    if (ok) wait_next();
     __syncthreads();
 #pragma unroll 1
     for (int s = 0; s <= last; ++s) {
-      if (issued < npair) issue(issued++);
-      // the next step reads up to pair s + 2; a wait that runs out fails the solve, and the
-      // block goes on without waiting
-      if (ok && waited < npair) ok = arrived(waited++);
+      if (next < npair) issue(next++);
+      if (ok && waited < npair) wait_next();   // the next step reads up to pair s + 2
       __syncthreads();
     }
     for (; waited < issued; ++waited) ok = arrived(waited) && ok;   // no copy in flight when the block ends
-    if (!ok && lane == 0) *a.fail = 1.0;
+    if (!ok) *a.fail = 1.0;
   } else {
     // ---- x += P x_c (prolong_delta's taps, weights and order)
     const int t0 = (warp - NPW - NOUT - kWaveCopy) * 32 + lane, r = t0 % RP, comp = (t0 / RP) & 1, h = t0 / (2 * RP);
@@ -2248,11 +2256,11 @@ __global__ void __launch_bounds__(256) k_update_s(Dims d, double* sc, const doub
   sc[SC_SNORM2] = ss;
   if (!h.on) return;
   sc[SC_LIN_IT] += 1.0;
-  const bool fin = isfinite(ss), done = fin && ss <= sc[SC_TARGET2];
+  const bool fin = isfinite(ss), late = sc[SC_TIMEOUT] != 0.0, done = fin && !late && ss <= sc[SC_TARGET2];
   if (!fin) sc[SC_NAN] = 1.0;
   sc[SC_HALFDONE] = done ? 1.0 : 0.0;
   if (done) sc[SC_RNORM2] = ss;
-  const bool go = fin && !done;
+  const bool go = fin && !late && !done;
   cudaGraphSetConditional(h.b, go ? 1u : 0u);
   if (!go) cudaGraphSetConditional(h.a, 0u);
 }
@@ -2302,7 +2310,8 @@ __global__ void __launch_bounds__(256) k_update_xr(Dims d, double* sc, double* x
   sc[SC_LIN_FULL] += 1.0;
   const bool fin = isfinite(rr);
   if (!fin) sc[SC_NAN] = 1.0;
-  cudaGraphSetConditional(h.a, (fin && rr > sc[SC_TARGET2] && sc[SC_LIN_IT] < (double)maxit) ? 1u : 0u);
+  const bool late = sc[SC_TIMEOUT] != 0.0;
+  cudaGraphSetConditional(h.a, (fin && !late && rr > sc[SC_TARGET2] && sc[SC_LIN_IT] < (double)maxit) ? 1u : 0u);
 }
 
 // p = r + beta (p - omega v)
@@ -2730,7 +2739,8 @@ static void launch_wave(Ctx* c, int l, const double* bu, const double* bv, doubl
   a.o = make_op(c, l);
   a.idu = L.idu; a.idv = L.idv; a.bu = bu; a.bv = bv;
   a.xu = L.tu; a.xv = L.tv; a.ru = L.ru; a.rv = L.rv;
-  a.fail = c->scal + SC_NAN;
+  a.fail = c->scal + SC_TIMEOUT;
+  a.drop = c->wave_drop;
   if (UP) {
     a.ou = ou; a.ov = ov;
     a.oc = make_op(c, l + 1);
@@ -3091,6 +3101,7 @@ int solver_solve(Ctx* c, const double* u0, const double* v0, double rtol, int ma
     launch_first_half(c, LoopHandles{});
     DIVA_LAUNCHED(c, "bicgstab half step");
     if ((st = read_scalars(c))) return st;
+    if (c->h_scal[SC_TIMEOUT] != 0.0) return set_error(c, DIVA_TIMEOUT, kTimeoutMessage);
     if (sqrt(c->h_scal[SC_SNORM2]) <= target) {
       half = 1;
       rnorm = sqrt(c->h_scal[SC_SNORM2]);
@@ -3101,6 +3112,7 @@ int solver_solve(Ctx* c, const double* u0, const double* v0, double rtol, int ma
     launch_second_half(c, LoopHandles{});
     DIVA_LAUNCHED(c, "bicgstab full step");
     if ((st = read_scalars(c))) return st;
+    if (c->h_scal[SC_TIMEOUT] != 0.0) return set_error(c, DIVA_TIMEOUT, kTimeoutMessage);
     rnorm = sqrt(c->h_scal[SC_RNORM2]);
     if (!std::isfinite(rnorm)) return set_error(c, DIVA_NAN_DETECTED, "NaN in the linear solve");
     done = rnorm <= target;
