@@ -356,11 +356,6 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3(ConvArgs a) {
 // dZ is staged [row][8-channel chunk][pixel], so the 16 chunk groups of a 128-row A operand
 // run on into the following dZ rows: one MMA forms 128 / COUT vertical taps at once
 // (COUT = 32: all three, the last 32 rows of D unused; 64: two and one; 128: one each).
-struct WgradTile {
-  int TW, TH, zp, xp;   // zp: pixels between dZ chunk groups; xp: of an X plane
-  int ncol, nrow, ntile;
-  int buf;              // bytes of one of the two tile buffers
-};
 struct WgradArgs {
   Input in;          // the layer's input
   const bf16* dz;    // masked gradient of the layer's output [n][H][W][CO]
@@ -369,18 +364,15 @@ struct WgradArgs {
   int* err;
   WgradTile t;
 };
-// Vertical tap sets of a layer; a CTA (blockIdx.y) takes one set and one horizontal tap.
-// The slices of the pixels (blockIdx.x) stay at 64 and the taps fill the GPU instead: the
-// tensor core truncates every addition to its FP32 accumulator, so the sum shrinks with the
-// length of the chain, and 64 slices give the chain lengths that the library has always had.
+// A CTA (blockIdx.y) takes one set of vertical taps of the layer and one horizontal tap; the
+// slices of the pixels (blockIdx.x) are as many as keep the chains short (wgrad_tile).
 template <int CO>
 __host__ __device__ constexpr int wgrad_sets() {
   return CO == 32 ? 1 : CO == 64 ? 2 : 3;
 }
-constexpr int kWgradSlices = 64;
 
-// Bound by the copies of its tiles and the MMA issue of the 64 slices' CTAs (about 3000 and
-// 2700 cycles a tile).  436 us for the 32 -> 32 layer on 8 samples of 561 x 321 with its bias
+// Bound by the copies of its tiles and the MMA issue of its CTAs (about 3000 and 2700 cycles a
+// tile).  436 us for the 32 -> 32 layer on 8 samples of 561 x 321 with its bias
 // gradient; one tap per CTA, with both operands transposed by 2-byte shared-memory stores, took
 // 958 us and 1 to 2 ms for the bias in a kernel of its own.
 template <int CI, int CO>
@@ -924,45 +916,16 @@ int launch_conv(ConvArgs a, cudaStream_t st) {
   return DIVA_OK;
 }
 
-// The tile of a weight gradient: a multiple of 16 pixels wide (zeros beyond the image), the
-// width with the fewest staged pixels; rows so that two tile buffers take about 110 KB at
-// most (two CTAs per SM).
-template <int CI, int CO>
-WgradTile wgrad_tile(int n, int H, int W) {
-  WgradTile t{};
-  long cost = 0;
-  for (int TW = 16; TW <= 64; TW += 16) {
-    const long c = (long)((W + TW - 1) / TW) * (TW * CO + (TW + 2) * CI);
-    if (!t.TW || c <= cost) {
-      cost = c;
-      t.TW = TW;
-    }
-  }
-  t.zp = plane_px(t.TW, CO);
-  for (t.TH = std::min(H, 8);; --t.TH) {
-    t.xp = plane_px(t.TH * (t.TW + 2), CI);
-    // dZ, then X; the last A operands run one or more dZ rows on (rows of D that nothing reads)
-    const int zrow = CO / 8 * t.zp * 16, xbytes = CI / 8 * t.xp * 16;
-    t.buf = ((t.TH + 2) * zrow + std::max(xbytes, 128 / CO * zrow) + 127) / 128 * 128;
-    if (2 * t.buf <= 110 * 1024 || t.TH <= 2) break;
-  }
-  t.ncol = (W + t.TW - 1) / t.TW;
-  t.nrow = (H + t.TH - 1) / t.TH;
-  t.ntile = n * t.ncol * t.nrow;
-  return t;
-}
-
 template <int CI, int CO>
 int launch_wgrad(WgradArgs a, long part_floats, int* nsplit, cudaStream_t st) {
   constexpr int NCOL = tmem_cols<CI>();
-  a.t = wgrad_tile<CI, CO>(a.n, a.H, a.W);
+  a.t = wgrad_tile(a.n, a.H, a.W, CI, CO);
   int smem = 2 * a.t.buf + 128;
   // no more CTAs on an SM than its tensor memory serves
   smem = std::max(smem, 227 * 1024 / (512 / NCOL + 1));
-  const int grid = std::min(a.t.ntile, kWgradSlices);
-  if ((long)grid * (9 * CI * CO + CO) > part_floats) return DIVA_BAD_INPUT;
-  *nsplit = grid;
-  k_conv3x3_wgrad<CI, CO><<<dim3(grid, 3 * wgrad_sets<CO>()), kConvThreads, smem, st>>>(a);
+  if (wgrad_part_floats(a.t, CI, CO) > part_floats) return DIVA_BAD_INPUT;
+  *nsplit = a.t.slices;
+  k_conv3x3_wgrad<CI, CO><<<dim3(a.t.slices, 3 * wgrad_sets<CO>()), kConvThreads, smem, st>>>(a);
   return DIVA_OK;
 }
 
@@ -1270,8 +1233,14 @@ int32_t diva_cnn_create(diva_cnn_t** out, int32_t ny, int32_t nx, int32_t nz, in
   off += kOut;
   N->nw = off;
 
-  // weight-gradient sums: up to 64 CTAs' of the largest layer (more of a smaller one); head sums
-  long part = 64L * (9 * 128 * 64 + 128);
+  // weight-gradient sums of the slices of any layer and minibatch size; head sums
+  long part = 0;
+  for (int b = 1; b <= batch; ++b)
+    for (const Layer& ly : N->L) {
+      const int lv = kTLevel[ly.out];
+      const WgradTile t = wgrad_tile(b, N->lvH(lv), N->lvW(lv), ly.cin, ly.cout);
+      part = std::max(part, wgrad_part_floats(t, ly.cin, ly.cout));
+    }
   const long hb = (long)nblk((long)batch * N->Hp * N->Wp, 128);
   if (hb > part) part = hb;
   if ((long)kHeadBlocks * kHeadGrad > part) part = (long)kHeadBlocks * kHeadGrad;

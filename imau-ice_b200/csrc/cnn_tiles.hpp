@@ -52,4 +52,51 @@ inline ConvTile conv_tile(int n, int H, int W, int KC, int NO) {
   return best;
 }
 
+// ---- weight gradient: a tile is TH rows of X (TW + 2 pixels, halo columns included) and the
+// TH + 2 rows of dZ (TW pixels) that they meet
+struct WgradTile {
+  int TW, TH, zp, xp;   // zp: pixels between dZ chunk groups; xp: of an X plane
+  int ncol, nrow, ntile;
+  int buf;              // bytes of one of the two tile buffers
+  int slices;           // CTAs the tiles are dealt to, each with its own sums
+};
+// The longest chain of additions to one accumulator, in pixels.  The tensor core truncates every
+// addition to its FP32 accumulator, so a sum shrinks with the length of its chain: no longer
+// than with 64 slices of whole 64-pixel chunks, for images of every size.
+inline long wgrad_chain(int n, int H, int W) {
+  const long chunks = ((long)n * H * W + 63) / 64;
+  return (chunks + 63) / 64 * 64;
+}
+// The tile of a weight gradient: a multiple of 16 pixels wide (zeros beyond the image), the width
+// with the fewest staged pixels; rows so that two tile buffers take about 110 KB at most (two
+// CTAs per SM) and a tile is no longer than a chain.
+inline WgradTile wgrad_tile(int n, int H, int W, int CI, int CO) {
+  WgradTile t{};
+  long cost = 0;
+  for (int TW = 16; TW <= 64; TW += 16) {
+    const long c = (long)((W + TW - 1) / TW) * (TW * CO + (TW + 2) * CI);
+    if (!t.TW || c <= cost) {
+      cost = c;
+      t.TW = TW;
+    }
+  }
+  const long chain = wgrad_chain(n, H, W);
+  auto pixels = [&] { return (long)std::min(t.TW, W) * t.TH; };   // of the image in a tile
+  t.zp = plane_px(t.TW, CO);
+  for (t.TH = std::min(H, 8);; --t.TH) {
+    t.xp = plane_px(t.TH * (t.TW + 2), CI);
+    // dZ, then X; the last A operands run one or more dZ rows on (rows of D that nothing reads)
+    const int zrow = CO / 8 * t.zp * 16, xbytes = CI / 8 * t.xp * 16;
+    t.buf = ((t.TH + 2) * zrow + std::max(xbytes, 128 / CO * zrow) + 127) / 128 * 128;
+    if ((2 * t.buf <= 110 * 1024 || t.TH <= 2) && (pixels() <= chain || t.TH == 1)) break;
+  }
+  t.ncol = (W + t.TW - 1) / t.TW;
+  t.nrow = (H + t.TH - 1) / t.TH;
+  t.ntile = n * t.ncol * t.nrow;
+  const int each = (int)(chain / pixels());   // tiles a chain holds (one row is 64 pixels at most, a chain at least)
+  t.slices = (t.ntile + each - 1) / each;
+  return t;
+}
+inline long wgrad_part_floats(const WgradTile& t, int CI, int CO) { return (long)t.slices * (9L * CI * CO + CO); }
+
 }  // namespace diva::cnn

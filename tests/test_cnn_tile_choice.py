@@ -1,7 +1,7 @@
 """The convolutions' choice of tiles (imau-ice_b200/csrc/cnn_tiles.hpp), compiled for the CPU and
 checked for every layer over image sizes from one row or column on: the tiles cover the image,
-their positions fit the accumulators, and the launch's shared memory stays within what a block
-may have."""
+their positions fit the accumulators, the launch's shared memory stays within what a block may
+have, and no weight-gradient sum runs over more pixels than 64 slices of 64-pixel chunks gave."""
 import ctypes as C
 import os
 import subprocess
@@ -19,6 +19,11 @@ using namespace diva::cnn;
 extern "C" void conv(int n, int H, int W, int KC, int NO, int* o) {
   const ConvTile t = conv_tile(n, H, W, KC, NO);
   const int v[] = {t.TW, t.TH, t.P, t.npx, t.ncol, t.nrow, t.ntile, conv_blocks(KC, NO), conv_smem(KC, NO, t.npx), kDynSmemMax};
+  for (int k = 0; k < 10; ++k) o[k] = v[k];
+}
+extern "C" void wgrad(int n, int H, int W, int CI, int CO, int* o) {
+  const WgradTile t = wgrad_tile(n, H, W, CI, CO);
+  const int v[] = {t.TW, t.TH, t.zp, t.xp, t.ncol, t.nrow, t.ntile, t.buf, t.slices, kDynSmemMax};
   for (int k = 0; k < 10; ++k) o[k] = v[k];
 }
 """
@@ -49,3 +54,20 @@ def test_convolution_tiles_cover_the_image_and_fit(tiles, cin, cout):
             assert ntile == 2 * ncol * nrow
             assert TH * P <= 128 * nb and (TH + 2) * P <= npx and 128 * nb - 1 + 2 * P + 2 < npx < 1 << 14
             assert smem <= limit <= 225 * 1024, (H, W, KC, NO, smem)
+
+
+@pytest.mark.parametrize("cin, cout", LAYERS)
+def test_weight_gradient_tiles_fit_and_keep_the_chains_short(tiles, cin, cout):
+    for n in (1, 2, 8):
+        for H, W in SIZES:
+            TW, TH, zp, xp, ncol, nrow, ntile, buf, slices, limit = ints(tiles.wgrad, n, H, W, cin, cout, n=10)
+            assert TW in (16, 32, 48, 64) and 1 <= TH <= 8
+            assert ncol * TW >= W and nrow * TH >= H and ntile == n * ncol * nrow
+            assert zp >= TW and xp >= TH * (TW + 2) and max(zp, xp) < 1 << 14
+            zrow = cout // 8 * zp * 16
+            assert buf >= (TH + 2) * zrow + max(cin // 8 * xp * 16, 128 // cout * zrow)
+            assert 2 * buf + 128 <= limit
+            assert 1 <= slices <= ntile
+            chunks = -(-n * H * W // 64)
+            before = 64 * -(-chunks // min(chunks, 64))     # chunks of the longest of up to 64 slices
+            assert -(-ntile // slices) * min(TW, W) * TH <= before, (n, H, W, slices)
