@@ -1009,6 +1009,13 @@ int diva_get_tile_edges(diva_ctx_t* h, int32_t* edges, int32_t n, int32_t* nlev)
   return DIVA_OK;
 }
 
+int diva_get_strip_rows(diva_ctx_t* h, int32_t* rows, int32_t n, int32_t* nlev) {
+  if (!h || !rows || !nlev || n < 0) return DIVA_BAD_INPUT;
+  *nlev = solver_strip_rows(&h->c, rows, n < kMaxLevels ? n : kMaxLevels);
+  for (int l = kMaxLevels; l < n; ++l) rows[l] = 0;
+  return DIVA_OK;
+}
+
 int diva_set_tile_edges(diva_ctx_t* h, const int32_t* edges, int32_t n) {
   if (!h || (n > 0 && !edges) || n < 0 || n > kMaxLevels) return DIVA_BAD_INPUT;
   for (int l = 0; l < n; ++l)

@@ -356,6 +356,7 @@ void solver_destroy_graphs(Ctx* c);
 // tile edge (16 or 32) of each level's smoothing kernels, 0 for levels not smoothed by
 // the tiled kernels; returns the number of levels
 int solver_tile_edges(const Ctx* c, int32_t* edges, int n);
+int solver_strip_rows(const Ctx* c, int32_t* rows, int n);
 
 }  // namespace diva
 

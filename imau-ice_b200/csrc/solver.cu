@@ -33,6 +33,7 @@
 #include <utility>
 #include <vector>
 #include "ctx.hpp"
+#include "wave_geom.hpp"
 
 namespace diva {
 namespace {
@@ -968,34 +969,6 @@ __global__ void __launch_bounds__(kTileThreads) k_smooth_up(OpT<R> o, Op oc, int
 // well, so every row reads its whole stencil as stored.  (Corner ghosts are read by no
 // interior row.  Periodic sides, whose sources lie across the domain, use the per-colour
 // kernels.)
-constexpr int kWavePre = 3;       // pairs of columns the copies run ahead
-constexpr int kWaveBars = 8;      // mbarriers: more than the pairs in flight
-constexpr int kWaveCopy = 5;      // copying warps: five of a pair's 20 plane columns each (a bulk copy takes about
-                                  // 110 cycles to issue), the last the coarse columns
-constexpr int kWaveCoarse = 8;    // coarse columns held (2 (kWavePre + 1) of a level not coarsened along i)
-constexpr int kWaveSpin = 1 << 16;   // polls before a wait gives up: 0.26 s, a poll lasting up to 4 us (a copy
-                                     // takes a few)
-
-struct WaveGeom {
-  static constexpr int NU = 2;   // sweeps per phase
-  static constexpr int NP = 4 * NU, H = NP + 1;
-  static constexpr int TJ = 64 - 2 * NP;              // largest tile height: pass 0's rows of a colour fill a warp
-  static constexpr int HB = (H + 3) / 4 * 4;          // ring rows before the tile (even: 16-byte aligned)
-  static constexpr int RP = (HB + TJ + H + 3) / 4 * 4;   // ring rows
-  static constexpr int NC = 2 * kWavePre + 3 * NP + 6;   // ring columns: from the copies' to the output's left neighbour
-  static constexpr int CP = RP + 8;                   // rows of a coarse column (a level not coarsened along j)
-  static constexpr size_t xk = (size_t)NC * 8 * RP * sizeof(double), b = (size_t)NC * 2 * RP * sizeof(double);
-  static constexpr size_t coarse = (size_t)kWaveCoarse * 2 * CP * sizeof(double);
-  static constexpr size_t smem_down = xk + b + 128, smem_up = xk + b + coarse + 128;
-  // two per pass (rows below and above the middle); output (descent: a warp per component, half
-  // of the rows and column, ascent: per half of the rows); copies; prolongation (ascent: a lane
-  // per row, component and column)
-  static_assert(NC % 2 == 0 && (8 * RP * sizeof(double)) % 128 == 0 && (2 * RP) % 16 == 0, "pairs of slots, whole banks");
-  static constexpr int passes = 2 * NP, out_down = 8, out_up = 2, pro = RP * 4 / 32;
-  static constexpr int warps_down = passes + out_down + kWaveCopy, warps_up = passes + out_up + kWaveCopy + pro;
-  static_assert(RP * 4 % 32 == 0 && warps_up <= 32 && warps_down <= 32, "warps of a block");
-};
-
 struct WaveArgs {
   Op o;
   const double *idu, *idv;
@@ -2597,7 +2570,6 @@ static int tile_edge(const Ctx* c, int l) {
   const long long b32 = (long long)((d.ny + 31) / 32) * ((d.nx + 31) / 32);
   return b32 >= 148 ? 32 : 16;
 }
-constexpr int kSMs = 148;   // B200
 // Whether level l's tiles are 1.5x wider along i (T x 3T/2): when square tiles give a little
 // more than one block per SM (e.g. 198 on the 321 x 561 ice cap's finest level, where 50 SMs
 // would run two blocks each and set the kernel's length) and the wider ones fit in one
@@ -2694,8 +2666,8 @@ static int tile_up(Ctx* c, int l, int fx, int fy, const double* bu, const double
   return DIVA_OK;
 }
 
-// Whether level l is smoothed by the streamed kernel: double, two sweeps per phase, and more
-// points than one round of 16 x 16 tiles covers (two per SM).  Smoothing pair, tiles against
+// Whether level l is smoothed by the streamed kernel: double, two sweeps per phase, more points
+// than one round of 16 x 16 tiles covers (two per SM), and no edge chosen by the caller.  Smoothing pair, tiles against
 // the streamed kernel: 24.7 / 30.8 us at 129 x 17, 33.1 / 37.6 at 201 x 351 (286 tiles: one
 // round), 49.6 / 39.0 at 229 x 401 (390 tiles: a second one), 53.3 / 48.2 at 321 x 561, 57.8 /
 // 57.4 at 501 x 501, 107.5 / 92.1 at 751 x 751, 408 / 312 at 1501 x 1501.  Float levels keep
@@ -2705,31 +2677,8 @@ constexpr long long kWavePoints = 2LL * kSMs * 16 * 16;
 static int level_nu(const Ctx* c, int l);
 static bool level_streamed(const Ctx* c, int l) {
   const Dims& d = c->lv[l].d;
-  return !level_fp32(c, l) && level_nu(c, l) == WaveGeom::NU && (long long)d.nx * d.ny >= kWavePoints;
-}
-// Strips and chunks of a streamed level: strips as high as two warps per pass allow (fewer halo
-// rows), or 16 rows where the caller chose that edge, evened out over the level; then the number of chunks with the
-// fewest steps in turn, each block (one per SM) taking half its chunk, halo and lag, and some to
-// start, over as many rounds as needed.
-static void wave_shape(const Ctx* c, int l, int* rows, int* chunk, dim3* grid) {
-  using G = WaveGeom;
-  const Dims& d = c->lv[l].d;
-  const int top = c->tile_override[l] == 16 ? 16 : G::TJ;
-  const int ns = (d.ny + top - 1) / top;
-  *rows = ((d.ny + ns - 1) / ns + 1) / 2 * 2;
-  const int nstrip = (d.ny + *rows - 1) / *rows;
-  long best = 0;
-  for (int n = 1; n <= d.nx; ++n) {
-    const int w = (d.nx + n - 1) / n, nc = (d.nx + w - 1) / w;
-    if (w < 4 && n > 1) break;
-    const long rounds = ((long)nstrip * nc + kSMs - 1) / kSMs;
-    const long cost = rounds * ((w + G::H + 3 * G::NP + 2) / 2 + 5);
-    if (best == 0 || cost < best) {
-      best = cost;
-      *chunk = w;
-      *grid = dim3(nstrip, nc);
-    }
-  }
+  const bool chosen = c->tile_override[l] == 16 || c->tile_override[l] == 32;
+  return !chosen && !level_fp32(c, l) && level_nu(c, l) == WaveGeom::NU && (long long)d.nx * d.ny >= kWavePoints;
 }
 template <bool UP>
 static void launch_wave(Ctx* c, int l, const double* bu, const double* bv, double* ou, double* ov) {
@@ -2747,8 +2696,10 @@ static void launch_wave(Ctx* c, int l, const double* bu, const double* bv, doubl
     a.xcu = c->lv[l + 1].xu; a.xcv = c->lv[l + 1].xv;
     factors(c, l, &a.fx, &a.fy);
   }
-  dim3 grid;
-  wave_shape(c, l, &a.rows, &a.chunk, &grid);
+  const WaveShape shape = wave_shape(L.d.ny, L.d.nx);
+  a.rows = shape.rows;
+  a.chunk = shape.chunk;
+  const dim3 grid(shape.nstrip, shape.nchunk);
   const auto kern = a.o.rtu ? k_wave<true, UP> : k_wave<false, UP>;   // 'BC' rows: the finest level
   kern<<<grid, 32 * (UP ? G::warps_up : G::warps_down), UP ? G::smem_up : G::smem_down, c->stream>>>(a);
   c->launches++;
@@ -3443,6 +3394,15 @@ int solver_tile_edges(const Ctx* c, int32_t* edges, int n) {
   const int first = sub_first_level(c);
   for (int l = 0; l < n; ++l)
     edges[l] = (l < c->nlev && c->tiled && c->nlev > 1 && l < first) ? tile_edge(c, l) : 0;
+  return c->nlev;
+}
+
+int solver_strip_rows(const Ctx* c, int32_t* rows, int n) {
+  const int first = sub_first_level(c);
+  for (int l = 0; l < n; ++l) {
+    const bool strips = l < c->nlev && c->tiled && c->nlev > 1 && l < first && level_streamed(c, l);
+    rows[l] = strips ? wave_shape(c->lv[l].d.ny, c->lv[l].d.nx).rows : 0;
+  }
   return c->nlev;
 }
 

@@ -345,15 +345,24 @@ class Context:
         return int(f(self.h))
 
     def get_tile_edges(self):
-        """(edge of each multigrid level's tiled smoother, 0 where untiled; level count)."""
+        """Edge of each multigrid level's tiles (those it would have where it is swept in
+        strips), 0 where untiled."""
         f = self.backend.lib.diva_get_tile_edges
         f.argtypes = [C.c_void_p, C.POINTER(C.c_int32), C.c_int32, C.POINTER(C.c_int32)]
         e, n = (C.c_int32 * 12)(), C.c_int32()
         self._check(f(self.h, e, 12, C.byref(n)), "get_tile_edges")
         return [int(e[k]) for k in range(n.value)]
 
+    def get_strip_rows(self):
+        """Rows of the strips each multigrid level is swept in, 0 where it is not."""
+        f = self.backend.lib.diva_get_strip_rows
+        f.argtypes = [C.c_void_p, C.POINTER(C.c_int32), C.c_int32, C.POINTER(C.c_int32)]
+        e, n = (C.c_int32 * 12)(), C.c_int32()
+        self._check(f(self.h, e, 12, C.byref(n)), "get_strip_rows")
+        return [int(e[k]) for k in range(n.value)]
+
     def set_tile_edges(self, edges):
-        """Fix the tile edge (16, 32, or 0 for the default) of levels 0..len(edges)-1."""
+        """Fix the tile edge (16, 32: square tiles; 0 for the default) of levels 0..len(edges)-1."""
         f = self.backend.lib.diva_set_tile_edges
         f.argtypes = [C.c_void_p, C.POINTER(C.c_int32), C.c_int32]
         e = (C.c_int32 * max(1, len(edges)))(*[int(v) for v in edges])

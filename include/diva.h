@@ -376,14 +376,17 @@ int  diva_complete_state(diva_ctx_t* ctx, int32_t sweeps);
  * are smoothed by tiled kernels of edge 16 or 32; by default a level takes 32 while
  * its 32 x 32 tiles still fill the GPU, and tiles 1.5x as wide along i (32 x 48,
  * 16 x 24) where the square ones give just over one block per SM and the wide ones
- * fit in one.  Large levels in double are swept in strips instead (two columns at a
- * time): 16 rows high for edge 16, up to 48 otherwise.  diva_get_tile_edges writes each level's edge along j (0 for levels not
- * smoothed by tiles) into edges[0..n) and the level count into *nlev;
- * diva_set_tile_edges fixes the edge of levels 0..n-1 (16 or 32: square tiles; 0 for
- * the default) until the next call, e.g. from an autotuner that times candidates
- * with diva_profile_kernel.  The solution does not depend on the shape, only the
- * time per V-cycle. */
+ * fit in one, and large levels in double are swept in strips instead, two columns at
+ * a time.  diva_get_tile_edges writes the edge along j of each level's tiles (of those
+ * it would have, where it is swept in strips; 0 for levels smoothed by neither) into
+ * edges[0..n) and the level count into *nlev; diva_get_strip_rows writes the rows of
+ * each level's strips (0 for levels not swept in strips) likewise.  diva_set_tile_edges
+ * fixes the edge of levels 0..n-1 (16 or 32: square tiles on every such level, in place
+ * of strips or wide tiles; 0 for the default) until the next call, e.g. from an
+ * autotuner that times candidates with diva_profile_kernel.  The solution does not
+ * depend on the shape, only the time per V-cycle. */
 int  diva_get_tile_edges(diva_ctx_t* ctx, int32_t* edges, int32_t n, int32_t* nlev);
+int  diva_get_strip_rows(diva_ctx_t* ctx, int32_t* rows, int32_t n, int32_t* nlev);
 int  diva_set_tile_edges(diva_ctx_t* ctx, const int32_t* edges, int32_t n);
 
 /* Snapshot / restore of the Picard state that persists across calls
