@@ -2562,25 +2562,14 @@ static int sub_first_level(const Ctx* c) {
 static int vcycle(Ctx* c, int l, double* xu, double* xv, const double* bu, const double* bv,
                   const Restriction& rs);
 
-// tile edge of level l's smoothing kernels: 32 x 32 while that still fills the GPU, else
-// 16 x 16, unless the caller chose one (diva_set_tile_edges, e.g. from an autotuner)
+// tile edge of level l's smoothing kernels, and whether they are 1.5x wider along i: by its size
+// (tile_choice), unless the caller chose an edge (diva_set_tile_edges, e.g. from an autotuner)
+static bool tile_chosen(const Ctx* c, int l) { return c->tile_override[l] == 16 || c->tile_override[l] == 32; }
 static int tile_edge(const Ctx* c, int l) {
-  if (c->tile_override[l] == 16 || c->tile_override[l] == 32) return c->tile_override[l];
-  const Dims& d = c->lv[l].d;
-  const long long b32 = (long long)((d.ny + 31) / 32) * ((d.nx + 31) / 32);
-  return b32 >= 148 ? 32 : 16;
+  return tile_chosen(c, l) ? c->tile_override[l] : tile_choice(c->lv[l].d.ny, c->lv[l].d.nx).edge;
 }
-// Whether level l's tiles are 1.5x wider along i (T x 3T/2): when square tiles give a little
-// more than one block per SM (e.g. 198 on the 321 x 561 ice cap's finest level, where 50 SMs
-// would run two blocks each and set the kernel's length) and the wider ones fit in one
-// block per SM, with less halo per point.  Not when the caller chose the edge.
 static bool tile_wide(const Ctx* c, int l) {
-  if (c->tile_override[l] == 16 || c->tile_override[l] == 32) return false;
-  const Dims& d = c->lv[l].d;
-  const int T = tile_edge(c, l), W = 3 * T / 2;
-  const long long sq = (long long)((d.ny + T - 1) / T) * ((d.nx + T - 1) / T);
-  const long long wide = (long long)((d.ny + T - 1) / T) * ((d.nx + W - 1) / W);
-  return sq > kSMs && wide <= kSMs;
+  return !tile_chosen(c, l) && tile_choice(c->lv[l].d.ny, c->lv[l].d.nx).wide;
 }
 
 // Which tile kernels a level uses: the edge (tile_edge), and whether the region's
@@ -2666,19 +2655,13 @@ static int tile_up(Ctx* c, int l, int fx, int fy, const double* bu, const double
   return DIVA_OK;
 }
 
-// Whether level l is smoothed by the streamed kernel: double, two sweeps per phase, more points
-// than one round of 16 x 16 tiles covers (two per SM), and no edge chosen by the caller.  Smoothing pair, tiles against
-// the streamed kernel: 24.7 / 30.8 us at 129 x 17, 33.1 / 37.6 at 201 x 351 (286 tiles: one
-// round), 49.6 / 39.0 at 229 x 401 (390 tiles: a second one), 53.3 / 48.2 at 321 x 561, 57.8 /
-// 57.4 at 501 x 501, 107.5 / 92.1 at 751 x 751, 408 / 312 at 1501 x 1501.  Float levels keep
-// the tiles, which hold the coefficients of a 32 x 32 tile in shared memory: 41 / 46 us at
-// 321 x 561.
-constexpr long long kWavePoints = 2LL * kSMs * 16 * 16;
+// Whether level l is smoothed by the streamed kernel: double, two sweeps per phase, a size at which
+// that pays, and no edge chosen by the caller.  Float levels keep the tiles, which hold the
+// coefficients of a 32 x 32 tile in shared memory: 41 / 46 us at 321 x 561.
 static int level_nu(const Ctx* c, int l);
 static bool level_streamed(const Ctx* c, int l) {
   const Dims& d = c->lv[l].d;
-  const bool chosen = c->tile_override[l] == 16 || c->tile_override[l] == 32;
-  return !chosen && !level_fp32(c, l) && level_nu(c, l) == WaveGeom::NU && (long long)d.nx * d.ny >= kWavePoints;
+  return !tile_chosen(c, l) && !level_fp32(c, l) && level_nu(c, l) == WaveGeom::NU && strips_pay(d.ny, d.nx);
 }
 template <bool UP>
 static void launch_wave(Ctx* c, int l, const double* bu, const double* bv, double* ou, double* ov) {

@@ -1,5 +1,6 @@
-// Sizes of the streamed smoother (k_wave in solver.cu) and the strips and chunks of a level, in
-// plain C++ so that they can be checked for every level size without a GPU.
+// Sizes of the streamed smoother (k_wave in solver.cu), the strips and chunks of a level, and
+// whether it is swept in strips or smoothed by tiles, in plain C++ so that they can be checked for
+// every level size without a GPU.
 #pragma once
 #include <cstddef>
 
@@ -38,6 +39,7 @@ struct WaveGeom {
 struct WaveShape {
   int rows, chunk;       // tile height and width
   int nstrip, nchunk;
+  long steps;            // in turn on an SM
 };
 // Strips as high as two warps per pass allow (fewer halo rows), evened out over the level; then the
 // number of chunks with the fewest steps in turn, each block (one per SM) taking half its chunk,
@@ -60,7 +62,46 @@ inline WaveShape wave_shape(int ny, int nx) {
       s.nchunk = nc;
     }
   }
+  s.steps = best;
   return s;
+}
+
+// Tiles of a level: 32 x 32 while that still fills the GPU, else 16 x 16, and 1.5x wider along i
+// (T x 3T/2) when square tiles give a little more than one block per SM (e.g. 198 of 32 x 32 at
+// 321 x 561, where 50 SMs would run two blocks each and set the kernel's length) and the wider
+// ones fit in one block per SM, with less halo per point.
+struct TileChoice {
+  int edge;
+  bool wide;
+  long n;   // tiles
+};
+inline TileChoice tile_choice(int ny, int nx) {
+  auto tiles = [&](int tj, int ti) { return (long)((ny + tj - 1) / tj) * ((nx + ti - 1) / ti); };
+  TileChoice t{};
+  t.edge = tiles(32, 32) >= kSMs ? 32 : 16;
+  const long square = tiles(t.edge, t.edge), wide = tiles(t.edge, 3 * t.edge / 2);
+  t.wide = square > kSMs && wide <= kSMs;
+  t.n = t.wide ? wide : square;
+  return t;
+}
+
+// Whether a level in double with two sweeps per phase is swept in strips: more points than one
+// round of 16 x 16 tiles covers (two per SM), and no more steps in turn than the tiles take time
+// for.  A smoothing pair takes 1.3 to 1.5 us a step.  Tiles take 33 us for one round of 16 x 16 ones
+// and 46 to 60 for two, 49 to 53 for one of 32 x 48, and of 32 x 32 ones, two per SM, 50 to 59 us for
+// one round, 70 to 105 for two and about 28 us for every 148 from there on.  Tiles against
+// strips: 33.1 / 37.6 us at 201 x 351 (286 tiles of 16 x 16), 49.6 / 39.0 at 229 x 401 (390),
+// 53.3 / 48.2 at 321 x 561 (126 of 32 x 48), 59.0 / 61.5 at 401 x 701 (286 of 32 x 32), 101 / 83 at
+// 501 x 875 (448), 408 / 312 at 1501 x 1501 (2209); on long grids, whose strips are low or
+// whose chunks are long, 47.2 / 64.7 at 6579 x 17, 50.1 / 63.6 at 49 x 4235, 82.8 / 102 at 41 x 8667,
+// but 98.6 / 57.2 at 12198 x 41 and 92.6 / 62.8 at 6168 x 33.
+inline bool strips_pay(int ny, int nx) {
+  if ((long long)nx * ny < 2LL * kSMs * 16 * 16) return false;
+  const TileChoice t = tile_choice(ny, nx);
+  if (t.edge == 16) return true;
+  const double per_sm = (double)t.n / kSMs;
+  const double steps = t.wide ? 37.0 : per_sm <= 2.0 ? 40.0 : per_sm < 52.0 / 19.5 ? 52.0 : 19.5 * per_sm;
+  return wave_shape(ny, nx).steps <= steps;
 }
 
 }  // namespace diva

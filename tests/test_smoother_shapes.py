@@ -24,22 +24,43 @@ extern "C" void shape(int ny, int nx, int* o) {
   const int v[] = {s.rows, s.chunk, s.nstrip, s.nchunk, WaveGeom::TJ};
   for (int k = 0; k < 5; ++k) o[k] = v[k];
 }
+extern "C" void choice(int ny, int nx, int* o) {
+  const TileChoice t = tile_choice(ny, nx);
+  const int v[] = {t.edge, t.wide, (int)t.n, (int)strips_pay(ny, nx)};
+  for (int k = 0; k < 4; ++k) o[k] = v[k];
+}
 """
 
 
 @pytest.fixture(scope="module")
-def shape(tmp_path_factory):
+def lib(tmp_path_factory):
     d = tmp_path_factory.mktemp("wave")
     (d / "w.cpp").write_text(PROGRAM)
     so = str(d / "w.so")
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, str(d / "w.cpp"), "-o", so], check=True)
-    lib = C.CDLL(so)
+    return C.CDLL(so)
 
+
+@pytest.fixture(scope="module")
+def shape(lib):
     def call(ny, nx):
         o = (C.c_int * 5)()
         lib.shape(ny, nx, o)
         return list(o)
     return call
+
+
+# ny, nx: the default tiles (edge, wide), and whether strips take the smoothing pair less time there
+@pytest.mark.parametrize("ny, nx, tiles, strips", [
+    (351, 201, (16, 0), 0), (401, 229, (16, 0), 1), (561, 321, (32, 1), 1), (701, 401, (32, 0), 0), (875, 501, (32, 0), 1),
+    (1501, 1501, (32, 0), 1), (9, 5005, (32, 1), 0), (9, 8710, (32, 0), 0), (8710, 9, (32, 0), 0), (17, 6579, (32, 1), 0),
+    (25, 8106, (32, 0), 0), (33, 2570, (32, 1), 1), (33, 6168, (32, 0), 1), (49, 4235, (32, 0), 0), (4235, 49, (32, 0), 0),
+    (65, 3078, (32, 0), 0), (3078, 65, (32, 0), 1), (8667, 41, (32, 0), 0), (41, 8667, (32, 0), 1), (113, 2691, (32, 0), 1),
+    (4485, 113, (32, 0), 0), (129, 4100, (32, 0), 1), (4100, 129, (32, 0), 0), (1025, 129, (32, 1), 1)])
+def test_the_faster_smoother_is_the_default(lib, ny, nx, tiles, strips):
+    o = (C.c_int * 4)()
+    lib.choice(ny, nx, o)
+    assert (o[0], o[1]) == tiles and o[3] == strips
 
 
 def test_strips_and_chunks_cover_every_level(shape):
