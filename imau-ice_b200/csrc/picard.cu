@@ -139,7 +139,7 @@ __device__ __forceinline__ int margin_mode(double H0, double H1) {
 }
 // K1 in three launches.  (a) k_column_prep, one thread per column: the strain rates
 // of the depth-averaged flow and which of the column's four shear faces have ice.
-// (b) k_layer_viscosity, one thread per column and kViscLayers layers, a warp over 32
+// (b) k_layer_viscosity, one thread per column and one or three layers, a warp over 32
 // neighbouring rows j of one grid column i: the shear of the column's own east and
 // north faces, the west face, and the south face as the north face of the lane below
 // (shuffle), then the viscosity of the layer.  (c) k_column_integrals, one thread per
@@ -209,14 +209,19 @@ __device__ __forceinline__ float rcbrt_t(float x) { return rcbrtf(x); }
 __device__ __forceinline__ double pow_t(double x, double y) { return pow(x, y); }
 __device__ __forceinline__ float pow_t(float x, float y) { return powf(x, y); }
 
-// A thread takes kViscLayers layers of its column, whose loads are in flight together and share
-// the column's flags and basal stress.  All of K1 in FP64, one
-// layer a thread against three: 76.8 / 72.5 us on 321 x 561, 780 / 687 us on 1501 x 1501, 23.5 /
-// 24.6 us on 129 x 17 (five layers: 84.9, 804, 27.8: too few warps for their registers).
+// A thread takes L layers of its column, whose loads are in flight together and share the
+// column's flags and basal stress.  All of K1 in FP64, 15 layers, one layer a thread against three:
+// 23.6 / 25.6 us on 129 x 17, 25.7 / 26.7 on 257 x 33, 26.7 / 28.2 on 81 x 141, 28.7 / 30.8 on
+// 115 x 201, 32.8 / 32.9 on 161 x 281, 38.0 / 36.9 on 201 x 351, 77.0 / 72.8 on 321 x 561, 198 / 175 on
+// 533 x 933.  Three where a GPU of 2048 threads per SM is full with them, one below: there a
+// thread's layers come one after the other while SMs are idle (two are between the others; five
+// at 321 x 561, 1501 x 1501 and 129 x 17 84.9, 804 and 27.8 us: too few warps for their registers).
 constexpr int kViscLayers = 3;
-template <bool WRITE_SHEAR, class R>
+inline int visc_layers(const Dims& d) {
+  return (long long)d.nx * d.ny * ((d.nz + kViscLayers - 1) / kViscLayers) >= 148LL * 2048 ? kViscLayers : 1;
+}
+template <bool WRITE_SHEAR, class R, int L>
 __global__ void __launch_bounds__(kColLanes * kColRows) k_layer_viscosity(CoefArgs a) {
-  constexpr int L = kViscLayers;
   const Dims d = a.d;
   const int lane = threadIdx.x, y = threadIdx.y;
   // the layers are the fastest grid index: blocks running together share their columns'
@@ -1100,16 +1105,14 @@ int launch_diva_coefficients(Ctx* c, const double* u, const double* v, bool diva
   k_column_prep<<<G2>>>(a); c->launches++;
   {
     const dim3 block(kColLanes, kColRows);
-    const dim3 grid((c->d.nz + kViscLayers - 1) / kViscLayers, (c->d.ny + kColLanes - 1) / kColLanes,
-                    (c->d.nx + kColRows - 1) / kColRows);
-    const bool f32 = k1_fp32(C);
-    if (what == K1_WRITE_SHEAR) {
-      if (f32) k_layer_viscosity<true, float><<<grid, block, 0, c->stream>>>(a);
-      else k_layer_viscosity<true, double><<<grid, block, 0, c->stream>>>(a);
-    } else {
-      if (f32) k_layer_viscosity<false, float><<<grid, block, 0, c->stream>>>(a);
-      else k_layer_viscosity<false, double><<<grid, block, 0, c->stream>>>(a);
-    }
+    const int L = visc_layers(c->d);
+    const dim3 grid((c->d.nz + L - 1) / L, (c->d.ny + kColLanes - 1) / kColLanes, (c->d.nx + kColRows - 1) / kColRows);
+    const bool f32 = k1_fp32(C), w = what == K1_WRITE_SHEAR;
+    auto kern = w ? (f32 ? (L == 1 ? k_layer_viscosity<true, float, 1> : k_layer_viscosity<true, float, kViscLayers>)
+                         : (L == 1 ? k_layer_viscosity<true, double, 1> : k_layer_viscosity<true, double, kViscLayers>))
+                  : (f32 ? (L == 1 ? k_layer_viscosity<false, float, 1> : k_layer_viscosity<false, float, kViscLayers>)
+                         : (L == 1 ? k_layer_viscosity<false, double, 1> : k_layer_viscosity<false, double, kViscLayers>));
+    kern<<<grid, block, 0, c->stream>>>(a);
     c->launches++;
   }
   if (k1_fp32(C)) {
