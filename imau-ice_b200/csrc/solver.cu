@@ -319,35 +319,6 @@ __global__ void k_gs(Op o, double* xu, double* xv, const double* bu, const doubl
   gs_point(o, xu, xv, bu, bv, idu, idv, comp, j, i);
 }
 
-// block-wide pass over all points of one colour (the caller synchronises)
-__device__ __forceinline__ void block_gs_pass(const Op& o, double* xu, double* xv, const double* bu, const double* bv,
-                                              const double* idu, const double* idv, int comp, int color) {
-  const Dims& d = o.d;
-  const int hj = (d.ny + 1) / 2, n = hj * d.nx;
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
-    const int i = t / hj, j = 2 * (t % hj) + ((i + color) & 1);
-    if (j < d.ny) gs_point(o, xu, xv, bu, bv, idu, idv, comp, j, i);
-  }
-}
-
-// relaxation of the coarsest level by one block: `sweeps` symmetric sweeps u0 u1 v0 v1 | v1 v0 u1 u0
-__device__ __forceinline__ void block_coarse_relax(const Op& o, double* xu, double* xv, const double* bu,
-                                                   const double* bv, const double* idu, const double* idv,
-                                                   int sweeps) {
-  for (int s = 0; s < sweeps; ++s) {
-    for (int pass = 0; pass < 8; ++pass) {
-      const int p = pass < 4 ? pass : 7 - pass;
-      block_gs_pass(o, xu, xv, bu, bv, idu, idv, p >> 1, p & 1);
-      __syncthreads();
-    }
-  }
-}
-
-__global__ void k_coarse_solve(Op o, double* xu, double* xv, const double* bu, const double* bv, const double* idu,
-                               const double* idv, int sweeps) {
-  block_coarse_relax(o, xu, xv, bu, bv, idu, idv, sweeps);
-}
-
 // r = b - A x on the interior (zero elsewhere)
 __device__ __forceinline__ void residual_point(const Op& o, const double* xu, const double* xv, const double* bu,
                                                const double* bv, double* ru, double* rv, int j, int i) {
@@ -1711,12 +1682,8 @@ __global__ void __launch_bounds__(kSubThreads) k_subcycle(const __grid_constant_
       }
       __syncthreads();
     }
-    if (l == sc.last) {
-      Op o = sc.L[l].o;
-      o.d.ld = m.ny;
-      o.d.plane = m.P1 - 1;
-      o.Na = m.plane(SA_NA); o.Nb = m.plane(SA_NB); o.Bx = m.plane(SA_BX); o.By = m.plane(SA_BY);
-      block_coarse_relax(o, xu, xv, m.plane(SA_BU), m.plane(SA_BV), m.plane(SA_IDU), m.plane(SA_IDV), sc.coarse_sweeps);
+    if (l == sc.last) {   // relaxed: symmetric sweeps u0 u1 v0 v1 | v1 v0 u1 u0
+      for (int s = 0; s < 8 * sc.coarse_sweeps; ++s) gs_pass(m, l, s & 4 ? 3 - (s & 3) : s & 3);
       break;
     }
     for (int s = 0; s < 4 * sc.nu1; ++s) gs_pass(m, l, s & 3);
@@ -2928,12 +2895,6 @@ static int vcycle(Ctx* c, int l, double* xu, double* xv, const double* bu, const
     k_subcycle<<<1, kSubThreads, sub_alloc(c, l), c->stream>>>(sc, xu, xv, bu, bv); c->launches++;
     DIVA_LAUNCHED(c, "k_subcycle");
     for (int q = l; q < c->nlev; ++q) c->fine_passes += 8.0 * (double)c->lv[q].d.plane / (double)c->d.plane;
-    return DIVA_OK;
-  }
-  if (l == c->nlev - 1) {
-    k_coarse_solve<<<1, 256, 0, c->stream>>>(make_op(c, l), xu, xv, bu, bv, c->lv[l].idu, c->lv[l].idv,
-                                             coarse_sweeps); c->launches++;
-    DIVA_LAUNCHED(c, "k_coarse_solve");
     return DIVA_OK;
   }
   const Level& L = c->lv[l];
