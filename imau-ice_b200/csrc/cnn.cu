@@ -896,8 +896,6 @@ __global__ void k_apply(Dims d, const float* pred, StatePtrs s, int Wp, int velo
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-constexpr int kSMs = 148;   // B200
-
 // CTAs of a persistent kernel that fit on the GPU: by its shared memory (228 KB per SM, 1 KB of
 // it per CTA) and by tensor memory (512 columns per SM)
 int resident_ctas(int smem, int ncols) {

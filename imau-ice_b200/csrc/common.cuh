@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "../../include/diva.h"
+#include "gpu.hpp"
 
 namespace diva {
 
@@ -112,7 +113,7 @@ __device__ __forceinline__ void block_sum(double (&v)[N]) {
 // at most kRedBlocks of them (the four that k_matvec's registers let an SM hold: with six a second
 // round starts half empty), so that the last block's sum over the blocks' partials stays at a
 // few microseconds (one partial per tile: 23 us at 1501 x 1501).
-constexpr int kRedBlocks = 148 * 4;
+constexpr int kRedBlocks = 4 * kSMs;
 inline int red_blocks(const Dims& d) {
   const int n = ((d.ny + kBX - 1) / kBX) * ((d.nx + kBY - 1) / kBY);
   return n < kRedBlocks ? n : kRedBlocks;

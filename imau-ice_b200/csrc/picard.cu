@@ -218,7 +218,7 @@ __device__ __forceinline__ float pow_t(float x, float y) { return powf(x, y); }
 // at 321 x 561, 1501 x 1501 and 129 x 17 84.9, 804 and 27.8 us: too few warps for their registers).
 constexpr int kViscLayers = 3;
 inline int visc_layers(const Dims& d) {
-  return (long long)d.nx * d.ny * ((d.nz + kViscLayers - 1) / kViscLayers) >= 148LL * 2048 ? kViscLayers : 1;
+  return (long long)d.nx * d.ny * ((d.nz + kViscLayers - 1) / kViscLayers) >= 2048LL * kSMs ? kViscLayers : 1;
 }
 template <bool WRITE_SHEAR, class R, int L>
 __global__ void __launch_bounds__(kColLanes * kColRows) k_layer_viscosity(CoefArgs a) {

@@ -21,10 +21,11 @@
 //   * smoothing is 4-colour Gauss-Seidel (u red/black, v red/black), with the
 //     exact diagonal of the reduced system;
 //   * the larger levels are smoothed by tile kernels, the largest of them in streamed strips
-//     (two launches per level and V-cycle, halo recomputed instead of exchanged), the coarse levels whose
-//     data fit in 200 KB run out of one thread block's shared memory (one launch
-//     per V-cycle), and the coarsest level is solved directly with its inverse,
-//     formed once per viscosity iteration.
+//     (halo recomputed instead of exchanged; two launches per level and V-cycle, three for a
+//     streamed level below the finest, whose right-hand side is restricted first), the coarse
+//     levels whose data fit in 200 KB run out of one thread block's shared memory (one launch
+//     per V-cycle), and the coarsest level is solved directly with its inverse, formed once per
+//     viscosity iteration, or relaxed where it has none.
 // All reductions are two-stage (block partials, then one fixed-order sum) so
 // results are bit-reproducible from run to run.
 #include <cmath>
@@ -2476,7 +2477,7 @@ static size_t sub_points(const Ctx* c, int l) {
 }
 static size_t sub_rows(const Ctx* c, int l) {
   size_t n = 0;
-  for (int q = l; q < c->nlev; ++q) n += ((size_t)13 * level_rows(c->lv[q].d) + 7) / 8 * 8;
+  for (int q = l; q < c->nlev; ++q) n += ((size_t)(kTabReads + 1 + kTabProlong) * level_rows(c->lv[q].d) + 7) / 8 * 8;
   return n;
 }
 static int sub_first_fit(const Ctx* c);

@@ -3,10 +3,9 @@
 // every level size without a GPU.
 #pragma once
 #include <cstddef>
+#include "gpu.hpp"
 
 namespace diva {
-
-constexpr int kSMs = 148;   // B200
 
 constexpr int kWavePre = 3;       // pairs of columns the copies run ahead
 constexpr int kWaveBars = 8;      // mbarriers: more than the pairs in flight
