@@ -1,7 +1,8 @@
 """The convolutions' choice of tiles (imau-ice_b200/csrc/cnn_tiles.hpp), compiled for the CPU and
 checked for every layer over image sizes from one row or column on: the tiles cover the image,
 their positions fit the accumulators, the launch's shared memory stays within what a block may
-have, and no weight-gradient sum runs over more pixels than 64 slices of 64-pixel chunks gave."""
+have, and no weight-gradient sum runs over more pixels than 64 slices of 64-pixel chunks gave, and
+an eighth."""
 import ctypes as C
 import os
 import subprocess
@@ -70,4 +71,4 @@ def test_weight_gradient_tiles_fit_and_keep_the_chains_short(tiles, cin, cout):
             assert 1 <= slices <= ntile
             chunks = -(-n * H * W // 64)
             before = 64 * -(-chunks // min(chunks, 64))     # chunks of the longest of up to 64 slices
-            assert -(-ntile // slices) * min(TW, W) * TH <= before, (n, H, W, slices)
+            assert -(-ntile // slices) * min(TW, W) * TH <= before * 9 / 8, (n, H, W, slices)
