@@ -13,10 +13,14 @@ pytestmark = [pytest.mark.gpu,
 FRONT = {"choice_ice_margin": "BC"}
 
 
-def long_channel(times):
-    """A 65 x 9 channel with every column repeated."""
-    g, cfg, f = helpers.make_case(1, dx=10e3)
-    return diva.Grid(g.nx * times, g.ny, g.dx, zeta=g.zeta), cfg, {k: np.repeat(v, times, axis=-1) for k, v in f.items()}
+def long_channel(times, dx=10e3, across=False):
+    """A channel (65 x 9 cells at 10 km) with every column repeated, along i or along j."""
+    g, cfg, f = helpers.make_case(1, dx=dx)
+    nx, ny = g.nx * times, g.ny
+    f = {k: np.repeat(v, times, axis=-1) for k, v in f.items()}
+    if across:
+        nx, ny, f = ny, nx, {k: np.swapaxes(v, -1, -2) for k, v in f.items()}
+    return diva.Grid(nx, ny, g.dx, zeta=g.zeta), cfg, f
 
 
 @pytest.mark.parametrize("case, over, edge, strips", [
@@ -26,11 +30,13 @@ def long_channel(times):
     (dict(cfg_id=2, dx=6.7e3), {}, 32, True),                          # 239 x 417
     (dict(cfg_id=2, dx=6.7e3), {}, 16, True),
     (dict(cfg_id=1, dx=0.75e3, calving_front=True), FRONT, 32, True),  # 853 x 107
-    (77, {}, None, False),                                             # 5005 x 9: 32 x 48 tiles
-    (77, {}, 32, False),
+    (dict(times=77), {}, None, False),                                 # 5005 x 9: 32 x 48 tiles
+    (dict(times=77), {}, 32, False),
+    (dict(times=36, dx=5e3), {}, None, True),                          # 4644 x 17: one strip of 18 rows
+    (dict(times=36, dx=5e3, across=True), {}, None, True),             # 17 x 4644: chunks as wide as the level
 ])
 def test_shapes_match_per_colour_kernels(monkeypatch, case, over, edge, strips):
-    g, cfg, f = long_channel(case) if isinstance(case, int) else helpers.make_case(**case)
+    g, cfg, f = long_channel(**case) if "times" in case else helpers.make_case(**case)
     cfg = dict(cfg, **over, DIVA_visc_it_nit=4, lin_rtol=1e-4)
     out = []
     for tiles in (True, False):
@@ -45,7 +51,7 @@ def test_shapes_match_per_colour_kernels(monkeypatch, case, over, edge, strips):
                 ctx.set_tile_edges([edge] * len(edges))
                 assert ctx.get_tile_edges()[0] == edge and not any(ctx.get_strip_rows())
             else:
-                assert edges[0] == 32
+                assert edges[0] == (16 if strips else 32)
         else:
             assert not any(ctx.get_tile_edges()) and not any(ctx.get_strip_rows())
         r = ctx.solve_DIVA()
