@@ -1192,6 +1192,9 @@ StatePtrs state_ptrs(Ctx* c) {
                    c->D(DIVA_F_VISC_EFF_3D_A)};
 }
 
+// the alignment diva_cnn.h asks of a caller's buffer (a misaligned access is a fault on the GPU)
+bool aligned(const void* p, size_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; }
+
 dim3 img_grid(int Hp, int Wp) { return dim3((Hp + kBX - 1) / kBX, (Wp + kBY - 1) / kBY); }
 
 }  // namespace
@@ -1414,6 +1417,7 @@ int32_t diva_cnn_predict(diva_cnn_t* N, diva_ctx_t* ctx, int32_t complete_sweeps
 
 int32_t diva_cnn_forward(diva_cnn_t* N, const void* feat, float* out, int32_t n) {
   if (!N || !feat || !out || n < 1 || n > N->batch) return DIVA_BAD_INPUT;
+  if (!aligned(feat, 16) || !aligned(out, sizeof(float))) return DIVA_BAD_INPUT;
   RET(forward(N, static_cast<const bf16*>(feat), out, n, N->stream));
   CK(cudaStreamSynchronize(N->stream));
   return check_err(N);
@@ -1421,6 +1425,7 @@ int32_t diva_cnn_forward(diva_cnn_t* N, const void* feat, float* out, int32_t n)
 
 int32_t diva_cnn_train_step(diva_cnn_t* N, const void* feat, const float* tgt, int32_t n, float lr, float* loss) {
   if (!N || !feat || !tgt || n < 1 || n > N->batch || !(lr >= 0.0f)) return DIVA_BAD_INPUT;
+  if (!aligned(feat, 16) || !aligned(tgt, sizeof(float))) return DIVA_BAD_INPUT;
   const bf16* in = static_cast<const bf16*>(feat);
   RET(forward(N, in, nullptr, n, N->stream));
   RET(backward(N, in, tgt, n, N->stream, N->loss));

@@ -99,7 +99,7 @@ int32_t diva_cnn_predict(diva_cnn_t* net, diva_ctx_t* ctx, int32_t complete_swee
 /* Device-buffer forms for tests and callers with their own data (pointers are device
  * memory; n <= batch).  feat: [n][Hp][Wp][16] BF16 with Hp, Wp = ny, nx rounded up to
  * multiples of 4, on a 16-byte boundary; out: [n][Hp][Wp][20] FP32, at any float's
- * address; tgt like out. */
+ * address; tgt like out.  A buffer aligned less is DIVA_BAD_INPUT. */
 int32_t diva_cnn_padded_shape(const diva_cnn_t* net, int32_t* Hp, int32_t* Wp);
 int32_t diva_cnn_forward(diva_cnn_t* net, const void* feat, float* out, int32_t n);
 

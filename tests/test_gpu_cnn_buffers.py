@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from imau_ice_b200 import diva, learned
+from imau_ice_b200 import _abi, diva, learned
 import cnn_reference as ref
 import helpers
 
@@ -36,6 +36,22 @@ def test_outputs_and_targets_at_any_float(shift):
     net.close()
     (o0, g0, l0), (o1, g1, l1) = res
     assert np.array_equal(o0, o1) and np.array_equal(g0, g1) and l0 == l1
+
+
+def test_buffers_aligned_less_are_refused_before_any_launch():
+    g = diva.Grid(9, 9, 10e3)
+    net = learned.WarmStartNet(g, batch=1, capacity=0, seed=1)
+    n = int(np.prod(net.padded_shape))
+    feat = torch.zeros(n * learned.IN_C + 8, dtype=torch.bfloat16, device="cuda")
+    out = torch.zeros(n * learned.N_OUT + 2, device="cuda")
+    for df, do in ((2, 0), (8, 0), (0, 1), (0, 2)):
+        for call in (lambda: net.forward(feat.data_ptr() + df, out.data_ptr() + do, 1),
+                     lambda: net.train_step(feat.data_ptr() + df, out.data_ptr() + do, 1, 0.0)):
+            with pytest.raises(diva.DivaError) as e:
+                call()
+            assert e.value.status == _abi.BAD_INPUT
+    net.forward(feat.data_ptr(), out.data_ptr(), 1)
+    net.close()
 
 
 @pytest.mark.parametrize("ny, nx", [(2, 400), (4, 372), (3, 1001)])
