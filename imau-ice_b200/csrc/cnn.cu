@@ -637,8 +637,9 @@ struct LossWeights {
 // every thread needs the same ones); read from global memory, one load per multiply-add made
 // the load unit the bound (326 us for 8 training samples of 561 x 321, whose tensors cross
 // HBM in 65 us).  With targets, gd1 is masked by the ReLU of d1.  out and tgt may be a caller's
-// buffers at any float's address: four floats at a time where both lie on 16 bytes, else one by
-// one.
+// buffers at any float's address: four floats at a time where both lie on 16 bytes (WIDE), else
+// one by one.
+template <bool WIDE>
 __global__ void __launch_bounds__(128) k_head(const bf16* d1, const float* wh, const float* bh, float* out,
                                               const float* tgt, float* dout, bf16* gd1, float* part, int n, int H,
                                               int W, int ny, int nx, int nz, float inv_count, LossWeights lw) {
@@ -664,13 +665,12 @@ __global__ void __launch_bounds__(128) k_head(const bf16* d1, const float* wh, c
 #pragma unroll
     for (int c = 0; c < kHeadC; ++c) gd[c] = 0.0f;
     const int x = (int)(p % W), y = (int)((p / W) % H);
-    const bool wide = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(tgt)) & 15) == 0;
 #pragma unroll
     for (int j4 = 0; j4 < kOut; j4 += 4) {
       float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f), o4, g4;
       if (tgt) {
         const float* t = tgt + p * kOut + j4;
-        t4 = wide ? *reinterpret_cast<const float4*>(t) : make_float4(t[0], t[1], t[2], t[3]);
+        t4 = WIDE ? *reinterpret_cast<const float4*>(t) : make_float4(t[0], t[1], t[2], t[3]);
       }
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(128) k_head(const bf16* d1, const float* wh, c
       }
       if (out) {
         float* o = out + p * kOut + j4;
-        if (wide) *reinterpret_cast<float4*>(o) = o4;
+        if (WIDE) *reinterpret_cast<float4*>(o) = o4;
         else o[0] = o4.x, o[1] = o4.y, o[2] = o4.z, o[3] = o4.w;
       }
       if (tgt) *reinterpret_cast<float4*>(dout + p * kOut + j4) = g4;
@@ -1054,6 +1054,9 @@ Input layer_input(const diva_cnn_t* N, int l, const bf16* in) {
   return Input{t == T_IN ? in : N->act[t], nullptr, 0};
 }
 
+// of a caller's buffer (a misaligned access is a fault on the GPU)
+bool aligned(const void* p, size_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; }
+
 int forward(diva_cnn_t* N, const bf16* in, float* out, int n, cudaStream_t st) {
   auto conv = [&](int l) {
     const Layer& ly = N->L[l];
@@ -1081,7 +1084,8 @@ int forward(diva_cnn_t* N, const bf16* in, float* out, int n, cudaStream_t st) {
   RET(conv(9));
   if (out) {
     const long npix = (long)n * N->Hp * N->Wp;
-    k_head<<<nblk(npix, 128), 128, 0, st>>>(N->act[T_D1], N->w + N->head_w, N->w + N->head_b, out, nullptr,
+    const auto head = aligned(out, 16) ? k_head<true> : k_head<false>;
+    head<<<nblk(npix, 128), 128, 0, st>>>(N->act[T_D1], N->w + N->head_w, N->w + N->head_b, out, nullptr,
                                             nullptr, nullptr, nullptr, n, N->Hp, N->Wp, N->ny, N->nx, N->nz, 0.0f,
                                             N->lw);
   }
@@ -1097,7 +1101,8 @@ int backward(diva_cnn_t* N, const bf16* in, const float* tgt, int n, cudaStream_
   auto sum_rows = [&](int rows, long cols, float* dst) {
     k_sum_rows<<<nblk(cols, 32), dim3(32, 8), 0, st>>>(N->part, rows, (int)cols, dst);
   };
-  k_head<<<hb, 128, 0, st>>>(N->act[T_D1], N->w + N->head_w, N->w + N->head_b, nullptr, tgt, N->dout,
+  const auto head = aligned(tgt, 16) ? k_head<true> : k_head<false>;
+  head<<<hb, 128, 0, st>>>(N->act[T_D1], N->w + N->head_w, N->w + N->head_b, nullptr, tgt, N->dout,
                              N->grad[T_D1], N->part, n, N->Hp, N->Wp, N->ny, N->nx, N->nz,
                              1.0f / (float)N->valid(n), N->lw);
   k_sum_all<<<1, 1024, 0, st>>>(N->part, (int)hb, loss_dst);
@@ -1191,9 +1196,6 @@ StatePtrs state_ptrs(Ctx* c) {
   return StatePtrs{c->D(DIVA_F_U_VAV_CX), c->D(DIVA_F_V_VAV_CY), c->D(DIVA_F_TAUB_CX), c->D(DIVA_F_TAUB_CY),
                    c->D(DIVA_F_VISC_EFF_3D_A)};
 }
-
-// the alignment diva_cnn.h asks of a caller's buffer (a misaligned access is a fault on the GPU)
-bool aligned(const void* p, size_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; }
 
 dim3 img_grid(int Hp, int Wp) { return dim3((Hp + kBX - 1) / kBX, (Wp + kBY - 1) / kBY); }
 
